@@ -531,26 +531,70 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
   return {C, pre, (int64_t)rc};
 }
 
-// x [M <= 16, K], w [N, K] (rows contiguous) -> y [M, N]; returns an empty optional if the kernel does not apply
-OptTensor gemv_small_m(const Tensor& x, const Tensor& w, const OptTensor& bias, int64_t act, int64_t out_dtype_code,
-                       double alpha) {
-  TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
+// x [1, K], w [N, K] (rows contiguous) -> y [1, N]; returns an empty optional if the kernel does not apply
+OptTensor gemv(const Tensor& x, const Tensor& w, const OptTensor& bias, int64_t act, int64_t out_dtype_code) {
+  TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(0) == 1 && x.size(1) == w.size(1));
   TORCH_CHECK(x.stride(1) == 1 && w.stride(1) == 1 && x.scalar_type() == w.scalar_type());
   c10::cuda::CUDAGuard guard(x.device());
-  const int M = x.size(0), K = x.size(1), N = w.size(0);
+  const int K = x.size(1), N = w.size(0);
   at::ScalarType odt = out_dtype_code == 0 ? at::kFloat : (out_dtype_code == 1 ? at::kBFloat16 : at::kHalf);
-  Tensor y = torch::empty({M, N}, x.options().dtype(odt));
+  Tensor y = torch::empty({1, N}, x.options().dtype(odt));
   int bias_code = 0;
   if (bias.has_value()) {
     check_cuda_contig(*bias, "bias");
     bias_code = dtype_code(*bias);
     TORCH_CHECK(bias->numel() == N);
   }
-  const bool ok = mb::gemv_small_m(x.data_ptr(), w.data_ptr(), opt_ptr(bias), bias_code, y.data_ptr(), M, N, K,
-                                   x.stride(0), w.stride(0), y.stride(0), (float)alpha, (int)act, dtype_code(x),
-                                   (int)out_dtype_code, stream());
+  const bool ok = mb::gemv(x.data_ptr(), w.data_ptr(), opt_ptr(bias), bias_code, y.data_ptr(), N, K, w.stride(0),
+                           (int)act, dtype_code(x), (int)out_dtype_code, stream());
   if (!ok) return OptTensor();
   return y;
+}
+
+// Up to four products over the same M rows: outs[i] = act_i(xs[i] ws[i]^T + biases[i]) + addends[i], act 0 none,
+// 1 SiLU, 2 SwiGLU with second weight w2s[i]; returns the launch status (0: done, -1: outside what the kernel handles)
+int64_t skinny_gemm(const std::vector<Tensor>& xs, const std::vector<Tensor>& ws, const std::vector<OptTensor>& w2s,
+                    const std::vector<OptTensor>& biases, const std::vector<OptTensor>& addends,
+                    const std::vector<int64_t>& acts, const std::vector<Tensor>& outs, bool pdl, const Tensor& err) {
+  const size_t n = xs.size();
+  TORCH_CHECK(n >= 1 && n <= (size_t)mb::kSkinnyJobs && ws.size() == n && w2s.size() == n && biases.size() == n &&
+              addends.size() == n && acts.size() == n && outs.size() == n);
+  c10::cuda::CUDAGuard guard(xs[0].device());
+  const int64_t M = xs[0].size(0);
+  if (M > mb::kSkinnyMaxRows) return -1;
+  mb::SkinnyJob jobs[mb::kSkinnyJobs] = {};
+  for (size_t i = 0; i < n; ++i) {
+    const Tensor &x = xs[i], &w = ws[i], &y = outs[i];
+    TORCH_CHECK(x.is_cuda() && w.is_cuda() && y.is_cuda() && x.dim() == 2 && w.dim() == 2 && y.dim() == 2);
+    TORCH_CHECK(x.size(0) == M && x.size(1) == w.size(1) && y.size(0) == M && y.size(1) == w.size(0));
+    TORCH_CHECK(x.scalar_type() == xs[0].scalar_type() && w.scalar_type() == x.scalar_type());
+    TORCH_CHECK(x.stride(1) == 1 && w.stride(1) == 1 && y.stride(1) == 1);
+    TORCH_CHECK(y.scalar_type() == at::kFloat || y.scalar_type() == x.scalar_type());
+    mb::SkinnyJob& j = jobs[i];
+    j.x = x.data_ptr(); j.w = w.data_ptr(); j.y = y.data_ptr();
+    j.ldx = M == 1 ? x.size(1) : x.stride(0); j.ldw = w.size(0) == 1 ? w.size(1) : w.stride(0); j.ldy = y.stride(0);
+    j.N = w.size(0); j.K = w.size(1); j.act = acts[i]; j.out_f32 = y.scalar_type() == at::kFloat;
+    TORCH_CHECK((acts[i] == mb::kSkinnySwiGLU) == w2s[i].has_value());
+    if (w2s[i].has_value()) {
+      TORCH_CHECK(w2s[i]->sizes() == w.sizes() && w2s[i]->strides() == w.strides() && w2s[i]->scalar_type() == w.scalar_type());
+      j.w2 = w2s[i]->data_ptr();
+    }
+    if (biases[i].has_value()) {
+      check_cuda_contig(*biases[i], "bias");
+      TORCH_CHECK(biases[i]->numel() == j.N);
+      j.bias = biases[i]->data_ptr(); j.bias_dtype = dtype_code(*biases[i]);
+    }
+    if (addends[i].has_value()) {
+      const Tensor& a = *addends[i];
+      TORCH_CHECK(a.is_cuda() && a.sizes() == y.sizes() && a.stride(1) == 1 && a.scalar_type() == x.scalar_type());
+      j.addend = a.data_ptr(); j.ld_add = a.stride(0);
+    }
+    if (x.scalar_type() == at::kFloat ||
+        !mb::skinny_gemm_ok((int)M, j.N, j.K, j.ldx, j.ldw, j.x, j.w, dtype_code(x)))
+      return -1;
+  }
+  return mb::skinny_gemm(jobs, (int)n, (int)M, dtype_code(xs[0]), pdl, err.data_ptr<int>(),
+                         at::cuda::getCurrentDeviceProperties()->multiProcessorCount, stream());
 }
 
 // ------------------------------------------------------------------ FFT long convolution
@@ -649,12 +693,122 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_buf, const Tensor& v_bu
   TORCH_CHECK(k_buf.scalar_type() == q.scalar_type() && v_buf.scalar_type() == q.scalar_type());
   const int B = q.size(0), H = q.size(1), dk = q.size(2), C = k_buf.size(2), dv = v_buf.size(3);
   TORCH_CHECK(k_buf.size(0) == B && k_buf.size(1) == H && k_buf.size(3) == dk && v_buf.size(2) == C && dk % 8 == 0);
-  TORCH_CHECK(C * 4 <= 200 * 1024, "key buffer too long for the score array in shared memory");
+  TORCH_CHECK(C <= 51200 && dv % 8 == 0, "decode_attention: key buffer too long or value width not a multiple of 8");
+  for (const Tensor* t : {&k_buf, &v_buf})
+    TORCH_CHECK((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "decode_attention: buffers must be 16-byte aligned");
   Tensor out = torch::empty({B, H, dv}, q.options());
-  mb::decode_attention(q.data_ptr(), k_buf.data_ptr(), v_buf.data_ptr(),
-                       reinterpret_cast<const long long*>(pos.data_ptr<int64_t>()), out.data_ptr(), B * H,
-                       C, dk, dv, (float)scale, dtype_code(q), stream());
+  const int splits = mb::decode_attend_splits(B * H, C, at::cuda::getCurrentDeviceProperties()->multiProcessorCount);
+  Tensor acc = torch::empty({(int64_t)B * H * splits, dv}, q.options().dtype(at::kFloat));
+  Tensor ml = torch::empty({(int64_t)B * H * splits, 2}, acc.options());
+  mb::DecodeAttend a{};
+  a.q = q.data_ptr(); a.k_buf = k_buf.data_ptr(); a.v_buf = v_buf.data_ptr();
+  a.pos = reinterpret_cast<const long long*>(pos.data_ptr<int64_t>());
+  a.out = out.data_ptr(); a.part_acc = acc.data_ptr<float>(); a.part_ml = ml.data_ptr<float>();
+  a.scale = (float)scale; a.H = H; a.C = C; a.dk = dk; a.dv = dv;
+  TORCH_CHECK(mb::decode_attend(a, B, splits, dtype_code(q), false, stream()) == 0, "decode_attention: launch failed");
   return out;
+}
+
+// ---- links of the decode chain (decoding.py): every tensor is checked here, outputs and state are the caller's
+void check_link(const Tensor& t, const char* name, at::ScalarType st, std::vector<int64_t> shape) {
+  check_cuda_contig(t, name);
+  TORCH_CHECK(t.scalar_type() == st && t.sizes().vec() == shape, name, ": unexpected type or shape");
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, name, " must be 16-byte aligned");
+}
+
+// x [B, D]: TimestepNorm step (count, mean, var updated) -> t_out; with hx also the EMA step (hx updated) and RMSNorm
+// -> mx_out, otherwise `pos` (if given) moves on modulo `chunk`
+void decode_norm_ema(const Tensor& x, const Tensor& w, const Tensor& b, Tensor count, Tensor mean, Tensor var,
+                     Tensor t_out, const OptTensor& p, const OptTensor& q, const OptTensor& gamma,
+                     const OptTensor& omega, const OptTensor& hx, const OptTensor& rms_w, const OptTensor& mx_out,
+                     const OptTensor& pos, int64_t chunk, double eps, double rms_eps, bool pdl) {
+  TORCH_CHECK(x.dim() == 2 && mean.dim() == 2);
+  const int64_t B = x.size(0), D = x.size(1), G = mean.size(1);
+  const auto T = x.scalar_type();
+  TORCH_CHECK(T == at::kBFloat16 || T == at::kHalf);
+  check_link(x, "x", T, {B, D});
+  check_link(w, "w", T, {D});
+  check_link(b, "b", T, {D});
+  check_link(count, "count", at::kLong, {B});
+  check_link(mean, "mean", at::kFloat, {B, G});
+  check_link(var, "var", at::kFloat, {B, G});
+  check_link(t_out, "t_out", T, {B, D});
+  c10::cuda::CUDAGuard guard(x.device());
+  mb::DecodeNormEma a{};
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.b = b.data_ptr();
+  a.count = reinterpret_cast<long long*>(count.data_ptr<int64_t>());
+  a.mean = mean.data_ptr<float>(); a.var = var.data_ptr<float>(); a.t_out = t_out.data_ptr();
+  a.eps = (float)eps; a.rms_eps = (float)rms_eps; a.D = (int)D; a.G = (int)G; a.N = 2; a.chunk = (int)chunk;
+  if (hx.has_value()) {
+    TORCH_CHECK(p.has_value() && q.has_value() && gamma.has_value() && omega.has_value() && mx_out.has_value() && p->dim() == 2);
+    const int64_t N = p->size(1);
+    check_link(*p, "p", at::kFloat, {D, N});
+    check_link(*q, "q", at::kFloat, {D, N, 2});
+    check_link(*gamma, "gamma", at::kFloat, {D, N, 2});
+    check_link(*omega, "omega", T, {D});
+    check_link(*hx, "hx", at::kFloat, {B, D, N, 2});
+    check_link(*mx_out, "mx_out", T, {B, D});
+    if (rms_w.has_value()) check_link(*rms_w, "rms_w", T, {D});
+    a.p = p->data_ptr<float>(); a.q = q->data_ptr<float>(); a.gamma = gamma->data_ptr<float>();
+    a.omega = omega->data_ptr(); a.hx = hx->data_ptr<float>(); a.rms_w = opt_ptr(rms_w);
+    a.mx_out = mx_out->data_ptr(); a.N = (int)N;
+  } else if (pos.has_value()) {
+    TORCH_CHECK(pos->is_cuda() && pos->scalar_type() == at::kLong && pos->numel() == 1 && chunk > 0);
+    a.pos = reinterpret_cast<long long*>(pos->data_ptr<int64_t>());
+  }
+  TORCH_CHECK(mb::decode_norm_ema_ok(a.D, a.G, a.N), "decode_norm_ema: shape not supported");
+  TORCH_CHECK(mb::decode_norm_ema(a, (int)B, dtype_code(x), pdl, stream()) == 0, "decode_norm_ema: launch failed");
+}
+bool decode_norm_ema_ok(int64_t D, int64_t G, int64_t N) { return mb::decode_norm_ema_ok((int)D, (int)G, (int)N); }
+int64_t decode_attend_splits(int64_t BH, int64_t C) {
+  return mb::decode_attend_splits((int)BH, (int)C, at::cuda::getCurrentDeviceProperties()->multiProcessorCount);
+}
+
+// z [B, H * dk] -> normalised, rotated query and key; key and v_new [B, H * dv] go to slot pos of the buffers
+// [B, H, C, .]; out [B, H * dv] = gate * attention over slots 0 .. pos.  part: fp32 scratch, B * H * splits * (dv + 2)
+void decode_attend(const Tensor& z, const Tensor& gamma, const Tensor& beta, const Tensor& freqs, const Tensor& v_new,
+                   Tensor k_buf, Tensor v_buf, const Tensor& pos, const Tensor& gate, Tensor out, Tensor part,
+                   double eps, bool pdl) {
+  TORCH_CHECK(k_buf.dim() == 4 && v_buf.dim() == 4);
+  const int64_t B = k_buf.size(0), H = k_buf.size(1), C = k_buf.size(2), dk = k_buf.size(3), dv = v_buf.size(3);
+  const auto T = z.scalar_type();
+  TORCH_CHECK((T == at::kBFloat16 || T == at::kHalf) && dk % 8 == 0 && dv % 8 == 0 && C <= 51200);
+  check_link(z, "z", T, {B, H * dk});
+  check_link(gamma, "gamma", T, {2, H * dk});
+  check_link(beta, "beta", T, {2, H * dk});
+  check_link(freqs, "freqs", at::kFloat, {C, dk / 2, 2});
+  check_link(v_new, "v_new", T, {B, H * dv});
+  check_link(k_buf, "k_buf", T, {B, H, C, dk});
+  check_link(v_buf, "v_buf", T, {B, H, C, dv});
+  check_link(gate, "gate", T, {B, H * dv});
+  check_link(out, "out", T, {B, H * dv});
+  TORCH_CHECK(pos.is_cuda() && pos.scalar_type() == at::kLong && pos.numel() == 1);
+  c10::cuda::CUDAGuard guard(z.device());
+  const int64_t splits = decode_attend_splits(B * H, C);
+  check_cuda_contig(part, "part");
+  TORCH_CHECK(part.scalar_type() == at::kFloat && part.numel() >= B * H * splits * (dv + 2));
+  mb::DecodeAttend a{};
+  a.z = z.data_ptr(); a.gamma = gamma.data_ptr(); a.beta = beta.data_ptr(); a.freqs = freqs.data_ptr<float>();
+  a.v_new = v_new.data_ptr(); a.k_buf = k_buf.data_ptr(); a.v_buf = v_buf.data_ptr();
+  a.pos = reinterpret_cast<const long long*>(pos.data_ptr<int64_t>());
+  a.gate = gate.data_ptr(); a.out = out.data_ptr();
+  a.part_acc = part.data_ptr<float>(); a.part_ml = a.part_acc + B * H * splits * dv;
+  a.scale = 1.f; a.eps = (float)eps; a.H = (int)H; a.C = (int)C; a.dk = (int)dk; a.dv = (int)dv;
+  TORCH_CHECK(mb::decode_attend(a, (int)B, (int)splits, dtype_code(z), pdl, stream()) == 0, "decode_attend: launch failed");
+}
+
+void decode_layer_norm(const Tensor& x, const OptTensor& w, const OptTensor& b, Tensor y, double eps, bool pdl) {
+  TORCH_CHECK(x.dim() == 2 && x.size(1) % 8 == 0 && x.size(1) <= 16384);
+  const int64_t B = x.size(0), D = x.size(1);
+  const auto T = x.scalar_type();
+  TORCH_CHECK(T == at::kBFloat16 || T == at::kHalf);
+  check_link(x, "x", T, {B, D});
+  check_link(y, "y", T, {B, D});
+  if (w.has_value()) check_link(*w, "w", T, {D});
+  if (b.has_value()) check_link(*b, "b", T, {D});
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(mb::decode_layer_norm(x.data_ptr(), opt_ptr(w), opt_ptr(b), y.data_ptr(), (int)B, (int)D, (float)eps,
+                                    dtype_code(x), pdl, stream()) == 0, "decode_layer_norm: launch failed");
 }
 
 // dout, out [B, L, H, dv] (16-bit), rowsum [B, H, L] fp32 -> (dout / rowsum, delta [B, H, L] = dout . out)
@@ -981,7 +1135,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_gather_supported", [](int64_t M, int64_t N, int64_t K, int64_t world) {
     return mb::gemm_gather_supported((int)M, (int)N, (int)K, (int)world);
   });
-  m.def("gemv_small_m", checked(&gemv_small_m));
+  m.def("gemv", checked(&gemv));
+  m.def("skinny_gemm", checked(&skinny_gemm));
   m.def("rfft_rows", checked(&rfft_rows), py::arg("x"), py::arg("flip"), py::arg("packed") = -1);
   m.def("irfft_rows", checked(&irfft_rows), py::arg("spec"), py::arg("L"), py::arg("packed") = -1);
   m.def("fftconv_apply", checked(&fftconv_apply), py::arg("x"), py::arg("kf"), py::arg("conj_k"), py::arg("packed") = -1);
@@ -1005,6 +1160,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_softmax_bwd", checked(&attn_softmax_bwd));
   m.def("attn_bwd_prep", checked(&attn_bwd_prep));
   m.def("decode_attention", checked(&decode_attention));
+  m.def("decode_norm_ema", checked(&decode_norm_ema));
+  m.def("decode_norm_ema_ok", &decode_norm_ema_ok);
+  m.def("decode_attend_splits", &decode_attend_splits);
+  m.def("decode_attend", checked(&decode_attend));
+  m.def("decode_layer_norm", checked(&decode_layer_norm));
   m.def("p2p_send", checked(&p2p_send));
   m.def("p2p_recv", checked(&p2p_recv), py::arg("dst"), py::arg("local_slot"), py::arg("nbytes"), py::arg("local_flag"),
         py::arg("seq"), py::arg("remote_ack"), py::arg("counter"), py::arg("timeout_ns"), py::arg("abort"),

@@ -83,6 +83,25 @@ void sum_squares(const void* g, long long n, double* out, int dtype, cudaStream_
 void scale_by_ptr(void* g, long long n, const float* scale, int dtype, cudaStream_t st);
 void clip_coef(const double* sumsq, float max_norm, float* norm_out, float* coef_out, cudaStream_t st);
 
+// ---- products with few rows (skinny_gemm.cu): up to four over the same number of rows in one launch
+constexpr int kSkinnyJobs = 4;
+constexpr int kSkinnyMaxRows = 256;
+enum SkinnyAct : int { kSkinnyNone = 0, kSkinnySilu = 1, kSkinnySwiGLU = 2 };
+struct SkinnyJob {
+  const void* x;        // [M, K], row stride ldx
+  const void* w;        // [N, K], row stride ldw
+  const void* w2;       // second weight of a SwiGLU product (layout of w), else null
+  const void* bias;     // [N] or null
+  const void* addend;   // [M, N] in the input type, row stride ld_add, added after the activation; or null
+  void* y;              // [M, N], row stride ldy
+  long long ldx, ldw, ld_add, ldy;
+  int N, K, act, bias_dtype, out_f32;
+};
+bool skinny_gemm_ok(int M, int N, int K, long long ldx, long long ldw, const void* x, const void* w, int in_dtype);
+// pdl: the launch may overlap the end of the kernel before it (only inside a chain of such launches)
+int skinny_gemm(const SkinnyJob* jobs, int njobs, int M, int in_dtype, bool pdl, int* err, int num_sms,
+                cudaStream_t st);
+
 // ---- tcgen05 GEMM (gemm_sm100.cu): C[M,N] = act(A B^T + bias)
 // lda / ldb / ldc: row strides in elements (multiples of 8).  mode: 0 dense, 1..3 causal tile structure
 // (see gemm_sm100.cu).  The result is scaled by alpha before bias / activation.  `batch` independent
@@ -147,10 +166,48 @@ void fftconv_rows(const void* x, const float* kf, void* y, long long rows, int L
 // the gradient w.r.t. the kernel in one pass; rows of at most 8192 samples (longer: rfft_rows + irfft_rows)
 void fftconv_dk(const void* dy, const void* x, float* acc_spec, float* dk, long long rows, int L, int D, int dtype,
                 cudaStream_t st);
-// y = act(alpha x w^T + bias) for M <= 16 rows of x (gemv_kernels.cu); false if the shapes do not qualify
-bool gemv_small_m(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int M, int N, int K,
-                  long long ldx, long long ldw, long long ldy, float alpha, int act, int in_dtype, int out_dtype,
-                  cudaStream_t st);
+// y [N] = act(x w^T + bias) for one row x [K] (gemv_kernels.cu); false if the shapes do not qualify
+bool gemv(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int N, int K, long long ldw, int act,
+          int in_dtype, int out_dtype, cudaStream_t st);
+
+// ---- one token against a fixed-shape state (decode_kernels.cu); 16-bit activations and weights, fp32 state
+struct DecodeNormEma {
+  const void* x;                        // [B, D]
+  const void *w, *b;                    // [D] TimestepNorm weight (applied as w + 1) and bias
+  long long* count;                     // [B], updated
+  float *mean, *var;                    // [B, G], updated
+  void* t_out;                          // [B, D] normalised input
+  // complex EMA and RMSNorm; hx null: the norm alone
+  const float *p, *q, *gamma;           // [D, N], [D, N, 2], [D, N, 2]
+  const void* omega;                    // [D]
+  float* hx;                            // [B, D, N, 2], updated
+  const void* rms_w;                    // [D] or null
+  void* mx_out;                         // [B, D]
+  long long* pos;                       // with hx null: advanced modulo `chunk` after the last layer; or null
+  float eps, rms_eps;
+  int D, G, N, chunk;
+};
+bool decode_norm_ema_ok(int D, int G, int N);
+int decode_norm_ema(const DecodeNormEma& p, int B, int dtype, bool pdl, cudaStream_t st);
+
+constexpr int kDecodeMaxSplits = 64;
+struct DecodeAttend {
+  const void* q;                        // [B, H, dk] ready query, or null with z [B, H, dk] below
+  const void *z, *gamma, *beta;         // gamma, beta [2, H * dk]
+  const float* freqs;                   // [C, dk / 2, 2] cos, sin by position in the chunk
+  const void* v_new;                    // [B, H, dv] with z: this token's values
+  void *k_buf, *v_buf;                  // [B, H, C, dk], [B, H, C, dv]
+  const long long* pos;                 // [1]: slots 0 .. pos take part
+  const void* gate;                     // [B, H, dv] multiplied into the result, or null
+  void* out;                            // [B, H, dv]
+  float *part_acc, *part_ml;            // [B * H, splits, dv], [B * H, splits, 2]
+  float scale, eps;
+  int H, C, dk, dv;
+};
+int decode_attend_splits(int BH, int C, int num_sms);
+int decode_attend(const DecodeAttend& p, int B, int splits, int dtype, bool pdl, cudaStream_t st);
+int decode_layer_norm(const void* x, const void* w, const void* b, void* y, int rows, int D, float eps, int dtype,
+                      bool pdl, cudaStream_t st);
 // reduce-scatter fused with the sharded AdamW update (comm_kernels.cu); false if the shapes do not qualify
 bool reduce_scatter_adamw(const void* const* bufs, int rank, int world, long long shard_n, float scale, float* p,
                           float* m, float* v, void* low, double* sumsq, float lr, float beta1, float beta2, float eps,
@@ -168,10 +225,6 @@ void attn_softmax_fwd(void* s_inout, float* lse, long long rows, int L1, int L2,
                       cudaStream_t st);
 void attn_softmax_bwd(const void* p, void* dp_inout, long long rows, int L1, int L2, long long ld, bool causal,
                       int dtype, cudaStream_t st);
-// one decode step against fixed key / value buffers [BH, C, dk] / [BH, C, dv], keys 0 .. *pos valid (device scalar);
-// dk a multiple of 8, 16-bit types; out [BH, dv]
-void decode_attention(const void* q, const void* kb, const void* vb, const long long* pos, void* out, int BH, int C,
-                      int dk, int dv, float scale, int dtype, cudaStream_t st);
 // delta[b, h, l] = dO . O and dO' = dO / rowsum[b, h, l] over rows of dv values (dv a multiple of 8, 16-bit types)
 void attn_bwd_prep(const void* dout, const void* out, const float* rowsum, void* dos, float* delta, int B, int L,
                    int H, int dv, int dtype, cudaStream_t st);

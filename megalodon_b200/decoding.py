@@ -17,6 +17,11 @@ shapes never change -
 captures the step in a CUDA graph; from then on a token is one graph launch.
 On CPU, with tensor-parallel ranks, or with `use_graph=False` the same code
 runs eagerly, which is what the tests compare against the regular cache path.
+
+On one GPU with 16-bit weights the step is a chain of native launches
+(`_native_step`): per layer four products and five kernels for everything
+between them, each a link of a programmatic dependent launch chain, instead of
+some thirty-five launches through the modules.
 """
 from __future__ import annotations
 
@@ -62,7 +67,9 @@ class DecodeSession:
         G = first.timenorm.groups_per_partition
         D, N = first.local_mdim, first.cema.ndim
         dev = self.device
-        stat_dtype = dtype
+        self._native = self._native_ok()
+        # the native step keeps the running statistics in fp32, the modules hand them on in the compute dtype
+        stat_dtype = torch.float32 if self._native else dtype
 
         def norm_state(groups):
             return [torch.zeros(batch_size, dtype=torch.int64, device=dev),
@@ -84,6 +91,8 @@ class DecodeSession:
         self._graph = None
         self._eager_steps = 0
         self._fresh = True           # no statistics yet: the norms start from their priors
+        if self._native:
+            self._native_buffers()
 
     # ------------------------------------------------------------------ state import
     @torch.no_grad()
@@ -107,10 +116,131 @@ class DecodeSession:
         self.pos.fill_(n)
         self._fresh = False
 
+    # ------------------------------------------------------------------ one token, native chain
+    def _native_ok(self) -> bool:
+        """Whether every layer is inside what the native step covers: one GPU's worth of 16-bit parameters
+        in the session's dtype, plain MEGA blocks, sizes the kernels take."""
+        from .models.mega import MegaBlock
+        from .ops import native_for
+        from .ops._ext import require
+        m = self.mega
+        if self.device.type != "cuda" or self.dtype not in (torch.bfloat16, torch.float16) or self._small is not None:
+            return False
+        w = m.embed.weight
+        if w is None or w.dtype != self.dtype or not native_for(w) or self.B > 64:
+            return False
+        from .ops import cuda_ops
+        if cuda_ops.gemm_backend() != "tcgen05" or m.embed.weight.shape[1] != m.model_dim:
+            return False
+        C = require()
+        for layer in m.layers:
+            block = _unwrap(layer)
+            if type(block) is not MegaBlock or block.nffn.alpha is not None:
+                return False
+            a = block.mega
+            dims = (a.mdim, a.z_head_dim, a.local_v_head_dim, block.nffn.hidden_dim)
+            if (a.head_split != 1 or a.local_heads != a.num_heads or a.local_mdim != a.mdim or a.mdim > 16384
+                    or any(d % 8 for d in dims) or m.chunk_size > 51200
+                    or not C.decode_norm_ema_ok(a.mdim, a.timenorm.groups_per_partition, a.cema.ndim)):
+                return False
+            if any(p.dtype != self.dtype or not p.is_contiguous() or p.data_ptr() % 16
+                   for p in self._layer_params(block)):
+                return False
+        fn, out = m.output.final_norm, m.output.output
+        return (C.decode_norm_ema_ok(m.model_dim, fn.groups_per_partition, 2) and out.weight.dtype == self.dtype
+                and out.weight.shape[1] == m.model_dim and out.bias is None)
+
+    @staticmethod
+    def _layer_params(block):
+        a, f = block.mega, block.nffn
+        ps = [a.gamma, a.beta, a.timenorm.weight, a.timenorm.bias, a.rmsnorm.weight, a.cema.omega, a.wv.weight, a.wv.bias,
+              a.wz.weight, a.wz.bias, a.wr.weight, a.wr.bias, a.wh1.weight, a.wh1.bias, a.wh2.weight,
+              f.norm.weight, f.norm.bias, f.fc1.weight, f.fc2.weight]
+        if f.fc3 is not None:
+            ps.append(f.fc3.weight)
+        return [p for p in ps if p is not None]
+
+    def _native_buffers(self) -> None:
+        """Activations of a step.  They are shared by all layers: a link writes only after its predecessor is
+        complete, and by then everything that read the buffer is."""
+        m, B, dev = self.mega, self.B, self.device
+        a = _unwrap(m.layers[0]).mega
+        D, S, V, F = m.model_dim, a.num_heads * a.z_head_dim, a.num_heads * a.local_v_head_dim, \
+            _unwrap(m.layers[0]).nffn.hidden_dim
+        from .ops._ext import require
+        splits = require().decode_attend_splits(B * a.num_heads, m.chunk_size)
+        self._buf = {n: torch.empty(B, k, dtype=self.dtype, device=dev) for n, k in
+                     dict(t=D, mx=D, z=S, r=V, v=V, h=D, attn=V, y=D, f=D, u=F, x0=D, x1=D).items()}
+        self._buf["logits"] = torch.empty(B, m.output_size, dtype=torch.float32, device=dev)
+        self._buf["part"] = torch.empty(B * a.num_heads * splits * (a.local_v_head_dim + 2), device=dev)
+
+    def _start_stats(self) -> None:
+        """A sequence without a past starts from the priors of its norms."""
+        for layer, st in zip(self.mega.layers, self.layers):
+            for dst, src in zip(st["norm"], _unwrap(layer).mega.timenorm.initial_stats(self.B, torch.float32)):
+                dst.copy_(src)
+        for dst, src in zip(self.out_norm, self.mega.output.final_norm.initial_stats(self.B, torch.float32)):
+            dst.copy_(src)
+
+    def _native_step(self) -> Tensor:
+        from .ops import cuda_ops
+        from .ops._ext import require
+        C, m, b = require(), self.mega, self._buf
+        err = cuda_ops._err_flag(self.device)
+        if self._fresh:
+            self._start_stats()
+        table = torch.view_as_real(m.rope.get_freqs_cis(0, m.chunk_size))
+        keep = [table]               # what a captured graph reads besides the session's buffers and the weights
+
+        def products(xs, ws, biases, addends, acts, outs, w2=None):
+            rc = C.skinny_gemm(xs, ws, [w2] if w2 is not None else [None] * len(xs), biases, addends, acts, outs, True,
+                               err)
+            if rc != 0:
+                raise RuntimeError(f"decode products: launch failed with code {rc}")
+
+        x = torch.nn.functional.embedding(self.tok[:, 0], m.embed.weight)
+        if m.emb_scale is not None:
+            x = x * m.emb_scale
+        n = 0
+        for layer, st in zip(m.layers, self.layers):
+            block = _unwrap(layer)
+            a, f = block.mega, block.nffn
+            p, q, gamma = a.cema.coeffs()
+            coeffs = [p.reshape(a.mdim, -1).float().contiguous(),
+                      torch.view_as_real(q.reshape(a.mdim, -1).contiguous()),
+                      torch.view_as_real(gamma.reshape(a.mdim, -1).contiguous()),
+                      a.cema.omega.view(a.mdim)]
+            keep += coeffs
+            count, mean, var = st["norm"]
+            C.decode_norm_ema(x, a.timenorm.weight, a.timenorm.bias, count, mean, var, b["t"], *coeffs,
+                              torch.view_as_real(st["hx"]), a.rmsnorm.weight, b["mx"], None, 0, a.timenorm.eps,
+                              a.rmsnorm.eps, n > 0)
+            products([b["mx"], b["mx"], b["t"], b["mx"]], [a.wh1.weight, a.wr.weight, a.wv.weight, a.wz.weight],
+                     [a.wh1.bias, a.wr.bias, a.wv.bias, a.wz.bias], [x, None, None, None], [0, 1, 1, 0],
+                     [b["h"], b["r"], b["v"], b["z"]])
+            C.decode_attend(b["z"], a.gamma, a.beta, table, b["v"], st["k"], st["v"], self.pos, b["r"], b["attn"],
+                            b["part"], a.znorm.eps, True)
+            products([b["attn"]], [a.wh2.weight], [None], [b["h"]], [0], [b["y"]])
+            C.decode_layer_norm(b["y"], f.norm.weight, f.norm.bias, b["f"], f.norm.eps, True)
+            products([b["f"]], [f.fc1.weight], [None], [None], [2 if f.swiglu else 1], [b["u"]],
+                     f.fc3.weight if f.swiglu else None)
+            nxt = b["x0"] if n % 2 == 0 else b["x1"]
+            products([b["u"]], [f.fc2.weight], [None], [x], [0], [nxt])
+            x = nxt
+            n += 1
+        norm, (count, mean, var) = m.output.final_norm, self.out_norm
+        C.decode_norm_ema(x, norm.weight, norm.bias, count, mean, var, b["t"], None, None, None, None, None, None, None,
+                          self.pos, m.chunk_size, norm.eps, 0.0, True)
+        products([b["t"]], [m.output.output.weight], [None], [None], [0], [b["logits"]])
+        cuda_ops._bump(9 * n + 2)
+        self._keep = keep
+        return b["logits"]
+
     # ------------------------------------------------------------------ one token
     def _step_body(self) -> Tensor:
+        if self._native:
+            return self._native_step()
         m = self.mega
-        from . import ops
         x = m.embed(self.tok)
         if m.emb_scale is not None:
             x = x * m.emb_scale
@@ -142,6 +272,8 @@ class DecodeSession:
         try:
             if self._fresh or not self.use_graph or self._eager_steps < 2:
                 self.logits = self._step_body()
+                if self._native:             # the chain's logits buffer belongs to the next step
+                    self.logits = self.logits.clone()
                 self._fresh = False
                 self._eager_steps += 1
                 return self.logits

@@ -27,7 +27,15 @@ def _C():
 # ----------------------------------------------------------------------------- GEMM / linear
 _GEMM_ERR = {}
 _GEMM_BACKEND = [os.environ.get("MEGALODON_B200_GEMM", "tcgen05")]
-_GEMV_MAX_ROWS = 4          # up to this many rows a product runs on the weight-streaming CUDA-core kernel
+# Products with few rows (K-major operands, nothing kept for backward) leave the 256-wide tiles, whose CTAs
+# walk K alone at one memory latency per ring of stages and leave most SMs without a tile.  Measured (us, 256 MiB
+# rewritten before each call, 8192 x 4096 / 4096 x 11264 / 1024 x 1024 weights):
+#   1 row     gemv 26.7 / 37.9 /  8.2   skinny 23.6 / 29.7 / 11.1
+#   16 rows   gemv  193 /  326 / 34.8   skinny 25.6 / 29.7 / 11.2   tiles 42.0 / 82.9 / 17.3
+#   37 rows                             skinny 29.7 / 33.8 / 13.3   tiles 42.1 / 82.9 / 17.4
+#   128 rows                            skinny 58.4 / 72.7 / 19.5   tiles 44.2 / 85.0 / 19.5
+_SKINNY_MAX_ROWS = 64
+_GEMV_MAX_K = 4096          # one row: the CUDA-core kernel needs no tensor maps and starts sooner
 _launches = [0]          # kernels launched by this framework (bench bookkeeping)
 
 
@@ -126,13 +134,9 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
                 out.copy_(res)
             res = out
         return res.to(out_dtype), (pre.to(out_dtype) if want_preact else None)
-    if (a.dim() == 2 and a.shape[0] <= _GEMV_MAX_ROWS and not a_mn and not b_mn and mode == 0 and out is None
-            and not want_preact and not accumulate and not softmax):
-        # a few rows (decoding): one pass over the weights on the CUDA cores beats a 128-row MMA tile; its
-        # time grows with the rows (7B decode: 6.3 / 12.7 / 42 ms per token at 1 / 4 / 16 rows), the MMA
-        # tile's does not, and from about five rows the tile wins
-        _bump()
-        res = _C().gemv_small_m(a, b, bias, 1 if act == "silu" else 0, _DT[out_dtype], alpha)
+    if (a.dim() == 2 and a.shape[0] <= _SKINNY_MAX_ROWS and not a_mn and not b_mn and mode == 0 and alpha == 1.0
+            and not want_preact and not accumulate and (not softmax or list(softmax) == ["aux"])):
+        res = _few_rows(a, b, bias, act, out_dtype, out, softmax["aux"] if softmax else None)
         if res is not None:
             return res, None
     _bump()
@@ -142,6 +146,28 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
     if rc != 0:
         raise RuntimeError(f"tcgen05 GEMM launch failed with code {rc}")
     return res, pre
+
+
+def _few_rows(a: Tensor, b: Tensor, bias, act, out_dtype, out, addend) -> Optional[Tensor]:
+    """act(a b^T + bias) + addend for at most `_SKINNY_MAX_ROWS` rows; None if the kernels do not take the operands."""
+    if a.shape[0] == 1 and b.shape[1] <= _GEMV_MAX_K and out is None and addend is None:
+        res = _C().gemv(a, b, bias, 1 if act == "silu" else 0, _DT[out_dtype])
+        if res is not None:
+            _bump()
+        return res
+    if addend is not None and (addend.dtype != a.dtype or act is not None):
+        return None
+    if out_dtype not in (a.dtype, torch.float32):
+        return None
+    res = out if out is not None else torch.empty(a.shape[0], b.shape[0], dtype=out_dtype, device=a.device)
+    rc = _C().skinny_gemm([a], [b], [None], [bias], [addend], [1 if act == "silu" else 0], [res], False,
+                          _err_flag(a.device))
+    if rc == -1:
+        return None
+    if rc != 0:
+        raise RuntimeError(f"few-row product: launch failed with code {rc}")
+    _bump()
+    return res
 
 
 def _gemm_gathering(x2: Tensor, w: Tensor, b, act, **kw):
@@ -209,8 +235,8 @@ def linear_add(x: Tensor, w: Tensor, b: Optional[Tensor], addend: Tensor) -> Ten
     """x w^T + b + addend; `addend` has the shape of the result."""
     rows = x.numel() // x.shape[-1]
     if (x.dtype == torch.float32 or _GEMM_BACKEND[0] != "tcgen05" or addend.dtype != x.dtype
-            or w.shape[0] % 8 != 0 or rows <= _GEMV_MAX_ROWS or not _tma_ok(x.reshape(-1, x.shape[-1]))):
-        # (a few rows - decoding - stay on the weight-streaming kernel behind `linear`)
+            or w.shape[0] % 8 != 0 or rows <= 1 or not _tma_ok(x.reshape(-1, x.shape[-1]))):
+        # (one row stays on the weight-streaming kernel behind `linear`)
         return linear(x, w, b) + addend
     return _LinearAdd.apply(x, w, b, addend)
 
@@ -751,7 +777,7 @@ class _Attention(torch.autograd.Function):
 
 
 def decode_attention(q, k_buf, v_buf, pos, scale):
-    _bump()
+    _bump(2)
     return _C().decode_attention(q.contiguous(), k_buf, v_buf.contiguous(), pos, float(scale))
 
 

@@ -1,0 +1,158 @@
+"""Products with few rows and the kernels of the native decode step, against 64-bit / module references."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(got, want):
+    return ((got.double() - want.double()).norm() / want.double().norm()).item()
+
+
+# rows around the padding to 16 and the largest accepted; features around the 128-row tile; K with a ragged
+# 64-block, fewer blocks than a split would need, and a long one
+@pytest.mark.parametrize("M", [1, 16, 17, 64, 129, 256])
+@pytest.mark.parametrize("N,K", [(8, 8), (100, 72), (136, 4104), (2056, 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_skinny_products(M, N, K, dtype):
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(M + N + K)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def rand(*s):
+        return torch.randn(*s, device="cuda")
+    x = rand(M, K).to(dtype)
+    w, w2 = (rand(N, K) / K ** 0.5).to(dtype), (rand(N, K) / K ** 0.5).to(dtype)
+    b, add = rand(N).to(dtype), rand(M, N + 8).to(dtype)[:, :N]
+    lin, lin2 = x.double() @ w.double().t(), x.double() @ w2.double().t()
+    outs = [torch.full((M, N), float("nan"), device="cuda") for _ in range(3)]
+    # three jobs of one launch: bias + addend, SiLU, SwiGLU
+    rc = cuda_ops._C().skinny_gemm([x, x, x], [w, w, w], [None, None, w2], [b, b, None], [add, None, None], [0, 1, 2],
+                                   outs, False, err)
+    assert rc == 0 and err.item() == 0
+    silu = torch.nn.functional.silu
+    # fp32 accumulation: the tensor core adds 16 products at a time and truncates, which a sum of K terms of
+    # either sign shows as up to K / 16 steps of 2^-24 each, far below sqrt(K) * 2^-20 of the result's norm
+    tol = max(4e-6, K ** 0.5 * 2.0 ** -20)
+    for got, want in zip(outs, (lin + b.double() + add.double(), silu(lin + b.double()), silu(lin) * lin2)):
+        assert _rel(got, want) < tol, (_rel(got, want), tol)
+    low = torch.empty(M, N, dtype=dtype, device="cuda")
+    assert cuda_ops._C().skinny_gemm([x], [w], [None], [None], [None], [0], [low], False, err) == 0
+    assert _rel(low, lin) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+
+
+def test_few_row_rule_agrees_with_the_tiles():
+    """`gemm` sends 1 row, few rows and many rows to three kernels; strided rows and an addend included."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(3)
+    w = (torch.randn(264, 520, device="cuda") / 520 ** 0.5).bfloat16()
+    big = torch.randn(200, 3, 520, device="cuda").bfloat16()
+    add = torch.randn(200, 264, device="cuda").bfloat16()
+    for M in (1, 2, 63, 64, 65, 200):
+        x = big[:M, 1]                                  # row stride 1560
+        ref = x.double() @ w.double().t()
+        y, _ = cuda_ops.gemm(x, w)
+        assert _rel(y, ref) < 2.0 ** -8
+        z = cuda_ops.linear_add(x, w, None, add[:M])
+        assert _rel(z, ref + add[:M].double()) < 2.0 ** -7
+    cuda_ops.check_kernel_errors()
+
+
+@pytest.mark.parametrize("D,G,N,B", [(512, 32, 16, 1), (1024, 32, 16, 3), (96, 3, 4, 2), (4096, 64, 16, 2), (64, 1, 32, 1)])
+def test_decode_norm_ema(D, G, N, B):
+    from megalodon_b200.ops import cuda_ops, reference
+    torch.manual_seed(D)
+    dev = "cuda"
+    x = torch.randn(B, D, device=dev).bfloat16()
+    w, b, rw, omega = (torch.randn(D, device=dev).mul_(0.1).bfloat16() for _ in range(4))
+    count = torch.tensor([0, 5, 1000][:B], device=dev)
+    mean, var = torch.randn(B, G, device=dev) * 0.1, torch.rand(B, G, device=dev) + 0.5
+    p = torch.rand(D, N, device=dev)
+    q = torch.polar(torch.rand(D, N, device=dev), torch.randn(D, N, device=dev))
+    ga = torch.view_as_complex(torch.randn(D, N, 2, device=dev))
+    hx = torch.view_as_complex(torch.randn(B, D, N, 2, device=dev))
+    ty, c1, m1, v1 = reference.timestep_norm(x.double()[:, None], count, mean.double(), var.double(), w.double(),
+                                             b.double(), None, G, 1e-5, 1.0)
+    t_ref = ty[:, 0].to(torch.bfloat16)
+    h_ref = q.to(torch.complex128) * hx.to(torch.complex128) + p.double() * t_ref.double()[:, :, None]
+    y_ref = ((ga.to(torch.complex128) * h_ref).sum(-1).real + omega.double() * t_ref.double())
+    mx_ref = y_ref * torch.rsqrt(y_ref.pow(2).mean(-1, keepdim=True) + 1e-5) * (rw.double() + 1.0)
+    t, mx = torch.empty_like(x), torch.empty_like(x)
+    cuda_ops._C().decode_norm_ema(x, w, b, count, mean, var, t, p, torch.view_as_real(q), torch.view_as_real(ga), omega,
+                                  torch.view_as_real(hx), rw, mx, None, 0, 1e-5, 1e-5, False)
+    assert torch.equal(count, c1) and _rel(mean, m1) < 1e-6 and _rel(var, v1) < 1e-6
+    # one rounding to 8 bits each way (t), and of y and mx
+    assert _rel(t, ty[:, 0]) < 2.0 ** -8 and _rel(torch.view_as_real(hx), torch.view_as_real(h_ref)) < 2.0 ** -8
+    assert _rel(mx, mx_ref) < 2.0 ** -7
+    pos = torch.tensor([6], device=dev)
+    cuda_ops._C().decode_norm_ema(x, w, b, count, mean, var, t, None, None, None, None, None, None, None, pos, 7, 1e-5,
+                                  0.0, False)
+    assert pos.item() == 0 and torch.equal(count, c1 + 1)
+
+
+@pytest.mark.parametrize("B,H,C,dk,dv,pos", [(1, 1, 40, 8, 8, 0), (2, 3, 100, 72, 200, 99), (1, 4, 4096, 256, 2048, 700),
+                                             (33, 2, 64, 16, 4096, 31)])
+def test_decode_attend(B, H, C, dk, dv, pos):
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(pos)
+    dev = "cuda"
+
+    def rand(*s):
+        return torch.randn(*s, device=dev)
+    z, v, gate = rand(B, H * dk).bfloat16(), rand(B, H * dv).bfloat16(), rand(B, H * dv).bfloat16()
+    gamma, beta = (rand(2, H * dk) * 0.3).bfloat16(), (rand(2, H * dk) * 0.3).bfloat16()
+    kb, vb = rand(B, H, C, dk).bfloat16(), rand(B, H, C, dv).bfloat16()
+    kb[:, :, pos:] = float("nan")                      # neither the stale slots nor slot `pos` may be read
+    vb[:, :, pos:] = float("nan")
+    ang = torch.outer(torch.arange(C, device=dev).float(), torch.rand(dk // 2, device=dev))
+    freqs = torch.polar(torch.ones_like(ang), ang)
+    zn = z.double().view(B, H, dk)
+    zn = zn * torch.rsqrt(zn.pow(2).mean(-1, keepdim=True) + 1e-5)
+    qk = []
+    for i in range(2):
+        u = zn * (gamma[i].double().view(H, dk) + 1.0) / dk ** 0.5 + beta[i].double().view(H, dk)
+        u = torch.view_as_complex(u.view(B, H, dk // 2, 2).contiguous()) * freqs[pos].to(torch.complex128)
+        qk.append(torch.view_as_real(u).reshape(B, H, dk))
+    keys = torch.cat([kb[:, :, :pos].double(), qk[1].bfloat16().double()[:, :, None]], 2)
+    vals = torch.cat([vb[:, :, :pos].double(), v.double().view(B, H, 1, dv)], 2)
+    pr = torch.softmax(torch.einsum("bhd,bhcd->bhc", qk[0], keys), -1)
+    ref = torch.einsum("bhc,bhcd->bhd", pr, vals).reshape(B, -1) * gate.double()
+    out = torch.empty(B, H * dv, device=dev, dtype=torch.bfloat16)
+    splits = cuda_ops._C().decode_attend_splits(B * H, C)
+    part = torch.empty(B * H * splits * (dv + 2), device=dev)
+    cuda_ops._C().decode_attend(z, gamma, beta, torch.view_as_real(freqs), v, kb, vb, torch.tensor([pos], device=dev),
+                                gate, out, part, 1e-5, False)
+    # fp32 scores; one rounding of the result (and a key that may round the other way)
+    assert _rel(out, ref) < 2.0 ** -7
+    assert _rel(kb[:, :, pos], qk[1]) < 2.0 ** -8 and torch.equal(vb[:, :, pos].reshape(B, -1), v)
+
+
+@pytest.mark.parametrize("swiglu,B,D,H,share", [(True, 1, 256, 2, False), (False, 5, 512, 1, True)])
+def test_native_session_matches_cache_path(swiglu, B, D, H, share):
+    """The native chain, eager and replayed, against the growing cache; one step across the chunk boundary."""
+    from megalodon_b200.config import ModelConf
+    from megalodon_b200.decoding import DecodeSession
+    from megalodon_b200.models.mega import build_model
+    from megalodon_b200.ops import cuda_ops
+    from megalodon_b200.utils import init_cache, set_random_seed
+    cfg = ModelConf(num_layers=2, model_dim=D, num_heads=H, z_dim=128, value_dim=512, ffn_hidden_dim=384,
+                    chunk_size=64, vocab_size=520, swiglu=swiglu, norm_num_groups=16, efficient_attn="fused",
+                    share_emb=share, scale_emb=share)
+    set_random_seed(1)
+    model = build_model(cfg, "bf16", False, False).eval()
+    tok = torch.randint(0, 520, (B, 76), device="cuda")
+    with torch.no_grad():
+        fresh = DecodeSession(model, B, use_graph=False)
+        assert fresh._native
+        cache = init_cache(B, model, torch.bfloat16)
+        for i in range(3):                              # from no past at all
+            ref, cache = model(tok[:, i:i + 1], cache=cache)
+            assert _rel(fresh.step(tok[:, i]), ref[:, -1]) < 3e-2
+        _, cache = model(tok[:, 3:60], cache=cache)
+        sess = DecodeSession(model, B)
+        sess.load_cache(cache)
+        for i in range(60, 72):
+            ref, cache = model(tok[:, i:i + 1], cache=cache)
+            assert _rel(sess.step(tok[:, i]), ref[:, -1]) < 3e-2, i
+        assert sess._graph is not None
+    cuda_ops.check_kernel_errors()
