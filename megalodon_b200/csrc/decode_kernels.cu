@@ -39,6 +39,18 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
   float* gr = gm + gl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row0 = (long long)b * p.D + rank * dl;
+  if (p.hx != nullptr) {
+    // state and coefficients on their way into L2 while the previous kernel finishes
+    const long long f0 = (long long)rank * dl * p.N;
+    const int nb = dl * p.N * 4;                                     // bytes of one float per state
+    for (int i = threadIdx.x * 128; i < 2 * nb; i += kDecThreads * 128) {
+      const char* h = reinterpret_cast<const char*>(p.hx + 2 * ((long long)b * p.D * p.N + f0)) + i;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(h));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.q + 2 * f0) + i));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.gamma + 2 * f0) + i));
+      if (i < nb) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.p + f0) + i));
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
   for (int i = threadIdx.x; i < dl; i += kDecThreads) xs[i] = to_f(reinterpret_cast<const T*>(p.x)[row0 + i]);
@@ -154,12 +166,23 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   float* kn = qs + p.dk;                // dk: this token's key
   float* red = kn + p.dk;               // kDecThreads * 8: partial rows of the thread groups
   float* sc = red + kDecThreads * 8;    // scores of this split
-  pdl_wait();
-  pdl_launch_dependents();
+  // In the chain `pos` and the older slots were written by launches long before the predecessor, which itself
+  // waited for them: they may be read, and the split's keys and values fetched into L2, ahead of the wait.
+  if (p.z == nullptr) pdl_wait();
   const int at = (int)min(p.pos[0], (long long)p.C - 1);
   const int n = at + 1;
   const int per = keys_per_split(n, gridDim.x);
   const int lo = blockIdx.x * per, hi = min(n, lo + per);
+  if (lo < hi && warp == 0) {
+    const T* k0 = reinterpret_cast<const T*>(p.k_buf) + ((long long)bh * p.C + lo) * p.dk;
+    const T* v0 = reinterpret_cast<const T*>(p.v_buf) + ((long long)bh * p.C + lo) * p.dv;
+    for (int j = lane; j < hi - lo; j += 32) {
+      bulk_prefetch_l2(v0 + (long long)j * p.dv, p.dv * sizeof(T));
+      bulk_prefetch_l2(k0 + (long long)j * p.dk, p.dk * sizeof(T));
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
   if (lo >= hi) return;
   T* krow = reinterpret_cast<T*>(p.k_buf) + (long long)bh * p.C * p.dk;
   T* vrow = reinterpret_cast<T*>(p.v_buf) + (long long)bh * p.C * p.dv;
@@ -420,7 +443,7 @@ int decode_norm_ema(const DecodeNormEma& p, int B, int dtype, bool pdl, cudaStre
 }
 
 int decode_attend_splits(int BH, int C, int num_sms) {
-  int s = div_up(2 * num_sms, BH > 0 ? BH : 1);
+  int s = 2 * num_sms / (BH > 0 ? BH : 1);         // one wave of two CTAs per SM
   const int least = div_up(C, 16384);              // the scores of a split sit in shared memory
   if (s < least) s = least;
   return s < 1 ? 1 : (s > kDecodeMaxSplits ? kDecodeMaxSplits : s);

@@ -85,7 +85,7 @@ void clip_coef(const double* sumsq, float max_norm, float* norm_out, float* coef
 
 // ---- products with few rows (skinny_gemm.cu): up to four over the same number of rows in one launch
 constexpr int kSkinnyJobs = 4;
-constexpr int kSkinnyMaxRows = 256;
+constexpr int kSkinnyMaxRows = 64;
 enum SkinnyAct : int { kSkinnyNone = 0, kSkinnySilu = 1, kSkinnySwiGLU = 2 };
 struct SkinnyJob {
   const void* x;        // [M, K], row stride ldx

@@ -1,6 +1,6 @@
 // Linear layers for few rows (decoding, short prompts, the last position of a prefill):
 //
-//   y[m, n] = act(sum_k x[m, k] w[n, k] + bias[n]) + addend[m, n]              m < M <= 256
+//   y[m, n] = act(sum_k x[m, k] w[n, k] + bias[n]) + addend[m, n]              m < M <= 64
 //
 // One pass over the weights is what such a product costs, so the kernel is organised as a stream of
 // weight tiles over all SMs.  The operands are swapped: 128 weight rows are the M side of the tcgen05.mma,
@@ -11,8 +11,9 @@
 // Up to four products over the same rows share a launch (the four projections of a MEGA layer), and a
 // product may carry a second weight for SwiGLU: y = silu(x w^T) * (x w2^T).
 //
-// In a chain of programmatic dependent launches the weight tiles of the first ring round are requested
-// before the previous kernel has finished: weights do not depend on it, x does.
+// In a chain of programmatic dependent launches the weight tiles of the first ring round are requested and the
+// rest of the CTA's weights prefetched into L2 before the previous kernel has finished: weights do not depend
+// on it, x does.
 //
 // All waits are bounded; a timeout sets `*err` and the CTA unwinds.
 #include <cuda.h>
@@ -41,7 +42,7 @@ struct SkinnyMaps {
 struct SkinnyParams {
   SkinnyJob job[kSkinnyJobs];
   int tile0[kSkinnyJobs];                // first tile of each product
-  int njobs, M, mpad, split, stages, stage_bytes, tmem_cols, fmt;
+  int njobs, M, mpad, split, stages, stage_bytes, tmem_cols, fmt, chained, red_bytes;
   int* err;
 };
 
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kSkThreads)
 skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ SkinnyParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.stages * p.stage_bytes);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.stages * p.stage_bytes + p.red_bytes);
   uint64_t* empty_bar = full_bar + kSkMaxStages;
   uint64_t* acc_bar = empty_bar + kSkMaxStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_bar + 1);
@@ -118,6 +119,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if (S > 1) cluster_arrive();       // awaited before the first store into another CTA: by then all have started
 
   if (warp == 0) {
     if (elect_one()) {
@@ -128,6 +130,12 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
         mbar_expect_tx(full_bar + i, tx_bytes);
         tma_load_3d(st, &maps.w[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0);
         if (dual) tma_load_3d(st + w_bytes, &maps.w2[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0);
+      }
+      if (p.chained) {
+        for (int i = first; i < total; ++i) {
+          tma_prefetch_3d(&maps.w[ji], (kb0 + i) * kSkBK, n0, 0);
+          if (dual) tma_prefetch_3d(&maps.w2[ji], (kb0 + i) * kSkBK, n0, 0);
+        }
       }
       pdl_wait();
       for (int i = 0; i < first; ++i)
@@ -207,10 +215,10 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
       }
     }
   } else {
-    // every CTA of the cluster is past its last MMA here: the ring is free to hold partial sums
-    cluster_sync_all();
+    cluster_wait();
     const int R = kSkRows / S;                     // features finished by each CTA
-    const uint32_t red = smem_u32(smem);
+    uint8_t* red_smem = smem + p.stages * p.stage_bytes;      // partial sums have memory of their own
+    const uint32_t red = smem_u32(red_smem);
     const int plane = p.mpad * R;                  // floats of one (source, accumulator)
     const int naccs = dual ? 2 : 1;
     if (warp >= 2) {
@@ -228,7 +236,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
     }
     cluster_sync_all();
     if (warp >= 2 && ok) {
-      const float* part = reinterpret_cast<const float*>(smem);
+      const float* part = reinterpret_cast<const float*>(red_smem);
       for (int idx = threadIdx.x - 64; idx < R * p.M; idx += kSkThreads - 64) {
         const int fl = idx % R, m = idx / R;
         const int n = n0 + rank * R + fl;
@@ -316,20 +324,20 @@ int skinny_gemm(const SkinnyJob* jobs, int njobs, int M, int in_dtype, bool pdl,
     if (!make_tmap_3d(&maps.x[i], j.x, j.K, M, 1, j.ldx, 0, kSkBK, p.mpad, in_dtype)) return -4;
   }
   p.stage_bytes = (dual ? 2 : 1) * kSkRows * kSkBK * 2 + p.mpad * kSkBK * 2;
+  // K is split until the tiles cover every SM; at least two k-blocks are left to each CTA
+  p.split = 1;
+  while (p.split < 8 && tiles * p.split < num_sms && min_nk >= 4 * p.split) p.split *= 2;
+  p.red_bytes = p.split > 1 ? (dual ? 2 : 1) * p.mpad * kSkRows * 4 : 0;
   // two CTAs share an SM as long as a ring of at least four stages fits half of its shared memory
-  const int half = 110 * 1024, whole = 224 * 1024;
+  const int half = 110 * 1024 - p.red_bytes, whole = 224 * 1024 - p.red_bytes;
   const int budget = 4 * p.stage_bytes <= half ? half : whole;
   p.stages = budget / p.stage_bytes;
   if (p.stages > kSkMaxStages) p.stages = kSkMaxStages;
   const int ring = p.stages * p.stage_bytes;
-  // K is split until the tiles cover every SM; at least two k-blocks are left to each CTA, and the partial
-  // sums of a split tile have to fit the ring
-  const int red = (dual ? 2 : 1) * p.mpad * kSkRows * 4;
-  p.split = 1;
-  while (p.split < 8 && tiles * p.split < num_sms && min_nk >= 4 * p.split && red <= ring) p.split *= 2;
+  p.chained = pdl ? 1 : 0;
   p.tmem_cols = 32;
   while (p.tmem_cols < p.mpad * (dual ? 2 : 1)) p.tmem_cols *= 2;
-  const size_t smem = 1024 + ring + (2 * kSkMaxStages + 1) * 8 + 16;
+  const size_t smem = 1024 + ring + p.red_bytes + (2 * kSkMaxStages + 1) * 8 + 16;
   if (in_dtype == kBF16) return launch_skinny<__nv_bfloat16>(maps, p, tiles, smem, pdl, st);
   return launch_skinny<__half>(maps, p, tiles, smem, pdl, st);
 }

@@ -99,20 +99,21 @@ class DecodeSession:
     def load_cache(self, cache) -> None:
         """Take over the state of a regular cache (e.g. after prefilling the prompt)."""
         layers, out_norm = cache
+        n = 0
+        dsts, srcs = list(self.out_norm), list(out_norm)
         for st, (kv, norm, hx) in zip(self.layers, layers):
-            st["k"].zero_()
-            st["v"].zero_()
+            if not self._native:     # (the native step reads no slot past `pos`)
+                st["k"].zero_()
+                st["v"].zero_()
             n = 0
             if kv is not None and kv[0] is not None:
                 n = int(kv[2])
                 if n > 0:
                     st["k"][:, :, :n].copy_(kv[0][:, -n:].transpose(1, 2))
                     st["v"][:, :, :n].copy_(kv[1][:, -n:].transpose(1, 2))
-            for dst, src in zip(st["norm"], norm):
-                dst.copy_(src)
-            st["hx"].copy_(hx)
-        for dst, src in zip(self.out_norm, out_norm):
-            dst.copy_(src)
+            dsts += [*st["norm"], torch.view_as_real(st["hx"])]
+            srcs += [*norm, torch.view_as_real(hx)]
+        torch._foreach_copy_(dsts, srcs)
         self.pos.fill_(n)
         self._fresh = False
 

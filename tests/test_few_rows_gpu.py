@@ -11,7 +11,7 @@ def _rel(got, want):
 
 # rows around the padding to 16 and the largest accepted; features around the 128-row tile; K with a ragged
 # 64-block, fewer blocks than a split would need, and a long one
-@pytest.mark.parametrize("M", [1, 16, 17, 64, 129, 256])
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64])
 @pytest.mark.parametrize("N,K", [(8, 8), (100, 72), (136, 4104), (2056, 1024)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_skinny_products(M, N, K, dtype):
