@@ -71,29 +71,31 @@ std::tuple<Tensor, OptTensor> rms_norm_bwd(const Tensor& dy, const Tensor& x, co
   OptTensor dw;
   int wc = 0;
   if (w.has_value()) {
-    dw = torch::zeros({D}, x.options().dtype(at::kFloat));
+    dw = torch::empty({D}, w->options());
     wc = weight_code(x, *w);
   }
-  Tensor ws;     // partial column sums of the wide-row kernel (caching allocator: no device call)
-  if (w.has_value() && D > 1024) ws = torch::empty({(long long)mb::kColsumRows * D}, x.options().dtype(at::kFloat));
+  Tensor ws;     // partial column sums (caching allocator: no device call)
+  if (w.has_value()) ws = torch::empty({(long long)mb::kColsumRows * D}, x.options().dtype(at::kFloat));
   mb::rms_norm_bwd(dy.data_ptr(), x.data_ptr(), opt_ptr(w), (float)w_off, rstd.data_ptr<float>(), dx.data_ptr(),
-                   dw.has_value() ? dw->data_ptr<float>() : nullptr, M, D, dtype_code(x), wc, stream(),
+                   dw.has_value() ? dw->data_ptr() : nullptr, M, D, dtype_code(x), wc, stream(),
                    ws.defined() ? ws.data_ptr<float>() : nullptr);
   return {dx, dw};
 }
 
-// fp32 column sums of a 16-bit matrix [M, N] (the bias gradient of a linear layer)
-Tensor colsum(const Tensor& g) {
+// column sums (fp32 arithmetic) of a 16-bit matrix [M, N], the bias gradient of a linear layer, in `out_dtype`
+Tensor colsum(const Tensor& g, int64_t out_dtype_code) {
   check_cuda_contig(g, "g");
   TORCH_CHECK(g.dim() == 2, "colsum: a matrix");
   c10::cuda::CUDAGuard guard(g.device());
   const int N = g.size(1);
   const long long M = g.size(0);
-  Tensor out = torch::zeros({N}, g.options().dtype(at::kFloat));
+  const at::ScalarType odt = out_dtype_code == 0 ? at::kFloat : (out_dtype_code == 1 ? at::kBFloat16 : at::kHalf);
+  Tensor out = torch::empty({N}, g.options().dtype(odt));
   Tensor ws = torch::empty({(long long)mb::kColsumRows * N}, g.options().dtype(at::kFloat));
-  const bool done = g.element_size() == 2 &&
-                    mb::colsum_16bit(g.data_ptr(), M, N, ws.data_ptr<float>(), out.data_ptr<float>(), dtype_code(g), stream());
-  if (!done) return g.sum(0, /*keepdim=*/false, at::kFloat);
+  const bool done = g.element_size() == 2 && M > 0 &&
+                    mb::colsum_16bit(g.data_ptr(), M, N, ws.data_ptr<float>(), out.data_ptr(), (int)out_dtype_code,
+                                     dtype_code(g), stream());
+  if (!done) return g.sum(0, /*keepdim=*/false, at::kFloat).to(odt);
   return out;
 }
 
@@ -126,15 +128,15 @@ std::tuple<Tensor, OptTensor, OptTensor> layer_norm_bwd(const Tensor& dy, const 
   OptTensor dw, db;
   int wc = 0;
   if (w.has_value()) {
-    dw = torch::zeros({D}, x.options().dtype(at::kFloat));
-    db = torch::zeros({D}, x.options().dtype(at::kFloat));
+    dw = torch::empty({D}, w->options());
+    db = torch::empty({D}, w->options());
     wc = weight_code(x, *w);
   }
   Tensor ws;
-  if (w.has_value() && D > 1024) ws = torch::empty({2LL * mb::kColsumRows * D}, x.options().dtype(at::kFloat));
+  if (w.has_value()) ws = torch::empty({2LL * mb::kColsumRows * D}, x.options().dtype(at::kFloat));
   mb::layer_norm_bwd(dy.data_ptr(), x.data_ptr(), opt_ptr(w), (float)w_off, mean.data_ptr<float>(),
-                     rstd.data_ptr<float>(), dx.data_ptr(), dw.has_value() ? dw->data_ptr<float>() : nullptr,
-                     db.has_value() ? db->data_ptr<float>() : nullptr, M, D, dtype_code(x), wc, stream(),
+                     rstd.data_ptr<float>(), dx.data_ptr(), dw.has_value() ? dw->data_ptr() : nullptr,
+                     db.has_value() ? db->data_ptr() : nullptr, M, D, dtype_code(x), wc, stream(),
                      ws.defined() ? ws.data_ptr<float>() : nullptr);
   return {dx, dw, db};
 }
@@ -177,34 +179,34 @@ std::vector<Tensor> timestep_norm_fwd(const Tensor& x, const Tensor& prev_count,
   return {y, count, mean, var, cummean, cumrstd};
 }
 
-// returns dx, dprev_mean, dprev_var, dgamma(fp32), dbeta(fp32)
-std::vector<Tensor> timestep_norm_bwd(const Tensor& dy, const Tensor& dmean, const Tensor& dvar, const Tensor& x,
+// returns dx, dprev_mean, dprev_var, dgamma, dbeta (in gamma's type)
+std::vector<Tensor> timestep_norm_bwd(const Tensor& dy, const OptTensor& dmean, const OptTensor& dvar, const Tensor& x,
                                       const Tensor& prev_mean, const Tensor& count, const Tensor& cummean,
                                       const Tensor& cumrstd, const Tensor& gamma, double gamma_off,
                                       const OptTensor& mask, int64_t G) {
   check_cuda_contig(dy, "dy");
   check_cuda_contig(x, "x");
-  check_cuda_contig(dmean, "dmean");
-  check_cuda_contig(dvar, "dvar");
+  if (dmean.has_value()) check_cuda_contig(*dmean, "dmean");
+  if (dvar.has_value()) check_cuda_contig(*dvar, "dvar");
   c10::cuda::CUDAGuard guard(x.device());
   const int B = x.size(0), L = x.size(1), H = x.size(2);
   auto f32 = x.options().dtype(at::kFloat);
   Tensor dx = torch::empty_like(x);
   Tensor dpm = torch::empty_like(prev_mean);
   Tensor dpv = torch::empty_like(prev_mean);
-  Tensor dgamma = torch::zeros({H}, f32);
-  Tensor dbeta = torch::zeros({H}, f32);
+  Tensor dgamma = torch::empty({H}, gamma.options());
+  Tensor dbeta = torch::empty({H}, gamma.options());
   Tensor scratch = torch::empty({5, B, L, G}, f32);
   float* sp = scratch.data_ptr<float>();
   const long long n = (long long)B * L * G;
   Tensor seg = torch::empty({4LL * B * mb::tsn_num_segments(L) * G}, x.options().dtype(at::kDouble));
   Tensor cumvalid = torch::empty({mask.has_value() ? (long long)B * L : 0}, x.options().dtype(at::kInt));
   Tensor ws = torch::empty({2LL * mb::kColsumRows * H}, f32);    // partial sums of dgamma | dbeta per CTA
-  mb::timestep_norm_bwd(dy.data_ptr(), dmean.data_ptr(), dvar.data_ptr(), x.data_ptr(), prev_mean.data_ptr(),
+  mb::timestep_norm_bwd(dy.data_ptr(), opt_ptr(dmean), opt_ptr(dvar), x.data_ptr(), prev_mean.data_ptr(),
                         (const long long*)count.data_ptr<int64_t>(), cummean.data_ptr<float>(),
                         cumrstd.data_ptr<float>(), gamma.data_ptr(), (float)gamma_off,
                         mask.has_value() ? mask->data_ptr<bool>() : nullptr, dx.data_ptr(), dpm.data_ptr(),
-                        dpv.data_ptr(), dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), sp, sp + n, sp + 2 * n,
+                        dpv.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), sp, sp + n, sp + 2 * n,
                         sp + 3 * n, sp + 4 * n, seg.data_ptr<double>(), cumvalid.data_ptr<int>(), B, L, H, (int)G,
                         dtype_code(x), weight_code(x, gamma), stream(), ws.data_ptr<float>());
   return {dx, dpm, dpv, dgamma, dbeta};
@@ -244,10 +246,13 @@ std::vector<Tensor> cema_bwd(const Tensor& dy, const Tensor& x, const Tensor& p,
   const int B = x.size(0), L = x.size(1), D = x.size(2), N = p.size(1);
   auto f32 = x.options().dtype(at::kFloat);
   Tensor dx = torch::empty_like(x);
-  Tensor dp = torch::zeros({D, N}, f32);
-  Tensor dq = torch::zeros({D, N, 2}, f32);
-  Tensor dgamma = torch::zeros({D, N, 2}, f32);
-  Tensor domega = torch::zeros({D}, f32);
+  // one fill for the four sums
+  const int64_t dn = (int64_t)D * N;
+  Tensor sums = torch::zeros({5 * dn + D}, f32);
+  Tensor dq = sums.narrow(0, 0, 2 * dn).view({D, N, 2});
+  Tensor dgamma = sums.narrow(0, 2 * dn, 2 * dn).view({D, N, 2});
+  Tensor dp = sums.narrow(0, 4 * dn, dn).view({D, N});
+  Tensor domega = sums.narrow(0, 5 * dn, D);
   Tensor dhx = torch::empty({B, D, N, 2}, f32);
   const int S = mb::cema_num_segments(L);
   const long long cn = S > 1 ? (long long)B * S * N * D * 2 : 0;

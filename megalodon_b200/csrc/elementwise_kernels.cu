@@ -210,6 +210,67 @@ __global__ void ce_bwd_kernel(const T* __restrict__ logits, const long long* __r
   }
 }
 
+// 16-byte forms (V % 8 == 0, rows aligned): the forward pass reads the row once, every thread keeping a running
+// maximum and the sum of exponentials relative to it (rescaled when the maximum moves), instead of two scalar
+// passes.  4000 x 32000 bf16 logits: forward 333 us, backward 271 us before; both are bound by memory (39 and
+// 78 us at the measured copy bandwidth).
+constexpr int kCeThreads = 512;
+template <typename T>
+__global__ void __launch_bounds__(kCeThreads)
+ce_fwd_vec_kernel(const T* __restrict__ logits, const long long* __restrict__ target, float* __restrict__ loss,
+                  float* __restrict__ lse, int V, long long ignore_index) {
+  __shared__ float scratch[32];
+  const long long row = blockIdx.x;
+  const T* lr = logits + row * V;
+  float m = -INFINITY, s = 0.f;
+#pragma unroll 4
+  for (int j = threadIdx.x * 8; j < V; j += kCeThreads * 8) {
+    float v[8];
+    load8(lr + j, v);
+    float vm = m;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) vm = fmaxf(vm, v[i]);
+    const float ref = vm == -INFINITY ? 0.f : vm;      // nothing but weights of zero so far
+    s = m == vm ? s : s * __expf(m - ref);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += __expf(v[i] - ref);
+    m = vm;
+  }
+  const float rm = block_max(m, scratch);
+  const float ref = rm == -INFINITY ? 0.f : rm;
+  s = block_sum(m == -INFINITY ? s : s * __expf(m - ref), scratch);
+  if (threadIdx.x == 0) {
+    const float l = rm + logf(s);
+    lse[row] = l;
+    const long long t = target[row];
+    loss[row] = (t == ignore_index || t < 0 || t >= V) ? 0.f : l - to_f(lr[t]);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCeThreads)
+ce_bwd_vec_kernel(const T* __restrict__ logits, const long long* __restrict__ target, const float* __restrict__ lse,
+                  const float* __restrict__ dloss, T* __restrict__ dlogits, int V, long long ignore_index) {
+  const long long row = blockIdx.x;
+  const long long t = target[row];
+  const bool skip = (t == ignore_index || t < 0 || t >= V);
+  const float g = skip ? 0.f : dloss[row];
+  const float l = lse[row];
+  const T* lr = logits + row * V;
+  T* dr = dlogits + row * V;
+#pragma unroll 4
+  for (int j = threadIdx.x * 8; j < V; j += kCeThreads * 8) {
+    float v[8];
+    load8(lr + j, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float p = __expf(v[i] - l);
+      v[i] = (j + i == t ? p - 1.f : p) * g;
+    }
+    store8(dr + j, v);
+  }
+}
+
 __device__ __forceinline__ void load4(const float* p, float (&o)[4]) {
   const float4 t = *reinterpret_cast<const float4*>(p);
   o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
@@ -288,11 +349,19 @@ __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, flo
 }
 
 template <typename T>
-__global__ void sumsq_kernel(const T* __restrict__ g, long long n, double* __restrict__ out) {
+__global__ void sumsq_kernel(const T* __restrict__ g, long long n, long long n8, double* __restrict__ out) {
   __shared__ float scratch[32];
-  float acc = 0.f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  float part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (long long i = tid; i < n8; i += stride) {
+    float v[8];
+    load8(g + 8 * i, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[j] = fmaf(v[j], v[j], part[j]);
+  }
+  float acc = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+  for (long long i = 8 * n8 + tid; i < n; i += stride) {
     const float v = to_f(g[i]);
     acc += v * v;
   }
@@ -300,13 +369,21 @@ __global__ void sumsq_kernel(const T* __restrict__ g, long long n, double* __res
   if (threadIdx.x == 0) atomicAdd(out, (double)acc);
 }
 
+// 16-byte accesses: 1.6 GB of bf16 gradients took 1415 us with one element per access
 template <typename T>
-__global__ void scale_by_ptr_kernel(T* __restrict__ g, long long n, const float* __restrict__ scale) {
+__global__ void scale_by_ptr_kernel(T* __restrict__ g, long long n, long long n8, const float* __restrict__ scale) {
   const float s = *scale;
   if (s == 1.f) return;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    g[i] = from_f<T>(to_f(g[i]) * s);
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (long long i = tid; i < n8; i += stride) {
+    float v[8];
+    load8(g + 8 * i, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] *= s;
+    store8(g + 8 * i, v);
+  }
+  for (long long i = 8 * n8 + tid; i < n; i += stride) g[i] = from_f<T>(to_f(g[i]) * s);
 }
 
 // coef = min(1, max_norm / (sqrt(sumsq) + 1e-6)); also writes the norm
@@ -390,6 +467,11 @@ void qk_rotary_bwd(const void* dq, const void* dk, const void* z, const void* ga
 void cross_entropy_fwd(const void* logits, const long long* target, float* loss, float* lse, long long rows,
                        int V, long long ignore_index, int dtype, cudaStream_t st) {
   if (rows == 0) return;
+  if (V % 8 == 0 && aligned32(logits)) {
+    MB_DISPATCH_DTYPE(dtype, (ce_fwd_vec_kernel<scalar_t><<<(unsigned)rows, kCeThreads, 0, st>>>(
+                                 (const scalar_t*)logits, target, loss, lse, V, ignore_index)));
+    return;
+  }
   MB_DISPATCH_DTYPE(dtype, (ce_fwd_kernel<scalar_t><<<(unsigned)rows, 256, 0, st>>>(
                                (const scalar_t*)logits, target, loss, lse, V, ignore_index)));
 }
@@ -398,6 +480,11 @@ void cross_entropy_bwd(const void* logits, const long long* target, const float*
                        void* dlogits, long long rows, int V, long long ignore_index, int dtype,
                        cudaStream_t st) {
   if (rows == 0) return;
+  if (V % 8 == 0 && aligned32(logits) && aligned32(dlogits)) {
+    MB_DISPATCH_DTYPE(dtype, (ce_bwd_vec_kernel<scalar_t><<<(unsigned)rows, kCeThreads, 0, st>>>(
+                                 (const scalar_t*)logits, target, lse, dloss, (scalar_t*)dlogits, V, ignore_index)));
+    return;
+  }
   MB_DISPATCH_DTYPE(dtype, (ce_bwd_kernel<scalar_t><<<(unsigned)rows, 256, 0, st>>>(
                                (const scalar_t*)logits, target, lse, dloss, (scalar_t*)dlogits, V, ignore_index)));
 }
@@ -426,12 +513,16 @@ void adamw_step(float* p, const void* g, float* m, float* v, void* low, long lon
 
 void sum_squares(const void* g, long long n, double* out, int dtype, cudaStream_t st) {
   if (n == 0) return;
-  MB_DISPATCH_DTYPE(dtype, (sumsq_kernel<scalar_t><<<ew_grid(n), 256, 0, st>>>((const scalar_t*)g, n, out)));
+  const long long n8 = aligned32(g) ? n / 8 : 0;
+  MB_DISPATCH_DTYPE(dtype, (sumsq_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+                               (const scalar_t*)g, n, n8, out)));
 }
 
 void scale_by_ptr(void* g, long long n, const float* scale, int dtype, cudaStream_t st) {
   if (n == 0) return;
-  MB_DISPATCH_DTYPE(dtype, (scale_by_ptr_kernel<scalar_t><<<ew_grid(n), 256, 0, st>>>((scalar_t*)g, n, scale)));
+  const long long n8 = aligned32(g) ? n / 8 : 0;
+  MB_DISPATCH_DTYPE(dtype, (scale_by_ptr_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+                               (scalar_t*)g, n, n8, scale)));
 }
 
 void clip_coef(const double* sumsq, float max_norm, float* norm_out, float* coef_out, cudaStream_t st) {

@@ -9,22 +9,21 @@ namespace mb {
 // ---- row-wise norms (norm_kernels.cu); weight dtype is fp32 or the activation dtype
 void rms_norm_fwd(const void* x, const void* w, float w_off, void* y, float* rstd, long long M, int D,
                   float eps, int x_dtype, int w_dtype, cudaStream_t st);
-// `colsum_ws`: kColsumRows * D floats (2 * kColsumRows * D for LayerNorm and TimestepNorm) or null.  With
-// it, every CTA of the wide-row kernels stores its partial column sums (the weight / bias gradients) as one
-// plain row and `colsum_finish` adds the rows up; without it the partial sums go out as atomics.  Either
-// way the sums are ADDED to dw / db.
+// `colsum_ws`: kColsumRows * D floats (2 * kColsumRows * D for LayerNorm and TimestepNorm), null without parameter
+// gradients.  Every CTA of the vectorised kernels stores its partial column sums (the weight / bias gradients)
+// as one plain row and `colsum_finish` adds the rows up (the other paths use atomics on one row); dw / db are
+// written in the type of the weight.
 constexpr int kColsumRows = 296;
-void colsum_finish(const float* ws, int rows, int D, float* out0, float* out1, cudaStream_t st);
-// out[j] += sum over rows of a row-major 16-bit matrix [M, N] (bias gradients); false: shape not covered
-bool colsum_16bit(const void* g, long long M, int N, float* ws, float* out, int dtype, cudaStream_t st);
+void colsum_finish(const float* ws, int rows, int D, void* out0, void* out1, int out_dtype, cudaStream_t st);
+// out[j] = sum over rows of a row-major 16-bit matrix [M, N] (bias gradients); false: shape not covered
+bool colsum_16bit(const void* g, long long M, int N, float* ws, void* out, int out_dtype, int dtype, cudaStream_t st);
 void rms_norm_bwd(const void* dy, const void* x, const void* w, float w_off, const float* rstd, void* dx,
-                  float* dw, long long M, int D, int x_dtype, int w_dtype, cudaStream_t st,
-                  float* colsum_ws = nullptr);
+                  void* dw, long long M, int D, int x_dtype, int w_dtype, cudaStream_t st, float* colsum_ws);
 void layer_norm_fwd(const void* x, const void* w, const void* b, float w_off, void* y, float* mean,
                     float* rstd, long long M, int D, float eps, int x_dtype, int w_dtype, cudaStream_t st);
 void layer_norm_bwd(const void* dy, const void* x, const void* w, float w_off, const float* mean,
-                    const float* rstd, void* dx, float* dw, float* db, long long M, int D, int x_dtype,
-                    int w_dtype, cudaStream_t st, float* colsum_ws = nullptr);
+                    const float* rstd, void* dx, void* dw, void* db, long long M, int D, int x_dtype,
+                    int w_dtype, cudaStream_t st, float* colsum_ws);
 
 // ---- TimestepNorm (timestep_norm_kernels.cu)
 void timestep_norm_fwd(const void* x, const long long* prev_count, const void* prev_mean,
@@ -38,10 +37,10 @@ int tsn_num_segments(int L);
 void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_out, const void* x,
                        const void* prev_mean, const long long* count_final, const float* cummean,
                        const float* cumrstd, const void* gamma, float gamma_offset, const bool* mask,
-                       void* dx, void* dprev_mean, void* dprev_var, float* dgamma, float* dbeta,
+                       void* dx, void* dprev_mean, void* dprev_var, void* dgamma, void* dbeta,
                        float* ux, float* ds, float* db, float* dux, float* dvx, double* seg_scratch,
                        int* cumvalid, int B, int L, int H, int G, int x_dtype, int w_dtype, cudaStream_t st,
-                       float* colsum_ws = nullptr);
+                       float* colsum_ws);
 
 // ---- CEMA (cema_kernels.cu); complex tensors are interleaved (re, im) fp32
 constexpr int kCemaSegLen = 128;

@@ -148,6 +148,7 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
 // t, t + ROW_THREADS, ... (at most VPT of them), so x and dy are read once and every access is 16
 // bytes (two for fp32).  Needs D % 8 == 0, D <= ROW_THREADS * 8 * VPT and 32-byte aligned pointers.
 constexpr int kMaxVecVPT = 4;
+constexpr int kNarrowThreads = 256;      // backward with a warp per row: eight rows per CTA iteration
 
 template <typename T, typename W, bool LAYER, int ROW_THREADS, int kVecVPT>
 __global__ void norm_fwd_vec_kernel(const T* __restrict__ x, const W* __restrict__ weight,
@@ -230,8 +231,7 @@ template <typename T, typename W, bool LAYER, int ROW_THREADS, int kVecVPT>
 __global__ void norm_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                     const W* __restrict__ weight, float weight_offset,
                                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
-                                    T* __restrict__ dx, float* __restrict__ dweight, float* __restrict__ dbias,
-                                    long long M, int D, float* __restrict__ colsum_ws) {
+                                    T* __restrict__ dx, long long M, int D, float* __restrict__ colsum_ws) {
   __shared__ float scratch[32];
   const int rows_per_cta = blockDim.x / ROW_THREADS;
   const int sub = threadIdx.x / ROW_THREADS;
@@ -296,10 +296,38 @@ __global__ void norm_bwd_vec_kernel(const T* __restrict__ dy, const T* __restric
       }
     }
   }
-  if (dweight != nullptr && colsum_ws != nullptr) {
-    // one row of partial sums per CTA (one row per CTA iteration on this path: ROW_THREADS == blockDim.x)
+  if (colsum_ws != nullptr) {
+    // one row of partial sums per CTA
     constexpr int kSets = LAYER ? 2 : 1;
     float* mine = colsum_ws + (long long)blockIdx.x * kSets * D;
+    if constexpr (ROW_THREADS == 32) {
+      // the warps' sums meet in shared memory, half of them folding into the other half each round.  As one
+      // atomic per column and warp (2368 warps on 1024 columns) they were nearly all of the kernel's time:
+      // LayerNorm of 4000 x 1024, 232 us.
+      constexpr int kHalf = kNarrowThreads / 64;
+      __shared__ float part[kHalf][32 * 8 * kVecVPT];
+#pragma unroll
+      for (int set = 0; set < kSets; ++set) {
+        float (&acc)[kVecVPT][8] = set == 0 ? acc_w : acc_b;
+        for (int half = kHalf; half > 0; half /= 2) {
+          if (sub >= half && sub < 2 * half) {
+#pragma unroll
+            for (int i = 0; i < kVecVPT; ++i)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) part[sub - half][(i * 8 + j) * 32 + t] = acc[i][j];
+          }
+          __syncthreads();
+          if (sub < half) {
+#pragma unroll
+            for (int i = 0; i < kVecVPT; ++i)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[i][j] += part[sub][(i * 8 + j) * 32 + t];
+          }
+          __syncthreads();
+        }
+      }
+      if (sub != 0) return;
+    }
 #pragma unroll
     for (int i = 0; i < kVecVPT; ++i) {
       const int g = t + i * ROW_THREADS;
@@ -308,25 +336,15 @@ __global__ void norm_bwd_vec_kernel(const T* __restrict__ dy, const T* __restric
         if (LAYER) store8(mine + D + 8 * g, acc_b[i]);
       }
     }
-  } else if (dweight != nullptr) {
-#pragma unroll
-    for (int i = 0; i < kVecVPT; ++i) {
-      const int g = t + i * ROW_THREADS;
-      if (g < nvec) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          atomicAdd(dweight + 8 * g + j, acc_w[i][j]);
-          if (LAYER && dbias != nullptr) atomicAdd(dbias + 8 * g + j, acc_b[i][j]);
-        }
-      }
-    }
   }
 }
 
-// out0[j] += sum over rows of ws[row][0][j] (and out1 from ws[row][1][j] when given): a warp owns 32
-// adjacent columns (128-byte reads), the 8 warps of a CTA take every 8th row and meet in shared memory.
-__global__ void colsum_finish_kernel(const float* __restrict__ ws, int rows, int D, float* __restrict__ out0,
-                                     float* __restrict__ out1) {
+// out0[j] = sum over rows of ws[row][0][j] (and out1 from ws[row][1][j] when given), in the type of the parameter
+// whose gradient it is: a warp owns 32 adjacent columns (128-byte reads), the 8 warps of a CTA take every 8th
+// row and meet in shared memory.
+template <typename O>
+__global__ void colsum_finish_kernel(const float* __restrict__ ws, int rows, int D, O* __restrict__ out0,
+                                     O* __restrict__ out1) {
   __shared__ float part[2][8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
@@ -348,8 +366,8 @@ __global__ void colsum_finish_kernel(const float* __restrict__ ws, int rows, int
       s0 += part[0][w][lane];
       s1 += part[1][w][lane];
     }
-    out0[j] += s0;
-    if (out1 != nullptr) out1[j] += s1;
+    out0[j] = from_f<O>(s0);
+    if (out1 != nullptr) out1[j] = from_f<O>(s1);
   }
 }
 
@@ -397,37 +415,42 @@ void launch_fwd(const void* x, const void* w, const void* b, float off, void* y,
   }
 }
 
+// ws: the workspace of the column sums, null without parameter gradients; its first row serves as the target of
+// the atomics on the paths that have no partial rows
 template <typename T, typename W, bool LAYER>
 void launch_bwd(const void* dy, const void* x, const void* w, float off, const float* mean,
-                const float* rstd, void* dx, float* dw, float* db, long long M, int D, cudaStream_t st,
+                const float* rstd, void* dx, void* dw, void* db, long long M, int D, int w_dtype, cudaStream_t st,
                 float* ws) {
+  float *aw = ws, *ab = ws != nullptr && LAYER ? ws + D : nullptr;
   if (D <= 1024 && vec_ok(D, 32, {dy, x, w, dx})) {
-    const int threads = 128, rows = threads / 32;
-    const int grid = (int)std::min<long long>((M + rows - 1) / rows, 148LL * 4);
-    VPT_SWITCH(D, 32, (norm_bwd_vec_kernel<T, W, LAYER, 32, VPT><<<grid, threads, 0, st>>>(
-                           (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, dw, db, M, D, nullptr)));
+    const int rows = kNarrowThreads / 32;
+    const int grid = (int)std::min<long long>((M + rows - 1) / rows, (long long)kColsumRows);
+    VPT_SWITCH(D, 32, (norm_bwd_vec_kernel<T, W, LAYER, 32, VPT><<<grid, kNarrowThreads, 0, st>>>(
+                           (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, M, D, ws)));
+    if (ws != nullptr) colsum_finish(ws, grid, D, dw, LAYER ? db : nullptr, w_dtype, st);
     return;
   }
   if (D > 1024 && vec_ok(D, 256, {dy, x, w, dx})) {
     // one resident wave (the accumulators of the column sums cap the kernel at two CTAs per SM)
     const int grid = (int)std::min<long long>(M, (long long)kColsumRows);
-    float* use_ws = (dw != nullptr && (!LAYER || db != nullptr)) ? ws : nullptr;
     VPT_SWITCH(D, 256, (norm_bwd_vec_kernel<T, W, LAYER, 256, VPT><<<grid, 256, 0, st>>>(
-                            (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, dw, db, M, D, use_ws)));
-    if (use_ws != nullptr) colsum_finish(use_ws, grid, D, dw, LAYER ? db : nullptr, st);
+                            (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, M, D, ws)));
+    if (ws != nullptr) colsum_finish(ws, grid, D, dw, LAYER ? db : nullptr, w_dtype, st);
     return;
   }
+  if (ws != nullptr) cudaMemsetAsync(ws, 0, sizeof(float) * (LAYER ? 2 : 1) * D, st);
   if (D <= 1024) {
     const int threads = 128, rows = threads / 32;
     const int grid = (int)std::min<long long>((M + rows - 1) / rows, 148LL * 4);
     norm_bwd_kernel<T, W, LAYER, 32><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const W*)w, off,
-                                                               mean, rstd, (T*)dx, dw, db, M, D);
+                                                               mean, rstd, (T*)dx, aw, ab, M, D);
   } else {
     const int threads = 256;
     const int grid = (int)std::min<long long>(M, 148LL * 4);
     norm_bwd_kernel<T, W, LAYER, 256><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const W*)w, off,
-                                                                mean, rstd, (T*)dx, dw, db, M, D);
+                                                                mean, rstd, (T*)dx, aw, ab, M, D);
   }
+  if (ws != nullptr) colsum_finish(ws, 1, D, dw, LAYER ? db : nullptr, w_dtype, st);
 }
 
 }  // namespace
@@ -480,9 +503,9 @@ __global__ void colsum_partial_kernel(const T* __restrict__ g, long long M, int 
   }
 }
 
-// out[j] += sum_m g[m, j]; needs N % 8 == 0, N <= 8192, g 16-byte aligned; ws: kColsumRows * N floats.
+// out[j] = sum_m g[m, j]; needs N % 8 == 0, N <= 8192, g 16-byte aligned; ws: kColsumRows * N floats.
 // Returns false (nothing launched) when the shape is not covered.
-bool colsum_16bit(const void* g, long long M, int N, float* ws, float* out, int dtype, cudaStream_t st) {
+bool colsum_16bit(const void* g, long long M, int N, float* ws, void* out, int out_dtype, int dtype, cudaStream_t st) {
   if (N % 8 != 0 || N > 8192 || (reinterpret_cast<uintptr_t>(g) & 15) != 0 || (dtype != kBF16 && dtype != kF16))
     return false;
   const int grid = (int)std::min<long long>(M, (long long)kColsumRows);
@@ -496,18 +519,19 @@ bool colsum_16bit(const void* g, long long M, int N, float* ws, float* out, int 
   if (dtype == kBF16) MB_COLSUM(__nv_bfloat16);
   else MB_COLSUM(__half);
 #undef MB_COLSUM
-  colsum_finish_kernel<<<(N + 31) / 32, 256, 0, st>>>(ws, grid, N, out, nullptr);
+  colsum_finish(ws, grid, N, out, nullptr, out_dtype, st);
   return true;
 }
 
-void colsum_finish(const float* ws, int rows, int D, float* out0, float* out1, cudaStream_t st) {
-  colsum_finish_kernel<<<(D + 31) / 32, 256, 0, st>>>(ws, rows, D, out0, out1);
+void colsum_finish(const float* ws, int rows, int D, void* out0, void* out1, int out_dtype, cudaStream_t st) {
+  MB_DISPATCH_DTYPE(out_dtype, (colsum_finish_kernel<scalar_t><<<(D + 31) / 32, 256, 0, st>>>(
+                                   ws, rows, D, (scalar_t*)out0, (scalar_t*)out1)));
 }
 
 void rms_norm_bwd(const void* dy, const void* x, const void* w, float w_off, const float* rstd, void* dx,
-                  float* dw, long long M, int D, int x_dtype, int w_dtype, cudaStream_t st, float* colsum_ws) {
+                  void* dw, long long M, int D, int x_dtype, int w_dtype, cudaStream_t st, float* colsum_ws) {
   NORM_DISPATCH(x_dtype, w_dtype,
-                (launch_bwd<T, W, false>(dy, x, w, w_off, nullptr, rstd, dx, dw, nullptr, M, D, st, colsum_ws)));
+                (launch_bwd<T, W, false>(dy, x, w, w_off, nullptr, rstd, dx, dw, nullptr, M, D, w_dtype, st, colsum_ws)));
 }
 
 void layer_norm_fwd(const void* x, const void* w, const void* b, float w_off, void* y, float* mean,
@@ -516,10 +540,10 @@ void layer_norm_fwd(const void* x, const void* w, const void* b, float w_off, vo
 }
 
 void layer_norm_bwd(const void* dy, const void* x, const void* w, float w_off, const float* mean,
-                    const float* rstd, void* dx, float* dw, float* db, long long M, int D, int x_dtype,
+                    const float* rstd, void* dx, void* dw, void* db, long long M, int D, int x_dtype,
                     int w_dtype, cudaStream_t st, float* colsum_ws) {
   NORM_DISPATCH(x_dtype, w_dtype,
-                (launch_bwd<T, W, true>(dy, x, w, w_off, mean, rstd, dx, dw, db, M, D, st, colsum_ws)));
+                (launch_bwd<T, W, true>(dy, x, w, w_off, mean, rstd, dx, dw, db, M, D, w_dtype, st, colsum_ws)));
 }
 
 }  // namespace mb

@@ -417,7 +417,7 @@ __global__ void tsn_bwd_seg_prefix_kernel(double* __restrict__ maps, const T* __
   if (i >= B * G) return;
   const int g = i % G, b = i / G;
   const long long total = (long long)B * nseg * G;
-  double u = to_f(dmean_out[i]), v = to_f(dvar_out[i]);
+  double u = dmean_out != nullptr ? to_f(dmean_out[i]) : 0.f, v = dvar_out != nullptr ? to_f(dvar_out[i]) : 0.f;
 #pragma unroll 4
   for (int k = nseg - 1; k >= 0; --k) {
     const long long idx = ((long long)b * nseg + k) * G + g;
@@ -524,7 +524,8 @@ tsn_bwd_scan_fused_kernel(StepIn in, const bool* __restrict__ mask, const int* _
     __syncthreads();
   }
   if (!live) return;
-  const double iu = to_f(dmean_out[b * G + g]), iv = to_f(dvar_out[b * G + g]);
+  const double iu = dmean_out != nullptr ? to_f(dmean_out[b * G + g]) : 0.f;
+  const double iv = dvar_out != nullptr ? to_f(dvar_out[b * G + g]) : 0.f;
   if (sgi == 0) {   // every segment applied: the gradient of the carried statistics
     dprev_mean[b * G + g] = from_f<T>((float)(sh[0][slot] * iu + sh[1][slot] * iv + sh[2][slot]));
     dprev_var[b * G + g] = from_f<T>((float)(sh[0][slot] * iv + sh[3][slot]));
@@ -709,7 +710,7 @@ __global__ void tsn_bwd_apply_vec_kernel(const T* __restrict__ dy, const T* __re
                                          const float* __restrict__ ux, const float* __restrict__ dux,
                                          const float* __restrict__ dvx, const W* __restrict__ gamma,
                                          float gamma_offset, const bool* __restrict__ mask, T* __restrict__ dx,
-                                         float* __restrict__ dgamma, float* __restrict__ dbeta, long long rows,
+                                         long long rows,
                                          int H, int G, float* __restrict__ colsum_ws) {
   const int Dg = H / G;
   const int hv = H / 8;
@@ -754,27 +755,14 @@ __global__ void tsn_bwd_apply_vec_kernel(const T* __restrict__ dy, const T* __re
       store8(dx + e, o);
     }
   }
-  if (colsum_ws != nullptr) {   // one row of partial sums per CTA: [dgamma | dbeta]
-    float* mine = colsum_ws + (long long)blockIdx.x * 2 * H;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * kBwdThreads;
-      if (c < hv) {
-        store8(mine + c * 8, acc_g[i]);
-        store8(mine + H + c * 8, acc_b[i]);
-      }
-    }
-    return;
-  }
+  // one row of partial sums per CTA: [dgamma | dbeta]
+  float* mine = colsum_ws + (long long)blockIdx.x * 2 * H;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * kBwdThreads;
     if (c < hv) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        atomicAdd(dgamma + c * 8 + j, acc_g[i][j]);
-        atomicAdd(dbeta + c * 8 + j, acc_b[i][j]);
-      }
+      store8(mine + c * 8, acc_g[i]);
+      store8(mine + H + c * 8, acc_b[i]);
     }
   }
 }
@@ -881,7 +869,7 @@ void timestep_norm_fwd(const void* x, const long long* prev_count, const void* p
 void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_out, const void* x,
                        const void* prev_mean, const long long* count_final, const float* cummean,
                        const float* cumrstd, const void* gamma, float gamma_offset, const bool* mask,
-                       void* dx, void* dprev_mean, void* dprev_var, float* dgamma, float* dbeta,
+                       void* dx, void* dprev_mean, void* dprev_var, void* dgamma, void* dbeta,
                        float* ux, float* ds, float* db, float* dux, float* dvx, double* seg_scratch,
                        int* cumvalid, int B, int L, int H, int G, int x_dtype, int w_dtype, cudaStream_t st,
                        float* colsum_ws) {
@@ -926,20 +914,23 @@ void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_o
       if (hv <= kBwdThreads)
         tsn_bwd_apply_vec_kernel<T, W, 1><<<grid, kBwdThreads, 0, st>>>(
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
-            dgamma, dbeta, rows, H, G, colsum_ws);
+            rows, H, G, colsum_ws);
       else if (hv <= 2 * kBwdThreads)
         tsn_bwd_apply_vec_kernel<T, W, 2><<<grid, kBwdThreads, 0, st>>>(
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
-            dgamma, dbeta, rows, H, G, colsum_ws);
+            rows, H, G, colsum_ws);
       else
         tsn_bwd_apply_vec_kernel<T, W, 4><<<grid, kBwdThreads, 0, st>>>(
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
-            dgamma, dbeta, rows, H, G, colsum_ws);
-      if (colsum_ws != nullptr) colsum_finish(colsum_ws, grid, H, dgamma, dbeta, st);
-    } else
+            rows, H, G, colsum_ws);
+      colsum_finish(colsum_ws, grid, H, dgamma, dbeta, w_dtype, st);
+    } else {
+    cudaMemsetAsync(colsum_ws, 0, sizeof(float) * 2 * H, st);
     tsn_bwd_apply_kernel<T, W><<<grid, kBwdThreads, 0, st>>>((const T*)dy, (const T*)x, cummean, cumrstd, ux, dux,
                                                      dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
-                                                     dgamma, dbeta, rows, H, G);
+                                                     colsum_ws, colsum_ws + H, rows, H, G);
+    colsum_finish(colsum_ws, 1, H, dgamma, dbeta, w_dtype, st);
+    }
   });
 }
 

@@ -219,16 +219,16 @@ class _LinearAdd(torch.autograd.Function):
             else:
                 dw, _ = gemm(g, x2, None, None, a_mn=True, b_mn=True)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = _bias_grad(g).to(ctx.bias_dtype)
+            db = _bias_grad(g, ctx.bias_dtype)
         return dx, dw, db, (dy if ctx.needs_input_grad[3] else None)
 
 
-def _bias_grad(g: Tensor) -> Tensor:
-    """fp32 column sums of the output gradient [rows, features]."""
+def _bias_grad(g: Tensor, dtype: torch.dtype = torch.float32) -> Tensor:
+    """Column sums (in fp32) of the output gradient [rows, features], in the bias's type."""
     if g.is_cuda and g.dtype in (torch.bfloat16, torch.float16) and g.dim() == 2 and g.is_contiguous():
-        _bump()
-        return _C().colsum(g)
-    return g.sum(0, dtype=torch.float32)
+        _bump(2)
+        return _C().colsum(g, _DT[dtype])
+    return g.sum(0, dtype=torch.float32).to(dtype)
 
 
 def linear_add(x: Tensor, w: Tensor, b: Optional[Tensor], addend: Tensor) -> Tensor:
@@ -285,7 +285,7 @@ class _Linear(torch.autograd.Function):
             else:
                 dw, _ = gemm(g, x2, None, None, a_mn=True, b_mn=True)   # [M, N]^T x [M, K] -> [N, K]
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = _bias_grad(g).to(ctx.bias_dtype)
+            db = _bias_grad(g, ctx.bias_dtype)
         return dx, dw, db, None
 
 
@@ -396,13 +396,16 @@ class _TimestepNorm(torch.autograd.Function):
         ctx.offset = offset
         ctx.stat_dtypes = (prev_mean.dtype, prev_var.dtype)
         ctx.mark_non_differentiable(count)
+        ctx.set_materialize_grads(False)
         return y, count, mean, var
 
     @staticmethod
     def backward(ctx, dy, _dcount, dmean, dvar):
         xc, pm, count, cummean, cumrstd, gm, mk = ctx.saved_tensors
-        dmean = torch.zeros_like(pm) if dmean is None else dmean.to(pm.dtype).contiguous()
-        dvar = torch.zeros_like(pm) if dvar is None else dvar.to(pm.dtype).contiguous()
+        if dy is None:                      # only the statistics were used
+            dy = torch.zeros_like(xc)
+        dmean = None if dmean is None else dmean.to(pm.dtype).contiguous()
+        dvar = None if dvar is None else dvar.to(pm.dtype).contiguous()
         _bump(3)
         dx, dpm, dpv, dgamma, dbeta = _C().timestep_norm_bwd(
             dy.contiguous(), dmean, dvar, xc, pm, count, cummean, cumrstd, gm, ctx.offset,
@@ -529,6 +532,7 @@ class _CEMA(torch.autograd.Function):
         ctx.shapes = (p.shape, q.shape, gamma.shape, omega.shape)
         ctx.dtypes = (p.dtype, omega.dtype)
         ctx.S = S
+        ctx.set_materialize_grads(False)
         if h_last is None:
             return y, None
         return y, torch.view_as_complex(h_last)
@@ -536,6 +540,8 @@ class _CEMA(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dh_last):
         xc, p2, q2, g2, om, h2 = ctx.saved_tensors
+        if dy is None:                      # only the last state was used
+            dy = torch.zeros_like(xc)
         dh = None if dh_last is None else _c2r(dh_last)
         _bump(6 if ctx.S > 1 else 2)
         dx, dp, dq, dg, dom, dhx = _C().cema_bwd(dy.contiguous(), xc, p2, q2, g2, om,
