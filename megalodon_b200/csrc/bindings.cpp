@@ -432,12 +432,14 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
                                             const OptTensor& row_out, const OptTensor& aux, int64_t causal_off) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda(), "operands must be CUDA tensors");
   c10::cuda::CUDAGuard guard(A.device());
-  TORCH_CHECK((A.dim() == 2 || A.dim() == 3) && A.dim() == B.dim(), "operands must both be 2-D or both 3-D");
+  TORCH_CHECK(A.dim() >= 2 && A.dim() <= 4 && A.dim() == B.dim(), "operands must both be 2-D, 3-D or 4-D");
   TORCH_CHECK(A.scalar_type() == B.scalar_type());
   TORCH_CHECK(A.scalar_type() == at::kBFloat16 || A.scalar_type() == at::kHalf, "tcgen05 GEMM takes bf16/fp16");
   TORCH_CHECK(A.stride(-1) == 1 && B.stride(-1) == 1, "last dim of the operands must be contiguous");
-  const int batch = A.dim() == 3 ? (int)A.size(0) : 1;
-  TORCH_CHECK(A.dim() == 2 || B.size(0) == batch, "batch sizes differ");
+  const int batch = A.dim() >= 3 ? (int)A.size(-3) : 1;
+  mb::GemmOuterBatch outer;
+  outer.count = A.dim() == 4 ? (int)A.size(0) : 1;
+  TORCH_CHECK((A.dim() == 2 || B.size(-3) == batch) && (A.dim() < 4 || B.size(0) == outer.count), "batch sizes differ");
   // with a gathered A, `A` is this rank's piece [M, K / parts] and only supplies shape, stride and dtype
   const int a_parts = a_part_ptrs.empty() ? 1 : (int)a_part_ptrs.size();
   const int M = a_mn ? A.size(-1) : A.size(-2);
@@ -451,14 +453,18 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
   if (out.has_value()) {
     C = *out;
     TORCH_CHECK(C.is_cuda() && C.scalar_type() == odt && C.dim() == A.dim() && C.stride(-1) == 1);
-    TORCH_CHECK(C.size(-2) == M && C.size(-1) == N && (A.dim() == 2 || C.size(0) == batch), "bad output shape");
+    TORCH_CHECK(C.size(-2) == M && C.size(-1) == N && (A.dim() == 2 || C.size(-3) == batch) &&
+                (A.dim() < 4 || C.size(0) == outer.count), "bad output shape");
     TORCH_CHECK(reinterpret_cast<uintptr_t>(C.data_ptr()) % 16 == 0, "output must be 16-byte aligned");
   } else {
-    C = A.dim() == 3 ? torch::empty({batch, M, N}, A.options().dtype(odt)) : torch::empty({M, N}, A.options().dtype(odt));
+    auto shape = A.sizes().vec();
+    shape[shape.size() - 2] = M;
+    shape[shape.size() - 1] = N;
+    C = torch::empty(shape, A.options().dtype(odt));
   }
   OptTensor pre;
   if (want_preact) {
-    TORCH_CHECK(batch == 1 && !out.has_value(), "pre-activation output is only available for plain 2-D calls");
+    TORCH_CHECK(A.dim() == 2 && !out.has_value(), "pre-activation output is only available for plain 2-D calls");
     pre = torch::empty({M, N}, A.options().dtype(odt));
   }
   int bias_code = 0;
@@ -467,8 +473,11 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
     bias_code = dtype_code(*bias);
     TORCH_CHECK(bias->numel() == N);
   }
-  const long long a_bs = A.dim() == 3 ? A.stride(0) : 0, b_bs = B.dim() == 3 ? B.stride(0) : 0;
-  const long long c_bs = C.dim() == 3 ? C.stride(0) : 0;
+  const long long a_bs = A.dim() >= 3 ? A.stride(-3) : 0, b_bs = B.dim() >= 3 ? B.stride(-3) : 0;
+  const long long c_bs = C.dim() >= 3 ? C.stride(-3) : 0;
+  if (A.dim() == 4) {
+    outer.a_stride = A.stride(0); outer.b_stride = B.stride(0); outer.c_stride = C.stride(0);
+  }
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   mb::GemmPeerSpec peers;
   TORCH_CHECK(a_part_ptrs.size() <= 8 && c_part_ptrs.size() <= 8, "at most 8 peers");
@@ -508,7 +517,7 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
   if (epi_kind != 0) {
     auto rowvec = [&](const OptTensor& t, const char* what) -> float* {
       TORCH_CHECK(t.has_value() && t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() &&
-                  t->numel() == (int64_t)batch * M, what, ": expected a contiguous fp32 [batch, M] CUDA tensor");
+                  t->numel() == (int64_t)outer.count * batch * M, what, ": expected a contiguous fp32 [batch, M] CUDA tensor");
       return t->data_ptr<float>();
     };
     sm.kind = (int)epi_kind;
@@ -531,7 +540,8 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
                                        (int)out_dtype_code, err.data_ptr<int>(), sms, stream(),
                                        (a_parts > 1 || c_part_ptrs.size() > 1) ? &peers : nullptr,
                                        accumulate && out.has_value(), gather.world > 0 ? &gather : nullptr,
-                                       (sm.kind != 0 || with_addend) ? &sm : nullptr);
+                                       (sm.kind != 0 || with_addend) ? &sm : nullptr,
+                                       A.dim() == 4 ? &outer : nullptr);
   // the launcher's status goes back to Python, which raises on a non-zero code
   return {C, pre, (int64_t)rc};
 }

@@ -72,7 +72,9 @@ struct GemmParams {
   float alpha;         // C = alpha * acc (+ bias)
   int accumulate;      // 1: C += alpha * acc (+ bias); the old C is read in the epilogue
   int batch;           // independent problems sharing shapes (tensor maps carry their strides)
-  long long c_batch_stride;   // elements between consecutive C (and preact) matrices
+  int batch_in;        // problem i is (i / batch_in, i % batch_in): two batch strides per operand (sequence, head)
+  long long c_batch_stride;   // elements between consecutive C (and preact) matrices of the inner batch index
+  long long c_outer_stride;   // and of the outer one
   // all-gather -> GEMM: A is the concatenation along K of `a_parts` pieces of `a_part_k` columns, piece i
   // read through tensor map i (a peer GPU's memory); the walk over K starts at piece `a_first`
   int a_parts, a_part_k, a_first;
@@ -104,6 +106,11 @@ struct GemmParams {
   const void* aux;
   int causal_off;
 };
+
+__device__ __forceinline__ long long c_base(const GemmParams& p, int bz) {
+  const int bo = bz / p.batch_in;
+  return bo * p.c_outer_stride + (bz - bo * p.batch_in) * p.c_batch_stride;
+}
 
 struct TmapArray {
   CUtensorMap m[kMaxPeers];
@@ -338,7 +345,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileCoord tc = decode_tile<BN>(tile, num_m, tiles_per_batch);
-        const int m0 = tc.m0, n0 = tc.n0, bz = tc.bz;
+        const int m0 = tc.m0, n0 = tc.n0, bo = tc.bz / p.batch_in, bi = tc.bz - bo * p.batch_in;
         if (tile_skipped<BN>(p, m0, n0)) continue;
         int kb0, kb1;
         k_range(p, m0, num_k, kb0, kb1);
@@ -354,16 +361,16 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
           const int ka = p.a_parts > 1 ? k0 - part * p.a_part_k : k0;     // column inside the piece
           const CUtensorMap* tmap_a = &tmaps_a.m[part];
           if constexpr (!A_MN) {
-            tma_load_3d(sa, tmap_a, full_bar + stage, ka, m0, bz);
+            tma_load_4d(sa, tmap_a, full_bar + stage, ka, m0, bi, bo);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_3d(sa + j * 8192, tmap_a, full_bar + stage, m0 + 64 * j, ka, bz);
+            for (int j = 0; j < BM / 64; ++j) tma_load_4d(sa + j * 8192, tmap_a, full_bar + stage, m0 + 64 * j, ka, bi, bo);
           }
           if constexpr (!B_MN) {
-            tma_load_3d(sb, &tmap_b, full_bar + stage, k0, n0, bz);
+            tma_load_4d(sb, &tmap_b, full_bar + stage, k0, n0, bi, bo);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) tma_load_3d(sb + j * 8192, &tmap_b, full_bar + stage, n0 + 64 * j, k0, bz);
+            for (int j = 0; j < BN / 64; ++j) tma_load_4d(sb + j * 8192, &tmap_b, full_bar + stage, n0 + 64 * j, k0, bi, bo);
           }
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -427,6 +434,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
       const int row = m0 + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       const long long ridx = (long long)tc.bz * p.M + row;
+      const long long cb = c_base(p, tc.bz);
       EpiRow er;
       if (p.epi != kEpiStd) epi_row_begin(p, ridx, row < p.M, er);
 #pragma unroll 1
@@ -442,7 +450,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
         const int nvalid = min(32, p.N - col0);
         if (p.epi != kEpiStd) {
           if (row < p.M)
-            epi_chunk<OutT>(p, v, row, col0, nvalid, (long long)tc.bz * p.c_batch_stride + (long long)row * p.ldc + col0,
+            epi_chunk<OutT>(p, v, row, col0, nvalid, cb + (long long)row * p.ldc + col0,
                             C, er);
           continue;
         }
@@ -465,7 +473,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
             OutT* slot = reinterpret_cast<OutT*>(p.c_parts[owner]);
             store_row32<OutT>(slot + (long long)row * p.c_part_cols + (col0 - owner * p.c_part_cols), v, nvalid);
           } else {
-            const long long off = (long long)tc.bz * p.c_batch_stride + (long long)row * p.ldc + col0;
+            const long long off = cb + (long long)row * p.ldc + col0;
             if (p.accumulate) add_row32<OutT>(C + off, v, nvalid);
             if (p.aux != nullptr) add_row32<OutT>(reinterpret_cast<const OutT*>(p.aux) + off, v, nvalid);   // + addend
             if (P != nullptr) store_row32<OutT>(P + off, v, nvalid);
@@ -837,6 +845,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
         pair_tile_coords(p, tile, num_m, num_n, tiles_per_batch, num_pairs, m0, n0, bz);
         if (pair_tile_skipped(p, m0, n0)) continue;
         const int my_m = m0 + (int)rank * BM;
+        const int bo = bz / p.batch_in, bi = bz - bo * p.batch_in;
         const int my_n = n0 + (int)rank * (kPairBN / 2);
         int kb0, kb1;
         pair_k_range(p, m0, num_k, kb0, kb1);
@@ -856,17 +865,17 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
           const int ka = p.a_parts > 1 ? k0 - part * p.a_part_k : k0;
           const CUtensorMap* tmap_a = &tmaps_a.m[part];
           if constexpr (!A_MN) {
-            tma_load_3d_pair(sa, tmap_a, full0, ka, my_m, bz);
+            tma_load_4d_pair(sa, tmap_a, full0, ka, my_m, bi, bo);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_3d_pair(sa + j * 8192, tmap_a, full0, my_m + 64 * j, ka, bz);
+            for (int j = 0; j < BM / 64; ++j) tma_load_4d_pair(sa + j * 8192, tmap_a, full0, my_m + 64 * j, ka, bi, bo);
           }
           if constexpr (!B_MN) {
-            tma_load_3d_pair(sb, &tmap_b, full0, k0, my_n, bz);
+            tma_load_4d_pair(sb, &tmap_b, full0, k0, my_n, bi, bo);
           } else {
 #pragma unroll
             for (int j = 0; j < kPairBN / 128; ++j)
-              tma_load_3d_pair(sb + j * 8192, &tmap_b, full0, my_n + 64 * j, k0, bz);
+              tma_load_4d_pair(sb + j * 8192, &tmap_b, full0, my_n + 64 * j, k0, bi, bo);
           }
           if (++stage == kPairStages) { stage = 0; phase ^= 1; }
         }
@@ -939,6 +948,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
       const int row = m0 + (int)rank * BM + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + acc * kPairBN + ((uint32_t)(quarter * 32) << 16);
       const long long ridx = (long long)bz * p.M + row;
+      const long long cb = c_base(p, bz);
       EpiRow er;
       if (p.epi != kEpiStd) epi_row_begin(p, ridx, row < p.M, er);
       // chunk c (32 columns) written straight from the registers: partial groups, fp32 outputs, split C
@@ -954,7 +964,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
         const int nvalid = min(32, p.N - col0);
         if (p.epi != kEpiStd) {
           if (row < p.M)
-            epi_chunk<OutT>(p, v, row, col0, nvalid, (long long)bz * p.c_batch_stride + (long long)row * p.ldc + col0,
+            epi_chunk<OutT>(p, v, row, col0, nvalid, cb + (long long)row * p.ldc + col0,
                             C, er);
           return;
         }
@@ -976,7 +986,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
             OutT* slot = reinterpret_cast<OutT*>(p.c_parts[owner]);
             store_row32<OutT>(slot + (long long)row * p.c_part_cols + (col0 - owner * p.c_part_cols), v, nvalid);
           } else {
-            const long long off = (long long)bz * p.c_batch_stride + (long long)row * p.ldc + col0;
+            const long long off = cb + (long long)row * p.ldc + col0;
             if (p.accumulate) add_row32<OutT>(C + off, v, nvalid);
             if (p.aux != nullptr) add_row32<OutT>(reinterpret_cast<const OutT*>(p.aux) + off, v, nvalid);   // + addend
             if (P != nullptr) store_row32<OutT>(P + off, v, nvalid);
@@ -995,7 +1005,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
       // results pass through the warp's staging buffer and leave as whole 128-byte row segments
       const bool can_group = sizeof(OutT) == 2 && P == nullptr && p.c_nparts <= 1 &&
                              !(p.epi == kEpiStd && p.accumulate && p.aux != nullptr) &&
-                             ((p.ldc | p.c_batch_stride) & 7) == 0 &&
+                             ((p.ldc | p.c_batch_stride | p.c_outer_stride) & 7) == 0 &&
                              ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(p.aux)) & 15) == 0 &&
                              n0 + kPairBN <= p.N && !(p.epi == kEpiRowMax && p.alpha < 0.f);
       // (the gathering variant, whose 320 threads leave fewer registers each, keeps the direct form: a
@@ -1006,7 +1016,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
       } else if constexpr (!GATHER) {
         const bool need_in = p.epi == kEpiDS || std_in;
         const OutT* src = (p.epi == kEpiDS || !p.accumulate) ? reinterpret_cast<const OutT*>(p.aux) : C;
-        const long long off_row0 = (long long)bz * p.c_batch_stride + (long long)row_base * p.ldc + n0;
+        const long long off_row0 = cb + (long long)row_base * p.ldc + n0;
         const int last = p.mode == 1 ? row + p.causal_off : 0x7fffffff;
         // does any row of this warp end inside the tile?  (warp-uniform)
         const bool masked = p.mode == 1 && n0 + kPairBN - 1 > row_base + p.causal_off;
@@ -1109,11 +1119,11 @@ EncodeTiledFn get_encode_fn() {
 
 }  // namespace
 
-// 2-D bf16/fp16 tensor map: `inner` contiguous elements per row, `outer` rows, 128-byte swizzle.
-// 3-D bf16/fp16 tensor map [batch, outer, inner] (inner contiguous) with a {1, box_outer, box_inner} box
-// and 128-byte swizzle.  Strides are in elements and must be multiples of 8 (16 bytes).
-bool make_tmap_3d(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
-                  long long row_stride, long long batch_stride, int box_inner, int box_outer, int elem_dtype) {
+// 4-D bf16/fp16 tensor map [outer batch, batch, outer, inner] (inner contiguous) with a {1, 1, box_outer,
+// box_inner} box and 128-byte swizzle.  Strides are in elements and must be multiples of 8 (16 bytes).
+bool make_tmap_4d(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
+                  long long batch2, long long row_stride, long long batch_stride, long long batch2_stride,
+                  int box_inner, int box_outer, int elem_dtype) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return false;
   // The encoder is a driver entry point and needs a current context; a thread that has made no
@@ -1124,19 +1134,23 @@ bool make_tmap_3d(CUtensorMap* out, const void* base, long long inner, long long
     context_bound = true;
   }
   if (batch <= 1) batch_stride = row_stride * outer;      // unused, but must be a valid stride
-  const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)outer, (cuuint64_t)(batch < 1 ? 1 : batch)};
-  const cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)batch_stride * 2};
-  const cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
+  if (batch2 <= 1) batch2_stride = batch_stride;
+  const cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)outer, (cuuint64_t)(batch < 1 ? 1 : batch),
+                              (cuuint64_t)(batch2 < 1 ? 1 : batch2)};
+  const cuuint64_t strides[3] = {(cuuint64_t)row_stride * 2, (cuuint64_t)batch_stride * 2, (cuuint64_t)batch2_stride * 2};
+  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUtensorMapDataType dt = elem_dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const CUresult res = fn(out, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const CUresult res = fn(out, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (res != CUDA_SUCCESS)
     fprintf(stderr,
-            "tensor map encode failed (CUresult %d): base %p dims {%llu, %llu, %llu} strides {%llu, %llu} B box {%u, %u}\n",
+            "tensor map encode failed (CUresult %d): base %p dims {%llu, %llu, %llu, %llu} strides {%llu, %llu, %llu} B "
+            "box {%u, %u}\n",
             (int)res, base, (unsigned long long)dims[0], (unsigned long long)dims[1], (unsigned long long)dims[2],
-            (unsigned long long)strides[0], (unsigned long long)strides[1], box[0], box[1]);
+            (unsigned long long)dims[3], (unsigned long long)strides[0], (unsigned long long)strides[1],
+            (unsigned long long)strides[2], box[0], box[1]);
   return res == CUDA_SUCCESS;
 }
 
@@ -1202,17 +1216,21 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
                       bool b_mn, int mode, float alpha, int batch, long long a_bs, long long b_bs, long long c_bs,
                       int in_dtype, int out_dtype, int* err, int num_sms, cudaStream_t st,
                       const GemmPeerSpec* peers, bool accumulate, const GemmGatherSpec* gather,
-                      const GemmSoftmaxSpec* softmax) {
+                      const GemmSoftmaxSpec* softmax, const GemmOuterBatch* outer) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
   // TMA wants 16-byte strides; the vectorised epilogue wants 16-byte aligned rows of C
   if (lda % 8 != 0 || ldb % 8 != 0 || ldc % 8 != 0) return -1;
   if (batch > 1 && (a_bs % 8 != 0 || b_bs % 8 != 0 || c_bs % 8 != 0)) return -1;
+  const int nb2 = outer != nullptr ? outer->count : 1;
+  const long long a_bs2 = outer != nullptr ? outer->a_stride : 0, b_bs2 = outer != nullptr ? outer->b_stride : 0;
+  if (nb2 < 1 || (nb2 > 1 && (a_bs2 % 8 != 0 || b_bs2 % 8 != 0 || outer->c_stride % 8 != 0))) return -1;
   const int BN = 256;
   TmapArray ta;
   CUtensorMap tb;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.C = C; p.preact = preact; p.bias = bias; p.bias_dtype = bias_dtype; p.act = act;
-  p.err = err; p.ldc = ldc; p.mode = mode; p.alpha = alpha; p.batch = batch; p.c_batch_stride = c_bs;
+  p.err = err; p.ldc = ldc; p.mode = mode; p.alpha = alpha; p.batch = batch * nb2; p.batch_in = batch;
+  p.c_batch_stride = c_bs; p.c_outer_stride = outer != nullptr ? outer->c_stride : 0;
   p.a_parts = 1; p.a_part_k = K; p.a_first = 0; p.c_nparts = 1; p.c_part_cols = N;
   p.accumulate = accumulate ? 1 : 0;
   if (softmax != nullptr && softmax->kind == 0 && softmax->aux != nullptr) {
@@ -1229,19 +1247,19 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
   bool ok = true;
   if (peers != nullptr && peers->a_parts > 1) {
     // gathered A: K-major pieces [M, K / parts] living on different GPUs
-    if (a_mn || batch != 1 || peers->a_parts > kMaxPeers || K % peers->a_parts != 0) return -6;
+    if (a_mn || p.batch != 1 || peers->a_parts > kMaxPeers || K % peers->a_parts != 0) return -6;
     p.a_parts = peers->a_parts;
     p.a_part_k = K / peers->a_parts;
     p.a_first = peers->a_first;
     if (p.a_part_k % BK != 0) return -6;
     for (int i = 0; i < p.a_parts; ++i)
-      ok = ok && make_tmap_3d(&ta.m[i], peers->a_ptrs[i], p.a_part_k, M, 1, lda, 0, BK, BM, in_dtype);
+      ok = ok && make_tmap_4d(&ta.m[i], peers->a_ptrs[i], p.a_part_k, M, 1, 1, lda, 0, 0, BK, BM, in_dtype);
   } else {
-    ok = a_mn ? make_tmap_3d(&ta.m[0], A, M, K, batch, lda, a_bs, 64, 64, in_dtype)
-              : make_tmap_3d(&ta.m[0], A, K, M, batch, lda, a_bs, BK, BM, in_dtype);
+    ok = a_mn ? make_tmap_4d(&ta.m[0], A, M, K, batch, nb2, lda, a_bs, a_bs2, 64, 64, in_dtype)
+              : make_tmap_4d(&ta.m[0], A, K, M, batch, nb2, lda, a_bs, a_bs2, BK, BM, in_dtype);
   }
   if (peers != nullptr && peers->c_nparts > 1) {
-    if (batch != 1 || peers->c_nparts > kMaxPeers || N % peers->c_nparts != 0) return -7;
+    if (p.batch != 1 || peers->c_nparts > kMaxPeers || N % peers->c_nparts != 0) return -7;
     p.c_nparts = peers->c_nparts;
     p.c_part_cols = N / peers->c_nparts;
     if (p.c_part_cols % 32 != 0) return -7;
@@ -1251,14 +1269,14 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
   if (!ok) return -41;
   if (gather != nullptr && gather->world > 0) {
     // B must be the whole K-major weight, contiguous, its row blocks whole 128-row chunks
-    if (!gemm_gather_supported(M, N, K, gather->world) || !pair || a_mn || b_mn || batch != 1 || mode != 0 ||
+    if (!gemm_gather_supported(M, N, K, gather->world) || !pair || a_mn || b_mn || p.batch != 1 || mode != 0 ||
         p.a_parts != 1 || ldb != K || gather->world > kMaxPeers || gather->flags == nullptr || B != gather->dst)
       return -9;
     p.g_world = gather->world; p.g_rank = gather->rank; p.g_dst = gather->dst; p.g_flags = gather->flags;
     for (int i = 0; i < gather->world; ++i) p.g_src[i] = gather->src[i];
   }
-  ok = ok && (b_mn ? make_tmap_3d(&tb, B, N, K, batch, ldb, b_bs, 64, 64, in_dtype)
-                   : make_tmap_3d(&tb, B, K, N, batch, ldb, b_bs, BK, pair ? kPairBN / 2 : BN, in_dtype));
+  ok = ok && (b_mn ? make_tmap_4d(&tb, B, N, K, batch, nb2, ldb, b_bs, b_bs2, 64, 64, in_dtype)
+                   : make_tmap_4d(&tb, B, K, N, batch, nb2, ldb, b_bs, b_bs2, BK, pair ? kPairBN / 2 : BN, in_dtype));
   if (!ok) return -4;
   const int fmt = in_dtype == kBF16 ? 1 : 0;
   if (p.g_world > 0) {

@@ -147,12 +147,19 @@ struct GemmSoftmaxSpec {
 };
 bool gemm_gather_supported(int M, int N, int K, int world);
 int gemm_gather_flag_words(int N);
+// a second batch index: `count` groups of `batch` problems each (attention: sequences of heads); row vectors of the
+// fused softmax are then [count, batch, M]
+struct GemmOuterBatch {
+  int count = 1;
+  long long a_stride = 0, b_stride = 0, c_stride = 0;
+};
 int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const void* bias, int bias_dtype,
                       int act, int M, int N, int K, long long lda, long long ldb, long long ldc, bool a_mn,
                       bool b_mn, int mode, float alpha, int batch, long long a_bs, long long b_bs, long long c_bs,
                       int in_dtype, int out_dtype, int* err, int num_sms, cudaStream_t st,
                       const GemmPeerSpec* peers = nullptr, bool accumulate = false,
-                      const GemmGatherSpec* gather = nullptr, const GemmSoftmaxSpec* softmax = nullptr);
+                      const GemmGatherSpec* gather = nullptr, const GemmSoftmaxSpec* softmax = nullptr,
+                      const GemmOuterBatch* outer = nullptr);
 // ---- FFT long convolution (fftconv_kernels.cu); spectra are [rows, N2/2 + 1] complex, N2 = 1 << fftconv_logn(L)
 int fftconv_logn(int L);
 bool fftconv_supported(int L);          // L <= 16384

@@ -24,8 +24,9 @@
 
 namespace mb {
 
-bool make_tmap_3d(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
-                  long long row_stride, long long batch_stride, int box_inner, int box_outer, int elem_dtype);
+bool make_tmap_4d(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
+                  long long batch2, long long row_stride, long long batch_stride, long long batch2_stride,
+                  int box_inner, int box_outer, int elem_dtype);
 
 namespace {
 
@@ -128,18 +129,18 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
       for (int i = 0; i < first; ++i) {
         uint8_t* st = smem + i * p.stage_bytes;
         mbar_expect_tx(full_bar + i, tx_bytes);
-        tma_load_3d(st, &maps.w[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0);
-        if (dual) tma_load_3d(st + w_bytes, &maps.w2[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0);
+        tma_load_4d(st, &maps.w[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0, 0);
+        if (dual) tma_load_4d(st + w_bytes, &maps.w2[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0, 0);
       }
       if (p.chained) {
         for (int i = first; i < total; ++i) {
-          tma_prefetch_3d(&maps.w[ji], (kb0 + i) * kSkBK, n0, 0);
-          if (dual) tma_prefetch_3d(&maps.w2[ji], (kb0 + i) * kSkBK, n0, 0);
+          tma_prefetch_4d(&maps.w[ji], (kb0 + i) * kSkBK, n0, 0, 0);
+          if (dual) tma_prefetch_4d(&maps.w2[ji], (kb0 + i) * kSkBK, n0, 0, 0);
         }
       }
       pdl_wait();
       for (int i = 0; i < first; ++i)
-        tma_load_3d(smem + i * p.stage_bytes + x_off, &maps.x[ji], full_bar + i, (kb0 + i) * kSkBK, 0, 0);
+        tma_load_4d(smem + i * p.stage_bytes + x_off, &maps.x[ji], full_bar + i, (kb0 + i) * kSkBK, 0, 0, 0);
       bool ok = true;
       int stage = 0, issued = first;
       uint32_t phase = 0;
@@ -148,9 +149,9 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
         uint8_t* st = smem + stage * p.stage_bytes;
         const int k = (kb0 + i) * kSkBK;
         mbar_expect_tx(full_bar + stage, tx_bytes);
-        tma_load_3d(st, &maps.w[ji], full_bar + stage, k, n0, 0);
-        if (dual) tma_load_3d(st + w_bytes, &maps.w2[ji], full_bar + stage, k, n0, 0);
-        tma_load_3d(st + x_off, &maps.x[ji], full_bar + stage, k, 0, 0);
+        tma_load_4d(st, &maps.w[ji], full_bar + stage, k, n0, 0, 0);
+        if (dual) tma_load_4d(st + w_bytes, &maps.w2[ji], full_bar + stage, k, n0, 0, 0);
+        tma_load_4d(st + x_off, &maps.x[ji], full_bar + stage, k, 0, 0, 0);
         ++issued;
         if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
@@ -316,12 +317,12 @@ int skinny_gemm(const SkinnyJob* jobs, int njobs, int M, int in_dtype, bool pdl,
     p.tile0[i] = tiles;
     tiles += div_up(j.N, kSkRows);
     min_nk = min_nk < div_up(j.K, kSkBK) ? min_nk : div_up(j.K, kSkBK);
-    if (!make_tmap_3d(&maps.w[i], j.w, j.K, j.N, 1, j.ldw, 0, kSkBK, kSkRows, in_dtype)) return -4;
+    if (!make_tmap_4d(&maps.w[i], j.w, j.K, j.N, 1, 1, j.ldw, 0, 0, kSkBK, kSkRows, in_dtype)) return -4;
     if (j.act == kSkinnySwiGLU) {
       dual = true;
-      if (!aligned16(j.w2) || !make_tmap_3d(&maps.w2[i], j.w2, j.K, j.N, 1, j.ldw, 0, kSkBK, kSkRows, in_dtype)) return -4;
+      if (!aligned16(j.w2) || !make_tmap_4d(&maps.w2[i], j.w2, j.K, j.N, 1, 1, j.ldw, 0, 0, kSkBK, kSkRows, in_dtype)) return -4;
     }
-    if (!make_tmap_3d(&maps.x[i], j.x, j.K, M, 1, j.ldx, 0, kSkBK, p.mpad, in_dtype)) return -4;
+    if (!make_tmap_4d(&maps.x[i], j.x, j.K, M, 1, 1, j.ldx, 0, 0, kSkBK, p.mpad, in_dtype)) return -4;
   }
   p.stage_bytes = (dual ? 2 : 1) * kSkRows * kSkBK * 2 + p.mpad * kSkBK * 2;
   // K is split until the tiles cover every SM; at least two k-blocks are left to each CTA

@@ -212,12 +212,7 @@ class Mega(nn.Module):
             x = x * self.emb_scale
         x = ops.memory_efficient_dropout(x, self.dropout, self.training)
 
-        if self.efficient_attn:
-            mask = None
-        else:
-            m = min(seq_len, c)
-            mask = torch.full((1, 1, m, m + cache_len), float("-inf"), device=tokens.device)
-            mask = torch.triu(mask, diagonal=cache_len + 1).to(x.dtype)
+        mask = self._causal_mask(x, min(seq_len, c), cache_len)
         freqs_cis = self.rope.get_freqs_cis(cache_len, min(cache_len + seq_len, c))
 
         piece_len = None
@@ -276,9 +271,7 @@ class Mega(nn.Module):
         k = getattr(self, "seq_microbatch_chunks", None) or (seq_len // c)
         piece_len = min(seq_len, k * c)
         n = seq_len // piece_len
-        mask = None
-        if not self.efficient_attn:
-            mask = torch.triu(torch.full((1, 1, c, c), float("-inf"), device=tokens.device), diagonal=1).to(x.dtype)
+        mask = self._causal_mask(x, c, 0)
         freqs_cis = self.rope.get_freqs_cis(0, c)
         pieces = list(torch.split(x, piece_len, dim=1))
         layer_states = []
@@ -309,6 +302,12 @@ class Mega(nn.Module):
                   torch.empty((bsz, 0, self.local_heads, self.local_v_head_dim), dtype=dt, device=x.device), 0)
             cache_layers.append((kv, (count, mean, var), hx))
         return logits, (cache_layers, tuple(out_state))
+
+    def _causal_mask(self, x: Tensor, rows: int, past: int):
+        first = self.layers[0]
+        while hasattr(first, "_wrapped"):
+            first = first._wrapped
+        return first.mega.inner_attention.causal_mask(x, rows, past)
 
     def _piece_loss(self, xn: Tensor, targets: Tensor) -> Tensor:
         logits = self.output.output(xn)

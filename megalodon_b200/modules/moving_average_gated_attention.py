@@ -48,6 +48,16 @@ _c2r = torch.view_as_real
 _r2c = torch.view_as_complex
 
 
+class _CausalMask:
+    """Stands for the additive causal mask where it does not have to be materialised."""
+
+    def __repr__(self):
+        return "CAUSAL"
+
+
+CAUSAL = _CausalMask()
+
+
 class _InnerAttention(nn.Module):
     """Causal attention restricted to fixed-size chunks.  Sequences longer than
     a chunk are folded to [(B * n_chunks), chunk, H, d]; the KV cache only ever
@@ -96,7 +106,7 @@ class _InnerAttention(nn.Module):
         if slen > c and freqs_cis is not None:
             xq, xk = apply_rotary_emb(xq, xk, freqs_cis, backward=False)
 
-        if self.efficient_attn is None:
+        if self.efficient_attn is None and mask is not CAUSAL:
             # unfused path: post-softmax dropout, explicit additive mask
             assert mask is not None
             q, k, v = xq.transpose(1, 2), xk.transpose(1, 2), xv.transpose(1, 2)
@@ -105,8 +115,9 @@ class _InnerAttention(nn.Module):
             scores = ops.memory_efficient_dropout(scores, self.dropout, self.training)
             out = torch.matmul(scores, v).transpose(1, 2).contiguous()
         else:
+            # (without an explicit mask the unfused model has no dropout: the products are the same ones)
             causal = not (slen == 1 and cache is not None)
-            out = ops.attention(xq, xk, xv, 1.0, self.dropout, causal, self.training)
+            out = ops.attention(xq, xk, xv, 1.0, self.dropout if self.efficient_attn else 0.0, causal, self.training)
         return out.reshape(bs, slen, -1), new_cache
 
     def _static_step(self, xq: Tensor, xk: Tensor, xv: Tensor, cache):
@@ -130,6 +141,19 @@ class _InnerAttention(nn.Module):
         probs = torch.softmax(scores.masked_fill(hidden, float("-inf")), dim=-1).to(xq.dtype)
         out = torch.matmul(probs, v_buf)                                                 # [B, H, 1, dv]
         return out.transpose(1, 2).reshape(bs, 1, -1), cache
+
+    def causal_mask(self, x: Tensor, rows: int, past: int):
+        """Mask argument for `rows` queries after `past` cached keys on activations like x [.., D]: None for the
+        fused implementations; otherwise the additive mask, or `CAUSAL` where no dropout acts on the
+        probabilities and the attention kernels take the shapes - softmax(q k^T + mask) v is what they compute,
+        with the scores kept in fp32."""
+        if self.efficient_attn:
+            return None
+        if not (self.training and self.dropout > 0.0) and ops.attention_native(x, self.z_head_dim, self.v_head_dim,
+                                                                               rows + past):
+            return CAUSAL
+        mask = torch.full((1, 1, rows, rows + past), float("-inf"), device=x.device)
+        return torch.triu(mask, diagonal=past + 1).to(x.dtype)
 
     def extra_repr(self) -> str:
         return (f"heads={self.n_heads}, z_head_dim={self.z_head_dim}, "

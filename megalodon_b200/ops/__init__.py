@@ -211,6 +211,11 @@ def attention(q, k, v, scale: float = 1.0, dropout: float = 0.0, use_causal_mask
     return reference.attention(q, k, v, scale, dropout, use_causal_mask, training)
 
 
+def attention_native(x: Tensor, dk: int, dv: int, keys: int) -> bool:
+    """Whether `attention` runs on the kernels for activations like x, head widths dk / dv and that many keys."""
+    return native_for(x) and _cuda().attention_shapes_ok(x.dtype, dk, dv, keys)
+
+
 swift_efficient_attention = attention
 
 

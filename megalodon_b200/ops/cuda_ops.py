@@ -79,8 +79,13 @@ def check_kernel_errors(device: Optional[torch.device] = None) -> None:
 
 
 def _tma_ok(t: Tensor) -> bool:
-    return (t.stride(-1) == 1 and t.stride(-2) % 8 == 0 and t.data_ptr() % 16 == 0
-            and (t.dim() == 2 or t.stride(0) % 8 == 0))
+    *outer, last = t.stride()
+    if last != 1 or t.data_ptr() & 15:
+        return False
+    for s in outer:
+        if s & 7:
+            return False
+    return True
 
 
 def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str] = None, *,
@@ -94,13 +99,14 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
     while it computes (FSDP all-gather fused into the consuming GEMM).  `softmax = dict(epi_kind=..,
     row_in=.., row_in2=.., row_out=.., aux=.., causal_off=..)`: one of the fused-softmax epilogues of the
     attention products (csrc/kernels.h, GemmSoftmaxSpec); native path only.
-    Operands may be 2-D or 3-D (batched) strided views with a contiguous last
+    Operands may be 2-D, 3-D or 4-D (one or two batch dims) strided views with a contiguous last
     dim.  `mode` 1..3 exploits causal structure (see gemm_sm100.cu).  Returns
     (C, preact | None)."""
     out_dtype = out_dtype or (out.dtype if out is not None else a.dtype)
     native = (_GEMM_BACKEND[0] == "tcgen05" and a.dtype in (torch.bfloat16, torch.float16)
-              and _tma_ok(a) and _tma_ok(b) and (out is None or _tma_ok(out))
-              and (b.shape[-1] if b_mn else b.shape[-2]) % 8 == 0)
+              and _tma_ok(a) and _tma_ok(b)
+              # the epilogue stores 16-byte pieces of rows that start on a 16-byte boundary
+              and (_tma_ok(out) if out is not None else (b.shape[-1] if b_mn else b.shape[-2]) % 8 == 0))
     if a_part_ptrs or c_part_ptrs or b_gather:
         if not native:
             raise RuntimeError("peer-memory GEMM needs the tcgen05 backend and TMA-compatible operands")
@@ -665,17 +671,24 @@ def rfft(x, flip=False):
 # Chunk-local attention as five tensor-core products around an in-place softmax:
 #   S = scale Q K^T -> P = softmax_causal(S) -> O = P V
 #   dV = P^T dO,  dP = dO V^T,  dS = P (dP - rowsum(P dP)),  dQ = scale dS K,  dK = scale dS^T Q
-# All products run on the tcgen05 GEMM, batched over heads through strided 3-D
-# views of the [B, L, H, d] tensors (no per-head copies) and, for square causal
-# blocks, restricted to the tiles on or below the diagonal.
-def _heads_view(t: Tensor, b: int) -> Tensor:
-    """[B, L, H, d] -> view [H, L, d] of batch element b (strides d, H*d, 1)."""
-    return t[b].permute(1, 0, 2)
+# All products run on the tcgen05 GEMM, one launch for all sequences and heads
+# through strided 4-D views of the [B, L, H, d] tensors (no per-head copies; a
+# launch per sequence left the causal tiles of a 2048-token chunk to a part of
+# the CTA pairs) and, for square causal blocks, restricted to the tiles on or
+# below the diagonal.
+def _heads_view(t: Tensor, b: Optional[int] = None) -> Tensor:
+    """[B, L, H, d] -> view [B, H, L, d] (both batch indices of a product over all sequences and heads), or
+    [H, L, d] of sequence `b`."""
+    return t.permute(0, 2, 1, 3) if b is None else t[b].permute(1, 0, 2)
+
+
+def attention_shapes_ok(dtype: torch.dtype, dk: int, dv: int, keys: int) -> bool:
+    return (dtype in (torch.bfloat16, torch.float16) and dk % 8 == 0 and dv % 8 == 0 and keys <= 8192
+            and _GEMM_BACKEND[0] == "tcgen05")
 
 
 def _attention_native_ok(q, k, v) -> bool:
-    return (q.dtype in (torch.bfloat16, torch.float16) and q.shape[-1] % 8 == 0 and v.shape[-1] % 8 == 0
-            and k.shape[1] <= 8192 and _GEMM_BACKEND[0] == "tcgen05")
+    return attention_shapes_ok(q.dtype, q.shape[-1], v.shape[-1], k.shape[1])
 
 
 class _Attention(torch.autograd.Function):
@@ -695,22 +708,18 @@ class _Attention(torch.autograd.Function):
         B, L1, H, dk = q.shape
         L2, dv = k.shape[1], v.shape[-1]
         square = causal and L1 == L2
-        # (key counts that are not a multiple of 8 leave the tensor-core path, see `gemm`)
-        fused = drop_p == 0.0 and (square or not causal) and _FUSED_SOFTMAX[0] and L2 % 8 == 0
+        fused = drop_p == 0.0 and (square or not causal) and _FUSED_SOFTMAX[0]
         ld = -(-L2 // 128) * 128                     # padded row length of the score buffer
         P = torch.empty(B, H, L1, ld, dtype=q.dtype, device=q.device)
         out = torch.empty(B, L1, H, dv, dtype=q.dtype, device=q.device)
         mode_s, mode_o = (1, 2) if square else (0, 0)
+        Pv, qh, kh, vh, oh = P[..., :L2], _heads_view(q), _heads_view(k), _heads_view(v), _heads_view(out)
         if fused:
             rmax = torch.full((B, H, L1), float("-inf"), dtype=torch.float32, device=q.device)
             rsum = torch.zeros((B, H, L1), dtype=torch.float32, device=q.device)
-            for b in range(B):
-                Pb, qb, kb = P[b][:, :, :L2], _heads_view(q, b), _heads_view(k, b)
-                gemm(qb, kb, out=Pb, mode=mode_s, alpha=scale, softmax=dict(epi_kind=1, row_out=rmax[b]))
-                gemm(qb, kb, out=Pb, mode=mode_s, alpha=scale,
-                     softmax=dict(epi_kind=2, row_in=rmax[b], row_out=rsum[b]))
-                gemm(Pb, _heads_view(v, b), b_mn=True, out=_heads_view(out, b), mode=mode_o,
-                     softmax=dict(epi_kind=3, row_in=rsum[b]))
+            gemm(qh, kh, out=Pv, mode=mode_s, alpha=scale, softmax=dict(epi_kind=1, row_out=rmax))
+            gemm(qh, kh, out=Pv, mode=mode_s, alpha=scale, softmax=dict(epi_kind=2, row_in=rmax, row_out=rsum))
+            gemm(Pv, vh, b_mn=True, out=oh, mode=mode_o, softmax=dict(epi_kind=3, row_in=rsum))
             if _RECOMPUTE_SCORES[0]:
                 # keep the row maxima (16 KB per head) instead of the 32 MB of P~ per head: backward runs
                 # the second score pass again
@@ -723,12 +732,11 @@ class _Attention(torch.autograd.Function):
             seed = offset = 0
             if drop_p > 0.0:
                 seed = int(torch.randint(0, 2 ** 62, (1,)).item())
-            for b in range(B):
-                Pb = P[b][:, :, :L2]
-                gemm(_heads_view(q, b), _heads_view(k, b), out=Pb, mode=mode_s, alpha=scale)
+            gemm(qh, kh, out=Pv, mode=mode_s, alpha=scale)
+            for i, part in enumerate([Pv] if drop_p == 0.0 else Pv.unbind(0)):    # (a sequence, a Philox offset)
                 _bump()
-                _C().attn_softmax_fwd(Pb, L1, L2, causal, drop_p, seed, offset + b)
-                gemm(Pb, _heads_view(v, b), b_mn=True, out=_heads_view(out, b), mode=mode_o)
+                _C().attn_softmax_fwd(part, L1, L2, causal, drop_p, seed, offset + i)
+            gemm(Pv, vh, b_mn=True, out=oh, mode=mode_o)
             ctx.save_for_backward(q, k, v, P)
         ctx.meta = (scale, causal, square, L2, fused)
         return out
@@ -742,43 +750,35 @@ class _Attention(torch.autograd.Function):
                 rmax, (Bq, Lq, Hq, _) = P, q.shape
                 ld = -(-L2 // 128) * 128
                 P = torch.empty(Bq, Hq, Lq, ld, dtype=q.dtype, device=q.device)
-                scratch = torch.empty_like(rsum)
-                for b in range(Bq):
-                    gemm(_heads_view(q, b), _heads_view(k, b), out=P[b][:, :, :L2], mode=1 if square else 0,
-                         alpha=scale, softmax=dict(epi_kind=2, row_in=rmax[b], row_out=scratch[b]))
+                gemm(_heads_view(q), _heads_view(k), out=P[..., :L2], mode=1 if square else 0, alpha=scale,
+                     softmax=dict(epi_kind=2, row_in=rmax, row_out=torch.empty_like(rsum)))
         else:
             q, k, v, P = ctx.saved_tensors
         dout = dout.contiguous()
         B, L1, H, dk = q.shape
         dq, dk_, dv_ = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         m1, m2, m3 = (1, 2, 3) if square else (0, 0, 0)
+        Pv, doh, vh = P[..., :L2], _heads_view(dout), _heads_view(v)
         if fused:
             # delta_i = dO_i . O_i (what sum_j P_ij dP_ij equals) and dO' = dO / rowsum, in one pass
             _bump()
             dos, delta = _C().attn_bwd_prep(dout, out, rsum)                                      # delta [B, H, L1]
+            # dV = P~^T (dO / l); dS = P~ / l * (dO V^T - delta) written over P~; dQ, dK from dS
+            gemm(Pv, _heads_view(dos), a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)
+            gemm(doh, vh, out=Pv, mode=m1, softmax=dict(epi_kind=4, row_in=rsum, row_in2=delta, aux=Pv))
+            dS = Pv
         else:
-            dP = torch.empty_like(P[0])
-        for b in range(B):
-            Pb = P[b][:, :, :L2]
-            if fused:
-                # dV = P~^T (dO / l); dS = P~ / l * (dO V^T - delta) written over P~; dQ, dK from dS
-                gemm(Pb, _heads_view(dos, b), a_mn=True, b_mn=True, out=_heads_view(dv_, b), mode=m3)
-                gemm(_heads_view(dout, b), _heads_view(v, b), out=Pb, mode=m1,
-                     softmax=dict(epi_kind=4, row_in=rsum[b], row_in2=delta[b], aux=Pb))
-                dSb = Pb
-            else:
-                dPb = dP[:, :, :L2]
-                dOb = _heads_view(dout, b)
-                # dV = P^T dO   (A = P stored [q, key] = [K, M]; B = dO stored [q, dv] = [K, N])
-                gemm(Pb, dOb, a_mn=True, b_mn=True, out=_heads_view(dv_, b), mode=m3)
-                # dP = dO V^T
-                gemm(dOb, _heads_view(v, b), out=dPb, mode=m1)
-                _bump()
-                _C().attn_softmax_bwd(Pb, dPb, L1, L2, causal)      # dP <- dS in place
-                dSb = dPb
-            # dQ = scale dS K ; dK = scale dS^T Q
-            gemm(dSb, _heads_view(k, b), b_mn=True, out=_heads_view(dq, b), mode=m2, alpha=scale)
-            gemm(dSb, _heads_view(q, b), a_mn=True, b_mn=True, out=_heads_view(dk_, b), mode=m3, alpha=scale)
+            dP = torch.empty_like(P)
+            dS = dP[..., :L2]
+            # dV = P^T dO   (A = P stored [q, key] = [K, M]; B = dO stored [q, dv] = [K, N])
+            gemm(Pv, doh, a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)
+            # dP = dO V^T
+            gemm(doh, vh, out=dS, mode=m1)
+            _bump()
+            _C().attn_softmax_bwd(Pv, dS, L1, L2, causal)      # dP <- dS in place
+        # dQ = scale dS K ; dK = scale dS^T Q
+        gemm(dS, _heads_view(k), b_mn=True, out=_heads_view(dq), mode=m2, alpha=scale)
+        gemm(dS, _heads_view(q), a_mn=True, b_mn=True, out=_heads_view(dk_), mode=m3, alpha=scale)
         return dq, dk_, dv_, None, None, None
 
 

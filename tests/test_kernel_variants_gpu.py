@@ -63,3 +63,48 @@ def test_gradient_norm_and_scale(n):
     want = (g.float() * 0.3).bfloat16()
     cuda_ops.scale_by_ptr(g, torch.tensor([0.3], device="cuda"))
     assert torch.equal(g, want)
+
+
+# lengths around the 8-column pieces, the 128-row tile (one CTA / CTA pair) and the 256-column tile; several
+# sequences and heads in one launch
+@pytest.mark.parametrize("B,L,H,dk,dv", [(1, 5, 2, 16, 24), (3, 37, 1, 64, 64), (2, 128, 2, 32, 40), (2, 129, 3, 64, 72),
+                                         (2, 257, 2, 128, 256), (3, 777, 1, 64, 128)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_any_length(B, L, H, dk, dv, causal):
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(L)
+    q, k, v = _rand(B, L, H, dk, scale=dk ** -0.25), _rand(B, L, H, dk, scale=dk ** -0.25), _rand(B, L, H, dv)
+    g = _rand(B, L, H, dv)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    out = ops.attention(*leaves, 0.7, 0.0, causal, True)
+    out.backward(g)
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    s = torch.einsum("blhd,bmhd->bhlm", ref[0], ref[1]) * 0.7
+    if causal:
+        s = s.masked_fill(torch.ones(L, L, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.einsum("bhlm,bmhd->blhd", torch.softmax(s, -1), ref[2])
+    want.backward(g.double())
+    # probabilities, scores' gradients and results are rounded to 8 bits once each
+    assert _rel(out, want) < 2.0 ** -7
+    for a, b in zip(leaves, ref):
+        assert _rel(a.grad, b.grad) < 2.0 ** -6
+    cuda_ops.check_kernel_errors()
+
+
+@pytest.mark.parametrize("slen,past", [(37, 0), (96, 0), (33, 20), (192, 0)])
+def test_causal_marker_equals_the_explicit_mask(slen, past):
+    """The unfused model without dropout: `CAUSAL` against the additive mask it stands for."""
+    from megalodon_b200.modules.moving_average_gated_attention import CAUSAL, _InnerAttention
+    torch.manual_seed(slen)
+    H, dk, dv, c, B = 2, 32, 64, 96, 2
+    inner = _InnerAttention(dk, dv, H, c, 0.1, None).eval()
+    q, k, v = _rand(B, slen, H * dk, scale=0.5), _rand(B, slen, H * dk, scale=0.5), _rand(B, slen, H * dv)
+    kv = (_rand(B, past, H, dk, scale=0.5), _rand(B, past, H, dv), past)
+    rows = min(slen, c)
+    assert inner.causal_mask(q, rows, past) is CAUSAL
+    mask = torch.full((1, 1, rows, rows + past), float("-inf"), device="cuda").triu(past + 1).bfloat16()
+    got, kv1 = inner(q, k, v, CAUSAL, None, kv)
+    want, kv2 = inner(q, k, v, mask, None, kv)
+    assert _rel(got, want) < 2.0 ** -6 and torch.equal(kv1[0], kv2[0]) and kv1[2] == kv2[2]
+    assert torch.is_tensor(inner.train().causal_mask(q, rows, past))       # dropout acts on the probabilities
