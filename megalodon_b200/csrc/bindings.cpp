@@ -266,6 +266,44 @@ std::vector<Tensor> cema_bwd(const Tensor& dy, const Tensor& x, const Tensor& p,
   return {dx, dp, dq, dgamma, domega, dhx};
 }
 
+// alpha, delta [D, N, 1], theta [D, 1, 1], gamma [D, N, 2] of one type -> p [D, N, 1], q, gamma [D, N, 2] (fp32)
+std::tuple<Tensor, Tensor, Tensor> cema_coeffs_fwd(const Tensor& alpha, const Tensor& delta, const Tensor& theta,
+                                                   const Tensor& gamma, double scale) {
+  for (const Tensor* t : {&alpha, &delta, &theta, &gamma}) {
+    check_cuda_contig(*t, "cema parameter");
+    TORCH_CHECK(t->scalar_type() == alpha.scalar_type(), "cema parameters must share a type");
+  }
+  const int64_t D = alpha.size(0), N = alpha.size(1);
+  TORCH_CHECK(N >= 1 && N <= 32 && alpha.numel() == D * N && delta.numel() == D * N && theta.numel() == D &&
+              gamma.numel() == 2 * D * N);
+  c10::cuda::CUDAGuard guard(alpha.device());
+  auto f32 = alpha.options().dtype(at::kFloat);
+  Tensor p = torch::empty({D, N, 1}, f32), q = torch::empty({D, N, 2}, f32), g = torch::empty({D, N, 2}, f32);
+  mb::cema_coeffs_fwd(alpha.data_ptr(), delta.data_ptr(), theta.data_ptr(), gamma.data_ptr(), (float)scale,
+                      p.data_ptr<float>(), q.data_ptr<float>(), g.data_ptr<float>(), (int)D, (int)N, dtype_code(alpha),
+                      stream());
+  return {p, q, g};
+}
+
+// gradients of p, q, gamma (fp32, any may be absent) -> those of the four parameters, in their type
+std::vector<Tensor> cema_coeffs_bwd(const OptTensor& dp, const OptTensor& dq, const OptTensor& dg, const Tensor& alpha,
+                                    const Tensor& delta, const Tensor& theta, double scale) {
+  const int64_t D = alpha.size(0), N = alpha.size(1);
+  auto grad = [&](const OptTensor& t, int64_t n) -> const float* {
+    if (!t.has_value()) return nullptr;
+    check_cuda_contig(*t, "cema coefficient gradient");
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->numel() == n);
+    return t->data_ptr<float>();
+  };
+  c10::cuda::CUDAGuard guard(alpha.device());
+  Tensor da = torch::empty_like(alpha), dd = torch::empty_like(delta), dt = torch::empty_like(theta);
+  Tensor dgo = torch::empty({D, N, 2}, alpha.options());
+  mb::cema_coeffs_bwd(grad(dp, D * N), grad(dq, 2 * D * N), grad(dg, 2 * D * N), alpha.data_ptr(), delta.data_ptr(),
+                      theta.data_ptr(), (float)scale, da.data_ptr(), dd.data_ptr(), dt.data_ptr(), dgo.data_ptr(), (int)D,
+                      (int)N, dtype_code(alpha), stream());
+  return {da, dd, dt, dgo};
+}
+
 // ------------------------------------------------------------------ element-wise
 Tensor swiglu_fwd(const Tensor& a, const Tensor& b) {
   check_cuda_contig(a, "a");
@@ -1126,6 +1164,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("layer_norm_bwd", checked(&layer_norm_bwd));
   m.def("timestep_norm_fwd", checked(&timestep_norm_fwd));
   m.def("timestep_norm_bwd", checked(&timestep_norm_bwd));
+  m.def("cema_coeffs_fwd", checked(&cema_coeffs_fwd));
+  m.def("cema_coeffs_bwd", checked(&cema_coeffs_bwd));
   m.def("cema_fwd", checked(&cema_fwd));
   m.def("cema_bwd", checked(&cema_bwd));
   m.def("swiglu_fwd", checked(&swiglu_fwd));

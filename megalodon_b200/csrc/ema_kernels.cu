@@ -138,4 +138,81 @@ void ema_parameters_bwd(const float* dk, const float* dbias, const float* p, con
                                            dp, (cfloat*)dq, (cfloat*)dgamma, (cfloat*)dh, B, D, N, L);
 }
 
+// ---- coefficients of the recurrence from the layer's parameters; a thread owns state n of feature d.
+//   p = s(alpha), r = 1 - s(alpha) s(delta), phi = n s(theta) 2 pi / N, q = r e^(i phi), gamma_out = scale gamma
+namespace {
+__device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
+
+template <typename T>
+__global__ void cema_coeffs_fwd_kernel(const T* __restrict__ alpha, const T* __restrict__ delta,
+                                       const T* __restrict__ theta, const T* __restrict__ gamma, float scale,
+                                       float* __restrict__ p, float2* __restrict__ q, float2* __restrict__ g, int D, int N) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= D * N) return;
+  const int d = i / N, n = i - d * N + 1;
+  const float sa = sigmoid_f(to_f(alpha[i])), sd = sigmoid_f(to_f(delta[i]));
+  const float phi = (float)n * (sigmoid_f(to_f(theta[d])) * (6.283185307179586f / N));
+  float s, c;
+  sincosf(phi, &s, &c);
+  const float r = 1.f - sa * sd;
+  p[i] = sa;
+  q[i] = make_float2(r * c, r * s);
+  g[i] = make_float2(to_f(gamma[2 * i]) * scale, to_f(gamma[2 * i + 1]) * scale);
+}
+
+// the N <= 32 states of a feature are added up for d theta by the feature's first thread through shared memory
+template <typename T>
+__global__ void cema_coeffs_bwd_kernel(const float* __restrict__ dp, const float2* __restrict__ dq,
+                                       const float2* __restrict__ dg, const T* __restrict__ alpha,
+                                       const T* __restrict__ delta, const T* __restrict__ theta, float scale,
+                                       T* __restrict__ dalpha, T* __restrict__ ddelta, T* __restrict__ dtheta,
+                                       T* __restrict__ dgamma, int D, int N) {
+  __shared__ float dphi[256];
+  const int per = blockDim.x / N;                    // features of a block
+  const int fl = threadIdx.x / N, n = threadIdx.x - fl * N;
+  const int d = blockIdx.x * per + fl;
+  const bool on = fl < per && d < D;
+  const float w = 6.283185307179586f / N;
+  float st = 0.f;
+  if (on) {
+    const int i = d * N + n;
+    const float sa = sigmoid_f(to_f(alpha[i])), sd = sigmoid_f(to_f(delta[i]));
+    st = sigmoid_f(to_f(theta[d]));
+    float s, c;
+    sincosf((float)(n + 1) * (st * w), &s, &c);
+    const float r = 1.f - sa * sd;
+    const float2 gq = dq != nullptr ? dq[i] : make_float2(0.f, 0.f);
+    const float dr = gq.x * c + gq.y * s;
+    dphi[threadIdx.x] = r * (gq.y * c - gq.x * s) * (float)(n + 1);
+    dalpha[i] = from_f<T>(((dp != nullptr ? dp[i] : 0.f) - sd * dr) * sa * (1.f - sa));
+    ddelta[i] = from_f<T>(-sa * dr * sd * (1.f - sd));
+    const float2 gg = dg != nullptr ? dg[i] : make_float2(0.f, 0.f);
+    dgamma[2 * i] = from_f<T>(gg.x * scale);
+    dgamma[2 * i + 1] = from_f<T>(gg.y * scale);
+  }
+  __syncthreads();
+  if (on && n == 0) {
+    float t = 0.f;
+    for (int k = 0; k < N; ++k) t += dphi[threadIdx.x + k];
+    dtheta[d] = from_f<T>(t * w * st * (1.f - st));
+  }
+}
+}  // namespace
+
+void cema_coeffs_fwd(const void* alpha, const void* delta, const void* theta, const void* gamma, float scale, float* p,
+                     float* q, float* g, int D, int N, int dtype, cudaStream_t st) {
+  MB_DISPATCH_DTYPE(dtype, (cema_coeffs_fwd_kernel<scalar_t><<<div_up((long long)D * N, 256), 256, 0, st>>>(
+                               (const scalar_t*)alpha, (const scalar_t*)delta, (const scalar_t*)theta,
+                               (const scalar_t*)gamma, scale, p, (float2*)q, (float2*)g, D, N)));
+}
+
+void cema_coeffs_bwd(const float* dp, const float* dq, const float* dg, const void* alpha, const void* delta,
+                     const void* theta, float scale, void* dalpha, void* ddelta, void* dtheta, void* dgamma, int D, int N,
+                     int dtype, cudaStream_t st) {
+  MB_DISPATCH_DTYPE(dtype, (cema_coeffs_bwd_kernel<scalar_t><<<div_up(D, 256 / N), 256, 0, st>>>(
+                               dp, (const float2*)dq, (const float2*)dg, (const scalar_t*)alpha, (const scalar_t*)delta,
+                               (const scalar_t*)theta, scale, (scalar_t*)dalpha, (scalar_t*)ddelta, (scalar_t*)dtheta,
+                               (scalar_t*)dgamma, D, N)));
+}
+
 }  // namespace mb

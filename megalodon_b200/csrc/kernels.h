@@ -56,6 +56,14 @@ void cema_bwd(const void* dy, const void* x, const float* p, const float* q, con
               float* dgamma, float* domega, float* dhx, float* carry_a, float* carry_b, int B, int L,
               int D, int N, int x_dtype, cudaStream_t st);
 
+// coefficients p [D, N], q, gamma [D, N, 2] from alpha, delta [D, N], theta [D], gamma [D, N, 2] and the gradients
+// back (null: no gradient); N <= 32
+void cema_coeffs_fwd(const void* alpha, const void* delta, const void* theta, const void* gamma, float scale, float* p,
+                     float* q, float* g, int D, int N, int dtype, cudaStream_t st);
+void cema_coeffs_bwd(const float* dp, const float* dq, const float* dg, const void* alpha, const void* delta,
+                     const void* theta, float scale, void* dalpha, void* ddelta, void* dtheta, void* dgamma, int D, int N,
+                     int dtype, cudaStream_t st);
+
 // ---- element-wise (elementwise_kernels.cu)
 void swiglu_fwd(const void* a, const void* b, void* out, long long n, int dtype, cudaStream_t st);
 void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cudaStream_t st);

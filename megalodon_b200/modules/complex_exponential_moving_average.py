@@ -31,8 +31,6 @@ from .. import ops
 from ..parallel.initialize import get_model_parallel_rank, get_model_parallel_world_size
 from ..parallel.utils import comm_device, divide_and_check_no_remainder
 
-_r2c = torch.view_as_complex
-
 
 def _global_permutation(n: int) -> torch.Tensor:
     idx = torch.randperm(n)
@@ -88,15 +86,7 @@ class MultiHeadComplexEMA(nn.Module):
                 dst.copy_(src[lo:lo + self.dim_per_partition])
 
     def _calc_coeffs(self):
-        theta = torch.sigmoid(self.theta.float()) * (2.0 * math.pi / self.ndim)
-        n = torch.arange(1, self.ndim + 1, dtype=theta.dtype, device=theta.device).view(1, self.ndim, 1)
-        theta = n * theta                                     # D x N x 1
-        alpha = torch.sigmoid(self.alpha.float())
-        delta = torch.sigmoid(self.delta.float())
-        p = alpha
-        q = torch.polar(1.0 - alpha * delta, theta)
-        gamma = _r2c(self.gamma.float()) * self.scale         # D x N
-        return p, q, gamma
+        return ops.cema_coeffs(self.alpha, self.delta, self.theta, self.gamma, self.scale)
 
     def coeffs(self):
         if self.training:

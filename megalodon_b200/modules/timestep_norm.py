@@ -67,7 +67,8 @@ class TimestepNorm(nn.Module):
         prev_var: Optional[torch.Tensor] = None,
         padding_mask: Optional[torch.Tensor] = None,
     ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
-        c0, m0, v0 = self.initial_stats(x.size(0), x.dtype)
+        if prev_count is None or prev_mean is None or prev_var is None:
+            c0, m0, v0 = self.initial_stats(x.size(0), x.dtype)
         prev_count = c0 if prev_count is None else prev_count
         prev_mean = m0 if prev_mean is None else prev_mean
         prev_var = v0 if prev_var is None else prev_var

@@ -67,6 +67,13 @@ def linear_add(x: Tensor, w: Tensor, b: Optional[Tensor], addend: Tensor) -> Ten
     return reference.linear(x, w, b, None) + addend
 
 
+def linear_group(x: Tensor, layers):
+    """Several linear layers of one input: [(w, b, addend or None), ...] -> [x w^T + b (+ addend), ...]."""
+    if native_for(x):
+        return _cuda().linear_group(x, layers)
+    return [reference.linear(x, w, b, None) if a is None else reference.linear(x, w, b, None) + a for w, b, a in layers]
+
+
 def qk_rotary(z: Tensor, gamma: Tensor, beta: Tensor, freqs_cis: Tensor, head_dim: int):
     """Shared q / k of the MEGA attention: (z (gamma + 1) / sqrt(head_dim) + beta) for the two rows of
     gamma / beta [2, S], then the rotary rotation; z [B, L, S], position of (b, l) = (b L + l) % len(freqs_cis)."""
@@ -165,6 +172,15 @@ def ema_parameters(p, q, gamma, hx, length: int):
         from . import cpu_native
         return cpu_native.ema_parameters(p, q, gamma, hx, length)
     return reference.ema_parameters(p, q, gamma, hx, length)
+
+
+def cema_coeffs(alpha, delta, theta, gamma, scale: float):
+    """Parameters alpha, delta [D, N, 1], theta [D, 1, 1], gamma [D, N, 2] -> p [D, N, 1] fp32, q [D, N, 1] and
+    gamma [D, N] complex:  p = sigmoid(alpha),  q = (1 - p sigmoid(delta)) e^(i n theta'),  theta' =
+    sigmoid(theta) 2 pi / N,  gamma scale."""
+    if native_for(alpha) and all(t.dtype == alpha.dtype for t in (delta, theta, gamma)) and alpha.shape[1] <= 32:
+        return _cuda().cema_coeffs(alpha, delta, theta, gamma, scale)
+    return reference.cema_coeffs(alpha, delta, theta, gamma, scale)
 
 
 def ema_hidden(x, p, q, hx):

@@ -218,15 +218,82 @@ class _LinearAdd(torch.autograd.Function):
             dx, _ = gemm(g, w, None, None, b_mn=True)
             dx = dx.view(ctx.x_shape)
         if ctx.needs_input_grad[1]:
-            sink = ctx.wgrad_sink
-            if sink is not None and w.dtype == g.dtype:
-                target, add = sink()
-                gemm(g, x2, None, None, a_mn=True, b_mn=True, out=target, accumulate=add)
-            else:
-                dw, _ = gemm(g, x2, None, None, a_mn=True, b_mn=True)
+            dw = _weight_grad(g, x2, w, ctx.wgrad_sink)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = _bias_grad(g, ctx.bias_dtype)
         return dx, dw, db, (dy if ctx.needs_input_grad[3] else None)
+
+
+class _LinearGroup(torch.autograd.Function):
+    """Several linear layers of one input, some with an addend: (x w_i^T + b_i [+ addend_i])_i.  Backward adds up
+    the input gradients in the epilogues of the data-gradient products, so the sum over the layers costs no
+    pass of its own.  Arguments after x: w, b, addend per layer."""
+
+    @staticmethod
+    def forward(ctx, x, *layers):
+        x2 = x.reshape(-1, x.shape[-1])
+        ws, bs, adds = layers[0::3], layers[1::3], layers[2::3]
+        outs = [torch.empty(*x.shape[:-1], w.shape[0], dtype=x.dtype, device=x.device) for w in ws]
+        ys = [o.view(-1, o.shape[-1]) for o in outs]
+        a2 = [None if a is None else a.reshape(-1, a.shape[-1]).contiguous() for a in adds]
+        pending = any(getattr(w, "_gather_spec", None) is not None and w._gather_spec.pending for w in ws)
+        rc = -1
+        if x2.shape[0] <= _SKINNY_MAX_ROWS and len(ws) <= 4 and not pending:
+            rc = _C().skinny_gemm([x2] * len(ws), list(ws), [None] * len(ws), list(bs), a2, [0] * len(ws), ys, False,
+                                  _err_flag(x.device))
+            if rc not in (0, -1):
+                raise RuntimeError(f"few-row products: launch failed with code {rc}")
+            _bump(1 if rc == 0 else 0)
+        if rc != 0:
+            for w, b, a, y in zip(ws, bs, a2, ys):
+                _gemm_gathering(x2, w, b, None, out=y, **({} if a is None else {"softmax": dict(aux=a)}))
+        ctx.save_for_backward(x2, *ws)
+        ctx.sinks = [getattr(w, "_wgrad_sink", None) for w in ws]
+        ctx.bias_dtypes = [None if b is None else b.dtype for b in bs]
+        ctx.x_shape = x.shape
+        ctx.set_materialize_grads(False)
+        return tuple(outs)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x2, *ws = ctx.saved_tensors
+        dx, grads = None, []
+        for i, (dy, w) in enumerate(zip(dys, ws)):
+            need_w, need_b, need_a = ctx.needs_input_grad[1 + 3 * i:4 + 3 * i]
+            if dy is None:
+                grads += [None, None, None]
+                continue
+            g = dy.reshape(-1, dy.shape[-1]).contiguous()
+            if ctx.needs_input_grad[0]:
+                if dx is None:
+                    dx, _ = gemm(g, w, None, None, b_mn=True)
+                else:
+                    gemm(g, w, None, None, b_mn=True, out=dx, accumulate=True)
+            dw = _weight_grad(g, x2, w, ctx.sinks[i]) if need_w else None
+            db = _bias_grad(g, ctx.bias_dtypes[i]) if need_b and ctx.bias_dtypes[i] is not None else None
+            grads += [dw, db, dy if need_a else None]
+        return (None if dx is None else dx.view(ctx.x_shape), *grads)
+
+
+def linear_group(x: Tensor, layers):
+    """[(w, b, addend or None), ...] of one input -> the list of x w^T + b (+ addend)."""
+    x2 = x.reshape(-1, x.shape[-1])
+    if (x.dtype == torch.float32 or _GEMM_BACKEND[0] != "tcgen05" or x2.shape[0] <= 1 or not _tma_ok(x2)
+            or any(w.dtype != x.dtype or w.shape[0] % 8 != 0 or not _tma_ok(w) or (a is not None and a.dtype != x.dtype)
+                   for w, _, a in layers)):
+        return [linear(x, w, b) if a is None else linear_add(x, w, b, a) for w, b, a in layers]
+    return list(_LinearGroup.apply(x, *[t for layer in layers for t in layer]))
+
+
+def _weight_grad(g: Tensor, x2: Tensor, w: Tensor, sink) -> Optional[Tensor]:
+    """g^T x.  A weight that is a view into an FSDP unit's flat buffer carries the matching view of the unit's
+    flat gradient (`sink`): the product lands there in the GEMM's epilogue - the first one of an iteration
+    writes, later ones accumulate - and nothing is handed to autograd."""
+    if sink is not None and w.dtype == g.dtype:
+        target, add = sink()
+        gemm(g, x2, None, None, a_mn=True, b_mn=True, out=target, accumulate=add)
+        return None
+    return gemm(g, x2, None, None, a_mn=True, b_mn=True)[0]          # [M, N]^T x [M, K] -> [N, K]
 
 
 def _bias_grad(g: Tensor, dtype: torch.dtype = torch.float32) -> Tensor:
@@ -281,15 +348,7 @@ class _Linear(torch.autograd.Function):
             dx, _ = gemm(g, w, None, None, b_mn=True)          # [M, N] x [N, K] -> [M, K]
             dx = dx.view(ctx.x_shape)
         if ctx.needs_input_grad[1]:
-            # A weight that is a view into an FSDP unit's flat buffer carries the matching view of the
-            # unit's flat gradient: the weight gradient is accumulated there by the GEMM epilogue and
-            # nothing is handed to autograd (no per-parameter tensor, no concatenation, no add).
-            sink = ctx.wgrad_sink
-            if sink is not None and w.dtype == g.dtype:
-                target, add = sink()        # first product of the iteration writes, later ones accumulate
-                gemm(g, x2, None, None, a_mn=True, b_mn=True, out=target, accumulate=add)
-            else:
-                dw, _ = gemm(g, x2, None, None, a_mn=True, b_mn=True)   # [M, N]^T x [M, K] -> [N, K]
+            dw = _weight_grad(g, x2, w, ctx.wgrad_sink)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = _bias_grad(g, ctx.bias_dtype)
         return dx, dw, db, None
@@ -517,6 +576,34 @@ def dropout(x, p):
 # ----------------------------------------------------------------------------- CEMA
 def _c2r(t: Tensor) -> Tensor:
     return torch.view_as_real(t.to(torch.complex64).contiguous())
+
+
+class _CEMACoeffs(torch.autograd.Function):
+    """p, q, gamma of the EMA recurrence from the layer's parameters, one kernel each way (as separate
+    element-wise operations 14 launches forward and some 25 backward per layer and call)."""
+
+    @staticmethod
+    def forward(ctx, alpha, delta, theta, gamma, scale):
+        a, d, t, g = (x.contiguous() for x in (alpha, delta, theta, gamma))
+        _bump()
+        p, q, go = _C().cema_coeffs_fwd(a, d, t, g, scale)
+        ctx.save_for_backward(a, d, t)
+        ctx.scale = scale
+        ctx.set_materialize_grads(False)
+        return p, torch.view_as_complex(q).unsqueeze(-1), torch.view_as_complex(go)
+
+    @staticmethod
+    def backward(ctx, dp, dq, dg):
+        a, d, t = ctx.saved_tensors
+        real = [None if x is None else _c2r(x) for x in (dq, dg)]
+        _bump()
+        da, dd, dt, dgo = _C().cema_coeffs_bwd(None if dp is None else dp.float().contiguous(), *real, a, d, t,
+                                               ctx.scale)
+        return da, dd, dt, dgo, None
+
+
+def cema_coeffs(alpha, delta, theta, gamma, scale: float):
+    return _CEMACoeffs.apply(alpha, delta, theta, gamma, float(scale))
 
 
 class _CEMA(torch.autograd.Function):

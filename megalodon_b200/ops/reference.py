@@ -128,6 +128,15 @@ def _powers(q: Tensor, start: int, length: int) -> Tensor:
     return torch.exp(logq.unsqueeze(-1) * j)
 
 
+def cema_coeffs(alpha: Tensor, delta: Tensor, theta: Tensor, gamma: Tensor, scale: float):
+    N = alpha.shape[1]
+    ang = torch.sigmoid(theta.float()) * (2.0 * math.pi / N)
+    n = torch.arange(1, N + 1, dtype=ang.dtype, device=ang.device).view(1, N, 1)
+    p = torch.sigmoid(alpha.float())
+    q = torch.polar(1.0 - p * torch.sigmoid(delta.float()), n * ang)
+    return p, q, torch.view_as_complex(gamma.float()) * scale
+
+
 def ema_parameters(p: Tensor, q: Tensor, gamma: Tensor, hx: Optional[Tensor], length: int):
     """CEMA convolution kernel k [D, L] and carried-state bias b [B, D, L].
 

@@ -108,3 +108,61 @@ def test_causal_marker_equals_the_explicit_mask(slen, past):
     want, kv2 = inner(q, k, v, mask, None, kv)
     assert _rel(got, want) < 2.0 ** -6 and torch.equal(kv1[0], kv2[0]) and kv1[2] == kv2[2]
     assert torch.is_tensor(inner.train().causal_mask(q, rows, past))       # dropout acts on the probabilities
+
+
+@pytest.mark.parametrize("D,N", [(1, 1), (37, 16), (512, 32), (100, 5)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_cema_coefficients(D, N, dtype):
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import reference
+    torch.manual_seed(D)
+    ps = [_rand(D, N, 1, dtype=dtype), _rand(D, N, 1, dtype=dtype), _rand(D, 1, 1, dtype=dtype, scale=3.0),
+          _rand(D, N, 2, dtype=dtype)]
+    a = [t.clone().requires_grad_(True) for t in ps]
+    b = [t.double().requires_grad_(True) for t in ps]
+    sc = N ** -0.5
+    p, q, g = ops.cema_coeffs(*a, sc)
+    pd = torch.sigmoid(b[0])
+    qd = torch.polar(1.0 - pd * torch.sigmoid(b[1]),
+                     torch.sigmoid(b[2]) * (2 * torch.pi / N) * torch.arange(1, N + 1, device="cuda").view(1, N, 1))
+    gd = torch.view_as_complex(b[3]) * sc
+    rp, rq, rg = reference.cema_coeffs(*ps, sc)
+    for got, ref, want in ((p, rp, pd), (q, rq, qd), (g, rg, gd)):
+        assert got.shape == ref.shape and got.dtype == ref.dtype
+        assert ((got - want).abs().norm() / want.abs().norm()).item() < 4e-7
+    cp, cq, cg = torch.randn_like(pd), torch.randn_like(qd), torch.randn_like(gd)
+    for outs in ((p, q, g), (pd, qd, gd)):
+        loss = (outs[0] * cp).sum() + (outs[1] * cq.conj()).real.sum() + (outs[2] * cg.conj()).real.sum()
+        loss.backward()
+    for x, y in zip(a, b):
+        assert _rel(x.grad, y.grad) < (2e-5 if dtype == torch.float32 else 2.0 ** -8)
+    p, q, g = ops.cema_coeffs(*a, sc)                       # one output alone
+    assert torch.autograd.grad(p.sum(), a[0])[0].shape == a[0].shape
+
+
+@pytest.mark.parametrize("rows", [1, 2, 64, 65, 300])
+def test_linear_group_matches_separate_layers(rows):
+    from megalodon_b200 import ops
+    torch.manual_seed(rows)
+    K, sizes = 264, (64, 136, 264)
+    x, add = _rand(rows, K), _rand(rows, sizes[2])
+    ws, bs = [_rand(n, K, scale=K ** -0.5) for n in sizes], [_rand(n) for n in sizes]
+    gs = [_rand(rows, n) for n in sizes]
+    leaves = [t.clone().requires_grad_(True) for t in (x, add, *ws, *bs)]
+    lw, lb = leaves[2:5], leaves[5:]
+    outs = ops.linear_group(leaves[0], [(lw[0], lb[0], None), (lw[1], None, None), (lw[2], lb[2], leaves[1])])
+    torch.autograd.backward(outs, gs)
+    ref = [t.double().requires_grad_(True) for t in (x, add, *ws, *bs)]
+    rw, rb = ref[2:5], ref[5:]
+    want = [ref[0] @ rw[0].t() + rb[0], ref[0] @ rw[1].t(), ref[0] @ rw[2].t() + rb[2] + ref[1]]
+    torch.autograd.backward(want, [g.double() for g in gs])
+    for o, w in zip(outs, want):
+        assert _rel(o, w) < 2.0 ** -7
+    for i, (a, r) in enumerate(zip(leaves, ref)):
+        if i != 6:
+            assert _rel(a.grad, r.grad) < 2.0 ** -7, i      # dx: rounded after each of the three products
+    # an output that nobody used
+    out = ops.linear_group(leaves[0], [(lw[0], lb[0], None), (lw[1], None, None)])
+    leaves[0].grad = None
+    out[1].backward(gs[1])
+    assert _rel(leaves[0].grad, gs[1].double() @ ws[1].double()) < 2.0 ** -7
