@@ -173,13 +173,17 @@ __global__ void tsn_seg_apply_kernel(const float* __restrict__ gu, const float* 
 }
 
 // ---- the same scan as ONE kernel when a sequence's segments fit one CTA (L <= 16384): a CTA owns GT
-// groups of one batch row, thread (segment, group) keeps its kSegLen samples in registers, the exclusive
+// groups of one batch row, thread (segment, group) keeps its SEG samples in registers, the exclusive
 // prefix over segments runs in shared memory (log2(nseg) doubling steps), and the running statistics are
 // written from the registers.  Three dependent launches and the round trip of the segment sums through
 // global memory become one launch.
+// What bounds it is the serial chain of a thread - every step ends in 64-bit reciprocals and roots - so the
+// segments are as short as a CTA has threads for (`tsn_fused_seg`), and a step takes one reciprocal and one
+// reciprocal root instead of three divisions and a root.  With 32-step segments throughout: 37 us for 4096 steps
+// of 64 groups, 18 us for 37 steps.
 constexpr int kScanMaxThreads = 512;   // 128 registers per thread: the segment's samples stay in registers
 
-template <typename T>
+template <typename T, int SEG>
 __global__ void __launch_bounds__(kScanMaxThreads)
 tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv, const bool* __restrict__ mask,
                       const long long* __restrict__ prev_count, const T* __restrict__ prev_mean,
@@ -191,14 +195,14 @@ tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv
   const int gl = tid % GT, sgi = tid / GT;
   const int g = blockIdx.x * GT + gl, b = blockIdx.y;
   const bool live = g < G;
-  const int t0 = sgi * kSegLen, t1 = min(L, t0 + kSegLen);
+  const int t0 = sgi * SEG, t1 = min(L, t0 + SEG);
   const long long off = (long long)b * L * G + (live ? g : 0);
   const bool* mb_ = mask ? mask + (long long)b * L : nullptr;
-  float us[kSegLen], vs[kSegLen];
+  float us[SEG], vs[SEG];
   unsigned valid = 0;   // bit j: step t0 + j exists and is not padded
   double n = 0, a = 0, c = 0;
 #pragma unroll
-  for (int j = 0; j < kSegLen; ++j) {
+  for (int j = 0; j < SEG; ++j) {
     const int t = t0 + j;
     const bool in = live && t < t1;
     us[j] = in ? gu[off + (long long)t * G] : 0.f;
@@ -206,7 +210,7 @@ tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv
     if (in && !(mb_ && mb_[t])) valid |= 1u << j;
   }
 #pragma unroll
-  for (int j = 0; j < kSegLen; ++j)
+  for (int j = 0; j < SEG; ++j)
     if (valid >> j & 1u) {
       const double u = us[j], v = vs[j];
       n += 1.0;
@@ -258,7 +262,7 @@ tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv
     var = fmax(s2 / cn - mean * mean, 0.0);
   }
 #pragma unroll
-  for (int j = 0; j < kSegLen; ++j) {
+  for (int j = 0; j < SEG; ++j) {
     const int t = t0 + j;
     if (t >= t1) break;
     if (valid >> j & 1u) {
@@ -266,17 +270,23 @@ tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv
       cn += 1.0;
       s1 += u;
       s2 += v + u * u;
-      mean = s1 / cn;
-      var = fmax(s2 / cn - mean * mean, 0.0);
+      const double inv = 1.0 / cn;
+      mean = s1 * inv;
+      var = fmax(s2 * inv - mean * mean, 0.0);
     }
     cummean[off + (long long)t * G] = (float)mean;
-    cumrstd[off + (long long)t * G] = (float)(1.0 / sqrt(var + (double)eps));
+    cumrstd[off + (long long)t * G] = (float)rsqrt(var + (double)eps);
   }
 }
 
-// groups per CTA of the fused scans: as many as keep the CTA near 512 threads (0: the sequence is too long)
+// steps per segment of the fused scans (0: the sequence is too long): the fewest whose segments fit a CTA
+inline int tsn_fused_seg(int L) {
+  for (int seg = 4; seg <= 32; seg *= 2)
+    if ((L + seg - 1) / seg <= kScanMaxThreads) return seg;
+  return 0;
+}
+// groups per CTA of the fused scans: as many as keep the CTA near 512 threads
 inline int tsn_fused_groups(int nseg) {
-  if (nseg > kScanMaxThreads) return 0;
   int gt = 1;
   while (gt * 2 * nseg <= kScanMaxThreads && gt < 32) gt *= 2;
   return gt;
@@ -366,18 +376,39 @@ struct StepIn {
   const float *ux, *ds, *db, *cummean, *cumrstd;
 };
 
-__device__ __forceinline__ Affine tsn_step_map(const StepIn& in, long long i, int G, int t, double pm, double m0) {
-  const double c1 = (m0 - 1.0) / m0, c2 = 1.0 / m0;
-  const double prev_u = t == 0 ? pm : (double)in.cummean[i - G];
-  const double delta = (double)in.ux[i] - prev_u;
-  const double r = in.cumrstd[i];
-  const double r3ds = r * r * r * (double)in.ds[i];
+// what a step's map and its replay need, as read from memory
+struct StepVal {
+  float ux, ds, db, prev_u, r;
+};
+__device__ __forceinline__ StepVal tsn_step_load(const StepIn& in, long long i, int G, int t, float pm) {
+  return {in.ux[i], in.ds[i], in.db[i], t == 0 ? pm : in.cummean[i - G], in.cumrstd[i]};
+}
+__device__ __forceinline__ Affine tsn_step_map(const StepVal& s, double m0) {
+  const double c2 = 1.0 / m0, c1 = 1.0 - c2;
+  const double delta = (double)s.ux - (double)s.prev_u;
+  const double r = s.r;
+  const double r3ds = r * r * r * (double)s.ds;
   Affine m;
   m.a = c1;
   m.b = -2.0 * c1 * c2 * delta;
-  m.o1 = -c1 * r * (double)in.db[i] + c1 * c2 * delta * r3ds;
+  m.o1 = -c1 * r * (double)s.db + c1 * c2 * delta * r3ds;
   m.o2 = -0.5 * c1 * r3ds;
   return m;
+}
+__device__ __forceinline__ Affine tsn_step_map(const StepIn& in, long long i, int G, int t, float pm, double m0) {
+  return tsn_step_map(tsn_step_load(in, i, G, t, pm), m0);
+}
+// the step's input gradients from the incoming (u, v), which become those of the step before
+__device__ __forceinline__ void tsn_step_replay(const StepVal& s, double m0, double& u, double& v, float* dux, float* dvx) {
+  const double c2 = 1.0 / m0, c1 = 1.0 - c2;
+  const double delta = (double)s.ux - (double)s.prev_u;
+  const double r = s.r;
+  const double du = u - r * (double)s.db;
+  const double dv = v - 0.5 * r * r * r * (double)s.ds;
+  *dux = (float)(c2 * du + 2.0 * c1 * c2 * dv * delta);
+  *dvx = (float)(c2 * dv);
+  u = c1 * du - 2.0 * c1 * c2 * dv * delta;
+  v = c1 * dv;
 }
 
 // (b, seg, g): composite map of the segment's valid steps, taken from its last step to its first
@@ -395,7 +426,7 @@ __global__ void tsn_bwd_seg_maps_kernel(StepIn in, const bool* __restrict__ mask
   const int t0 = sgi * kSegLen, t1 = min(L, t0 + kSegLen);
   const bool* mb_ = mask ? mask + (long long)b * L : nullptr;
   const long long first = count_final[b] - (cumvalid ? cumvalid[(long long)b * L + L - 1] : L);
-  const double pm = to_f(prev_mean[b * G + g]);
+  const float pm = to_f(prev_mean[b * G + g]);
   const long long off = (long long)b * L * G + g;
   Affine seg = affine_identity();
   for (int t = t1 - 1; t >= t0; --t) {
@@ -448,7 +479,7 @@ __global__ void tsn_bwd_seg_apply_kernel(StepIn in, const bool* __restrict__ mas
   const int t0 = sgi * kSegLen, t1 = min(L, t0 + kSegLen);
   const bool* mb_ = mask ? mask + (long long)b * L : nullptr;
   const long long first = count_final[b] - (cumvalid ? cumvalid[(long long)b * L + L - 1] : L);
-  const double pm = to_f(prev_mean[b * G + g]);
+  const float pm = to_f(prev_mean[b * G + g]);
   const long long off = (long long)b * L * G + g;
   double u = maps[i], v = maps[total + i];
   for (int t = t1 - 1; t >= t0; --t) {
@@ -458,24 +489,15 @@ __global__ void tsn_bwd_seg_apply_kernel(StepIn in, const bool* __restrict__ mas
       dvx[e] = 0.f;
       continue;
     }
-    const double md = count_at(cumvalid, first, b, L, t);
-    const double c1 = (md - 1.0) / md, c2 = 1.0 / md;
-    const double prev_u = t == 0 ? pm : (double)in.cummean[e - G];
-    const double delta = (double)in.ux[e] - prev_u;
-    const double r = in.cumrstd[e];
-    const double du = u - r * (double)in.db[e];
-    const double dv = v - 0.5 * r * r * r * (double)in.ds[e];
-    dux[e] = (float)(c2 * du + 2.0 * c1 * c2 * dv * delta);
-    dvx[e] = (float)(c2 * dv);
-    u = c1 * du - 2.0 * c1 * c2 * dv * delta;
-    v = c1 * dv;
+    tsn_step_replay(tsn_step_load(in, e, G, t, pm), count_at(cumvalid, first, b, L, t), u, v, dux + e, dvx + e);
   }
 }
 
 // The backward scan as ONE kernel under the same condition as the forward one: thread (segment, group)
 // composes its segment's map, the suffix composition over segments runs in shared memory (the maps do not
 // commute: the later segment's map is applied first), and the segment is replayed from its incoming state.
-template <typename T>
+// Short segments (`tsn_fused_seg`) are read once, all loads in flight together, and stay in registers.
+template <typename T, int SEG>
 __global__ void __launch_bounds__(kScanMaxThreads)
 tsn_bwd_scan_fused_kernel(StepIn in, const bool* __restrict__ mask, const int* __restrict__ cumvalid,
                           const long long* __restrict__ count_final, const T* __restrict__ prev_mean,
@@ -487,17 +509,32 @@ tsn_bwd_scan_fused_kernel(StepIn in, const bool* __restrict__ mask, const int* _
   const int gl = tid % GT, sgi = tid / GT;
   const int g = blockIdx.x * GT + gl, b = blockIdx.y;
   const bool live = g < G;
-  const int t0 = sgi * kSegLen, t1 = min(L, t0 + kSegLen);
+  const int t0 = sgi * SEG, t1 = min(L, t0 + SEG);
   const bool* mb_ = mask ? mask + (long long)b * L : nullptr;
   const long long first = count_final[b] - (cumvalid ? cumvalid[(long long)b * L + L - 1] : L);
-  const double pm = live ? (double)to_f(prev_mean[b * G + g]) : 0.0;
+  const float pm = live ? to_f(prev_mean[b * G + g]) : 0.f;
   const long long off = (long long)b * L * G + (live ? g : 0);
   Affine seg = affine_identity();
-  if (live)
+  constexpr bool kKeep = SEG <= 8;
+  StepVal keep[kKeep ? SEG : 1];
+  if constexpr (kKeep) {
+#pragma unroll
+    for (int i = 0; i < SEG; ++i) {
+      const int t = t0 + i;
+      if (live && t < t1) keep[i] = tsn_step_load(in, off + (long long)t * G, G, t, pm);
+    }
+#pragma unroll
+    for (int i = SEG - 1; i >= 0; --i) {
+      const int t = t0 + i;
+      if (live && t < t1 && !(mb_ && mb_[t]))
+        seg = affine_compose(tsn_step_map(keep[i], count_at(cumvalid, first, b, L, t)), seg);
+    }
+  } else if (live) {
     for (int t = t1 - 1; t >= t0; --t) {
       if (mb_ && mb_[t]) continue;
       seg = affine_compose(tsn_step_map(in, off + (long long)t * G, G, t, pm, count_at(cumvalid, first, b, L, t)), seg);
     }
+  }
   // position j = nseg - 1 - sgi counts the segments in the order the backward pass meets them
   const int j = nseg - 1 - sgi;
   const int slot = j * GT + gl;
@@ -536,6 +573,17 @@ tsn_bwd_scan_fused_kernel(StepIn in, const bool* __restrict__ mask, const int* _
     u = sh[0][e] * iu + sh[1][e] * iv + sh[2][e];
     v = sh[0][e] * iv + sh[3][e];
   }
+  if constexpr (kKeep) {
+#pragma unroll
+    for (int i = SEG - 1; i >= 0; --i) {
+      const int t = t0 + i;
+      if (t >= t1) continue;
+      const long long e = off + (long long)t * G;
+      if (mb_ && mb_[t]) dux[e] = dvx[e] = 0.f;
+      else tsn_step_replay(keep[i], count_at(cumvalid, first, b, L, t), u, v, dux + e, dvx + e);
+    }
+    return;
+  }
   for (int t = t1 - 1; t >= t0; --t) {
     const long long e = off + (long long)t * G;
     if (mb_ && mb_[t]) {
@@ -543,17 +591,7 @@ tsn_bwd_scan_fused_kernel(StepIn in, const bool* __restrict__ mask, const int* _
       dvx[e] = 0.f;
       continue;
     }
-    const double md = count_at(cumvalid, first, b, L, t);
-    const double c1 = (md - 1.0) / md, c2 = 1.0 / md;
-    const double prev_u = t == 0 ? pm : (double)in.cummean[e - G];
-    const double delta = (double)in.ux[e] - prev_u;
-    const double r = in.cumrstd[e];
-    const double du = u - r * (double)in.db[e];
-    const double dv = v - 0.5 * r * r * r * (double)in.ds[e];
-    dux[e] = (float)(c2 * du + 2.0 * c1 * c2 * dv * delta);
-    dvx[e] = (float)(c2 * dv);
-    u = c1 * du - 2.0 * c1 * c2 * dv * delta;
-    v = c1 * dv;
+    tsn_step_replay(tsn_step_load(in, e, G, t, pm), count_at(cumvalid, first, b, L, t), u, v, dux + e, dvx + e);
   }
 }
 
@@ -786,6 +824,14 @@ inline bool tsn_vec_ok(int H, int G, std::initializer_list<const void*> ptrs) {
     default: { constexpr int VL = 32; __VA_ARGS__; } break;  \
   }
 
+#define SEG_SWITCH(seg, ...)                                  \
+  switch (seg) {                                              \
+    case 4: { constexpr int SEG = 4; __VA_ARGS__; } break;    \
+    case 8: { constexpr int SEG = 8; __VA_ARGS__; } break;    \
+    case 16: { constexpr int SEG = 16; __VA_ARGS__; } break;  \
+    default: { constexpr int SEG = 32; __VA_ARGS__; } break;  \
+  }
+
 int pick_lpg(int Dg) {
   int l = 1;
   while (l * 2 <= Dg && l < 32) l *= 2;
@@ -838,14 +884,15 @@ void timestep_norm_fwd(const void* x, const long long* prev_count, const void* p
         tsn_group_stats_kernel<T, LPG><<<div_up(threads, 256), 256, 0, st>>>((const T*)x, gu, gv, rows, H, G);
       });
     }
+    const int seg = tsn_fused_seg(L);
+    if (seg > 0 && B <= 65535) {
+      const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
+      SEG_SWITCH(seg, (tsn_scan_fused_kernel<T, SEG><<<dim3(div_up(G, gt), B), gt * nseg, 0, st>>>(
+          gu, gv, mask, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
+          cummean, cumrstd, L, G, nseg, gt, eps)));
+    } else {
     const int nseg = tsn_num_segments(L);
     const long long nsg = (long long)B * nseg * G;
-    const int gt = tsn_fused_groups(nseg);
-    if (gt > 0 && B <= 65535) {
-      tsn_scan_fused_kernel<T><<<dim3(div_up(G, gt), B), gt * nseg, 0, st>>>(
-          gu, gv, mask, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
-          cummean, cumrstd, L, G, nseg, gt, eps);
-    } else {
     tsn_seg_sums_kernel<<<div_up(nsg, 256), 256, 0, st>>>(gu, gv, mask, seg_scratch, B, L, G, nseg);
     tsn_seg_prefix_kernel<T><<<div_up((long long)B * G, 128), 128, 0, st>>>(
         seg_scratch, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
@@ -890,17 +937,18 @@ void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_o
             (const T*)dy, (const T*)x, cummean, (const W*)gamma, gamma_offset, ux, ds, db, rows, H, G);
       });
     }
-    const int nseg = tsn_num_segments(L);
-    const long long nsg = (long long)B * nseg * G;
     if (mask != nullptr) tsn_cumvalid_kernel<<<div_up(B, 32), 32, 0, st>>>(mask, cumvalid, B, L);
     const int* cv = mask != nullptr ? cumvalid : nullptr;
     const StepIn in{ux, ds, db, cummean, cumrstd};
-    const int gt = tsn_fused_groups(nseg);
-    if (gt > 0 && B <= 65535) {
-      tsn_bwd_scan_fused_kernel<T><<<dim3(div_up(G, gt), B), gt * nseg, 0, st>>>(
+    const int seg = tsn_fused_seg(L);
+    if (seg > 0 && B <= 65535) {
+      const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
+      SEG_SWITCH(seg, (tsn_bwd_scan_fused_kernel<T, SEG><<<dim3(div_up(G, gt), B), gt * nseg, 0, st>>>(
           in, mask, cv, count_final, (const T*)prev_mean, (const T*)dmean_out, (const T*)dvar_out, (T*)dprev_mean,
-          (T*)dprev_var, dux, dvx, L, G, nseg, gt);
+          (T*)dprev_var, dux, dvx, L, G, nseg, gt)));
     } else {
+    const int nseg = tsn_num_segments(L);
+    const long long nsg = (long long)B * nseg * G;
     tsn_bwd_seg_maps_kernel<T><<<div_up(nsg, 256), 256, 0, st>>>(in, mask, cv, count_final, (const T*)prev_mean,
                                                                seg_scratch, B, L, G, nseg);
     tsn_bwd_seg_prefix_kernel<T><<<div_up((long long)B * G, 128), 128, 0, st>>>(

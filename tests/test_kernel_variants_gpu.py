@@ -166,3 +166,37 @@ def test_linear_group_matches_separate_layers(rows):
     leaves[0].grad = None
     out[1].backward(gs[1])
     assert _rel(leaves[0].grad, gs[1].double() @ ws[1].double()) < 2.0 ** -7
+
+
+# lengths at which the scans change the steps of a segment (4, 8, 16, 32 of at most 512 segments) and leave the
+# one-kernel form; a padded stretch and a carried past
+@pytest.mark.parametrize("L", [1, 3, 5, 37, 2048, 2049, 4097, 8193, 16385])
+@pytest.mark.parametrize("masked", [False, True])
+def test_timestep_norm_segments(L, masked):
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import reference
+    torch.manual_seed(L)
+    B, G, D = 2, 3, 24
+    x, g = _rand(B, L, D, dtype=torch.float32), _rand(B, L, D, dtype=torch.float32)
+    w, b = _rand(D, dtype=torch.float32, scale=0.2), _rand(D, dtype=torch.float32)
+    count = torch.tensor([0, 11], device="cuda")
+    mean, var = _rand(B, G, dtype=torch.float32, scale=0.3), torch.rand(B, G, device="cuda") + 0.5
+    mask = None
+    if masked:
+        mask = torch.zeros(B, L, dtype=torch.bool, device="cuda")
+        mask[0, : L // 3] = True
+        mask[1, L // 2: L // 2 + 5] = True
+    gm, gv = _rand(B, G, dtype=torch.float32), _rand(B, G, dtype=torch.float32)
+
+    def grads(f, dt):
+        leaves = [t.to(dt).requires_grad_(True) for t in (x, mean, var, w, b)]
+        y, c, m, v = f(leaves[0], count, leaves[1], leaves[2], leaves[3], leaves[4], mask, G, 1e-5, 1.0)
+        return (y, m, v), torch.autograd.grad((y * g.to(dt)).sum() + (m * gm.to(dt)).sum() + (v * gv.to(dt)).sum(),
+                                              leaves), c
+    got, dgot, c1 = grads(ops.timestep_norm, torch.float32)
+    want, dwant, c2 = grads(reference.timestep_norm, torch.float64)
+    assert torch.equal(c1, c2)
+    for a, r in zip(got, want):
+        assert _rel(a, r) < 2e-6
+    for a, r in zip(dgot, dwant):
+        assert _rel(a, r) < 2e-5, (a.shape, _rel(a, r))
