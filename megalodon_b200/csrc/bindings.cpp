@@ -467,7 +467,7 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
                                             const std::vector<int64_t>& c_part_ptrs, bool accumulate,
                                             const std::vector<int64_t>& b_gather_ptrs, int64_t b_gather_rank,
                                             int64_t epi_kind, const OptTensor& row_in, const OptTensor& row_in2,
-                                            const OptTensor& row_out, const OptTensor& aux, int64_t causal_off) {
+                                            const OptTensor& row_out, const OptTensor& aux, int64_t causal_off, int64_t tile) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda(), "operands must be CUDA tensors");
   c10::cuda::CUDAGuard guard(A.device());
   TORCH_CHECK(A.dim() >= 2 && A.dim() <= 4 && A.dim() == B.dim(), "operands must both be 2-D, 3-D or 4-D");
@@ -579,7 +579,7 @@ std::tuple<Tensor, OptTensor, int64_t> gemm(const Tensor& A, const Tensor& B, co
                                        (a_parts > 1 || c_part_ptrs.size() > 1) ? &peers : nullptr,
                                        accumulate && out.has_value(), gather.world > 0 ? &gather : nullptr,
                                        (sm.kind != 0 || with_addend) ? &sm : nullptr,
-                                       A.dim() == 4 ? &outer : nullptr);
+                                       A.dim() == 4 ? &outer : nullptr, (int)tile);
   // the launcher's status goes back to Python, which raises on a non-zero code
   return {C, pre, (int64_t)rc};
 }
@@ -1186,7 +1186,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("c_part_ptrs") = std::vector<int64_t>(), py::arg("accumulate") = false,
         py::arg("b_gather_ptrs") = std::vector<int64_t>(), py::arg("b_gather_rank") = 0, py::arg("epi_kind") = 0,
         py::arg("row_in") = py::none(), py::arg("row_in2") = py::none(), py::arg("row_out") = py::none(),
-        py::arg("aux") = py::none(), py::arg("causal_off") = 0);
+        py::arg("aux") = py::none(), py::arg("causal_off") = 0, py::arg("tile") = 0);
   m.def("gemm_gather_supported", [](int64_t M, int64_t N, int64_t K, int64_t world) {
     return mb::gemm_gather_supported((int)M, (int)N, (int)K, (int)world);
   });

@@ -39,13 +39,15 @@ using namespace ptx;
 constexpr int BM = 128;
 constexpr int BK = 64;          // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int kStages = 4;
 constexpr int kGemmThreads = 192;
 constexpr int kEpiWarps = 4;
 constexpr int kMaxPeers = 8;
 
+// Ring of the single-CTA kernel: a tile that walks K alone is bound by one memory latency per ring round, so the
+// narrow tiles spend their smaller stages on a deeper ring.
 template <int BN>
 struct SmemLayout {
+  static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
   static constexpr int a_bytes = BM * BK * 2;       // 16 KiB
   static constexpr int b_bytes = BN * BK * 2;       // 32 KiB at BN = 256
   static constexpr int stage_bytes = a_bytes + b_bytes;
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ GemmParams p, int in_fmt) {
   using L = SmemLayout<BN>;
+  constexpr int kStages = L::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::bar_offset);
@@ -311,7 +314,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
   const int tiles_per_batch = num_m * num_n;
   const int num_tiles = tiles_per_batch * p.batch;
   const int num_k = (p.K + BK - 1) / BK;
-  constexpr uint32_t kTmemCols = 2 * BN;     // two accumulators (power of two: 256 or 512)
+  constexpr uint32_t kTmemCols = 2 * BN;     // two accumulators (a power of two)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
@@ -511,6 +514,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
 constexpr int kPairStages = 6;
 constexpr int kPairBM = 256;      // rows of the pair's tile
 constexpr int kPairBN = 256;
+constexpr int kPairTile = 512;    // name of this variant among the tiles (the others go by their width)
 
 struct PairSmem {
   static constexpr int a_bytes = BM * BK * 2;                 // this CTA's 128 rows of A
@@ -1010,7 +1014,53 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
                              n0 + kPairBN <= p.N && !(p.epi == kEpiRowMax && p.alpha < 0.f);
       // (the gathering variant, whose 320 threads leave fewer registers each, keeps the direct form: a
       // register spilled between an asynchronous tensor-memory read and its wait would be read too early)
-      if (GATHER || !can_group) {
+      const bool can_group_f32 = !GATHER && sizeof(OutT) == 4 && p.epi == kEpiStd && P == nullptr && p.c_nparts <= 1 &&
+                                 !p.accumulate && p.aux == nullptr && n0 + kPairBN <= p.N &&
+                                 ((p.ldc | p.c_batch_stride | p.c_outer_stride) & 3) == 0 &&
+                                 (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+      if (can_group_f32) {
+        // fp32 results (logits): 32 columns are one staging buffer
+        float* dst = reinterpret_cast<float*>(p.C) + cb + (long long)row_base * p.ldc + n0;
+#pragma unroll 1
+        for (int c = 0; c < kPairBN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32(t_row + c * 32, r);
+          tmem_ld_wait();
+          float v[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+          if (p.bias != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const int col = n0 + c * 32 + i;
+              float bv;
+              if (p.bias_dtype == kF32) bv = reinterpret_cast<const float*>(p.bias)[col];
+              else if (p.bias_dtype == kBF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col]);
+              else bv = __half2float(reinterpret_cast<const __half*>(p.bias)[col]);
+              v[i] += bv;
+            }
+          }
+          if (p.act == 1) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 w = make_uint4(__float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]),
+                                       __float_as_uint(v[4 * i + 2]), __float_as_uint(v[4 * i + 3]));
+            sts128(epi_stage_addr(stage_buf, lane, i), w);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int rr = 4 * j + (lane >> 3), q = lane & 7;
+            uint4 w;
+            lds128(epi_stage_addr(stage_buf, rr, q), w);
+            if (rr < rows_valid) *reinterpret_cast<uint4*>(dst + (long long)rr * p.ldc + c * 32 + q * 4) = w;
+          }
+          __syncwarp();
+        }
+      } else if (GATHER || !can_group) {
 #pragma unroll 1
         for (int c = 0; c < kPairBN / 32; ++c) direct_chunk(c);
       } else if constexpr (!GATHER) {
@@ -1209,6 +1259,41 @@ static int launch_gemm_pair(const TmapArray& ta, const CUtensorMap& tb, const Ge
 
 static bool g_use_pair = true;
 
+// Which tile a product runs on: the one whose estimate is lowest,
+//   waves * max(k-blocks * t, e) + e,   t = max(latency of a ring round / its stages, bytes of resident tiles / rate).
+// Latency: a tile alone on its SM takes 0.30 us per k-block as a CTA pair (6 stages), 0.42 / 0.30 / 0.24 us as
+// 128 x 256 / 128 / 64 (4 / 6 / 8 stages; K from 1024 to 8192 at one tile per CTA, differences of event times).
+// Rate: what the big products draw from L2 in steady state, 64 KiB per pair and k-block at 0.45 us on 74 pairs.
+// `e` is a tile's epilogue, hidden behind the next tile's main loop except at the end.  Few wide tiles leave most
+// SMs without work and no tile is faster than its ring: 1024 x 512 x 512 is 8 pair tiles (20 us measured) and 64
+// tiles of 128 x 64.
+static int pick_tile(const GemmParams& p, int num_sms) {
+  const bool pair_ok = g_use_pair && p.M > BM && num_sms >= 2;
+  if (p.a_parts > 1 || p.c_nparts > 1) return pair_ok ? kPairTile : 256;
+  const double nk = (p.K + BK - 1) / BK, rate = 10.5e6;      // bytes per us
+  struct Tile { int name, bm, bn; double lat, bytes, tail; };
+  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.30, 65536, 3.0},
+                        {256, BM, 256, 0.42, 49152, 3.0},
+                        {128, BM, 128, 0.30, 32768, 2.0},
+                        {64, BM, 64, 0.24, 24576, 1.5}};
+  int best = 256;
+  double best_us = 1e30;
+  for (const Tile& t : tiles) {
+    if (t.name == kPairTile && !pair_ok) continue;
+    const long long n = (long long)((p.M + t.bm - 1) / t.bm) * ((p.N + t.bn - 1) / t.bn) * p.batch;
+    const int slots = t.name == kPairTile ? num_sms / 2 : num_sms;
+    const double resident = n < slots ? (double)n : (double)slots;
+    const double per_k = t.lat > t.bytes * resident / rate ? t.lat : t.bytes * resident / rate;
+    const double loop = nk * per_k > t.tail ? nk * per_k : t.tail;
+    const double us = (double)((n + slots - 1) / slots) * loop + t.tail;
+    if (us < best_us * 0.97) {
+      best_us = us;
+      best = t.name;
+    }
+  }
+  return best;
+}
+
 // Returns 0 on success, negative on a host-side failure.  `err` is a device int
 // that the kernel sets non-zero if one of its bounded waits gives up.
 int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const void* bias, int bias_dtype,
@@ -1216,7 +1301,7 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
                       bool b_mn, int mode, float alpha, int batch, long long a_bs, long long b_bs, long long c_bs,
                       int in_dtype, int out_dtype, int* err, int num_sms, cudaStream_t st,
                       const GemmPeerSpec* peers, bool accumulate, const GemmGatherSpec* gather,
-                      const GemmSoftmaxSpec* softmax, const GemmOuterBatch* outer) {
+                      const GemmSoftmaxSpec* softmax, const GemmOuterBatch* outer, int tile) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
   // TMA wants 16-byte strides; the vectorised epilogue wants 16-byte aligned rows of C
   if (lda % 8 != 0 || ldb % 8 != 0 || ldc % 8 != 0) return -1;
@@ -1224,7 +1309,6 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
   const int nb2 = outer != nullptr ? outer->count : 1;
   const long long a_bs2 = outer != nullptr ? outer->a_stride : 0, b_bs2 = outer != nullptr ? outer->b_stride : 0;
   if (nb2 < 1 || (nb2 > 1 && (a_bs2 % 8 != 0 || b_bs2 % 8 != 0 || outer->c_stride % 8 != 0))) return -1;
-  const int BN = 256;
   TmapArray ta;
   CUtensorMap tb;
   GemmParams p{};
@@ -1265,8 +1349,11 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
     if (p.c_part_cols % 32 != 0) return -7;
     for (int i = 0; i < p.c_nparts; ++i) p.c_parts[i] = peers->c_ptrs[i];
   }
-  const bool pair = g_use_pair && M > BM && num_sms >= 2;
   if (!ok) return -41;
+  if (gather != nullptr && gather->world > 0) tile = kPairTile;
+  if (tile == 0) tile = pick_tile(p, num_sms);
+  if (tile != kPairTile && tile != 64 && tile != 128 && tile != 256) return -11;
+  const bool pair = tile == kPairTile && g_use_pair;
   if (gather != nullptr && gather->world > 0) {
     // B must be the whole K-major weight, contiguous, its row blocks whole 128-row chunks
     if (!gemm_gather_supported(M, N, K, gather->world) || !pair || a_mn || b_mn || p.batch != 1 || mode != 0 ||
@@ -1276,7 +1363,7 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
     for (int i = 0; i < gather->world; ++i) p.g_src[i] = gather->src[i];
   }
   ok = ok && (b_mn ? make_tmap_4d(&tb, B, N, K, batch, nb2, ldb, b_bs, b_bs2, 64, 64, in_dtype)
-                   : make_tmap_4d(&tb, B, K, N, batch, nb2, ldb, b_bs, b_bs2, BK, pair ? kPairBN / 2 : BN, in_dtype));
+                   : make_tmap_4d(&tb, B, K, N, batch, nb2, ldb, b_bs, b_bs2, BK, pair ? kPairBN / 2 : tile, in_dtype));
   if (!ok) return -4;
   const int fmt = in_dtype == kBF16 ? 1 : 0;
   if (p.g_world > 0) {
@@ -1298,16 +1385,21 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
 #undef GEMM_PAIR_CASE
     return -5;
   }
-#define GEMM_CASE(AMN, BMN)                                                                              \
-  if (a_mn == AMN && b_mn == BMN) {                                                                      \
-    if (out_dtype == kBF16) return launch_gemm<256, AMN, BMN, __nv_bfloat16>(ta, tb, p, fmt, num_sms, st); \
-    if (out_dtype == kF16) return launch_gemm<256, AMN, BMN, __half>(ta, tb, p, fmt, num_sms, st);       \
-    return launch_gemm<256, AMN, BMN, float>(ta, tb, p, fmt, num_sms, st);                               \
+#define GEMM_CASE(BNV, AMN, BMN)                                                                         \
+  if (tile == BNV && a_mn == AMN && b_mn == BMN) {                                                       \
+    if (out_dtype == kBF16) return launch_gemm<BNV, AMN, BMN, __nv_bfloat16>(ta, tb, p, fmt, num_sms, st); \
+    if (out_dtype == kF16) return launch_gemm<BNV, AMN, BMN, __half>(ta, tb, p, fmt, num_sms, st);       \
+    return launch_gemm<BNV, AMN, BMN, float>(ta, tb, p, fmt, num_sms, st);                               \
   }
-  GEMM_CASE(false, false)
-  GEMM_CASE(false, true)
-  GEMM_CASE(true, true)
-  GEMM_CASE(true, false)
+#define GEMM_CASES(BNV)         \
+  GEMM_CASE(BNV, false, false)  \
+  GEMM_CASE(BNV, false, true)   \
+  GEMM_CASE(BNV, true, true)    \
+  GEMM_CASE(BNV, true, false)
+  GEMM_CASES(64)
+  GEMM_CASES(128)
+  GEMM_CASES(256)
+#undef GEMM_CASES
 #undef GEMM_CASE
   return -5;
 }

@@ -161,13 +161,14 @@ struct GemmOuterBatch {
   int count = 1;
   long long a_stride = 0, b_stride = 0, c_stride = 0;
 };
+// `tile`: 0 picks one; 512: 256 x 256 by a CTA pair; 64, 128, 256: 128 x tile by one CTA
 int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const void* bias, int bias_dtype,
                       int act, int M, int N, int K, long long lda, long long ldb, long long ldc, bool a_mn,
                       bool b_mn, int mode, float alpha, int batch, long long a_bs, long long b_bs, long long c_bs,
                       int in_dtype, int out_dtype, int* err, int num_sms, cudaStream_t st,
                       const GemmPeerSpec* peers = nullptr, bool accumulate = false,
                       const GemmGatherSpec* gather = nullptr, const GemmSoftmaxSpec* softmax = nullptr,
-                      const GemmOuterBatch* outer = nullptr);
+                      const GemmOuterBatch* outer = nullptr, int tile = 0);
 // ---- FFT long convolution (fftconv_kernels.cu); spectra are [rows, N2/2 + 1] complex, N2 = 1 << fftconv_logn(L)
 int fftconv_logn(int L);
 bool fftconv_supported(int L);          // L <= 16384

@@ -124,6 +124,12 @@ class MegaOutputLayer(nn.Module):
             return x, (prev_count.detach(), prev_mean.detach(), prev_var.detach())
         return x, None
 
+    def logits(self, x: Tensor) -> Tensor:
+        """fp32 logits of normalised activations."""
+        if torch.is_grad_enabled() or get_model_parallel_world_size() > 1:
+            return self.output(x).float()
+        return ops.linear_fp32_out(x, self.output.weight)
+
     def forward(self, x: Tensor, cache: Optional[Tuple[Tensor, Tensor, Tensor]] = None, carry=None,
                 piece=None):
         x, state = self.normalize(x, cache, carry, piece)
@@ -227,10 +233,10 @@ class Mega(nn.Module):
             if targets is not None:
                 xn, _ = self.output.normalize(x)
                 return self._gather_losses([self._piece_loss(xn, targets)]), None
-            out, cache_output = self.output(x, cache_output)
+            xn, cache_output = self.output.normalize(x, cache_output)
             if cache is not None:
                 cache = (cache_layers, cache_output)
-            return out.float(), cache
+            return self.output.logits(xn), cache
 
         # ---- sequence micro-batching (training / scoring without cache)
         pieces = list(torch.split(x, piece_len, dim=1))
@@ -244,7 +250,7 @@ class Mega(nn.Module):
         for i in range(n):
             xn, carry = self.output.normalize(pieces[i], None, carry, (i, n, seq_len))
             pieces[i] = None
-            outs.append(self._piece_loss(xn, tgt[i]) if targets is not None else self.output.output(xn).float())
+            outs.append(self._piece_loss(xn, tgt[i]) if targets is not None else self.output.logits(xn))
         if targets is not None:
             return self._gather_losses(outs), None
         return torch.cat(outs, dim=1), None
@@ -283,7 +289,7 @@ class Mega(nn.Module):
         carry = None
         for i in range(n):
             xn, carry = self.output.normalize(pieces[i], None, carry, (i, n, seq_len, True))
-        logits = self.output.output(xn[:, -1:]).float()[:, 0]
+        logits = self.output.logits(xn[:, -1:])[:, 0]
         out_state = carry
         if cp > 1:
             src = get_chunk_parallel_ranks()[-1]

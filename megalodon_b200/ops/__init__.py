@@ -67,6 +67,13 @@ def linear_add(x: Tensor, w: Tensor, b: Optional[Tensor], addend: Tensor) -> Ten
     return reference.linear(x, w, b, None) + addend
 
 
+def linear_fp32_out(x: Tensor, w: Tensor) -> Tensor:
+    """x @ w^T as fp32, for results nobody differentiates: on the GPU 16-bit products leave as accumulated."""
+    if native_for(x) and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype:
+        return _cuda().linear_fp32_out(x, w)
+    return linear(x, w).float()
+
+
 def linear_group(x: Tensor, layers):
     """Several linear layers of one input: [(w, b, addend or None), ...] -> [x w^T + b (+ addend), ...]."""
     if native_for(x):

@@ -360,6 +360,13 @@ def linear(x: Tensor, w: Tensor, b: Optional[Tensor] = None, act: Optional[str] 
     return _Linear.apply(x, w, b, act)
 
 
+def linear_fp32_out(x: Tensor, w: Tensor) -> Tensor:
+    """x w^T in fp32 as accumulated, without autograd (logits)."""
+    x2 = x.reshape(-1, x.shape[-1])
+    y, _ = _gemm_gathering(x2, w, None, None, out_dtype=torch.float32)
+    return y.view(*x.shape[:-1], w.shape[0])
+
+
 def silu_bwd(g: Tensor, pre: Tensor) -> Tensor:
     """g * silu'(pre): two reads and one write."""
     _bump()

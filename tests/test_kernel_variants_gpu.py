@@ -200,3 +200,22 @@ def test_timestep_norm_segments(L, masked):
         assert _rel(a, r) < 2e-6
     for a, r in zip(dgot, dwant):
         assert _rel(a, r) < 2e-5, (a.shape, _rel(a, r))
+
+
+@pytest.mark.parametrize("tile", [64, 128, 256, 512])
+@pytest.mark.parametrize("M,N,K", [(100, 72, 136), (128, 64, 64), (300, 200, 264), (777, 264, 1032), (513, 768, 264)])
+def test_tiles(tile, M, N, K):
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(M)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, b, bias = _rand(M, K), _rand(N, K, scale=K ** -0.5), _rand(N)
+    ref = a.double() @ b.double().t() + bias.double()
+    for a_mn, b_mn in ((False, False), (False, True), (True, True)):
+        if a_mn and M % 8:
+            continue
+        A = a.t().contiguous() if a_mn else a
+        B = b.t().contiguous() if b_mn else b
+        for dtype, tol in ((0, 2e-6), (1, 2.0 ** -8)):      # fp32 leaves through the staging buffers too
+            out, _, rc = cuda_ops._C().gemm(A, B, None, bias, 0, a_mn, b_mn, False, dtype, 0, 1.0, err, tile=tile)
+            assert rc == 0 and err.item() == 0
+            assert _rel(out, ref) < tol
