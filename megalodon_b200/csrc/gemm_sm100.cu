@@ -1260,22 +1260,25 @@ static int launch_gemm_pair(const TmapArray& ta, const CUtensorMap& tb, const Ge
 static bool g_use_pair = true;
 
 // Which tile a product runs on: the one whose estimate is lowest,
-//   waves * max(k-blocks * t, e) + e,   t = max(latency of a ring round / its stages, bytes of resident tiles / rate).
-// Latency: a tile alone on its SM takes 0.30 us per k-block as a CTA pair (6 stages), 0.42 / 0.30 / 0.24 us as
-// 128 x 256 / 128 / 64 (4 / 6 / 8 stages; K from 1024 to 8192 at one tile per CTA, differences of event times).
-// Rate: what the big products draw from L2 in steady state, 64 KiB per pair and k-block at 0.45 us on 74 pairs.
-// `e` is a tile's epilogue, hidden behind the next tile's main loop except at the end.  Few wide tiles leave most
-// SMs without work and no tile is faster than its ring: 1024 x 512 x 512 is 8 pair tiles (20 us measured) and 64
-// tiles of 128 x 64.
+//   (waves - 1) * max(k-blocks * t, e) + k-blocks * t + c,   t = max(latency, bytes of the resident tiles / rate).
+// Constants from graph-replayed launches over 65 shapes from 100 x 256 x 512 to 8192 x 4096 x 256 in three layouts:
+//   latency per k-block   0.285 us as a CTA pair or 128 x 256, 0.19 as 128 x 128, 0.185 as 128 x 64 (what a ring of
+//                         6, 4, 6, 8 stages leaves of a memory latency)
+//   epilogue e            3.5 / 6.3 / 3.5 / 2.0 us a tile, hidden behind the next tile's loop except at the end
+//   start and end c       7.8 / 9.7 / 6.7 / 4.8 us
+//   rate                  18 TB/s out of L2 and memory together, which the narrow tiles reach first
+// Few wide tiles leave most SMs without work: 1024 x 512 x 512 takes 8.6 us in 8 pair tiles and 5.5 us in 64 tiles of
+// 128 x 64, 2048 x 1024 x 4096 26.1 us in pairs and 18.7 us as 128 x 128; 4000 x 2048 x 4096 48 us in pairs, 66 as
+// 128 x 128 and 93 as 128 x 64.
 static int pick_tile(const GemmParams& p, int num_sms) {
   const bool pair_ok = g_use_pair && p.M > BM && num_sms >= 2;
   if (p.a_parts > 1 || p.c_nparts > 1) return pair_ok ? kPairTile : 256;
-  const double nk = (p.K + BK - 1) / BK, rate = 10.5e6;      // bytes per us
-  struct Tile { int name, bm, bn; double lat, bytes, tail; };
-  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.30, 65536, 3.0},
-                        {256, BM, 256, 0.42, 49152, 3.0},
-                        {128, BM, 128, 0.30, 32768, 2.0},
-                        {64, BM, 64, 0.24, 24576, 1.5}};
+  const double nk = (p.K + BK - 1) / BK, rate = 18e6;      // bytes per us
+  struct Tile { int name, bm, bn; double lat, bytes, e, c; };
+  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.285, 65536, 3.5, 7.8},
+                        {256, BM, 256, 0.285, 49152, 6.3, 9.7},
+                        {128, BM, 128, 0.19, 32768, 3.5, 6.7},
+                        {64, BM, 64, 0.185, 24576, 2.0, 4.8}};
   int best = 256;
   double best_us = 1e30;
   for (const Tile& t : tiles) {
@@ -1283,10 +1286,9 @@ static int pick_tile(const GemmParams& p, int num_sms) {
     const long long n = (long long)((p.M + t.bm - 1) / t.bm) * ((p.N + t.bn - 1) / t.bn) * p.batch;
     const int slots = t.name == kPairTile ? num_sms / 2 : num_sms;
     const double resident = n < slots ? (double)n : (double)slots;
-    const double per_k = t.lat > t.bytes * resident / rate ? t.lat : t.bytes * resident / rate;
-    const double loop = nk * per_k > t.tail ? nk * per_k : t.tail;
-    const double us = (double)((n + slots - 1) / slots) * loop + t.tail;
-    if (us < best_us * 0.97) {
+    const double loop = nk * (t.lat > t.bytes * resident / rate ? t.lat : t.bytes * resident / rate);
+    const double us = (double)((n + slots - 1) / slots - 1) * (loop > t.e ? loop : t.e) + loop + t.c;
+    if (us < best_us) {
       best_us = us;
       best = t.name;
     }

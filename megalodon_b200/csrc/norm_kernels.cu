@@ -340,19 +340,22 @@ __global__ void norm_bwd_vec_kernel(const T* __restrict__ dy, const T* __restric
 }
 
 // out0[j] = sum over rows of ws[row][0][j] (and out1 from ws[row][1][j] when given), in the type of the parameter
-// whose gradient it is: a warp owns 32 adjacent columns (128-byte reads), the 8 warps of a CTA take every 8th
-// row and meet in shared memory.
+// whose gradient it is: a warp owns 32 adjacent columns (128-byte reads), the 32 warps of a CTA take every 32nd
+// row, all its loads in flight at once, and meet in shared memory (with 8 warps and four loads in flight the kernel
+// took 7.5 us for 296 rows whatever their width).
+constexpr int kFinishWarps = 32;
 template <typename O>
-__global__ void colsum_finish_kernel(const float* __restrict__ ws, int rows, int D, O* __restrict__ out0,
+__global__ void __launch_bounds__(kFinishWarps * 32)
+colsum_finish_kernel(const float* __restrict__ ws, int rows, int D, O* __restrict__ out0,
                                      O* __restrict__ out1) {
-  __shared__ float part[2][8][32];
+  __shared__ float part[2][kFinishWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
   const int sets = out1 != nullptr ? 2 : 1;
   float s0 = 0.f, s1 = 0.f;
   if (j < D) {
-#pragma unroll 4
-    for (int r = warp; r < rows; r += 8) {
+#pragma unroll 10
+    for (int r = warp; r < rows; r += kFinishWarps) {
       s0 += ws[((long long)r * sets) * D + j];
       if (out1 != nullptr) s1 += ws[((long long)r * sets + 1) * D + j];
     }
@@ -362,7 +365,7 @@ __global__ void colsum_finish_kernel(const float* __restrict__ ws, int rows, int
   __syncthreads();
   if (warp == 0 && j < D) {
 #pragma unroll
-    for (int w = 1; w < 8; ++w) {
+    for (int w = 1; w < kFinishWarps; ++w) {
       s0 += part[0][w][lane];
       s1 += part[1][w][lane];
     }
@@ -524,7 +527,7 @@ bool colsum_16bit(const void* g, long long M, int N, float* ws, void* out, int o
 }
 
 void colsum_finish(const float* ws, int rows, int D, void* out0, void* out1, int out_dtype, cudaStream_t st) {
-  MB_DISPATCH_DTYPE(out_dtype, (colsum_finish_kernel<scalar_t><<<(D + 31) / 32, 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(out_dtype, (colsum_finish_kernel<scalar_t><<<(D + 31) / 32, kFinishWarps * 32, 0, st>>>(
                                    ws, rows, D, (scalar_t*)out0, (scalar_t*)out1)));
 }
 

@@ -12,6 +12,7 @@ from typing import Optional
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad as _forward_ad
 
 from . import reference
 from ._ext import require
@@ -37,6 +38,29 @@ _GEMM_BACKEND = [os.environ.get("MEGALODON_B200_GEMM", "tcgen05")]
 _SKINNY_MAX_ROWS = 64
 _GEMV_MAX_K = 4096          # one row: the CUDA-core kernel needs no tensor maps and starts sooner
 _launches = [0]          # kernels launched by this framework (bench bookkeeping)
+
+
+class _NoGradContext:
+    """What a forward pass sees as its `ctx` when nothing is recorded."""
+    needs_input_grad = (False,) * 64
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    mark_non_differentiable = save_for_backward
+
+    def set_materialize_grads(self, value):
+        pass
+
+
+def _apply(fn, *args):
+    """`fn.apply(*args)`; where no gradient is recorded the forward pass is called as it is, which saves the
+    autograd machinery's ten-odd microseconds an operator (a 12-layer forward call on a short prompt has 200).
+    Function transforms, forward-mode duals and tracing keep the full route, and with it their errors."""
+    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
+            or torch.compiler.is_compiling() or torch.jit.is_tracing()):
+        return fn.apply(*args)
+    return fn.forward(_NoGradContext(), *args)
 
 
 def count_launches() -> int:
@@ -282,7 +306,7 @@ def linear_group(x: Tensor, layers):
             or any(w.dtype != x.dtype or w.shape[0] % 8 != 0 or not _tma_ok(w) or (a is not None and a.dtype != x.dtype)
                    for w, _, a in layers)):
         return [linear(x, w, b) if a is None else linear_add(x, w, b, a) for w, b, a in layers]
-    return list(_LinearGroup.apply(x, *[t for layer in layers for t in layer]))
+    return list(_apply(_LinearGroup, x, *[t for layer in layers for t in layer]))
 
 
 def _weight_grad(g: Tensor, x2: Tensor, w: Tensor, sink) -> Optional[Tensor]:
@@ -311,7 +335,7 @@ def linear_add(x: Tensor, w: Tensor, b: Optional[Tensor], addend: Tensor) -> Ten
             or w.shape[0] % 8 != 0 or rows <= 1 or not _tma_ok(x.reshape(-1, x.shape[-1]))):
         # (one row stays on the weight-streaming kernel behind `linear`)
         return linear(x, w, b) + addend
-    return _LinearAdd.apply(x, w, b, addend)
+    return _apply(_LinearAdd, x, w, b, addend)
 
 
 def ensure_gathered(w: Tensor) -> Tensor:
@@ -357,7 +381,7 @@ class _Linear(torch.autograd.Function):
 def linear(x: Tensor, w: Tensor, b: Optional[Tensor] = None, act: Optional[str] = None) -> Tensor:
     if x.dtype == torch.float32:
         return reference.linear(x, w, b, act)
-    return _Linear.apply(x, w, b, act)
+    return _apply(_Linear, x, w, b, act)
 
 
 def linear_fp32_out(x: Tensor, w: Tensor) -> Tensor:
@@ -390,7 +414,7 @@ class _SwiGLU(torch.autograd.Function):
 
 
 def swiglu(a: Tensor, b: Tensor) -> Tensor:
-    return _SwiGLU.apply(a, b)
+    return _apply(_SwiGLU, a, b)
 
 
 # ----------------------------------------------------------------------------- norms
@@ -417,7 +441,7 @@ class _RMSNorm(torch.autograd.Function):
 
 
 def rms_norm(x, weight, eps, weight_offset: float = 0.0):
-    return _RMSNorm.apply(x, weight, eps, weight_offset)
+    return _apply(_RMSNorm, x, weight, eps, weight_offset)
 
 
 class _LayerNorm(torch.autograd.Function):
@@ -446,7 +470,7 @@ class _LayerNorm(torch.autograd.Function):
 
 
 def layer_norm(x, weight, bias, eps, weight_offset: float = 0.0):
-    return _LayerNorm.apply(x, weight, bias, eps, weight_offset)
+    return _apply(_LayerNorm, x, weight, bias, eps, weight_offset)
 
 
 class _TimestepNorm(torch.autograd.Function):
@@ -488,7 +512,7 @@ class _TimestepNorm(torch.autograd.Function):
 
 def timestep_norm(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, num_groups, eps,
                   gamma_offset: float = 0.0):
-    return _TimestepNorm.apply(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, num_groups,
+    return _apply(_TimestepNorm, x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, num_groups,
                                eps, gamma_offset)
 
 
@@ -555,7 +579,7 @@ class _SequenceNorm(torch.autograd.Function):
 
 
 def sequence_norm(x, gamma, beta, padding_mask, num_groups, eps, length_last):
-    return _SequenceNorm.apply(x, gamma, beta, padding_mask, num_groups, eps, length_last)
+    return _apply(_SequenceNorm, x, gamma, beta, padding_mask, num_groups, eps, length_last)
 
 
 class _Dropout(torch.autograd.Function):
@@ -577,7 +601,7 @@ class _Dropout(torch.autograd.Function):
 
 
 def dropout(x, p):
-    return _Dropout.apply(x, float(p))
+    return _apply(_Dropout, x, float(p))
 
 
 # ----------------------------------------------------------------------------- CEMA
@@ -610,7 +634,7 @@ class _CEMACoeffs(torch.autograd.Function):
 
 
 def cema_coeffs(alpha, delta, theta, gamma, scale: float):
-    return _CEMACoeffs.apply(alpha, delta, theta, gamma, float(scale))
+    return _apply(_CEMACoeffs, alpha, delta, theta, gamma, float(scale))
 
 
 class _CEMA(torch.autograd.Function):
@@ -656,7 +680,7 @@ def cema(x, p, q, gamma, omega, hx, compute_last_state: bool):
     N = p.reshape(x.shape[-1], -1).shape[1]
     if N not in (1, 2, 4, 8, 16, 32):
         return reference.cema(x, p, q, gamma, omega, hx, compute_last_state)
-    return _CEMA.apply(x, p, q, gamma, omega, hx, compute_last_state)
+    return _apply(_CEMA, x, p, q, gamma, omega, hx, compute_last_state)
 
 
 class _EMAParameters(torch.autograd.Function):
@@ -687,7 +711,7 @@ class _EMAParameters(torch.autograd.Function):
 
 
 def ema_parameters(p, q, gamma, hx, length):
-    return _EMAParameters.apply(p, q, gamma, hx, length)
+    return _apply(_EMAParameters, p, q, gamma, hx, length)
 
 
 def ema_hidden(x, p, q, hx):
@@ -698,7 +722,7 @@ def ema_hidden(x, p, q, hx):
         return reference.ema_hidden(x, p, q, hx)
     zg = torch.zeros(D, N, dtype=torch.complex64, device=x.device)
     zo = torch.zeros(D, device=x.device)
-    _, h = _CEMA.apply(x.transpose(1, 2), p, q, zg, zo, hx, True)
+    _, h = _apply(_CEMA, x.transpose(1, 2), p, q, zg, zo, hx, True)
     return h
 
 
@@ -749,7 +773,7 @@ def fftconv(x, k):
     if not _fft_native_ok(x, x.shape[-1]) or x.dim() not in (2, 3) or k.dim() != 2:
         return reference.fftconv(x, k)
     x3 = x if x.dim() == 3 else x.unsqueeze(0)
-    y = _FFTConv.apply(x3, k)
+    y = _apply(_FFTConv, x3, k)
     return y if x.dim() == 3 else y.squeeze(0)
 
 
@@ -900,7 +924,7 @@ def set_fused_attention_softmax(on: bool) -> None:
 def attention(q, k, v, scale, dropout, use_causal_mask, training):
     if not _attention_native_ok(q, k, v):
         return reference.attention(q, k, v, scale, dropout, use_causal_mask, training)
-    return _Attention.apply(q, k, v, float(scale), float(dropout) if training else 0.0, bool(use_causal_mask))
+    return _apply(_Attention, q, k, v, float(scale), float(dropout) if training else 0.0, bool(use_causal_mask))
 
 
 class _AttentionSoftmax(torch.autograd.Function):
@@ -932,7 +956,7 @@ class _AttentionSoftmax(torch.autograd.Function):
 def attention_softmax(x, dropout, use_causal_mask, training):
     if x.shape[-1] > 8192:
         return reference.attention_softmax(x, dropout, use_causal_mask, training)
-    return _AttentionSoftmax.apply(x, float(dropout) if training else 0.0, bool(use_causal_mask))
+    return _apply(_AttentionSoftmax, x, float(dropout) if training else 0.0, bool(use_causal_mask))
 
 
 class _Rotary(torch.autograd.Function):
@@ -978,12 +1002,12 @@ def qk_rotary(z, gamma, beta, freqs_cis, head_dim: int):
     """z [B, L, S] normalised per head; gamma, beta [2, S]; freqs_cis [P, head_dim / 2] complex with the
     position of (b, l) being (b L + l) % P.  Returns rotated q, k [B, L, S]."""
     freqs = torch.view_as_real(freqs_cis.to(torch.complex64).contiguous())
-    return _QKRotary.apply(z, gamma, beta, freqs, int(head_dim))
+    return _apply(_QKRotary, z, gamma, beta, freqs, int(head_dim))
 
 
 def rotary(x, freqs_cis, conj=False):
     freqs = torch.view_as_real(freqs_cis.to(torch.complex64).contiguous())
-    return _Rotary.apply(x, freqs, conj)
+    return _apply(_Rotary, x, freqs, conj)
 
 
 # ----------------------------------------------------------------------------- loss / optimiser
@@ -1006,7 +1030,7 @@ class _CrossEntropy(torch.autograd.Function):
 
 
 def cross_entropy(logits, target, ignore_index=-100):
-    return _CrossEntropy.apply(logits, target, ignore_index)
+    return _apply(_CrossEntropy, logits, target, ignore_index)
 
 
 def adamw_step(param, grad, m, v, *, lr, beta1, beta2, eps, weight_decay, step, grad_scale=1.0, low=None,

@@ -120,8 +120,7 @@ class _FlatViews(torch.autograd.Function):
     def forward(ctx, leaf: torch.Tensor, unit: "FullyShardedDataParallel"):
         ctx.unit = unit
         ctx.set_materialize_grads(False)
-        base = leaf.detach()
-        return tuple(base[info.offset:info.offset + info.numel].view(info.shape) for info in unit._infos)
+        return tuple(unit._param_views(leaf.detach()))
 
     @staticmethod
     def backward(ctx, *grads):
@@ -202,6 +201,8 @@ class FullyShardedDataParallel(nn.Module):
 
         self._flatten(module, compute_device)
         self.compute_device = self.flat_param.device
+        self._cuts = None                                  # how the flat buffer is cut into parameters
+        self._plain_views: Optional[torch.Tensor] = None   # buffer whose untracked views the modules hold
         self._full: Optional[torch.Tensor] = None          # gathered compute-dtype buffer
         self._full_leaf: Optional[torch.Tensor] = None
         self._flat_grad: Optional[torch.Tensor] = None     # this iteration's gradients, compute dtype
@@ -459,15 +460,37 @@ class FullyShardedDataParallel(nn.Module):
         if self.world_size > 1 and self._full is not None:
             self._full.untyped_storage().resize_(0)
 
+    def _param_views(self, flat: torch.Tensor) -> List[torch.Tensor]:
+        """One view per parameter; the flat buffer is cut in one call, at the parameters and the gaps behind them."""
+        if self._cuts is None:
+            sizes, at, pos = [], [], 0
+            for info in self._infos:                      # ascending offsets
+                if info.offset > pos:
+                    sizes.append(info.offset - pos)
+                at.append(len(sizes))
+                sizes.append(info.numel)
+                pos = info.offset + info.numel
+            if pos < self._numel_padded:
+                sizes.append(self._numel_padded - pos)
+            self._cuts = (sizes, at)
+        sizes, at = self._cuts
+        pieces = flat.split_with_sizes(sizes)
+        return [pieces[i].view(info.shape) for i, info in zip(at, self._infos)]
+
     def _set_views(self, leaf: torch.Tensor, track: bool = False) -> None:
         """Hand the wrapped modules views of `leaf`.  With `track` the views come out of `_FlatViews`
         so their gradients flow back into the unit's flat gradient buffer."""
+        fused_infos = getattr(self, "_fused_infos", ())
         if track:
             views = _FlatViews.apply(leaf, self)
+            self._plain_views = None
         else:
-            views = [leaf[info.offset:info.offset + info.numel].view(info.shape) for info in self._infos]
+            if self._plain_views is leaf and not fused_infos:
+                return                       # the modules hold plain views of this very buffer already
+            views = self._param_views(leaf)
+            self._plain_views = leaf
         direct = track and leaf.is_cuda and leaf.dtype in (torch.bfloat16, torch.float16)
-        fused = {i.name for i in getattr(self, "_fused_infos", ())}
+        fused = {i.name for i in fused_infos}
         for info, v in zip(self._infos, views):
             if direct and len(info.shape) == 2:
                 v._wgrad_sink = _WgradSink(self, info)

@@ -219,3 +219,20 @@ def test_tiles(tile, M, N, K):
             out, _, rc = cuda_ops._C().gemm(A, B, None, bias, 0, a_mn, b_mn, False, dtype, 0, 1.0, err, tile=tile)
             assert rc == 0 and err.item() == 0
             assert _rel(out, ref) < tol
+
+
+def test_operators_without_gradients_match_the_recorded_ones():
+    """The short route under no_grad against the autograd function, and what the latter refuses stays refused."""
+    from megalodon_b200 import ops
+    torch.manual_seed(0)
+    x, w, b = _rand(70, 64), _rand(128, 64, scale=0.1), _rand(128)
+    rec = ops.linear(x.clone().requires_grad_(True), w, b, "silu")
+    with torch.no_grad():
+        got = ops.linear(x, w.clone().requires_grad_(True), b, "silu")
+    assert rec.requires_grad and not got.requires_grad and torch.equal(rec, got)
+    with torch.no_grad(), torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+        with pytest.raises(Exception):
+            ops.linear(dual, w, b, "silu")
+    with torch.no_grad(), pytest.raises(Exception):
+        torch.func.vmap(lambda r: ops.rms_norm(r, None, 1e-5))(x)
