@@ -1273,6 +1273,10 @@ static bool g_use_pair = true;
 static int pick_tile(const GemmParams& p, int num_sms) {
   const bool pair_ok = g_use_pair && p.M > BM && num_sms >= 2;
   if (p.a_parts > 1 || p.c_nparts > 1) return pair_ok ? kPairTile : 256;
+  // The causal products of one attention write and read the same scores at the granularity of their row tiles:
+  // what Q K^T skips above the diagonal P V must not contract.  All of them see the same number of rows, so the row
+  // tile may depend on nothing else.
+  if (p.mode != 0 && pair_ok) return kPairTile;
   const double nk = (p.K + BK - 1) / BK, rate = 18e6;      // bytes per us
   struct Tile { int name, bm, bn; double lat, bytes, e, c; };
   const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.285, 65536, 3.5, 7.8},

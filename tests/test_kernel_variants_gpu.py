@@ -68,7 +68,8 @@ def test_gradient_norm_and_scale(n):
 # lengths around the 8-column pieces, the 128-row tile (one CTA / CTA pair) and the 256-column tile; several
 # sequences and heads in one launch
 @pytest.mark.parametrize("B,L,H,dk,dv", [(1, 5, 2, 16, 24), (3, 37, 1, 64, 64), (2, 128, 2, 32, 40), (2, 129, 3, 64, 72),
-                                         (2, 257, 2, 128, 256), (3, 777, 1, 64, 128)])
+                                         (2, 257, 2, 128, 256), (3, 777, 1, 64, 128),
+                                         (1, 907, 2, 256, 2048)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_attention_any_length(B, L, H, dk, dv, causal):
     from megalodon_b200 import ops
@@ -77,6 +78,10 @@ def test_attention_any_length(B, L, H, dk, dv, causal):
     q, k, v = _rand(B, L, H, dk, scale=dk ** -0.25), _rand(B, L, H, dk, scale=dk ** -0.25), _rand(B, L, H, dv)
     g = _rand(B, L, H, dv)
     leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    # the score buffer is uninitialised memory: whatever a product reads without another having written it is NaN
+    torch.cuda.empty_cache()
+    poison = [torch.full((B * H * L * (-(-L // 128) * 128),), float("nan"), dtype=q.dtype, device="cuda") for _ in range(3)]
+    del poison
     out = ops.attention(*leaves, 0.7, 0.0, causal, True)
     out.backward(g)
     ref = [t.double().requires_grad_(True) for t in (q, k, v)]
