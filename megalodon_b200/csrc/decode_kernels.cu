@@ -167,13 +167,15 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   float* red = kn + p.dk;               // kDecThreads * 8: partial rows of the thread groups
   float* sc = red + kDecThreads * 8;    // scores of this split
   // In the chain `pos` and the older slots were written by launches long before the predecessor, which itself
-  // waited for them: they may be read, and the split's keys and values fetched into L2, ahead of the wait.
+  // waited for them: they may be read, and the split's keys and values fetched into L2, ahead of the wait - as
+  // long as all of them leave room for the products' weights there (16 tokens at 1.4 MB a layer 9.0 -> 8.6 ms, at
+  // 103 MB 13.9 -> 14.3 ms, hence the line between).
   if (p.z == nullptr) pdl_wait();
   const int at = (int)min(p.pos[0], (long long)p.C - 1);
   const int n = at + 1;
   const int per = keys_per_split(n, gridDim.x);
   const int lo = blockIdx.x * per, hi = min(n, lo + per);
-  if (lo < hi && warp == 0) {
+  if (lo < hi && warp == 0 && (long long)n * gridDim.y * (p.dk + p.dv) * (long long)sizeof(T) <= (32 << 20)) {
     const T* k0 = reinterpret_cast<const T*>(p.k_buf) + ((long long)bh * p.C + lo) * p.dk;
     const T* v0 = reinterpret_cast<const T*>(p.v_buf) + ((long long)bh * p.C + lo) * p.dv;
     for (int j = lane; j < hi - lo; j += 32) {

@@ -11,9 +11,10 @@
 // Up to four products over the same rows share a launch (the four projections of a MEGA layer), and a
 // product may carry a second weight for SwiGLU: y = silu(x w^T) * (x w2^T).
 //
-// In a chain of programmatic dependent launches the weight tiles of the first ring round are requested and the
-// rest of the CTA's weights prefetched into L2 before the previous kernel has finished: weights do not depend
-// on it, x does.
+// In a chain of programmatic dependent launches the weight tiles of the first ring round are requested before the
+// previous kernel has finished: weights do not depend on it, x does.  (Prefetching the rest into L2 as well gained
+// nothing at 1024 features and cost the 4096-wide layers a tenth: 16 tokens 10.9 -> 12.0 ms.  So did one CTA per SM
+// with twice the ring, 12.9 ms, and splitting until there are two CTAs per SM, 11.4 ms.)
 //
 // All waits are bounded; a timeout sets `*err` and the CTA unwinds.
 #include <cuda.h>
@@ -43,7 +44,7 @@ struct SkinnyMaps {
 struct SkinnyParams {
   SkinnyJob job[kSkinnyJobs];
   int tile0[kSkinnyJobs];                // first tile of each product
-  int njobs, M, mpad, split, stages, stage_bytes, tmem_cols, fmt, chained, red_bytes;
+  int njobs, M, mpad, split, stages, stage_bytes, tmem_cols, fmt, red_bytes;
   int* err;
 };
 
@@ -131,12 +132,6 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
         mbar_expect_tx(full_bar + i, tx_bytes);
         tma_load_4d(st, &maps.w[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0, 0);
         if (dual) tma_load_4d(st + w_bytes, &maps.w2[ji], full_bar + i, (kb0 + i) * kSkBK, n0, 0, 0);
-      }
-      if (p.chained) {
-        for (int i = first; i < total; ++i) {
-          tma_prefetch_4d(&maps.w[ji], (kb0 + i) * kSkBK, n0, 0, 0);
-          if (dual) tma_prefetch_4d(&maps.w2[ji], (kb0 + i) * kSkBK, n0, 0, 0);
-        }
       }
       pdl_wait();
       for (int i = 0; i < first; ++i)
@@ -335,7 +330,6 @@ int skinny_gemm(const SkinnyJob* jobs, int njobs, int M, int in_dtype, bool pdl,
   p.stages = budget / p.stage_bytes;
   if (p.stages > kSkMaxStages) p.stages = kSkMaxStages;
   const int ring = p.stages * p.stage_bytes;
-  p.chained = pdl ? 1 : 0;
   p.tmem_cols = 32;
   while (p.tmem_cols < p.mpad * (dual ? 2 : 1)) p.tmem_cols *= 2;
   const size_t smem = 1024 + ring + p.red_bytes + (2 * kSkMaxStages + 1) * 8 + 16;

@@ -284,13 +284,8 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// L2 prefetches of memory that a later part of the kernel reads (no data returned, so they may run ahead of
+// L2 prefetch of memory that a later part of the kernel reads (no data returned, so it may run ahead of
 // pdl_wait whatever the predecessor does)
-__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* m, int x, int y, int z, int w) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(reinterpret_cast<uint64_t>(m)),
-               "r"(x), "r"(y), "r"(z), "r"(w)
-               : "memory");
-}
 // `bytes` a multiple of 16, `p` 16-byte aligned
 __device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
