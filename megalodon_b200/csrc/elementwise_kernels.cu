@@ -13,6 +13,7 @@ __global__ void swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__
                                   long long n, long long n8) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
   for (long long i = tid; i < n8; i += stride) {
     float av[8], bv[8], o[8];
     load8(a + 8 * i, av);
@@ -29,6 +30,7 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ g, const T* __restrict__
                                   T* __restrict__ da, T* __restrict__ db, long long n, long long n8) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 2
   for (long long i = tid; i < n8; i += stride) {
     float gv[8], av[8], bv[8], oa[8], ob[8];
     load8(g + 8 * i, gv);
@@ -55,6 +57,7 @@ __global__ void silu_bwd_kernel(const T* __restrict__ g, const T* __restrict__ a
                                 long long n8) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
   for (long long i = tid; i < n8; i += stride) {
     float gv[8], av[8], oa[8];
     load8(g + 8 * i, gv);
