@@ -25,8 +25,8 @@ constexpr int kDecThreads = 256;
 // the sum of squares of the RMSNorm crosses CTAs (through distributed shared memory).  The EMA state is the
 // bulk of the traffic (8 N bytes a feature read and written, 20 N bytes of coefficients): a thread owns two
 // states (16 bytes of h, q and gamma each), the N / 2 threads of a feature add up with shuffles.
-template <typename T>
-__global__ void __launch_bounds__(kDecThreads)
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
   extern __shared__ float sm[];
   __shared__ float scratch[32];
@@ -39,24 +39,45 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
   float* gr = gm + gl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row0 = (long long)b * p.D + rank * dl;
-  if (p.hx != nullptr) {
-    // state and coefficients on their way into L2 while the previous kernel finishes
-    const long long f0 = (long long)rank * dl * p.N;
-    const int nb = dl * p.N * 4;                                     // bytes of one float per state
-    for (int i = threadIdx.x * 128; i < 2 * nb; i += kDecThreads * 128) {
-      const char* h = reinterpret_cast<const char*>(p.hx + 2 * ((long long)b * p.D * p.N + f0)) + i;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(h));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.q + 2 * f0) + i));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.gamma + 2 * f0) + i));
-      if (i < nb) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.p + f0) + i));
+  // State, coefficients and statistics were last written long before the predecessor, which waited for that itself: the
+  // first items' are loaded and the rest requested in L2 while it finishes.
+  const int per = p.N / 2;         // threads of a feature
+  const int total = p.hx != nullptr ? dl * per : 0;
+  constexpr int kBatch = 4;        // items of a thread whose loads are in flight together
+  const long long c0 = (long long)rank * dl * per;           // first item of this CTA
+  float4* hx = reinterpret_cast<float4*>(p.hx) + (long long)b * p.D * per + c0;
+  float4 h[kBatch], q[kBatch], ga[kBatch];
+  float2 pp[kBatch];
+  auto load_items = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = base + u * THREADS + threadIdx.x;
+      if (i < total) {
+        h[u] = hx[i];
+        q[u] = __ldg(reinterpret_cast<const float4*>(p.q) + c0 + i);
+        ga[u] = __ldg(reinterpret_cast<const float4*>(p.gamma) + c0 + i);
+        pp[u] = __ldg(reinterpret_cast<const float2*>(p.p) + c0 + i);
+      }
     }
+  };
+  load_items(0);
+  for (int i = kBatch * THREADS + threadIdx.x * 8; i < total; i += THREADS * 8) {     // 8 items: 128 bytes
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(hx + i));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4*>(p.q) + c0 + i));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4*>(p.gamma) + c0 + i));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float2*>(p.p) + c0 + i));
+  }
+  const double n0 = (double)p.count[b];
+  float u_old = 0.f, v_old = 0.f;                             // of this warp's first group
+  if (warp < gl) {
+    u_old = p.mean[(long long)b * p.G + rank * gl + warp];
+    v_old = p.var[(long long)b * p.G + rank * gl + warp];
   }
   pdl_wait();
   pdl_launch_dependents();
-  for (int i = threadIdx.x; i < dl; i += kDecThreads) xs[i] = to_f(reinterpret_cast<const T*>(p.x)[row0 + i]);
-  const double n0 = (double)p.count[b];
+  for (int i = threadIdx.x; i < dl; i += THREADS) xs[i] = to_f(reinterpret_cast<const T*>(p.x)[row0 + i]);
   __syncthreads();
-  for (int g = warp; g < gl; g += kDecThreads / 32) {
+  for (int g = warp; g < gl; g += THREADS / 32) {
     float s = 0.f;
     for (int i = lane; i < gs; i += 32) s += xs[g * gs + i];
     const float u = warp_sum(s) / gs;
@@ -69,7 +90,7 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
     if (lane == 0) {
       // the group's features are one sample of weight one, merged into the running population
       const long long gi = (long long)b * p.G + rank * gl + g;
-      const double u0 = p.mean[gi], v0 = p.var[gi], ud = u;
+      const double u0 = g == warp ? u_old : p.mean[gi], v0 = g == warp ? v_old : p.var[gi], ud = u;
       const double mean = (n0 * u0 + ud) / (n0 + 1.0);
       const double var = fmax((n0 * (v0 + u0 * u0) + ((double)v + ud * ud)) / (n0 + 1.0) - mean * mean, 0.0);
       p.mean[gi] = (float)mean;
@@ -79,7 +100,7 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < dl; i += kDecThreads) {
+  for (int i = threadIdx.x; i < dl; i += THREADS) {
     const int f = rank * dl + i, g = i / gs;
     const T t = from_f<T>((xs[i] - gm[g]) * gr[g] * (to_f(reinterpret_cast<const T*>(p.w)[f]) + 1.f) +
                           to_f(reinterpret_cast<const T*>(p.b)[f]));
@@ -95,37 +116,31 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
     return;
   }
   __syncthreads();
-  const int per = p.N / 2;         // threads of a feature
-  const int total = dl * per;
   float sq = 0.f;
-#pragma unroll 4
-  for (int base = 0; base < total; base += kDecThreads) {
-    const int i = base + threadIdx.x;
-    const bool on = i < total;
-    const int fl = on ? i / per : 0, s = i % per;
-    float acc = 0.f;
-    const int f = rank * dl + fl;
-    if (on) {
-      const long long c = (long long)f * per + s;
-      float4* hp = reinterpret_cast<float4*>(p.hx) + (long long)b * p.D * per + c;
-      const float4 h = *hp;
-      const float4 q = __ldg(reinterpret_cast<const float4*>(p.q) + c);
-      const float4 ga = __ldg(reinterpret_cast<const float4*>(p.gamma) + c);
-      const float2 pp = __ldg(reinterpret_cast<const float2*>(p.p) + c);
+  for (int base = 0; base < total; base += kBatch * THREADS) {
+    if (base > 0) load_items(base);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = base + u * THREADS + threadIdx.x;
+      const bool on = i < total;
+      const int fl = on ? i / per : 0;
+      float acc = 0.f;
       const float t = ts[fl];
-      float4 n;
-      n.x = fmaf(q.x, h.x, fmaf(-q.y, h.y, pp.x * t));
-      n.y = fmaf(q.x, h.y, q.y * h.x);
-      n.z = fmaf(q.z, h.z, fmaf(-q.w, h.w, pp.y * t));
-      n.w = fmaf(q.z, h.w, q.w * h.z);
-      *hp = n;
-      acc = ga.x * n.x - ga.y * n.y + ga.z * n.z - ga.w * n.w;
-    }
-    for (int o = per / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (on && s == 0) {
-      const float y = to_f(from_f<T>(fmaf(to_f(reinterpret_cast<const T*>(p.omega)[f]), ts[fl], acc)));
-      xs[fl] = y;
-      sq = fmaf(y, y, sq);
+      if (on) {
+        float4 n;
+        n.x = fmaf(q[u].x, h[u].x, fmaf(-q[u].y, h[u].y, pp[u].x * t));
+        n.y = fmaf(q[u].x, h[u].y, q[u].y * h[u].x);
+        n.z = fmaf(q[u].z, h[u].z, fmaf(-q[u].w, h[u].w, pp[u].y * t));
+        n.w = fmaf(q[u].z, h[u].w, q[u].w * h[u].z);
+        hx[i] = n;
+        acc = ga[u].x * n.x - ga[u].y * n.y + ga[u].z * n.z - ga[u].w * n.w;
+      }
+      for (int o = per / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (on && i % per == 0) {
+        const float y = to_f(from_f<T>(fmaf(to_f(reinterpret_cast<const T*>(p.omega)[rank * dl + fl]), t, acc)));
+        xs[fl] = y;
+        sq = fmaf(y, y, sq);
+      }
     }
   }
   sq = block_sum(sq, scratch);     // (its barriers also publish xs)
@@ -136,7 +151,7 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
     for (int r = 0; r < cl; ++r) sq += csum[r];
   }
   const float rstd = rsqrtf(sq / p.D + p.rms_eps);
-  for (int i = threadIdx.x; i < dl; i += kDecThreads) {
+  for (int i = threadIdx.x; i < dl; i += THREADS) {
     const int f = rank * dl + i;
     float v = xs[i] * rstd;
     if (p.rms_w != nullptr) v *= to_f(reinterpret_cast<const T*>(p.rms_w)[f]) + 1.f;
@@ -150,13 +165,14 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
 __device__ __forceinline__ int keys_per_split(int n, int splits) { return max(8, (n + splits - 1) / splits); }
 
 // CTA = (split, sequence x head).  A split reads its keys once (a warp per key) and its value rows once
-// (16-byte pieces, eight rows in flight per thread), and leaves max, sum and the un-normalised fp32 row.  The
+// (16-byte pieces; eight rows in flight per thread while the eight before them are added up), and leaves max, sum and the un-normalised fp32 row.  The
 // number of splits is fixed by the buffers' shape (about two CTAs per SM), the keys per split by the
 // position, so the launch can sit in a CUDA graph; splits beyond the filled slots leave at once.
 // Before: one CTA per 256 value columns walked all keys with 2-byte loads - 177 us at 4 heads, 1100 keys,
-// d_v 2048 (18 MB of values).
+// d_v 2048 (18 MB of values), now 14.6 with the combination; 16 sequences of 2 heads, 700 keys (103 MB): 31.5 us
+// (54.5 with eight rows in flight and nothing behind them).
 template <typename T>
-__global__ void __launch_bounds__(kDecThreads)
+__global__ void __launch_bounds__(kDecThreads, 2)
 decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   extern __shared__ float sm[];
   __shared__ float scratch[32];
@@ -223,6 +239,20 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
     const T* qr = reinterpret_cast<const T*>(p.q) + (long long)bh * p.dk;
     for (int i = tid; i < p.dk; i += kDecThreads) qs[i] = to_f(qr[i]);
   }
+  // The first value rows of the first column block are under way while the scores are computed.
+  const T* vnew = fused ? reinterpret_cast<const T*>(p.v_new) + (long long)bh * p.dv : nullptr;
+  const int ct0 = min(kDecThreads, p.dv / 8), ng0 = kDecThreads / ct0, grp0 = tid / ct0;
+  const int c0 = (tid - grp0 * ct0) * 8;
+  auto load_rows = [&](uint4 (&raw)[8], int j0, int step, int c, bool on) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int j = j0 + u * step;
+      raw[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (on && j < hi) raw[u] = *reinterpret_cast<const uint4*>(mine && j == at ? vnew + c : vrow + (long long)j * p.dv + c);
+    }
+  };
+  uint4 next[8];
+  load_rows(next, lo + grp0, ng0, c0, grp0 < ng0);
   __syncthreads();
   for (int j0 = lo + warp * 4; j0 < hi; j0 += kDecThreads / 32 * 4) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -266,21 +296,18 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   const long long part = (long long)bh * gridDim.x + blockIdx.x;
   if (tid == 0) reinterpret_cast<float2*>(p.part_ml)[part] = make_float2(m, sum);
   float* dst = p.part_acc + part * p.dv;
-  const T* vnew = fused ? reinterpret_cast<const T*>(p.v_new) + (long long)bh * p.dv : nullptr;
   for (int col0 = 0; col0 < p.dv; col0 += kDecThreads * 8) {
     const int ct = min(kDecThreads, (p.dv - col0) / 8);     // threads across the columns
     const int ng = kDecThreads / ct;                        // groups of them, each every ng-th key
     const int grp = tid / ct, c = col0 + (tid - grp * ct) * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (grp < ng) {
+      if (col0 > 0) load_rows(next, lo + grp, ng, c, true);
       for (int j0 = lo + grp; j0 < hi; j0 += ng * 8) {
         uint4 raw[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int j = j0 + u * ng;
-          raw[u] = make_uint4(0u, 0u, 0u, 0u);
-          if (j < hi) raw[u] = *reinterpret_cast<const uint4*>(mine && j == at ? vnew + c : vrow + (long long)j * p.dv + c);
-        }
+        for (int u = 0; u < 8; ++u) raw[u] = next[u];
+        load_rows(next, j0 + ng * 8, ng, c, true);       // (nothing beyond the split's last key)
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int j = j0 + u * ng;
@@ -397,12 +424,12 @@ decode_layer_norm_kernel(const T* __restrict__ x, const T* __restrict__ w, const
   }
 }
 
-template <typename... KArgs, typename... Args>
+template <int THREADS = kDecThreads, typename... KArgs, typename... Args>
 cudaError_t launch_link(void (*kern)(KArgs...), dim3 grid, size_t smem, int cluster, bool pdl, cudaStream_t st,
                         Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(kDecThreads, 1, 1);
+  cfg.blockDim = dim3(THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -436,10 +463,19 @@ int decode_norm_ema(const DecodeNormEma& p, int B, int dtype, bool pdl, cudaStre
   while (cl > 1 && p.G % cl != 0) cl /= 2;
   const size_t smem = sizeof(float) * (2 * (p.D / cl) + 2 * (p.G / cl));
   cudaError_t e = cudaSuccess;
+  // Few rows: 512 threads, one CTA per SM.  A cluster of eight such CTAs takes half of a GPC, so from nine rows on
+  // some would wait for a second wave and 256 threads, two CTAs per SM, are the better ones (4096 features, one row:
+  // 9.4 against 14.2 us; 2048 features, 16 rows: 12.9 against 10.0 us).
   MB_DISPATCH_16BIT(dtype, {
-    auto kern = decode_norm_ema_kernel<scalar_t>;
-    if (smem > 40 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = launch_link(kern, dim3(B * cl), smem, cl, pdl, st, p, cl);
+    auto wide = decode_norm_ema_kernel<scalar_t, 512>;
+    auto narrow = decode_norm_ema_kernel<scalar_t, 256>;
+    if (smem > 40 * 1024) {
+      e = cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    }
+    if (e == cudaSuccess)
+      e = B <= 8 ? launch_link<512>(wide, dim3(B * cl), smem, cl, pdl, st, p, cl)
+                 : launch_link<256>(narrow, dim3(B * cl), smem, cl, pdl, st, p, cl);
   });
   return e == cudaSuccess ? 0 : -3;
 }

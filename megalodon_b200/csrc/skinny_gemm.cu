@@ -320,14 +320,18 @@ int skinny_gemm(const SkinnyJob* jobs, int njobs, int M, int in_dtype, bool pdl,
     if (!make_tmap_4d(&maps.x[i], j.x, j.K, M, 1, 1, j.ldx, 0, 0, kSkBK, p.mpad, in_dtype)) return -4;
   }
   p.stage_bytes = (dual ? 2 : 1) * kSkRows * kSkBK * 2 + p.mpad * kSkBK * 2;
-  // K is split until the tiles cover every SM; at least two k-blocks are left to each CTA
+  // K is split until the tiles cover every SM; at least two k-blocks are left to each CTA.  Two CTAs share an SM as
+  // long as a ring of at least four stages fits half of its shared memory.  Where it does not (SwiGLU, whose stages
+  // hold two weight tiles), the CTAs have to fit one per SM: a second wave of a few costs as much as the first
+  // (2 x 2560 x 1024 weights: 160 CTAs 8.9 us, 80 CTAs 5.1 us).
+  const int accs = dual ? 2 : 1, red_max = accs * p.mpad * kSkRows * 4;
+  const bool shared_sm = 4 * p.stage_bytes <= 110 * 1024 - red_max;
   p.split = 1;
-  while (p.split < 8 && tiles * p.split < num_sms && min_nk >= 4 * p.split) p.split *= 2;
-  p.red_bytes = p.split > 1 ? (dual ? 2 : 1) * p.mpad * kSkRows * 4 : 0;
-  // two CTAs share an SM as long as a ring of at least four stages fits half of its shared memory
-  const int half = 110 * 1024 - p.red_bytes, whole = 224 * 1024 - p.red_bytes;
-  const int budget = 4 * p.stage_bytes <= half ? half : whole;
-  p.stages = budget / p.stage_bytes;
+  while (p.split < 8 && min_nk >= 4 * p.split &&
+         (shared_sm ? tiles * p.split < num_sms : 2 * tiles * p.split <= num_sms))
+    p.split *= 2;
+  p.red_bytes = p.split > 1 ? red_max : 0;
+  p.stages = ((shared_sm ? 110 : 224) * 1024 - p.red_bytes) / p.stage_bytes;
   if (p.stages > kSkMaxStages) p.stages = kSkMaxStages;
   const int ring = p.stages * p.stage_bytes;
   p.tmem_cols = 32;

@@ -58,14 +58,15 @@ def test_few_row_rule_agrees_with_the_tiles():
     cuda_ops.check_kernel_errors()
 
 
-@pytest.mark.parametrize("D,G,N,B", [(512, 32, 16, 1), (1024, 32, 16, 3), (96, 3, 4, 2), (4096, 64, 16, 2), (64, 1, 32, 1)])
+@pytest.mark.parametrize("D,G,N,B", [(512, 32, 16, 1), (1024, 32, 16, 3), (96, 3, 4, 2), (4096, 64, 16, 2), (64, 1, 32, 1),
+                                     (2048, 32, 16, 9), (8192, 8, 32, 1)])
 def test_decode_norm_ema(D, G, N, B):
     from megalodon_b200.ops import cuda_ops, reference
     torch.manual_seed(D)
     dev = "cuda"
     x = torch.randn(B, D, device=dev).bfloat16()
     w, b, rw, omega = (torch.randn(D, device=dev).mul_(0.1).bfloat16() for _ in range(4))
-    count = torch.tensor([0, 5, 1000][:B], device=dev)
+    count = torch.tensor(([0, 5, 1000] * 3)[:B], device=dev)
     mean, var = torch.randn(B, G, device=dev) * 0.1, torch.rand(B, G, device=dev) + 0.5
     p = torch.rand(D, N, device=dev)
     q = torch.polar(torch.rand(D, N, device=dev), torch.randn(D, N, device=dev))
