@@ -81,9 +81,9 @@ def main():
     add("swiglu bwd", lambda: ext.swiglu_bwd(g3, a1, a2), 5 * ef)
     s = torch.randn(4, T, T, device=dev).to(bf)
     es = 2 * 4 * T * T
-    add("causal softmax fwd (in place)", lambda: ext.attn_softmax_fwd(s, T, T, True, 0.0, 0, 0), es)   # reads + writes the lower triangle
+    add("causal softmax fwd (in place)", lambda: ext.attn_softmax_fwd(s, T, T, True, 0.0, 0, 0, True), es)   # reads + writes the lower triangle
     ds = torch.randn(4, T, T, device=dev).to(bf)
-    add("causal softmax bwd (in place)", lambda: ext.attn_softmax_bwd(s, ds, T, T, True), es * 3 // 2)
+    add("causal softmax bwd (in place)", lambda: ext.attn_softmax_bwd(s, ds, T, T, True, True), es * 3 // 2)
     print(f"{'op':32s} {'us':>9s} {'MB':>9s} {'GB/s':>9s}  of {kind} {peak:.0f} GB/s")
     for name, us, mb, gbs in rows:
         print(f"{name:32s} {us:9.1f} {mb:9.1f} {gbs:9.0f}  {gbs / peak:5.2f}")

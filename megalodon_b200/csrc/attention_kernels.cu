@@ -9,10 +9,12 @@
 // dS = P * (dP - sum(P * dP)) needs no mask.
 //
 // Layout: `rows` rows of length L2 with row stride `ld`; row index modulo L1 is
-// the query position.  The forward pass also writes zeros to the masked columns
-// up to the next multiple of 256, because the causal GEMMs that follow read
-// whole diagonal tiles of up to 256 rows; columns further right are never read by them
-// and are left untouched (they may hold uninitialised scores).
+// the query position.  Masked columns are written as zeros.  With `tile` > 0 only
+// those up to the next multiple of `tile` are: the causal GEMMs around a square
+// block read whole diagonal tiles of at most that many rows, and what lies further
+// right (possibly uninitialised scores) is never read.  Everything else - blocks with
+// L1 != L2, whose products run over all columns, and the operator by itself - takes
+// whole rows (`tile` 0).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -20,8 +22,12 @@ namespace mb {
 namespace {
 
 constexpr int kSmThreads = 256;
-constexpr int kCausalTile = 256;      // row extent of the largest GEMM tile that reads the diagonal blocks
 constexpr int kSmMaxPerThread = 32;   // rows up to 8192 columns
+
+// columns of a row that are written: n visible ones and the masked ones that must read as 0
+__device__ __forceinline__ int written_columns(int n, int L2, bool causal, int tile) {
+  return causal && tile > 0 ? min(L2, (n + tile - 1) / tile * tile) : L2;
+}
 
 // Philox4x32-10 counter-based generator (Salmon et al. 2011): 4 x 32 random bits per counter.
 __device__ __forceinline__ uint4 philox4x32(uint4 ctr, uint2 key) {
@@ -49,13 +55,13 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
 
 template <typename T>
 __global__ void attn_softmax_fwd_kernel(T* __restrict__ s, float* __restrict__ lse, int L1, int L2,
-                                        long long ld, bool causal, float drop_p, unsigned long long seed,
-                                        unsigned long long offset) {
+                                        long long ld, bool causal, int tile, float drop_p,
+                                        unsigned long long seed, unsigned long long offset) {
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
   const int n = causal ? max(0, min(L2, L2 - L1 + pos + 1)) : L2;      // visible columns
-  const int zero_to = causal ? min(L2, ((n + kCausalTile - 1) / kCausalTile) * kCausalTile) : L2;  // masked columns that must read as 0
+  const int zero_to = written_columns(n, L2, causal, tile);
   T* sr = s + row * ld;
   float v[kSmMaxPerThread];
   float m = -INFINITY;
@@ -92,12 +98,12 @@ __global__ void attn_softmax_fwd_kernel(T* __restrict__ s, float* __restrict__ l
 
 template <typename T>
 __global__ void attn_softmax_bwd_kernel(const T* __restrict__ p, T* __restrict__ dp, int L1, int L2, long long ld,
-                                        bool causal) {
+                                        bool causal, int tile) {
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
   const int n = causal ? max(0, min(L2, L2 - L1 + pos + 1)) : L2;
-  const int zero_to = causal ? min(L2, ((n + kCausalTile - 1) / kCausalTile) * kCausalTile) : L2;
+  const int zero_to = written_columns(n, L2, causal, tile);
   const T* pr = p + row * ld;
   T* dr = dp + row * ld;
   float pv[kSmMaxPerThread], gv[kSmMaxPerThread];
@@ -124,18 +130,18 @@ __global__ void attn_softmax_bwd_kernel(const T* __restrict__ p, T* __restrict__
 
 // 16-byte variants: a thread owns up to kSmVecPerThread groups of 8 consecutive columns.  Requires
 // L2 % 8 == 0, ld % 8 == 0 and a 16-byte aligned base, so every group is either entirely inside or
-// entirely outside [0, zero_to) (zero_to is a multiple of 128 or L2 itself).
+// entirely outside [0, zero_to) (`tile` is a multiple of 8 too).
 constexpr int kSmVecPerThread = kSmMaxPerThread / 8;
 
 template <typename T>
 __global__ void attn_softmax_fwd_vec_kernel(T* __restrict__ s, float* __restrict__ lse, int L1, int L2,
-                                            long long ld, bool causal, float drop_p, unsigned long long seed,
-                                            unsigned long long offset) {
+                                            long long ld, bool causal, int tile, float drop_p,
+                                            unsigned long long seed, unsigned long long offset) {
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
   const int n = causal ? max(0, min(L2, L2 - L1 + pos + 1)) : L2;
-  const int zero_to = causal ? min(L2, ((n + kCausalTile - 1) / kCausalTile) * kCausalTile) : L2;
+  const int zero_to = written_columns(n, L2, causal, tile);
   T* sr = s + row * ld;
   float v[kSmVecPerThread][8];
   float m = -INFINITY;
@@ -187,12 +193,12 @@ __global__ void attn_softmax_fwd_vec_kernel(T* __restrict__ s, float* __restrict
 
 template <typename T>
 __global__ void attn_softmax_bwd_vec_kernel(const T* __restrict__ p, T* __restrict__ dp, int L1, int L2,
-                                            long long ld, bool causal) {
+                                            long long ld, bool causal, int tile) {
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
   const int n = causal ? max(0, min(L2, L2 - L1 + pos + 1)) : L2;
-  const int zero_to = causal ? min(L2, ((n + kCausalTile - 1) / kCausalTile) * kCausalTile) : L2;
+  const int zero_to = written_columns(n, L2, causal, tile);
   const T* pr = p + row * ld;
   T* dr = dp + row * ld;
   float pv[kSmVecPerThread][8], gv[kSmVecPerThread][8];
@@ -280,29 +286,29 @@ void attn_bwd_prep(const void* dout, const void* out, const float* rowsum, void*
                                dv)));
 }
 
-void attn_softmax_fwd(void* s_inout, float* lse, long long rows, int L1, int L2, long long ld, bool causal,
+void attn_softmax_fwd(void* s_inout, float* lse, long long rows, int L1, int L2, long long ld, bool causal, int tile,
                       float dropkey_p, unsigned long long seed, unsigned long long offset, int dtype,
                       cudaStream_t st) {
   if (rows == 0) return;
   if (softmax_vec_ok(s_inout, L2, ld, dtype)) {
     MB_DISPATCH_DTYPE(dtype, (attn_softmax_fwd_vec_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
-                                 (scalar_t*)s_inout, lse, L1, L2, ld, causal, dropkey_p, seed, offset)));
+                                 (scalar_t*)s_inout, lse, L1, L2, ld, causal, tile, dropkey_p, seed, offset)));
     return;
   }
   MB_DISPATCH_DTYPE(dtype, (attn_softmax_fwd_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
-                               (scalar_t*)s_inout, lse, L1, L2, ld, causal, dropkey_p, seed, offset)));
+                               (scalar_t*)s_inout, lse, L1, L2, ld, causal, tile, dropkey_p, seed, offset)));
 }
 
 void attn_softmax_bwd(const void* p, void* dp_inout, long long rows, int L1, int L2, long long ld, bool causal,
-                      int dtype, cudaStream_t st) {
+                      int tile, int dtype, cudaStream_t st) {
   if (rows == 0) return;
   if (softmax_vec_ok(p, L2, ld, dtype) && (reinterpret_cast<uintptr_t>(dp_inout) & 31) == 0) {
     MB_DISPATCH_DTYPE(dtype, (attn_softmax_bwd_vec_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
-                                 (const scalar_t*)p, (scalar_t*)dp_inout, L1, L2, ld, causal)));
+                                 (const scalar_t*)p, (scalar_t*)dp_inout, L1, L2, ld, causal, tile)));
     return;
   }
   MB_DISPATCH_DTYPE(dtype, (attn_softmax_bwd_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
-                               (const scalar_t*)p, (scalar_t*)dp_inout, L1, L2, ld, causal)));
+                               (const scalar_t*)p, (scalar_t*)dp_inout, L1, L2, ld, causal, tile)));
 }
 
 }  // namespace mb

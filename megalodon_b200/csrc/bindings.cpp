@@ -712,27 +712,29 @@ Tensor fftconv_dk(const Tensor& dy, const Tensor& x) {
 }
 
 // ------------------------------------------------------------------ attention softmax (in place)
-// s [..., L1, L2] with contiguous last dim and uniform row stride; returns lse [rows] (fp32)
+// s [..., L1, L2] with contiguous last dim and uniform row stride; returns lse [rows] (fp32).  `tiles`: masked columns
+// are cleared only as far as the triangular products of a square block read them
 Tensor attn_softmax_fwd(Tensor& s, int64_t L1, int64_t L2, bool causal, double drop_p, int64_t seed,
-                        int64_t offset) {
+                        int64_t offset, bool tiles) {
   TORCH_CHECK(s.is_cuda() && s.stride(-1) == 1 && L2 <= 8192, "attention softmax: bad input");
   c10::cuda::CUDAGuard guard(s.device());
   const long long ld = s.stride(-2);
   const long long rows = s.numel() / s.size(-1);
   for (int d = 0; d + 2 < s.dim(); ++d) TORCH_CHECK(s.stride(d) == s.stride(d + 1) * s.size(d + 1), "rows must be evenly strided");
   Tensor lse = torch::empty({rows}, s.options().dtype(at::kFloat));
-  mb::attn_softmax_fwd(s.data_ptr(), lse.data_ptr<float>(), rows, (int)L1, (int)L2, ld, causal, (float)drop_p,
+  mb::attn_softmax_fwd(s.data_ptr(), lse.data_ptr<float>(), rows, (int)L1, (int)L2, ld, causal,
+                       tiles ? mb::kCausalTile : 0, (float)drop_p,
                        (unsigned long long)seed, (unsigned long long)offset, dtype_code(s), stream());
   return lse;
 }
 
-void attn_softmax_bwd(const Tensor& p, Tensor& dp, int64_t L1, int64_t L2, bool causal) {
+void attn_softmax_bwd(const Tensor& p, Tensor& dp, int64_t L1, int64_t L2, bool causal, bool tiles) {
   TORCH_CHECK(p.is_cuda() && dp.is_cuda() && p.stride(-1) == 1 && dp.stride(-1) == 1);
   TORCH_CHECK(p.stride(-2) == dp.stride(-2) && p.scalar_type() == dp.scalar_type() && L2 <= 8192);
   c10::cuda::CUDAGuard guard(p.device());
   const long long rows = p.numel() / p.size(-1);
-  mb::attn_softmax_bwd(p.data_ptr(), dp.data_ptr(), rows, (int)L1, (int)L2, p.stride(-2), causal, dtype_code(p),
-                       stream());
+  mb::attn_softmax_bwd(p.data_ptr(), dp.data_ptr(), rows, (int)L1, (int)L2, p.stride(-2), causal,
+                       tiles ? mb::kCausalTile : 0, dtype_code(p), stream());
 }
 
 // q [B, H, dk], k_buf [B, H, C, dk], v_buf [B, H, C, dv] (16-bit, contiguous), pos int64 device tensor [1] -> [B, H, dv]

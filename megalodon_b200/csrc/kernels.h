@@ -234,12 +234,14 @@ int gemm_pair_max_active_clusters();
 // out[i] = sum over `world` slots of slot_w[i] (slots are consecutive, `n` elements each)
 void reduce_slots(const void* slots, void* out, long long n, int world, int dtype, cudaStream_t st);
 
-// ---- attention softmax (attention_kernels.cu)
-void attn_softmax_fwd(void* s_inout, float* lse, long long rows, int L1, int L2, long long ld, bool causal,
+// ---- attention softmax (attention_kernels.cu); tile > 0 (a multiple of 8): masked columns beyond the next multiple
+// of it stay as they are
+constexpr int kCausalTile = 256;      // row extent of the largest GEMM tile that reads the diagonal blocks
+void attn_softmax_fwd(void* s_inout, float* lse, long long rows, int L1, int L2, long long ld, bool causal, int tile,
                       float dropkey_p, unsigned long long seed, unsigned long long offset, int dtype,
                       cudaStream_t st);
 void attn_softmax_bwd(const void* p, void* dp_inout, long long rows, int L1, int L2, long long ld, bool causal,
-                      int dtype, cudaStream_t st);
+                      int tile, int dtype, cudaStream_t st);
 // delta[b, h, l] = dO . O and dO' = dO / rowsum[b, h, l] over rows of dv values (dv a multiple of 8, 16-bit types)
 void attn_bwd_prep(const void* dout, const void* out, const float* rowsum, void* dos, float* delta, int B, int L,
                    int H, int dv, int dtype, cudaStream_t st);

@@ -853,7 +853,7 @@ class _Attention(torch.autograd.Function):
             gemm(qh, kh, out=Pv, mode=mode_s, alpha=scale)
             for i, part in enumerate([Pv] if drop_p == 0.0 else Pv.unbind(0)):    # (a sequence, a Philox offset)
                 _bump()
-                _C().attn_softmax_fwd(part, L1, L2, causal, drop_p, seed, offset + i)
+                _C().attn_softmax_fwd(part, L1, L2, causal, drop_p, seed, offset + i, square)
             gemm(Pv, vh, b_mn=True, out=oh, mode=mode_o)
             ctx.save_for_backward(q, k, v, P)
         ctx.meta = (scale, causal, square, L2, fused)
@@ -893,7 +893,7 @@ class _Attention(torch.autograd.Function):
             # dP = dO V^T
             gemm(doh, vh, out=dS, mode=m1)
             _bump()
-            _C().attn_softmax_bwd(Pv, dS, L1, L2, causal)      # dP <- dS in place
+            _C().attn_softmax_bwd(Pv, dS, L1, L2, causal, square)      # dP <- dS in place
         # dQ = scale dS K ; dK = scale dS^T Q
         gemm(dS, _heads_view(k), b_mn=True, out=_heads_view(dq), mode=m2, alpha=scale)
         gemm(dS, _heads_view(q), a_mn=True, b_mn=True, out=_heads_view(dk_), mode=m3, alpha=scale)
@@ -934,7 +934,7 @@ class _AttentionSoftmax(torch.autograd.Function):
         y = x.contiguous().clone()
         seed = int(torch.randint(0, 2 ** 62, (1,)).item()) if drop_p > 0.0 else 0
         _bump()
-        _C().attn_softmax_fwd(y, L1, L2, causal, drop_p, seed, 0)
+        _C().attn_softmax_fwd(y, L1, L2, causal, drop_p, seed, 0, False)
         ctx.save_for_backward(y)
         ctx.causal = causal
         return y
@@ -945,11 +945,7 @@ class _AttentionSoftmax(torch.autograd.Function):
         L1, L2 = y.shape[-2:]
         dx = g.contiguous().clone()
         _bump()
-        _C().attn_softmax_bwd(y, dx, L1, L2, ctx.causal)
-        if ctx.causal:       # columns the kernel does not visit carry the incoming gradient: clear them
-            r = torch.arange(L1, device=y.device).unsqueeze(-1)
-            c = torch.arange(L2, device=y.device).unsqueeze(0)
-            dx = dx.masked_fill(c > r + (L2 - L1), 0)
+        _C().attn_softmax_bwd(y, dx, L1, L2, ctx.causal, False)
         return dx, None, None
 
 

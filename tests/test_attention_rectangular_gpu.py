@@ -1,0 +1,84 @@
+"""Causal attention of fewer (or more) queries than keys, wider than one 256-column tile: every product of that
+route contracts whole rows, so a masked column that is not zero is a key from the future."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(got, want):
+    return ((got.double() - want.double()).norm() / want.double().norm()).item()
+
+
+def _rand(*s, dtype=torch.bfloat16, scale=1.0):
+    return (torch.randn(*s, device="cuda") * scale).to(dtype)
+
+
+def _hidden(L1, L2):
+    """True where query r may not see key c."""
+    return torch.arange(L2, device="cuda") > torch.arange(L1, device="cuda").unsqueeze(-1) + (L2 - L1)
+
+
+def _probs(s):
+    """Causal softmax in the dtype of s; a row without keys gives zeros."""
+    hide = _hidden(*s.shape[-2:])
+    return torch.softmax(s.masked_fill(hide, -1e30), -1) * ~hide
+
+
+# 600 new tokens behind 500 cached ones; an odd key count (scalar rows); a single short query block; more queries
+# than keys (the first rows see nothing)
+@pytest.mark.parametrize("B,L1,L2,H", [(2, 600, 1100, 2), (1, 333, 905, 1), (1, 2, 777, 2), (1, 24, 2048, 1), (1, 300, 264, 2)])
+def test_rectangular_causal_attention(B, L1, L2, H):
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(L2)
+    dk, dv = 32, 72
+    q, k = _rand(B, L1, H, dk, scale=dk ** -0.25), _rand(B, L2, H, dk, scale=dk ** -0.25)
+    v, g = _rand(B, L2, H, dv), _rand(B, L1, H, dv)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    torch.cuda.empty_cache()        # the score buffers are uninitialised memory: make that NaN
+    poison = [torch.full((B * H * L1 * (-(-L2 // 128) * 128),), float("nan"), dtype=q.dtype, device="cuda") for _ in range(3)]
+    del poison
+    out = ops.attention(*leaves, 0.7, 0.0, True, True)
+    out.backward(g)
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    p = _probs(torch.einsum("blhd,bmhd->bhlm", ref[0], ref[1]) * 0.7)
+    want = torch.einsum("bhlm,bmhd->blhd", p, ref[2])
+    want.backward(g.double())
+    # scores, probabilities, their gradients and the results are rounded to 8 bits once each
+    assert _rel(out, want) < 2.0 ** -6
+    for a, b in zip(leaves, ref):
+        assert _rel(a.grad, b.grad) < 2.0 ** -5
+    cuda_ops.check_kernel_errors()
+
+
+@pytest.mark.parametrize("slen,past", [(600, 500), (401, 300)])
+def test_unfused_model_against_a_cached_prefix(slen, past):
+    """Several tokens behind a cached prefix: the marker that stands for the additive mask, and the mask itself."""
+    from megalodon_b200.modules.moving_average_gated_attention import CAUSAL, _InnerAttention
+    torch.manual_seed(slen)
+    H, dk, dv, c, B = 2, 32, 64, 1200, 2
+    inner = _InnerAttention(dk, dv, H, c, 0.1, None).eval()
+    q, k, v = _rand(B, slen, H * dk, scale=0.5), _rand(B, slen, H * dk, scale=0.5), _rand(B, slen, H * dv)
+    kv = (_rand(B, past, H, dk, scale=0.5), _rand(B, past, H, dv), past)
+    assert inner.causal_mask(q, slen, past) is CAUSAL
+    mask = torch.full((1, 1, slen, slen + past), float("-inf"), device="cuda").triu(past + 1).bfloat16()
+    got, _ = inner(q, k, v, CAUSAL, None, kv)
+    want, _ = inner(q, k, v, mask, None, kv)
+    assert _rel(got, want) < 2.0 ** -6
+
+
+# the operator by itself: rows wider than a tile, vectorised and scalar, square and not
+@pytest.mark.parametrize("L1,L2", [(600, 600), (40, 700), (40, 701), (300, 40)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_softmax_operator_clears_masked_columns(L1, L2, dtype):
+    from megalodon_b200 import ops
+    torch.manual_seed(L2)
+    x, g = _rand(2, L1, L2, dtype=dtype), _rand(2, L1, L2, dtype=dtype)
+    a, r = x.clone().requires_grad_(True), x.double().requires_grad_(True)
+    y, want = ops.attention_softmax(a, 0.0, True, True), _probs(r)
+    y.backward(g)
+    want.backward(g.double())
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8
+    assert _rel(y, want) < tol and _rel(a.grad, r.grad) < 4 * tol      # (the gradient starts from the rounded y)
+    assert (y[:, _hidden(L1, L2)] == 0).all() and (a.grad[:, _hidden(L1, L2)] == 0).all()
