@@ -39,8 +39,9 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
   float* gr = gm + gl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row0 = (long long)b * p.D + rank * dl;
-  // State, coefficients and statistics were last written long before the predecessor, which waited for that itself: the
-  // first items' are loaded and the rest requested in L2 while it finishes.
+  // State and statistics were last written, and the coefficients computed, before the first link of the chain, which
+  // waits for everything ahead of it (the caller launches nothing that writes them between two links): the first items'
+  // are loaded and the rest requested in L2 while the predecessor finishes.
   const int per = p.N / 2;         // threads of a feature
   const int total = p.hx != nullptr ? dl * per : 0;
   constexpr int kBatch = 4;        // items of a thread whose loads are in flight together

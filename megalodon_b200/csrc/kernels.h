@@ -185,7 +185,9 @@ void fftconv_dk(const void* dy, const void* x, float* acc_spec, float* dk, long 
 bool gemv(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int N, int K, long long ldw, int act,
           int in_dtype, int out_dtype, cudaStream_t st);
 
-// ---- one token against a fixed-shape state (decode_kernels.cu); 16-bit activations and weights, fp32 state
+// ---- one token against a fixed-shape state (decode_kernels.cu); 16-bit activations and weights, fp32 state.  With `pdl`
+// state, statistics and coefficients are read ahead of the wait for the predecessor: nothing in the chain but the
+// link itself may write them
 struct DecodeNormEma {
   const void* x;                        // [B, D]
   const void *w, *b;                    // [D] TimestepNorm weight (applied as w + 1) and bias

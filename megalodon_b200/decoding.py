@@ -183,6 +183,13 @@ class DecodeSession:
         for dst, src in zip(self.out_norm, self.mega.output.final_norm.initial_stats(self.B, torch.float32)):
             dst.copy_(src)
 
+    @staticmethod
+    def _coefficients(a):
+        """p, q, gamma, omega of the layer's EMA as the kernels take them."""
+        p, q, gamma = a.cema.coeffs()
+        return [p.reshape(a.mdim, -1).float().contiguous(), torch.view_as_real(q.reshape(a.mdim, -1).contiguous()),
+                torch.view_as_real(gamma.reshape(a.mdim, -1).contiguous()), a.cema.omega.view(a.mdim)]
+
     def _native_step(self) -> Tensor:
         from .ops import cuda_ops
         from .ops._ext import require
@@ -191,7 +198,10 @@ class DecodeSession:
         if self._fresh:
             self._start_stats()
         table = torch.view_as_real(m.rope.get_freqs_cis(0, m.chunk_size))
-        keep = [table]               # what a captured graph reads besides the session's buffers and the weights
+        # The links of the chain read these ahead of their wait, so whatever computes them (a model just put in eval
+        # mode has none yet) is launched before the first link, which waits for all of it.
+        coeffs = [self._coefficients(_unwrap(layer).mega) for layer in m.layers]
+        self._keep = [table, coeffs]     # what a captured graph reads besides the session's buffers and the weights
 
         def products(xs, ws, biases, addends, acts, outs, w2=None):
             rc = C.skinny_gemm(xs, ws, [w2] if w2 is not None else [None] * len(xs), biases, addends, acts, outs, True,
@@ -206,14 +216,8 @@ class DecodeSession:
         for layer, st in zip(m.layers, self.layers):
             block = _unwrap(layer)
             a, f = block.mega, block.nffn
-            p, q, gamma = a.cema.coeffs()
-            coeffs = [p.reshape(a.mdim, -1).float().contiguous(),
-                      torch.view_as_real(q.reshape(a.mdim, -1).contiguous()),
-                      torch.view_as_real(gamma.reshape(a.mdim, -1).contiguous()),
-                      a.cema.omega.view(a.mdim)]
-            keep += coeffs
             count, mean, var = st["norm"]
-            C.decode_norm_ema(x, a.timenorm.weight, a.timenorm.bias, count, mean, var, b["t"], *coeffs,
+            C.decode_norm_ema(x, a.timenorm.weight, a.timenorm.bias, count, mean, var, b["t"], *coeffs[n],
                               torch.view_as_real(st["hx"]), a.rmsnorm.weight, b["mx"], None, 0, a.timenorm.eps,
                               a.rmsnorm.eps, n > 0)
             products([b["mx"], b["mx"], b["t"], b["mx"]], [a.wh1.weight, a.wr.weight, a.wv.weight, a.wz.weight],
@@ -234,7 +238,6 @@ class DecodeSession:
                           self.pos, m.chunk_size, norm.eps, 0.0, True)
         products([b["t"]], [m.output.output.weight], [None], [None], [0], [b["logits"]])
         cuda_ops._bump(9 * n + 2)
-        self._keep = keep
         return b["logits"]
 
     # ------------------------------------------------------------------ one token

@@ -157,3 +157,35 @@ def test_native_session_matches_cache_path(swiglu, B, D, H, share):
             assert _rel(sess.step(tok[:, i]), ref[:, -1]) < 3e-2, i
         assert sess._graph is not None
     cuda_ops.check_kernel_errors()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("training,use_graph", [(False, False), (True, False), (True, True)])
+def test_native_session_without_cached_coefficients(dtype, training, use_graph):
+    """A session on a model whose EMA coefficients nobody has computed yet - just put in eval mode, or left in training
+    mode, where every eager step and the captured graph compute them anew - against the growing cache."""
+    from megalodon_b200.config import ModelConf
+    from megalodon_b200.decoding import DecodeSession
+    from megalodon_b200.models.mega import build_model
+    from megalodon_b200.ops import cuda_ops
+    from megalodon_b200.utils import init_cache, set_random_seed
+    cfg = ModelConf(num_layers=4, model_dim=1024, num_heads=1, z_dim=128, value_dim=1024, ffn_hidden_dim=1024,
+                    chunk_size=64, vocab_size=520, swiglu=True, norm_num_groups=32, efficient_attn="fused")
+    set_random_seed(2)
+    model = build_model(cfg, dtype, False, False)
+    t = torch.bfloat16 if dtype == "bf16" else torch.float16
+    tok = torch.randint(0, 520, (2, 40), device="cuda")
+    model.train(training)
+    sess = DecodeSession(model, 2, t, use_graph=use_graph)
+    assert sess._native
+    got = [sess.step(tok[:, i]).clone() for i in range(8)]
+    assert model.training == training and (sess._graph is not None) == use_graph
+    model.eval()
+    cache = init_cache(2, model, t)
+    eps = 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
+    with torch.no_grad():
+        for i in range(8):
+            ref, cache = model(tok[:, i:i + 1], cache=cache)
+            # some ten roundings to `eps` a layer on either side, adding up like a random walk
+            assert _rel(got[i], ref[:, -1]) < 2 * (10 * cfg.num_layers) ** 0.5 * eps, i
+    cuda_ops.check_kernel_errors()
