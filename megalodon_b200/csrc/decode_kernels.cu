@@ -31,6 +31,7 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
   extern __shared__ float sm[];
   __shared__ float scratch[32];
   __shared__ float csum[8];
+  if (cl > 1) cluster_arrive();    // awaited before the first store into another CTA: by then all have started
   const int rank = blockIdx.x % cl, b = blockIdx.x / cl;
   const int dl = p.D / cl, gl = p.G / cl, gs = p.D / p.G;
   float* xs = sm;                 // dl: input, later the EMA output
@@ -109,7 +110,12 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
     ts[i] = to_f(t);
   }
   if (p.hx == nullptr) {           // the norm alone (before the vocabulary projection)
-    if (cl > 1) cluster_sync_all(); else __syncthreads();
+    if (cl > 1) {
+      cluster_wait();
+      cluster_sync_all();          // every CTA of the row has read the count
+    } else {
+      __syncthreads();
+    }
     if (rank == 0 && threadIdx.x == 0) {
       p.count[b] += 1;
       if (b == 0 && p.pos != nullptr) p.pos[0] = (p.pos[0] + 1) % p.chunk;
@@ -146,6 +152,7 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
   }
   sq = block_sum(sq, scratch);     // (its barriers also publish xs)
   if (cl > 1) {
+    cluster_wait();
     if (threadIdx.x < cl) st_cluster_f32(map_to_cta(smem_u32(csum + rank), threadIdx.x), sq);
     cluster_sync_all();
     sq = 0.f;

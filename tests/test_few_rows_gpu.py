@@ -189,3 +189,26 @@ def test_native_session_without_cached_coefficients(dtype, training, use_graph):
             # some ten roundings to `eps` a layer on either side, adding up like a random walk
             assert _rel(got[i], ref[:, -1]) < 2 * (10 * cfg.num_layers) ** 0.5 * eps, i
     cuda_ops.check_kernel_errors()
+
+
+@pytest.mark.parametrize("D,G,B", [(2048, 32, 64), (4096, 64, 40), (1024, 2, 64)])
+def test_decode_norm_ema_with_more_clusters_than_fit(D, G, B):
+    """Clusters that wait for room start late and one by one; every row still gets the whole row's sum of squares."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(D)
+    N = 16
+    x = torch.randn(B, D, device="cuda").bfloat16()
+    w, b, rw, omega = (torch.randn(D, device="cuda").mul_(0.1).bfloat16() for _ in range(4))
+    p, q = torch.rand(D, N, device="cuda"), torch.randn(D, N, 2, device="cuda") * 0.5
+    ga = torch.randn(D, N, 2, device="cuda")
+    t, mx = torch.empty_like(x), torch.empty_like(x)
+    for _ in range(20):
+        count = torch.zeros(B, dtype=torch.int64, device="cuda")
+        mean, var = torch.zeros(B, G, device="cuda"), torch.ones(B, G, device="cuda")
+        hx = torch.zeros(B, D, N, 2, device="cuda")
+        cuda_ops._C().decode_norm_ema(x, w, b, count, mean, var, t, p, q, ga, omega, hx, rw, mx, None, 0, 1e-5, 1e-5, False)
+        y = ((ga[..., 0].double() * p.double()).sum(-1) + omega.double()) * t.double()      # no past: h = p t
+        ref = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * (rw.double() + 1.0)
+        rows = (mx.double() - ref).norm(dim=1) / ref.norm(dim=1)
+        assert rows.max() < 2.0 ** -7, rows
+        assert (count == 1).all()
