@@ -203,14 +203,13 @@ class MovingAverageGatedAttention(nn.Module):
         self.znorm = FusedRMSNorm(self.z_head_dim, elementwise_affine=False, eps=norm_eps)
 
         init_fn = get_init_fn(init_mode)
-        # v carries a SiLU that is fused into the GEMM epilogue; the one of the gate r is taken where the gate is
-        # applied (`ops.swiglu`), so that neither r nor its input has to be written out a second time
+        # v and r carry a SiLU that is fused into the GEMM epilogue
         self.wv = ColumnParallelLinear(mdim, hdim, bias=True, input_is_parallel=True,
                                        gather_output=False, init_method=init_fn, activation="silu")
         self.wz = ColumnParallelLinear(mdim, zdim, bias=True, input_is_parallel=False,
                                        gather_output=False, init_method=init_fn, partition=z_partition)
         self.wr = ColumnParallelLinear(mdim, hdim, bias=True, input_is_parallel=False,
-                                       gather_output=False, init_method=init_fn)
+                                       gather_output=False, init_method=init_fn, activation="silu")
         self.wh1 = ColumnParallelLinear(mdim, mdim, bias=True, input_is_parallel=False,
                                         gather_output=False, init_method=init_fn)
         self.wh2 = RowParallelLinear(hdim, mdim, bias=False, input_is_parallel=True,
@@ -294,11 +293,11 @@ class MovingAverageGatedAttention(nn.Module):
         # the epilogues of the projections around the attention
         fused_adds = get_model_parallel_world_size() == 1 and not (self.training and self.dropout > 0.0)
         if fused_adds:
-            z, r, h = ops.linear_group(mx, [(self.wz.weight, self.wz.bias, None), (self.wr.weight, self.wr.bias, None),
+            z, r, h = ops.linear_group(mx, [(self.wz.weight, self.wz.bias, None),
+                                            (self.wr.weight, self.wr.bias, None, "silu"),
                                             (self.wh1.weight, self.wh1.bias, residual)])
         else:
             z, r = self.wz(mx), self.wr(mx)
-        # (r is the gate before its SiLU)
         z = z.view(bsz, seq_len, self.local_heads, self.z_head_dim)
         z = self.znorm(z).view(bsz, seq_len, -1)
         # q, k = rotary(z (gamma + 1) / sqrt(d) + beta): one kernel; positions are those of the chunk
@@ -307,7 +306,7 @@ class MovingAverageGatedAttention(nn.Module):
         v = self.wv(out_tsn)          # SiLU fused
 
         attn, cache_attn = self.inner_attention(q, k, v, mask, None, cache_attn)
-        attn = ops.memory_efficient_dropout(ops.swiglu(r, attn), self.hidden_dropout, self.training)
+        attn = ops.memory_efficient_dropout(attn * r, self.hidden_dropout, self.training)
 
         if fused_adds:
             out = ops.linear_add(attn, self.wh2.weight, None, h)

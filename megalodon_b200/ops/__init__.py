@@ -75,10 +75,14 @@ def linear_fp32_out(x: Tensor, w: Tensor) -> Tensor:
 
 
 def linear_group(x: Tensor, layers):
-    """Several linear layers of one input: [(w, b, addend or None), ...] -> [x w^T + b (+ addend), ...]."""
+    """Several linear layers of one input: [(w, b, addend or None[, act]), ...] -> [act(x w^T + b) (+ addend), ...]; a
+    layer with an activation takes no addend."""
+    layers = [layer if len(layer) == 4 else (*layer, None) for layer in layers]
+    assert not any(a is not None and act is not None for _, _, a, act in layers)
     if native_for(x):
         return _cuda().linear_group(x, layers)
-    return [reference.linear(x, w, b, None) if a is None else reference.linear(x, w, b, None) + a for w, b, a in layers]
+    return [reference.linear(x, w, b, act) if a is None else reference.linear(x, w, b, None) + a
+            for w, b, a, act in layers]
 
 
 def qk_rotary(z: Tensor, gamma: Tensor, beta: Tensor, freqs_cis: Tensor, head_dim: int):

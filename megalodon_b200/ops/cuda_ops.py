@@ -249,45 +249,57 @@ class _LinearAdd(torch.autograd.Function):
 
 
 class _LinearGroup(torch.autograd.Function):
-    """Several linear layers of one input, some with an addend: (x w_i^T + b_i [+ addend_i])_i.  Backward adds up
-    the input gradients in the epilogues of the data-gradient products, so the sum over the layers costs no
-    pass of its own.  Arguments after x: w, b, addend per layer."""
+    """Several linear layers of one input: (act_i(x w_i^T + b_i) [+ addend_i])_i, a layer with an activation having no
+    addend.  Backward adds up the input gradients in the epilogues of the data-gradient products, so the sum over the
+    layers costs no pass of its own.  Arguments after x: w, b, addend, act per layer."""
 
     @staticmethod
     def forward(ctx, x, *layers):
         x2 = x.reshape(-1, x.shape[-1])
-        ws, bs, adds = layers[0::3], layers[1::3], layers[2::3]
+        ws, bs, adds, acts = (layers[i::4] for i in range(4))
         outs = [torch.empty(*x.shape[:-1], w.shape[0], dtype=x.dtype, device=x.device) for w in ws]
         ys = [o.view(-1, o.shape[-1]) for o in outs]
         a2 = [None if a is None else a.reshape(-1, a.shape[-1]).contiguous() for a in adds]
+        pres = [None] * len(ws)
+        keep_pre = any(ctx.needs_input_grad) and any(acts)
         pending = any(getattr(w, "_gather_spec", None) is not None and w._gather_spec.pending for w in ws)
         rc = -1
-        if x2.shape[0] <= _SKINNY_MAX_ROWS and len(ws) <= 4 and not pending:
-            rc = _C().skinny_gemm([x2] * len(ws), list(ws), [None] * len(ws), list(bs), a2, [0] * len(ws), ys, False,
-                                  _err_flag(x.device))
+        if x2.shape[0] <= _SKINNY_MAX_ROWS and len(ws) <= 4 and not pending and not keep_pre:
+            rc = _C().skinny_gemm([x2] * len(ws), list(ws), [None] * len(ws), list(bs), a2,
+                                  [1 if act == "silu" else 0 for act in acts], ys, False, _err_flag(x.device))
             if rc not in (0, -1):
                 raise RuntimeError(f"few-row products: launch failed with code {rc}")
             _bump(1 if rc == 0 else 0)
         if rc != 0:
-            for w, b, a, y in zip(ws, bs, a2, ys):
-                _gemm_gathering(x2, w, b, None, out=y, **({} if a is None else {"softmax": dict(aux=a)}))
-        ctx.save_for_backward(x2, *ws)
+            for i, (w, b, a, act) in enumerate(zip(ws, bs, a2, acts)):
+                if act is not None and keep_pre:
+                    y, pres[i] = _gemm_gathering(x2, w, b, act, want_preact=True)
+                    outs[i] = y.view(outs[i].shape)
+                else:
+                    _gemm_gathering(x2, w, b, act, out=ys[i], **({} if a is None else {"softmax": dict(aux=a)}))
+        ctx.save_for_backward(x2, *ws, *[p for p in pres if p is not None])
         ctx.sinks = [getattr(w, "_wgrad_sink", None) for w in ws]
         ctx.bias_dtypes = [None if b is None else b.dtype for b in bs]
+        ctx.has_pre = [p is not None for p in pres]
         ctx.x_shape = x.shape
         ctx.set_materialize_grads(False)
         return tuple(outs)
 
     @staticmethod
     def backward(ctx, *dys):
-        x2, *ws = ctx.saved_tensors
+        n = len(dys)
+        x2, saved = ctx.saved_tensors[0], ctx.saved_tensors[1:]
+        ws, pres = saved[:n], iter(saved[n:])
         dx, grads = None, []
         for i, (dy, w) in enumerate(zip(dys, ws)):
-            need_w, need_b, need_a = ctx.needs_input_grad[1 + 3 * i:4 + 3 * i]
+            need_w, need_b, need_a = ctx.needs_input_grad[1 + 4 * i:4 + 4 * i]
+            pre = next(pres) if ctx.has_pre[i] else None
             if dy is None:
-                grads += [None, None, None]
+                grads += [None] * 4
                 continue
             g = dy.reshape(-1, dy.shape[-1]).contiguous()
+            if pre is not None:
+                g = silu_bwd(g, pre)
             if ctx.needs_input_grad[0]:
                 if dx is None:
                     dx, _ = gemm(g, w, None, None, b_mn=True)
@@ -295,17 +307,17 @@ class _LinearGroup(torch.autograd.Function):
                     gemm(g, w, None, None, b_mn=True, out=dx, accumulate=True)
             dw = _weight_grad(g, x2, w, ctx.sinks[i]) if need_w else None
             db = _bias_grad(g, ctx.bias_dtypes[i]) if need_b and ctx.bias_dtypes[i] is not None else None
-            grads += [dw, db, dy if need_a else None]
+            grads += [dw, db, dy if need_a else None, None]
         return (None if dx is None else dx.view(ctx.x_shape), *grads)
 
 
 def linear_group(x: Tensor, layers):
-    """[(w, b, addend or None), ...] of one input -> the list of x w^T + b (+ addend)."""
+    """[(w, b, addend or None, act or None), ...] of one input -> the list of act(x w^T + b) (+ addend)."""
     x2 = x.reshape(-1, x.shape[-1])
     if (x.dtype == torch.float32 or _GEMM_BACKEND[0] != "tcgen05" or x2.shape[0] <= 1 or not _tma_ok(x2)
             or any(w.dtype != x.dtype or w.shape[0] % 8 != 0 or not _tma_ok(w) or (a is not None and a.dtype != x.dtype)
-                   for w, _, a in layers)):
-        return [linear(x, w, b) if a is None else linear_add(x, w, b, a) for w, b, a in layers]
+                   for w, _, a, _ in layers)):
+        return [linear(x, w, b, act) if a is None else linear_add(x, w, b, a) for w, b, a, act in layers]
     return list(_apply(_LinearGroup, x, *[t for layer in layers for t in layer]))
 
 

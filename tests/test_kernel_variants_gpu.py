@@ -241,3 +241,55 @@ def test_operators_without_gradients_match_the_recorded_ones():
             ops.linear(dual, w, b, "silu")
     with torch.no_grad(), pytest.raises(Exception):
         torch.func.vmap(lambda r: ops.rms_norm(r, None, 1e-5))(x)
+
+
+def test_gate_is_rounded_after_its_activation(monkeypatch):
+    """The gate SiLU(r) leaves the product's epilogue rounded once; rounding r first shows as up to |r| times that."""
+    from megalodon_b200.modules.moving_average_gated_attention import MovingAverageGatedAttention, ops
+    torch.manual_seed(5)
+    m = MovingAverageGatedAttention(mdim=64, zdim=16, hdim=128, num_heads=1, ndim=4, chunk_size=32,
+                                    efficient_attn="fused", norm_num_groups=4).cuda().bfloat16()
+    with torch.no_grad():
+        m.wr.weight.normal_(std=0.3)                       # r with a deviation of 2.4
+    x = _rand(3, 32, 64)
+    monkeypatch.setattr(m.inner_attention, "forward", lambda q, k, v, *a: (torch.ones_like(v), None))
+    seen = []
+    monkeypatch.setattr(ops, "memory_efficient_dropout", lambda t, p, training: (seen.append(t.detach()), t)[1])
+    freqs = torch.polar(torch.ones(32, 8, device="cuda"), torch.rand(32, 8, device="cuda"))
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            m(x, freqs)
+        mx, gate = seen
+        seen.clear()
+        want = torch.nn.functional.silu(mx.double() @ m.wr.weight.double().t() + m.wr.bias.double())
+        # one rounding to 8 significant bits is at most 2^-8 of the value; the sum behind it is fp32
+        assert ((gate.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 4e-6).all()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 64, 65, 300])
+def test_linear_group_with_an_activation(rows):
+    from megalodon_b200 import ops
+    torch.manual_seed(rows)
+    K, sizes = 264, (64, 136, 264)
+    x, add = _rand(rows, K), _rand(rows, sizes[2])
+    ws, bs = [_rand(n, K, scale=K ** -0.5) for n in sizes], [_rand(n) for n in sizes]
+    gs = [_rand(rows, n) for n in sizes]
+    leaves = [t.clone().requires_grad_(True) for t in (x, add, *ws, *bs)]
+
+    def outs(t):
+        return [t[0] @ t[2].t() + t[5], torch.nn.functional.silu(t[0] @ t[3].t() + t[6]), t[0] @ t[4].t() + t[7] + t[1]]
+
+    def group(t):
+        return ops.linear_group(t[0], [(t[2], t[5], None), (t[3], t[6], None, "silu"), (t[4], t[7], t[1], None)])
+    got = group(leaves)
+    torch.autograd.backward(got, gs)
+    ref = [t.double().requires_grad_(True) for t in (x, add, *ws, *bs)]
+    want = outs(ref)
+    torch.autograd.backward(want, [g.double() for g in gs])
+    with torch.no_grad():
+        again = group(leaves)
+    for o, n, w in zip(got, again, want):
+        assert _rel(o, w) < 2.0 ** -8 and _rel(n, w) < 2.0 ** -8
+    for i, (a, r) in enumerate(zip(leaves, ref)):
+        # dx and what comes through the activation: rounded once more on the way
+        assert _rel(a.grad, r.grad) < (2.0 ** -7 if i in (0, 3, 6) else 2.0 ** -8), i
