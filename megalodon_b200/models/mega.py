@@ -49,7 +49,7 @@ from ..parallel.chunk_parallel import (
     should_send_to_next,
 )
 from ..parallel.model_parallel import ParallelEmbedding, RowParallelLinear
-from ..utils import create_on_gpu, get_init_fn, get_torch_dtype
+from ..utils import create_on_gpu, get_init_fn, get_torch_dtype, is_plain
 
 
 class MegaBlock(nn.Module):
@@ -126,7 +126,8 @@ class MegaOutputLayer(nn.Module):
 
     def logits(self, x: Tensor) -> Tensor:
         """fp32 logits of normalised activations."""
-        if torch.is_grad_enabled() or get_model_parallel_world_size() > 1:
+        if (torch.is_grad_enabled() or get_model_parallel_world_size() > 1
+                or not is_plain(self.output, RowParallelLinear) or self.output.bias is not None):
             return self.output(x).float()
         return ops.linear_fp32_out(x, self.output.weight)
 
@@ -233,10 +234,14 @@ class Mega(nn.Module):
             if targets is not None:
                 xn, _ = self.output.normalize(x)
                 return self._gather_losses([self._piece_loss(xn, targets)]), None
-            xn, cache_output = self.output.normalize(x, cache_output)
+            if is_plain(self.output, MegaOutputLayer):
+                xn, cache_output = self.output.normalize(x, cache_output)
+                logits = self.output.logits(xn)
+            else:
+                logits, cache_output = self.output(x, cache_output)
             if cache is not None:
                 cache = (cache_layers, cache_output)
-            return self.output.logits(xn), cache
+            return logits.float(), cache
 
         # ---- sequence micro-batching (training / scoring without cache)
         pieces = list(torch.split(x, piece_len, dim=1))

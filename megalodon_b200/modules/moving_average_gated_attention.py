@@ -38,7 +38,7 @@ from ..parallel.chunk_parallel import (
     should_recv_from_prev,
     should_send_to_next,
 )
-from ..utils import get_init_fn
+from ..utils import get_init_fn, is_plain
 from .complex_exponential_moving_average import MultiHeadComplexEMA
 from .layer_norm import FusedRMSNorm
 from .rotary_positional_embedding import apply_rotary_emb
@@ -292,12 +292,13 @@ class MovingAverageGatedAttention(nn.Module):
         # one rank: the three projections of mx share their backward pass, and both residual additions ride in
         # the epilogues of the projections around the attention
         fused_adds = get_model_parallel_world_size() == 1 and not (self.training and self.dropout > 0.0)
-        if fused_adds:
+        if fused_adds and is_plain(self.wz, ColumnParallelLinear) and is_plain(self.wr, ColumnParallelLinear):
             z, r, h = ops.linear_group(mx, [(self.wz.weight, self.wz.bias, None),
                                             (self.wr.weight, self.wr.bias, None, "silu"),
                                             (self.wh1.weight, self.wh1.bias, residual)])
         else:
             z, r = self.wz(mx), self.wr(mx)
+            h = ops.linear_add(mx, self.wh1.weight, self.wh1.bias, residual) if fused_adds else None
         z = z.view(bsz, seq_len, self.local_heads, self.z_head_dim)
         z = self.znorm(z).view(bsz, seq_len, -1)
         # q, k = rotary(z (gamma + 1) / sqrt(d) + beta): one kernel; positions are those of the chunk

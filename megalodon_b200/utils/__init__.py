@@ -48,6 +48,15 @@ def get_torch_dtype(dtype: str) -> torch.dtype:
     return {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32}[dtype]
 
 
+def is_plain(module: nn.Module, cls: type) -> bool:
+    """Whether calling `module` does what `cls.forward` does and nothing else: a `cls` itself, no forward of its own,
+    no hooks.  Code that takes a module's parameters instead of calling it asks this first, so that adapters, observers
+    and hooks keep seeing their calls."""
+    return (type(module) is cls and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                     or module._backward_pre_hooks or nn.modules.module._has_any_global_hook()))
+
+
 def get_default_half() -> str:
     return "bf16"
 
