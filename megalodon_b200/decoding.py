@@ -30,6 +30,8 @@ from typing import List, Optional, Tuple
 import torch
 from torch import Tensor
 
+from .utils import is_plain
+
 
 def _unwrap(model):
     while hasattr(model, "_wrapped"):
@@ -121,7 +123,6 @@ class DecodeSession:
     def _native_ok(self) -> bool:
         """Whether every layer is inside what the native step covers: one GPU's worth of 16-bit parameters
         in the session's dtype, plain MEGA blocks, sizes the kernels take."""
-        from .models.mega import MegaBlock
         from .ops import native_for
         from .ops._ext import require
         m = self.mega
@@ -133,23 +134,66 @@ class DecodeSession:
         from .ops import cuda_ops
         if cuda_ops.gemm_backend() != "tcgen05" or m.embed.weight.shape[1] != m.model_dim:
             return False
+        # a sharded unit gives its gathered weights back after every call of its own
+        if hasattr(self.model, "_units") and any(u.reshard_after_forward and not u._is_root for u in self.model._units()):
+            return False
+        if not self._as_built():
+            return False
         C = require()
         for layer in m.layers:
             block = _unwrap(layer)
-            if type(block) is not MegaBlock or block.nffn.alpha is not None:
-                return False
             a = block.mega
             dims = (a.mdim, a.z_head_dim, a.local_v_head_dim, block.nffn.hidden_dim)
-            if (a.head_split != 1 or a.local_heads != a.num_heads or a.local_mdim != a.mdim or a.mdim > 16384
-                    or any(d % 8 for d in dims) or m.chunk_size > 51200
+            if (block.nffn.alpha is not None or a.head_split != 1 or a.local_heads != a.num_heads
+                    or a.local_mdim != a.mdim or a.mdim > 16384 or any(d % 8 for d in dims) or m.chunk_size > 51200
                     or not C.decode_norm_ema_ok(a.mdim, a.timenorm.groups_per_partition, a.cema.ndim)):
                 return False
-            if any(p.dtype != self.dtype or not p.is_contiguous() or p.data_ptr() % 16
-                   for p in self._layer_params(block)):
+            if not self._params_ok(self._layer_params(block)):
                 return False
         fn, out = m.output.final_norm, m.output.output
-        return (C.decode_norm_ema_ok(m.model_dim, fn.groups_per_partition, 2) and out.weight.dtype == self.dtype
-                and out.weight.shape[1] == m.model_dim and out.bias is None)
+        return (C.decode_norm_ema_ok(m.model_dim, fn.groups_per_partition, 2) and out.weight.shape[1] == m.model_dim
+                and self._params_ok([fn.weight, fn.bias, out.weight]))
+
+    def _params_ok(self, params) -> bool:
+        return all(p.dtype == self.dtype and p.is_contiguous() and p.data_ptr() % 16 == 0 for p in params)
+
+    def _as_built(self) -> bool:
+        """Whether every module whose call the native step stands for is the one that the model was built with,
+        without hooks, so that taking its parameters comes to the same thing."""
+        from .models.mega import MegaBlock, MegaOutputLayer
+        from .modules import MovingAverageGatedAttention, NormalizedFeedForwardNetwork, TimestepNorm
+        from .modules.complex_exponential_moving_average import MultiHeadComplexEMA
+        from .modules.layer_norm import FusedLayerNorm, FusedRMSNorm
+        from .modules.moving_average_gated_attention import _InnerAttention
+        from .parallel.model_parallel import ColumnParallelLinear, ParallelEmbedding, RowParallelLinear
+        m = self.mega
+        mods = [(m.embed, ParallelEmbedding), (m.output, MegaOutputLayer), (m.output.final_norm, TimestepNorm),
+                (m.output.output, RowParallelLinear)]
+        for layer in m.layers:
+            while hasattr(layer, "_wrapped"):
+                mods.append((layer, type(layer)))
+                layer = layer._wrapped
+            if type(layer) is not MegaBlock:
+                return False
+            a, f = layer.mega, layer.nffn
+            mods += [(layer, MegaBlock), (a, MovingAverageGatedAttention), (f, NormalizedFeedForwardNetwork),
+                     (a.timenorm, TimestepNorm), (a.cema, MultiHeadComplexEMA), (a.rmsnorm, FusedRMSNorm),
+                     (a.znorm, FusedRMSNorm), (a.wv, ColumnParallelLinear), (a.wz, ColumnParallelLinear),
+                     (a.wr, ColumnParallelLinear), (a.wh1, ColumnParallelLinear), (a.wh2, RowParallelLinear),
+                     (a.inner_attention, _InnerAttention), (f.norm, FusedLayerNorm), (f.fc1, ColumnParallelLinear),
+                     (f.fc2, RowParallelLinear)]
+            if f.fc3 is not None:
+                mods.append((f.fc3, ColumnParallelLinear))
+        if not all(is_plain(mod, cls) for mod, cls in mods) or m.embed.max_norm is not None:
+            return False
+        for layer in m.layers:
+            a, f = _unwrap(layer).mega, _unwrap(layer).nffn
+            acts = [a.wv.activation, a.wr.activation, a.wz.activation, a.wh1.activation, f.fc1.activation]
+            if (a.znorm.weight is not None or acts != ["silu", "silu", None, None, None if f.swiglu else "silu"]
+                    or (f.fc3 is not None) != bool(f.swiglu) or (f.swiglu and f.fc3.activation is not None)
+                    or any(p is not None and p.bias is not None for p in (a.wh2, f.fc1, f.fc2, f.fc3))):
+                return False
+        return m.output.output.bias is None
 
     @staticmethod
     def _layer_params(block):
@@ -242,7 +286,10 @@ class DecodeSession:
 
     # ------------------------------------------------------------------ one token
     def _step_body(self) -> Tensor:
-        if self._native:
+        if self._native and self._as_built():        # (a hook or an adapter may have come since)
+            # what the units' own calls would bring up to date after an optimiser step or a load
+            if hasattr(self.model, "_units") and not all(u._full_is_valid() for u in self.model._units()):
+                self.model.materialize_views()
             return self._native_step()
         m = self.mega
         x = m.embed(self.tok)
@@ -250,18 +297,23 @@ class DecodeSession:
             x = x * m.emb_scale
         freqs = m.rope.get_freqs_cis(0, m.chunk_size).index_select(0, self.pos)
         for layer, st in zip(m.layers, self.layers):
-            norm = tuple(st["norm"]) if not self._fresh else (None, None, None)
+            norm = self._stats(st["norm"]) if not self._fresh else (None, None, None)
             hx = st["hx"] if not self._fresh else None
             x, (_, new_norm, new_hx) = layer(x, freqs, None, ((st["k"], st["v"], self.pos), norm, hx))
             for dst, src in zip(st["norm"], new_norm):
                 dst.copy_(src)
             st["hx"].copy_(new_hx)
-        out_norm = tuple(self.out_norm) if not self._fresh else (None, None, None)
+        out_norm = self._stats(self.out_norm) if not self._fresh else (None, None, None)
         logits, new_out = m.output(x, out_norm)
         for dst, src in zip(self.out_norm, new_out):
             dst.copy_(src)
         self.pos.add_(1).remainder_(m.chunk_size)
         return logits[:, -1].float()
+
+    def _stats(self, norm):
+        """Running statistics as the modules take them."""
+        count, mean, var = norm
+        return count, mean.to(self.dtype), var.to(self.dtype)
 
     @torch.no_grad()
     def step(self, tokens: Tensor) -> Tensor:

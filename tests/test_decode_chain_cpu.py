@@ -60,3 +60,63 @@ def test_ema_coefficients_precede_the_chain(monkeypatch, training):
         # the first link waits for everything before it; only the later ones may run ahead
         links = [a[-1] for n, a in rec.calls if n == "decode_norm_ema"]
         assert links == [False, True, True, True]
+
+
+def _block(sess, i=1):
+    layer = sess.mega.layers[i]
+    while hasattr(layer, "_wrapped"):
+        layer = layer._wrapped
+    return layer
+
+
+def _spots(sess):
+    b, out = _block(sess), sess.mega.output
+    return {"embed": sess.mega.embed, "wrapper": sess.mega.layers[1], "block": b, "mega": b.mega, "wz": b.mega.wz,
+            "wr": b.mega.wr, "wv": b.mega.wv, "rmsnorm": b.mega.rmsnorm, "nffn": b.nffn, "fc1": b.nffn.fc1,
+            "fc3": b.nffn.fc3, "norm": b.nffn.norm, "output": out, "output.output": out.output}
+
+
+def test_hooks_and_adapters_take_the_step_through_the_modules(monkeypatch):
+    """Also when they come after the session was made; without them the chain runs again."""
+    sess, rec = _session(monkeypatch)
+    reached = []
+    monkeypatch.setattr(sess, "_native_step", lambda: (reached.append("chain"), torch.zeros(2, 96))[1])
+    tok = torch.tensor([1, 2])
+    for name, mod in _spots(sess).items():
+        h = mod.register_forward_hook(lambda m, a, o, name=name: (reached.append(name), None)[1])
+        assert not sess._as_built(), name
+        h.remove()
+        cls = type(mod)
+        mod.__class__ = type("Adapter", (cls,), {})
+        assert not sess._as_built() or name == "wrapper", name
+        mod.__class__ = cls
+    b = _block(sess)
+    b.nffn.fc1.bias = torch.nn.Parameter(torch.zeros(128))       # a bias that the chain has no place for
+    assert not sess._as_built()
+    b.nffn.fc1.bias = None
+    sess.step(tok)
+    assert reached == ["chain"]
+
+
+def test_updated_weights_are_gathered_before_the_chain(monkeypatch):
+    """An optimiser step or a load since the last token: the compute-dtype weights are brought up to date first."""
+    sess, rec = _session(monkeypatch)
+    events = []
+    inner = sess.model.materialize_views
+    monkeypatch.setattr(sess.model, "materialize_views", lambda: (events.append("gather"), inner())[1])
+    monkeypatch.setattr(sess, "_native_step", lambda: (events.append("chain"), torch.zeros(2, 96))[1])
+    tok = torch.tensor([1, 2])
+    sess.step(tok)
+    unit = sess.model._units()[1]
+    with torch.no_grad():
+        unit.flat_param.mul_(1.5)
+    sess.step(tok)
+    assert events == ["chain", "gather", "chain"] and all(u._full_is_valid() for u in sess.model._units())
+
+
+def test_step_through_the_modules_takes_fp32_statistics(monkeypatch):
+    """A native session's running statistics are fp32 whatever its dtype; the modules want them in the dtype."""
+    sess, _ = _session(monkeypatch)
+    sess.dtype = torch.bfloat16
+    count, mean, var = sess._stats(sess.layers[0]["norm"])
+    assert mean.dtype == var.dtype == torch.bfloat16 and count.dtype == torch.int64

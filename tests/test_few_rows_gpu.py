@@ -212,3 +212,71 @@ def test_decode_norm_ema_with_more_clusters_than_fit(D, G, B):
         rows = (mx.double() - ref).norm(dim=1) / ref.norm(dim=1)
         assert rows.max() < 2.0 ** -7, rows
         assert (count == 1).all()
+
+
+def test_native_session_with_hooks_adapters_and_new_weights():
+    """What the chain does not know about is left to the modules: hooks from the start or added later, an adapter in the
+    place of a projection; and weights changed between two eager steps are the ones used."""
+    from megalodon_b200.config import ModelConf
+    from megalodon_b200.decoding import DecodeSession
+    from megalodon_b200.models.mega import build_model
+    from megalodon_b200.parallel.model_parallel import ColumnParallelLinear
+    from megalodon_b200.utils import init_cache, set_random_seed
+    cfg = ModelConf(num_layers=2, model_dim=256, num_heads=1, z_dim=64, value_dim=256, ffn_hidden_dim=256,
+                    chunk_size=64, vocab_size=264, swiglu=True, norm_num_groups=8, efficient_attn="fused")
+    set_random_seed(4)
+    model = build_model(cfg, "fp16", False, False).eval()
+    tok = torch.randint(0, 264, (2, 12), device="cuda")
+
+    class Adapter(ColumnParallelLinear):
+        def forward(self, x):
+            return super().forward(x).roll(1, -1)
+
+    def run(steps, between=lambda i: None):
+        """the same steps through a session and through the growing cache, `between(i)` before step i of either"""
+        sess = DecodeSession(model, 2, torch.float16, use_graph=False)
+        outs = []
+        for session in (True, False):
+            cache = init_cache(2, model, torch.float16)
+            rows = []
+            with torch.no_grad():
+                for i in range(steps):
+                    undo = between(i)
+                    if session:
+                        rows.append(sess.step(tok[:, i]).clone())
+                    else:
+                        y, cache = model(tok[:, i:i + 1], cache=cache)
+                        rows.append(y[:, -1])
+                    if undo is not None:
+                        undo()
+            outs.append(torch.stack(rows))
+        # some ten roundings to 2^-11 a layer on either side, adding up like a random walk
+        assert _rel(*outs) < 2 * (10 * cfg.num_layers) ** 0.5 * 2.0 ** -11
+        return sess._native, outs[0]
+
+    block = model._wrapped.layers[1]
+    while hasattr(block, "_wrapped"):
+        block = block._wrapped
+    native, plain = run(4)
+    assert native
+    wr = block.mega.wr
+    wr.__class__ = Adapter                                   # from the start
+    native, adapted = run(4)
+    assert not native and _rel(adapted, plain) > 1e-2
+    wr.__class__ = ColumnParallelLinear
+
+    def hook(i):                                             # for some of the steps
+        if i % 2:
+            return block.nffn.fc1.register_forward_hook(lambda m, a, o: o * 0.5).remove
+    native, hooked = run(6, hook)
+    assert native and _rel(hooked[:4], plain) > 1e-2 and torch.equal(hooked[0], plain[0])
+
+    unit = model._units()[2]
+
+    def update(i):
+        if i == 2:
+            keep = unit.flat_param.detach().clone()
+            unit.flat_param.mul_(1.25)
+            return lambda: unit.flat_param.copy_(keep)       # (the steps run under no_grad)
+    native, moved = run(4, update)
+    assert native and torch.equal(moved[:2], plain[:2]) and _rel(moved[2:], plain[2:]) > 1e-3
