@@ -53,12 +53,17 @@ class _NoGradContext:
         pass
 
 
+def _transformed() -> bool:
+    """Function transforms, forward-mode duals or tracing are in effect."""
+    return (torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
+            or torch.compiler.is_compiling() or torch.jit.is_tracing())
+
+
 def _apply(fn, *args):
     """`fn.apply(*args)`; where no gradient is recorded the forward pass is called as it is, which saves the
     autograd machinery's ten-odd microseconds an operator (a 12-layer forward call on a short prompt has 200).
     Function transforms, forward-mode duals and tracing keep the full route, and with it their errors."""
-    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0
-            or torch.compiler.is_compiling() or torch.jit.is_tracing()):
+    if torch.is_grad_enabled() or _transformed():
         return fn.apply(*args)
     return fn.forward(_NoGradContext(), *args)
 
@@ -623,21 +628,29 @@ def _c2r(t: Tensor) -> Tensor:
 
 class _CEMACoeffs(torch.autograd.Function):
     """p, q, gamma of the EMA recurrence from the layer's parameters, one kernel each way (as separate
-    element-wise operations 14 launches forward and some 25 backward per layer and call)."""
+    element-wise operations 14 launches forward and some 25 backward per layer and call).  A backward pass that is
+    itself recorded goes through the element-wise operations, so that it can be differentiated."""
 
     @staticmethod
     def forward(ctx, alpha, delta, theta, gamma, scale):
-        a, d, t, g = (x.contiguous() for x in (alpha, delta, theta, gamma))
         _bump()
-        p, q, go = _C().cema_coeffs_fwd(a, d, t, g, scale)
-        ctx.save_for_backward(a, d, t)
+        p, q, go = _C().cema_coeffs_fwd(*(x.contiguous() for x in (alpha, delta, theta, gamma)), scale)
+        ctx.save_for_backward(alpha, delta, theta, gamma)
         ctx.scale = scale
         ctx.set_materialize_grads(False)
         return p, torch.view_as_complex(q).unsqueeze(-1), torch.view_as_complex(go)
 
     @staticmethod
     def backward(ctx, dp, dq, dg):
-        a, d, t = ctx.saved_tensors
+        params = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            outs = reference.cema_coeffs(*params, ctx.scale)
+            used = [(o, g) for o, g in zip(outs, (dp, dq, dg)) if g is not None]
+            wanted = [t for t, need in zip(params, ctx.needs_input_grad) if need]
+            grads = iter(torch.autograd.grad([o for o, _ in used], wanted, [g for _, g in used], create_graph=True,
+                                             allow_unused=True))
+            return (*[next(grads) if need else None for need in ctx.needs_input_grad[:4]], None)
+        a, d, t = (x.contiguous() for x in params[:3])
         real = [None if x is None else _c2r(x) for x in (dq, dg)]
         _bump()
         da, dd, dt, dgo = _C().cema_coeffs_bwd(None if dp is None else dp.float().contiguous(), *real, a, d, t,
@@ -646,6 +659,8 @@ class _CEMACoeffs(torch.autograd.Function):
 
 
 def cema_coeffs(alpha, delta, theta, gamma, scale: float):
+    if alpha.dtype not in _DT or _transformed():
+        return reference.cema_coeffs(alpha, delta, theta, gamma, scale)
     return _apply(_CEMACoeffs, alpha, delta, theta, gamma, float(scale))
 
 

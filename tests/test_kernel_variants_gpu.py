@@ -293,3 +293,55 @@ def test_linear_group_with_an_activation(rows):
     for i, (a, r) in enumerate(zip(leaves, ref)):
         # dx and what comes through the activation: rounded once more on the way
         assert _rel(a.grad, r.grad) < (2.0 ** -7 if i in (0, 3, 6) else 2.0 ** -8), i
+
+
+def _coefficient_args(dtype=torch.float32, D=12, N=4):
+    torch.manual_seed(D)
+    return [_rand(D, N, 1, dtype=dtype), _rand(D, N, 1, dtype=dtype), _rand(D, 1, 1, dtype=dtype),
+            _rand(D, N, 2, dtype=dtype)]
+
+
+def test_cema_coefficients_differentiate_twice():
+    """A penalty on the gradient of a function of p, q and gamma, against the element-wise operations in 64 bits."""
+    from megalodon_b200 import ops
+
+    def coeffs64(alpha, delta, theta, gamma, scale):
+        p = torch.sigmoid(alpha)
+        n = torch.arange(1, 5, device="cuda", dtype=torch.float64).view(1, 4, 1)
+        q = torch.polar(1.0 - p * torch.sigmoid(delta), torch.sigmoid(theta) * (2 * torch.pi / 4) * n)
+        return p, q, torch.view_as_complex(gamma) * scale
+
+    def second(f, args):
+        p, q, g = f(*args, 0.5)
+        loss = (p ** 2).sum() + (q.real ** 3).sum() + q.imag.abs().sum() + (g.abs() ** 4).sum()
+        first = torch.autograd.grad(loss, args, create_graph=True)
+        return [*first, *torch.autograd.grad(sum((x ** 2).sum() for x in first), args)]
+    base = _coefficient_args()
+    got = second(ops.cema_coeffs, [t.clone().requires_grad_(True) for t in base])
+    want = second(coeffs64, [t.double().requires_grad_(True) for t in base])
+    for a, b in zip(got, want):
+        assert _rel(a.detach(), b.detach()) < 2e-5
+    # some of the parameters, some of the outputs
+    alpha = base[0].clone().requires_grad_(True)
+    q = ops.cema_coeffs(alpha, *base[1:], 0.5)[1]
+    first, = torch.autograd.grad(q.real.sum(), alpha, create_graph=True)
+    assert torch.autograd.grad(first.sum(), alpha)[0].abs().sum() > 0
+
+
+def test_cema_coefficients_under_transforms_and_other_types():
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import reference
+    args = _coefficient_args()
+    want = reference.cema_coeffs(*args, 0.5)
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            got = ops.cema_coeffs(*[t.double() for t in args], 0.5)
+            assert all(_rel(torch.view_as_real(a) if a.is_complex() else a, torch.view_as_real(b) if b.is_complex() else b)
+                       < 1e-6 for a, b in zip(got, want))
+            _, tangents = torch.func.jvp(lambda a: ops.cema_coeffs(a, *args[1:], 0.5)[0], (args[0],),
+                                         (torch.ones_like(args[0]),))
+            s = torch.sigmoid(args[0])
+            assert _rel(tangents, s * (1 - s)) < 1e-6
+            batch = torch.stack([args[0], args[0] + 1.0])
+            ps = torch.func.vmap(lambda a: ops.cema_coeffs(a, *args[1:], 0.5)[0])(batch)
+            assert _rel(ps, torch.sigmoid(batch)) < 1e-6
