@@ -8,9 +8,24 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace mb {
 
 constexpr int kWarp = 32;
+
+// Lets a kernel use `bytes` of dynamic shared memory.  A function attribute belongs to the device that is current
+// when it is set, so `done` (one per kernel) keeps a bit for each device.
+template <typename Kernel>
+inline bool allow_dynamic_smem(Kernel kern, int bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if ((done.load(std::memory_order_acquire) & bit) != 0) return true;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+  done.fetch_or(bit, std::memory_order_release);
+  return true;
+}
 
 enum DType : int { kF32 = 0, kBF16 = 1, kF16 = 2 };
 

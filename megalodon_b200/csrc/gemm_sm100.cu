@@ -1209,11 +1209,8 @@ static int launch_gemm(const TmapArray& ta, const CUtensorMap& tb, const GemmPar
                        cudaStream_t st) {
   using L = SmemLayout<BN>;
   auto kern = gemm_tcgen05_kernel<BN, A_MN, B_MN, OutT>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total) != cudaSuccess) return -2;
-    configured = true;
-  }
+  static std::atomic<unsigned long long> configured{0};
+  if (!allow_dynamic_smem(kern, L::total, configured)) return -2;
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
   const int grid = tiles < sms ? tiles : sms;
   kern<<<grid, kGemmThreads, L::total, st>>>(ta, tb, p, in_fmt);
@@ -1227,11 +1224,8 @@ static int launch_gemm_pair_gather(const TmapArray& ta, const CUtensorMap& tb, c
                                    int sms, cudaStream_t st) {
   using L = PairSmem;
   auto kern = gemm_tcgen05_pair_kernel<false, false, OutT, true>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total) != cudaSuccess) return -2;
-    configured = true;
-  }
+  static std::atomic<unsigned long long> configured{0};
+  if (!allow_dynamic_smem(kern, L::total, configured)) return -2;
   if (cudaMemsetAsync(p.g_flags, 0, sizeof(unsigned int) * (1 + p.N / 128), st) != cudaSuccess) return -8;
   const int tiles = ((p.M + kPairBM - 1) / kPairBM) * ((p.N + kPairBN - 1) / kPairBN) * p.batch;
   const int pairs = sms / 2;
@@ -1245,11 +1239,8 @@ static int launch_gemm_pair(const TmapArray& ta, const CUtensorMap& tb, const Ge
                             cudaStream_t st) {
   using L = PairSmem;
   auto kern = gemm_tcgen05_pair_kernel<A_MN, B_MN, OutT>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total) != cudaSuccess) return -2;
-    configured = true;
-  }
+  static std::atomic<unsigned long long> configured{0};
+  if (!allow_dynamic_smem(kern, L::total, configured)) return -2;
   const int tiles = ((p.M + kPairBM - 1) / kPairBM) * ((p.N + kPairBN - 1) / kPairBN) * p.batch;
   const int pairs = sms / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);

@@ -257,11 +257,8 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
 template <typename T>
 int launch_skinny(const SkinnyMaps& maps, const SkinnyParams& p, int tiles, size_t smem, bool pdl, cudaStream_t st) {
   auto kern = skinny_gemm_kernel<T>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return -2;
-    configured = true;
-  }
+  static std::atomic<unsigned long long> configured{0};
+  if (!allow_dynamic_smem(kern, 227 * 1024, configured)) return -2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * p.split, 1, 1);
   cfg.blockDim = dim3(kSkThreads, 1, 1);
