@@ -836,6 +836,12 @@ def _attention_native_ok(q, k, v) -> bool:
     return attention_shapes_ok(q.dtype, q.shape[-1], v.shape[-1], k.shape[1])
 
 
+# One 4096-token chunk of four heads: what the backward pass without the fused softmax needs for a single sequence
+# anyway.  All sequences at once would be 1 GB for eight such chunks; a launch per sequence leaves short ones to a part
+# of the SMs.
+_DP_BYTES = 128 << 20
+
+
 class _Attention(torch.autograd.Function):
     """Chunk-local attention as matrix products on the tcgen05 GEMM (batched over heads).
 
@@ -911,19 +917,25 @@ class _Attention(torch.autograd.Function):
             # dV = P~^T (dO / l); dS = P~ / l * (dO V^T - delta) written over P~; dQ, dK from dS
             gemm(Pv, _heads_view(dos), a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)
             gemm(doh, vh, out=Pv, mode=m1, softmax=dict(epi_kind=4, row_in=rsum, row_in2=delta, aux=Pv))
-            dS = Pv
-        else:
-            dP = torch.empty_like(P)
-            dS = dP[..., :L2]
-            # dV = P^T dO   (A = P stored [q, key] = [K, M]; B = dO stored [q, dv] = [K, N])
-            gemm(Pv, doh, a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)
+            # dQ = scale dS K ; dK = scale dS^T Q
+            gemm(Pv, _heads_view(k), b_mn=True, out=_heads_view(dq), mode=m2, alpha=scale)
+            gemm(Pv, _heads_view(q), a_mn=True, b_mn=True, out=_heads_view(dk_), mode=m3, alpha=scale)
+            return dq, dk_, dv_, None, None, None
+        # dV = P^T dO   (A = P stored [q, key] = [K, M]; B = dO stored [q, dv] = [K, N])
+        gemm(Pv, doh, a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)
+        # dP needs memory of its own: as many sequences at a time as stay within `_DP_BYTES`
+        step = max(1, _DP_BYTES // max(1, P[:1].numel() * P.element_size()))
+        dP = torch.empty_like(P[:step])
+        for b0 in range(0, B, step):
+            s = slice(b0, min(b0 + step, B))
+            dS = dP[:s.stop - b0, ..., :L2]
             # dP = dO V^T
-            gemm(doh, vh, out=dS, mode=m1)
+            gemm(doh[s], vh[s], out=dS, mode=m1)
             _bump()
-            _C().attn_softmax_bwd(Pv, dS, L1, L2, causal, square)      # dP <- dS in place
-        # dQ = scale dS K ; dK = scale dS^T Q
-        gemm(dS, _heads_view(k), b_mn=True, out=_heads_view(dq), mode=m2, alpha=scale)
-        gemm(dS, _heads_view(q), a_mn=True, b_mn=True, out=_heads_view(dk_), mode=m3, alpha=scale)
+            _C().attn_softmax_bwd(Pv[s], dS, L1, L2, causal, square)      # dP <- dS in place
+            # dQ = scale dS K ; dK = scale dS^T Q
+            gemm(dS, _heads_view(k[s]), b_mn=True, out=_heads_view(dq[s]), mode=m2, alpha=scale)
+            gemm(dS, _heads_view(q[s]), a_mn=True, b_mn=True, out=_heads_view(dk_[s]), mode=m3, alpha=scale)
         return dq, dk_, dv_, None, None, None
 
 

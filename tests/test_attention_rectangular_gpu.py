@@ -82,3 +82,32 @@ def test_softmax_operator_clears_masked_columns(L1, L2, dtype):
     tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8
     assert _rel(y, want) < tol and _rel(a.grad, r.grad) < 4 * tol      # (the gradient starts from the rounded y)
     assert (y[:, _hidden(L1, L2)] == 0).all() and (a.grad[:, _hidden(L1, L2)] == 0).all()
+
+
+@pytest.mark.parametrize("L2", [2048, 2040])
+def test_backward_memory_without_the_fused_softmax(L2):
+    """The gradients of the probabilities are held for a bounded number of sequences, whatever the batch."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(0)
+    B, L1, H, d = 5, 2048, 8, 16
+    q, k, v, g = _rand(B, L1, H, d), _rand(B, L2, H, d), _rand(B, L2, H, d), _rand(B, L1, H, d)
+
+    def grads(s):
+        leaves = [t[s].clone().requires_grad_(True) for t in (q, k, v)]
+        out = cuda_ops.attention(*leaves, 0.25, 0.0, True, True)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        res = torch.autograd.grad(out, leaves, g[s])
+        torch.cuda.synchronize()
+        return res, torch.cuda.max_memory_allocated() - before
+    cuda_ops.set_fused_attention_softmax(False)
+    try:
+        whole, peak = grads(slice(0, B))
+        assert peak < (128 << 20) + (32 << 20), peak        # 64 MB a sequence, and the results
+        for b in range(B):
+            one, _ = grads(slice(b, b + 1))
+            for a, r in zip(one, whole):
+                assert torch.equal(a[0], r[b])
+    finally:
+        cuda_ops.set_fused_attention_softmax(True)
