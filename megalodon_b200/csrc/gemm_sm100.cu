@@ -1299,13 +1299,13 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
                       int in_dtype, int out_dtype, int* err, int num_sms, cudaStream_t st,
                       const GemmPeerSpec* peers, bool accumulate, const GemmGatherSpec* gather,
                       const GemmSoftmaxSpec* softmax, const GemmOuterBatch* outer, int tile) {
-  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
+  const int nb2 = outer != nullptr ? outer->count : 1;
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || nb2 <= 0) return 0;
   // TMA wants 16-byte strides; the vectorised epilogue wants 16-byte aligned rows of C
   if (lda % 8 != 0 || ldb % 8 != 0 || ldc % 8 != 0) return -1;
   if (batch > 1 && (a_bs % 8 != 0 || b_bs % 8 != 0 || c_bs % 8 != 0)) return -1;
-  const int nb2 = outer != nullptr ? outer->count : 1;
   const long long a_bs2 = outer != nullptr ? outer->a_stride : 0, b_bs2 = outer != nullptr ? outer->b_stride : 0;
-  if (nb2 < 1 || (nb2 > 1 && (a_bs2 % 8 != 0 || b_bs2 % 8 != 0 || outer->c_stride % 8 != 0))) return -1;
+  if (nb2 > 1 && (a_bs2 % 8 != 0 || b_bs2 % 8 != 0 || outer->c_stride % 8 != 0)) return -1;
   TmapArray ta;
   CUtensorMap tb;
   GemmParams p{};

@@ -821,6 +821,13 @@ def rfft(x, flip=False):
 # launch per sequence left the causal tiles of a 2048-token chunk to a part of
 # the CTA pairs) and, for square causal blocks, restricted to the tiles on or
 # below the diagonal.
+def _dense(t: Tensor) -> Tensor:
+    """`t` contiguous, aligned, and with the strides of its shape also along dimensions of size one, whose strides
+    `contiguous` leaves as they come and a tensor map may not take."""
+    t = t.contiguous()
+    return t if _tma_ok(t) else t.clone(memory_format=torch.contiguous_format)
+
+
 def _heads_view(t: Tensor, b: Optional[int] = None) -> Tensor:
     """[B, L, H, d] -> view [B, H, L, d] (both batch indices of a product over all sequences and heads), or
     [H, L, d] of sequence `b`."""
@@ -855,7 +862,7 @@ class _Attention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, scale, drop_p, causal):
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        q, k, v = _dense(q), _dense(k), _dense(v)
         B, L1, H, dk = q.shape
         L2, dv = k.shape[1], v.shape[-1]
         square = causal and L1 == L2
@@ -905,7 +912,7 @@ class _Attention(torch.autograd.Function):
                      softmax=dict(epi_kind=2, row_in=rmax, row_out=torch.empty_like(rsum)))
         else:
             q, k, v, P = ctx.saved_tensors
-        dout = dout.contiguous()
+        dout = _dense(dout)
         B, L1, H, dk = q.shape
         dq, dk_, dv_ = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         m1, m2, m3 = (1, 2, 3) if square else (0, 0, 0)

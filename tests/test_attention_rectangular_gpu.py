@@ -111,3 +111,30 @@ def test_backward_memory_without_the_fused_softmax(L2):
                 assert torch.equal(a[0], r[b])
     finally:
         cuda_ops.set_fused_attention_softmax(True)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("dropout", [0.0, 0.5])
+def test_attention_of_no_sequences(causal, dropout):
+    from megalodon_b200 import ops
+    leaves = [torch.empty(0, 16, 2, 16, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3)]
+    out = ops.attention(*leaves, 1.0, dropout, causal, True)
+    out.sum().backward()
+    assert out.shape == (0, 16, 2, 16) and all(t.grad.shape == t.shape for t in leaves)
+
+
+@pytest.mark.parametrize("shape,stride,offset", [((1, 16, 2, 16), (1001, 32, 16, 1), 0), ((2, 1, 2, 16), (32, 7, 16, 1), 0),
+                                                 ((2, 16, 1, 16), (256, 16, 13, 1), 0), ((2, 16, 2, 16), (512, 32, 16, 1), 3)])
+def test_attention_of_odd_strides(shape, stride, offset):
+    """Dimensions of size one may carry any stride and a view may start anywhere; both count as contiguous."""
+    from megalodon_b200 import ops
+    torch.manual_seed(0)
+    ts = [torch.as_strided(_rand(4096), shape, stride, offset) for _ in range(4)]
+    assert all(t.is_contiguous() for t in ts)
+    res = []
+    for norm in (lambda t: t, lambda t: t.clone(memory_format=torch.contiguous_format)):
+        leaves = [norm(t).detach().requires_grad_(True) for t in ts[:3]]
+        out = ops.attention(*leaves, 1.0, 0.0, True, True)
+        res.append([out, *torch.autograd.grad(out, leaves, norm(ts[3]))])
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
