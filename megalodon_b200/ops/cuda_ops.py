@@ -134,6 +134,7 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
     out_dtype = out_dtype or (out.dtype if out is not None else a.dtype)
     native = (_GEMM_BACKEND[0] == "tcgen05" and a.dtype in (torch.bfloat16, torch.float16)
               and _tma_ok(a) and _tma_ok(b)
+              and a.shape[-2 if a_mn else -1] > 0         # (an empty sum: no tile would write the zeros)
               # the epilogue stores 16-byte pieces of rows that start on a 16-byte boundary
               and (_tma_ok(out) if out is not None else (b.shape[-1] if b_mn else b.shape[-2]) % 8 == 0))
     if a_part_ptrs or c_part_ptrs or b_gather:
@@ -149,7 +150,8 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
         if rc != 0:
             raise RuntimeError(f"tcgen05 GEMM launch failed with code {rc}")
         return res, pre
-    if softmax and not native:
+    addend = softmax["aux"] if softmax and list(softmax) == ["aux"] else None
+    if softmax and addend is None and not native:
         raise RuntimeError("fused-softmax epilogues need the tcgen05 backend and TMA-compatible operands")
     if not native:
         A = a.transpose(-1, -2) if a_mn else a
@@ -160,6 +162,8 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
         if bias is not None:
             pre = pre + bias.to(pre.dtype)
         res = F.silu(pre) if act == "silu" else pre
+        if addend is not None:
+            res = res + addend
         if mode == 1:       # the kernel leaves tiles above the diagonal unwritten; nothing reads them
             pass
         if out is not None:
@@ -170,8 +174,8 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
             res = out
         return res.to(out_dtype), (pre.to(out_dtype) if want_preact else None)
     if (a.dim() == 2 and a.shape[0] <= _SKINNY_MAX_ROWS and not a_mn and not b_mn and mode == 0 and alpha == 1.0
-            and not want_preact and not accumulate and (not softmax or list(softmax) == ["aux"])):
-        res = _few_rows(a, b, bias, act, out_dtype, out, softmax["aux"] if softmax else None)
+            and not want_preact and not accumulate and (not softmax or addend is not None)):
+        res = _few_rows(a, b, bias, act, out_dtype, out, addend)
         if res is not None:
             return res, None
     _bump()

@@ -345,3 +345,27 @@ def test_cema_coefficients_under_transforms_and_other_types():
             batch = torch.stack([args[0], args[0] + 1.0])
             ps = torch.func.vmap(lambda a: ops.cema_coeffs(a, *args[1:], 0.5)[0])(batch)
             assert _rel(ps, torch.sigmoid(batch)) < 1e-6
+
+
+@pytest.mark.parametrize("rows", [1, 5, 300])
+def test_empty_sums(rows):
+    """No rows: every weight gradient is a sum of nothing, zero.  No features: bias and addend alone."""
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(0)
+    poison = [torch.full((1 << 14,), float("nan"), device="cuda") for _ in range(8)]
+    del poison
+    x, w, b = _rand(0, 64).requires_grad_(True), _rand(32, 64).requires_grad_(True), _rand(32).requires_grad_(True)
+    add = _rand(0, 32).requires_grad_(True)
+    for out in (ops.linear(x, w, b), ops.linear(x, w, b, "silu"), ops.linear_add(x, w, b, add),
+                ops.linear_group(x, [(w, b, None), (w, b, add)])[1]):
+        dx, dw, db = torch.autograd.grad(out.sum(), (x, w, b))
+        assert dx.shape == x.shape and (dw == 0).all() and (db == 0).all()
+    x, w, add = _rand(rows, 0), _rand(32, 0), _rand(rows, 32)
+    b = b.detach()
+    assert torch.equal(cuda_ops.gemm(x, w, b)[0], b.expand(rows, 32))
+    assert torch.equal(cuda_ops.gemm(x, w, b, softmax=dict(aux=add))[0], b + add)
+    target = _rand(32, 64)
+    for accumulate, want in ((True, target.clone()), (False, torch.zeros_like(target))):
+        cuda_ops.gemm(_rand(0, 32), _rand(0, 64), a_mn=True, b_mn=True, out=target, accumulate=accumulate)
+        assert torch.equal(target, want)
