@@ -748,12 +748,11 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_buf, const Tensor& v_bu
   TORCH_CHECK(k_buf.scalar_type() == q.scalar_type() && v_buf.scalar_type() == q.scalar_type());
   const int B = q.size(0), H = q.size(1), dk = q.size(2), C = k_buf.size(2), dv = v_buf.size(3);
   TORCH_CHECK(k_buf.size(0) == B && k_buf.size(1) == H && k_buf.size(3) == dk && v_buf.size(2) == C && dk % 8 == 0);
-  TORCH_CHECK(C <= 51200 && dv % 8 == 0, "decode_attention: key buffer too long or value width not a multiple of 8");
-  for (const Tensor* t : {&k_buf, &v_buf})
-    TORCH_CHECK((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "decode_attention: buffers must be 16-byte aligned");
+  TORCH_CHECK(C <= 51200, "decode_attention: key buffer too long");
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(k_buf.data_ptr()) & 15) == 0, "decode_attention: keys must be 16-byte aligned");
   Tensor out = torch::empty({B, H, dv}, q.options());
   const int splits = mb::decode_attend_splits(B * H, C, at::cuda::getCurrentDeviceProperties()->multiProcessorCount);
-  Tensor acc = torch::empty({(int64_t)B * H * splits, dv}, q.options().dtype(at::kFloat));
+  Tensor acc = torch::empty({(int64_t)B * H * splits, (dv + 7) / 8 * 8}, q.options().dtype(at::kFloat));
   Tensor ml = torch::empty({(int64_t)B * H * splits, 2}, acc.options());
   mb::DecodeAttend a{};
   a.q = q.data_ptr(); a.k_buf = k_buf.data_ptr(); a.v_buf = v_buf.data_ptr();

@@ -179,7 +179,11 @@ __device__ __forceinline__ int keys_per_split(int n, int splits) { return max(8,
 // Before: one CTA per 256 value columns walked all keys with 2-byte loads - 177 us at 4 heads, 1100 keys,
 // d_v 2048 (18 MB of values), now 14.6 with the combination; 16 sequences of 2 heads, 700 keys (103 MB): 31.5 us
 // (54.5 with eight rows in flight and nothing behind them).
-template <typename T>
+// VEC: value rows of whole 16-byte pieces.  Otherwise (a width that is no multiple of 8, or a buffer that starts
+// anywhere) their pieces are put together element by element; the partial rows are padded to `padded_width`.
+__host__ __device__ __forceinline__ int padded_width(int dv) { return (dv + 7) & ~7; }
+
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(kDecThreads, 2)
 decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   extern __shared__ float sm[];
@@ -199,7 +203,7 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   const int n = at + 1;
   const int per = keys_per_split(n, gridDim.x);
   const int lo = blockIdx.x * per, hi = min(n, lo + per);
-  if (lo < hi && warp == 0 && (long long)n * gridDim.y * (p.dk + p.dv) * (long long)sizeof(T) <= (32 << 20)) {
+  if (VEC && lo < hi && warp == 0 && (long long)n * gridDim.y * (p.dk + p.dv) * (long long)sizeof(T) <= (32 << 20)) {
     const T* k0 = reinterpret_cast<const T*>(p.k_buf) + ((long long)bh * p.C + lo) * p.dk;
     const T* v0 = reinterpret_cast<const T*>(p.v_buf) + ((long long)bh * p.C + lo) * p.dv;
     for (int j = lane; j < hi - lo; j += 32) {
@@ -249,14 +253,25 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   }
   // The first value rows of the first column block are under way while the scores are computed.
   const T* vnew = fused ? reinterpret_cast<const T*>(p.v_new) + (long long)bh * p.dv : nullptr;
-  const int ct0 = min(kDecThreads, p.dv / 8), ng0 = kDecThreads / ct0, grp0 = tid / ct0;
+  const int dvp = padded_width(p.dv);
+  const int ct0 = min(kDecThreads, dvp / 8), ng0 = kDecThreads / ct0, grp0 = tid / ct0;
   const int c0 = (tid - grp0 * ct0) * 8;
   auto load_rows = [&](uint4 (&raw)[8], int j0, int step, int c, bool on) {
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int j = j0 + u * step;
       raw[u] = make_uint4(0u, 0u, 0u, 0u);
-      if (on && j < hi) raw[u] = *reinterpret_cast<const uint4*>(mine && j == at ? vnew + c : vrow + (long long)j * p.dv + c);
+      if (!on || j >= hi) continue;
+      const T* src = mine && j == at ? vnew + c : vrow + (long long)j * p.dv + c;
+      if constexpr (VEC) {
+        raw[u] = *reinterpret_cast<const uint4*>(src);
+      } else {
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (c + i < p.dv) w[i / 2] |= (uint32_t)reinterpret_cast<const unsigned short*>(src)[i] << (16 * (i & 1));
+        raw[u] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
   };
   uint4 next[8];
@@ -303,9 +318,9 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
   __syncthreads();
   const long long part = (long long)bh * gridDim.x + blockIdx.x;
   if (tid == 0) reinterpret_cast<float2*>(p.part_ml)[part] = make_float2(m, sum);
-  float* dst = p.part_acc + part * p.dv;
-  for (int col0 = 0; col0 < p.dv; col0 += kDecThreads * 8) {
-    const int ct = min(kDecThreads, (p.dv - col0) / 8);     // threads across the columns
+  float* dst = p.part_acc + part * dvp;
+  for (int col0 = 0; col0 < dvp; col0 += kDecThreads * 8) {
+    const int ct = min(kDecThreads, (dvp - col0) / 8);     // threads across the columns
     const int ng = kDecThreads / ct;                        // groups of them, each every ng-th key
     const int grp = tid / ct, c = col0 + (tid - grp * ct) * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -320,7 +335,7 @@ decode_attend_kernel(const __grid_constant__ DecodeAttend p) {
         for (int u = 0; u < 8; ++u) {
           const int j = j0 + u * ng;
           if (j < hi) {
-            if (mine && j == at) *reinterpret_cast<uint4*>(vrow + (long long)j * p.dv + c) = raw[u];
+            if (VEC && mine && j == at) *reinterpret_cast<uint4*>(vrow + (long long)j * p.dv + c) = raw[u];
             float v[8];
             load8(reinterpret_cast<const T*>(&raw[u]), v);
             const float e = sc[j - lo];
@@ -371,11 +386,12 @@ decode_combine_kernel(const __grid_constant__ DecodeAttend p, int splits) {
   }
   __syncthreads();
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (c < p.dv) {
-    const float* src = p.part_acc + (long long)bh * splits * p.dv + c;
+  const int dvp = padded_width(p.dv);
+  if (c < dvp) {
+    const float* src = p.part_acc + (long long)bh * splits * dvp + c;
 #pragma unroll 4
     for (int s = strand; s < active; s += 8) {
-      const float4 v = *reinterpret_cast<const float4*>(src + (long long)s * p.dv);
+      const float4 v = *reinterpret_cast<const float4*>(src + (long long)s * dvp);
       const float w = wgt[s];
       a.x = fmaf(w, v.x, a.x); a.y = fmaf(w, v.y, a.y); a.z = fmaf(w, v.z, a.z); a.w = fmaf(w, v.w, a.w);
     }
@@ -497,12 +513,14 @@ int decode_attend_splits(int BH, int C, int num_sms) {
 
 int decode_attend(const DecodeAttend& p, int B, int splits, int dtype, bool pdl, cudaStream_t st) {
   if (B == 0) return 0;
+  if (p.z != nullptr && (p.dv % 8 != 0 || !aligned16(p.v_buf))) return -1;      // (the new value row leaves in pieces)
   const int BH = B * p.H;
   const int keys = div_up(p.C, splits) < 8 ? 8 : div_up(p.C, splits);
   const size_t smem = sizeof(float) * (2 * p.dk + kDecThreads * 8 + keys);
   cudaError_t e = cudaSuccess;
   MB_DISPATCH_16BIT(dtype, {
-    auto kern = decode_attend_kernel<scalar_t>;
+    const bool vec = p.dv % 8 == 0 && aligned16(p.v_buf);
+    auto kern = vec ? decode_attend_kernel<scalar_t, true> : decode_attend_kernel<scalar_t, false>;
     if (smem > 40 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
     if (e == cudaSuccess) e = launch_link(kern, dim3(splits, BH), smem, 1, pdl, st, p);
     if (e == cudaSuccess)

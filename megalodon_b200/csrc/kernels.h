@@ -217,7 +217,7 @@ struct DecodeAttend {
   const long long* pos;                 // [1]: slots 0 .. pos take part
   const void* gate;                     // [B, H, dv] multiplied into the result, or null
   void* out;                            // [B, H, dv]
-  float *part_acc, *part_ml;            // [B * H, splits, dv], [B * H, splits, 2]
+  float *part_acc, *part_ml;            // [B * H, splits, dv up to a multiple of 8], [B * H, splits, 2]
   float scale, eps;
   int H, C, dk, dv;
 };

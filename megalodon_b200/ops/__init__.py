@@ -102,16 +102,16 @@ def qk_rotary(z: Tensor, gamma: Tensor, beta: Tensor, freqs_cis: Tensor, head_di
     return q, k
 
 
-def decode_attention_native(q: Tensor, k_buf: Tensor, v_buf: Tensor) -> bool:
+def decode_attention_native(q: Tensor, k_buf: Tensor) -> bool:
     return (native_for(q) and q.dtype in (torch.bfloat16, torch.float16) and k_buf.dtype == q.dtype
-            and q.shape[-1] % 8 == 0 and v_buf.shape[-1] % 8 == 0 and k_buf.is_contiguous()
-            and k_buf.shape[2] * 4 <= 200 * 1024 and k_buf.data_ptr() % 16 == 0 and v_buf.data_ptr() % 16 == 0)
+            and q.shape[-1] % 8 == 0 and k_buf.is_contiguous() and k_buf.shape[2] * 4 <= 200 * 1024
+            and k_buf.data_ptr() % 16 == 0)
 
 
 def decode_attention(q: Tensor, k_buf: Tensor, v_buf: Tensor, pos: Tensor, scale: float) -> Tensor:
     """One decode step against fixed buffers: q [B, H, dk], k_buf [B, H, C, dk], v_buf [B, H, C, dv], `pos` a
     device index tensor [1]; keys 0 .. pos take part.  Returns [B, H, dv]."""
-    if decode_attention_native(q, k_buf, v_buf):
+    if decode_attention_native(q, k_buf):
         return _cuda().decode_attention(q, k_buf, v_buf, pos, scale)
     scores = torch.einsum("bhd,bhcd->bhc", q.float(), k_buf.float()) * scale
     hidden = torch.arange(k_buf.size(2), device=pos.device) > pos

@@ -280,3 +280,20 @@ def test_native_session_with_hooks_adapters_and_new_weights():
             return lambda: unit.flat_param.copy_(keep)       # (the steps run under no_grad)
     native, moved = run(4, update)
     assert native and torch.equal(moved[:2], plain[:2]) and _rel(moved[2:], plain[2:]) > 1e-3
+
+
+@pytest.mark.parametrize("B,H,C,dk,dv,pos,offset", [(2, 3, 40, 16, 12, 20, 0), (1, 2, 700, 64, 2061, 699, 0), (3, 1, 64, 8, 1, 5, 0),
+                                                    (2, 2, 300, 32, 64, 130, 1), (1, 1, 16, 8, 4100, 0, 3)])
+def test_decode_attention_of_any_value_width(B, H, C, dk, dv, pos, offset):
+    """Value rows that are no whole 16-byte pieces, or start between two."""
+    from megalodon_b200 import ops
+    torch.manual_seed(dv)
+    q, k = torch.randn(B, H, dk, device="cuda").bfloat16(), torch.randn(B, H, C, dk, device="cuda").bfloat16()
+    v = torch.randn(B * H * C * dv + offset, device="cuda").bfloat16()[offset:].view(B, H, C, dv)
+    k[:, :, pos + 1:] = float("nan")
+    v[:, :, pos + 1:] = float("nan")
+    assert ops.decode_attention_native(q, k)
+    out = ops.decode_attention(q, k, v, torch.tensor([pos], device="cuda"), 0.4)
+    s = torch.einsum("bhd,bhcd->bhc", q.double(), k[:, :, :pos + 1].double()) * 0.4
+    ref = torch.einsum("bhc,bhcd->bhd", torch.softmax(s, -1), v[:, :, :pos + 1].double())
+    assert out.shape == ref.shape and _rel(out, ref) < 2.0 ** -8       # fp32 throughout, one rounding
