@@ -202,7 +202,7 @@ class FullyShardedDataParallel(nn.Module):
         self._flatten(module, compute_device)
         self.compute_device = self.flat_param.device
         self._cuts = None                                  # how the flat buffer is cut into parameters
-        self._plain_views: Optional[torch.Tensor] = None   # buffer whose untracked views the modules hold
+        self._plain_views = None                           # the untracked views handed out last, see `_set_views`
         self._full: Optional[torch.Tensor] = None          # gathered compute-dtype buffer
         self._full_leaf: Optional[torch.Tensor] = None
         self._flat_grad: Optional[torch.Tensor] = None     # this iteration's gradients, compute dtype
@@ -483,12 +483,14 @@ class FullyShardedDataParallel(nn.Module):
         fused_infos = getattr(self, "_fused_infos", ())
         if track:
             views = _FlatViews.apply(leaf, self)
-            self._plain_views = None
         else:
-            if self._plain_views is leaf and not fused_infos:
-                return                       # the modules hold plain views of this very buffer already
+            # nothing to do where every module still holds the plain view of this memory that it was given (looked at
+            # one by one: a parameter may have been replaced since)
+            if (self._plain_views is not None and not fused_infos and self._plain_views[0] == leaf.data_ptr()
+                    and self._plain_views[1] is leaf
+                    and all(mod.__dict__.get(pname) is v for mod, pname, v in self._plain_views[2])):
+                return
             views = self._param_views(leaf)
-            self._plain_views = leaf
         direct = track and leaf.is_cuda and leaf.dtype in (torch.bfloat16, torch.float16)
         fused = {i.name for i in fused_infos}
         for info, v in zip(self._infos, views):
@@ -498,6 +500,8 @@ class FullyShardedDataParallel(nn.Module):
                 v._gather_spec = _GatherSpec(self, info)
             for mod, pname, _ in info.owners:
                 mod.__dict__[pname] = v
+        self._plain_views = None if track else (leaf.data_ptr(), leaf, [
+            (mod, pname, v) for info, v in zip(self._infos, views) for mod, pname, _ in info.owners])
 
     def _grad_buffer(self) -> torch.Tensor:
         """Flat gradient of this iteration in compute dtype.  Nothing is zero-filled up front: the first

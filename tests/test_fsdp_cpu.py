@@ -98,3 +98,24 @@ def test_flat_gradient_is_not_zero_filled_but_unused_parameters_and_gaps_end_up_
             else:
                 assert torch.allclose(got, want, atol=1e-5, rtol=1e-5), info.name
         assert bool((shard[~covered] == 0).all())
+
+
+def test_views_are_handed_out_again_where_a_module_lost_its_own():
+    """Without gradients the views of a call are kept for the next, as long as the modules still hold them."""
+    import copy
+    unit, ref = _unit(mixed=False)
+    x = torch.randn(4, 48)
+    with torch.no_grad():
+        want = unit(x)
+        held = unit._wrapped.weight
+        unit(x)
+        assert unit._wrapped.weight is held
+        unit._wrapped.__dict__["weight"] = torch.zeros(24, 48)
+        assert torch.equal(unit(x), want)
+        unit._wrapped.weight = nn.Parameter(torch.zeros(24, 48))
+        assert torch.equal(unit(x), want)
+        twin = copy.deepcopy(unit)
+        twin._wrapped.__dict__["weight"] = torch.zeros(24, 48)
+        assert torch.equal(twin(x), want)
+        unit.flat_param.mul_(2.0)
+        assert torch.allclose(unit(x), want * 2.0, rtol=1e-5, atol=1e-6)
