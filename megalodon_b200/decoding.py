@@ -310,6 +310,11 @@ class DecodeSession:
         self.pos.add_(1).remainder_(m.chunk_size)
         return logits[:, -1].float()
 
+    def _eager_step(self) -> Tensor:
+        logits = self._step_body()
+        # (the chain's logits buffer belongs to the next step)
+        return logits.clone() if self._native else logits
+
     def _stats(self, norm):
         """Running statistics as the modules take them."""
         count, mean, var = norm
@@ -327,9 +332,7 @@ class DecodeSession:
             self.model.eval()
         try:
             if self._fresh or not self.use_graph or self._eager_steps < 2:
-                self.logits = self._step_body()
-                if self._native:             # the chain's logits buffer belongs to the next step
-                    self.logits = self.logits.clone()
+                self.logits = self._eager_step()
                 self._fresh = False
                 self._eager_steps += 1
                 return self.logits
@@ -356,7 +359,7 @@ class DecodeSession:
                                             "continuing with eager fixed-shape steps")
                 torch.cuda.synchronize()
                 self.use_graph = False
-                self.logits = self._step_body()
+                self.logits = self._eager_step()
                 return self.logits
             self.logits = captured
             self._graph = graph

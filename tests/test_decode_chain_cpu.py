@@ -120,3 +120,20 @@ def test_step_through_the_modules_takes_fp32_statistics(monkeypatch):
     sess.dtype = torch.bfloat16
     count, mean, var = sess._stats(sess.layers[0]["norm"])
     assert mean.dtype == var.dtype == torch.bfloat16 and count.dtype == torch.int64
+
+
+def test_logits_of_a_step_outlive_the_next(monkeypatch):
+    """Eager steps hand out memory of their own, the one after a capture that did not work among them."""
+    import contextlib
+    sess, _ = _session(monkeypatch)
+    sess.use_graph = True
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: None)
+
+    @contextlib.contextmanager
+    def no_capture(*a, **k):
+        raise RuntimeError("not capturable")
+        yield
+    monkeypatch.setattr(torch.cuda, "graph", no_capture)
+    outs = [sess.step(torch.tensor([1, 2])) for _ in range(5)]
+    assert not sess.use_graph and len({o.data_ptr() for o in outs}) == 5
