@@ -136,4 +136,5 @@ def test_logits_of_a_step_outlive_the_next(monkeypatch):
         yield
     monkeypatch.setattr(torch.cuda, "graph", no_capture)
     outs = [sess.step(torch.tensor([1, 2])) for _ in range(5)]
-    assert not sess.use_graph and len({o.data_ptr() for o in outs}) == 5
+    held = {o.data_ptr() for o in outs}
+    assert not sess.use_graph and len(held) == 5 and sess._buf["logits"].data_ptr() not in held
