@@ -19,7 +19,7 @@ On CPU, with tensor-parallel ranks, or with `use_graph=False` the same code
 runs eagerly, which is what the tests compare against the regular cache path.
 
 On one GPU with 16-bit weights the step is a chain of native launches
-(`_native_step`): per layer four products and five kernels for everything
+(`_native_step`): per layer four products and four kernels for everything
 between them, each a link of a programmatic dependent launch chain, instead of
 some thirty-five launches through the modules.
 """
@@ -281,7 +281,7 @@ class DecodeSession:
         C.decode_norm_ema(x, norm.weight, norm.bias, count, mean, var, b["t"], None, None, None, None, None, None, None,
                           self.pos, m.chunk_size, norm.eps, 0.0, True)
         products([b["t"]], [m.output.output.weight], [None], [None], [0], [b["logits"]])
-        cuda_ops._bump(9 * n + 2)
+        cuda_ops._bump(8 * n + 2)        # (the EMA coefficients count themselves)
         return b["logits"]
 
     # ------------------------------------------------------------------ one token

@@ -138,3 +138,13 @@ def test_logits_of_a_step_outlive_the_next(monkeypatch):
     outs = [sess.step(torch.tensor([1, 2])) for _ in range(5)]
     held = {o.data_ptr() for o in outs}
     assert not sess.use_graph and len(held) == 5 and sess._buf["logits"].data_ptr() not in held
+
+
+def test_launches_are_counted(monkeypatch):
+    from megalodon_b200.ops import cuda_ops
+    sess, rec = _session(monkeypatch)
+    before = cuda_ops.count_launches()
+    sess.step(torch.tensor([1, 2]))
+    # (attention is two launches: the splits and their combination)
+    made = sum(2 if name == "decode_attend" else 1 for name, _ in rec.calls if name != "decode_attend_splits")
+    assert made == 8 * sess.mega.num_layers + 2 and cuda_ops.count_launches() - before == made
