@@ -305,12 +305,18 @@ std::vector<Tensor> cema_coeffs_bwd(const OptTensor& dp, const OptTensor& dq, co
 }
 
 // ------------------------------------------------------------------ element-wise
-Tensor swiglu_fwd(const Tensor& a, const Tensor& b) {
+void check_swiglu(const Tensor& a, const Tensor& b) {
   check_cuda_contig(a, "a");
   check_cuda_contig(b, "b");
+  TORCH_CHECK(a.numel() == b.numel() && (a.scalar_type() == b.scalar_type() || a.scalar_type() == at::kFloat),
+              "swiglu: a and b must match in size, and in type unless a is fp32");
+}
+
+Tensor swiglu_fwd(const Tensor& a, const Tensor& b) {
+  check_swiglu(a, b);
   c10::cuda::CUDAGuard guard(a.device());
-  Tensor out = torch::empty_like(a);
-  mb::swiglu_fwd(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), dtype_code(a), stream());
+  Tensor out = torch::empty_like(b);
+  mb::swiglu_fwd(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), dtype_code(a), dtype_code(b), stream());
   return out;
 }
 
@@ -326,10 +332,12 @@ Tensor silu_bwd(const Tensor& g, const Tensor& a) {
 
 std::tuple<Tensor, Tensor> swiglu_bwd(const Tensor& g, const Tensor& a, const Tensor& b) {
   check_cuda_contig(g, "g");
+  check_swiglu(a, b);
+  TORCH_CHECK(g.numel() == b.numel() && g.scalar_type() == b.scalar_type(), "swiglu_bwd: g and b must match");
   c10::cuda::CUDAGuard guard(a.device());
-  Tensor da = torch::empty_like(a), db = torch::empty_like(b);
+  Tensor da = torch::empty(a.sizes(), b.options()), db = torch::empty_like(b);
   mb::swiglu_bwd(g.data_ptr(), a.data_ptr(), b.data_ptr(), da.data_ptr(), db.data_ptr(), a.numel(), dtype_code(a),
-                 stream());
+                 dtype_code(b), stream());
   return {da, db};
 }
 

@@ -8,8 +8,11 @@ namespace mb {
 namespace {
 
 // n8 groups of 8 elements through 16-byte accesses, then a scalar tail of n - 8 * n8 elements
-template <typename T>
-__global__ void swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
+// a in the type of b, or in fp32: the MEGA gate's SiLU acts on what the product accumulated.  4096 x 8192 gates: forward
+// 48 us, backward 68 (45 and 62 with a 16-bit a, whose rounding costs up to |a| times its own error); the product before
+// it takes 191 us instead of 185, against 252 with the SiLU in its epilogue and 530 with the pre-activation kept as well.
+template <typename A, typename T>
+__global__ void swiglu_fwd_kernel(const A* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                                   long long n, long long n8) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -25,8 +28,8 @@ __global__ void swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__
   for (long long i = 8 * n8 + tid; i < n; i += stride) out[i] = from_f<T>(silu_f(to_f(a[i])) * to_f(b[i]));
 }
 
-template <typename T>
-__global__ void swiglu_bwd_kernel(const T* __restrict__ g, const T* __restrict__ a, const T* __restrict__ b,
+template <typename A, typename T>
+__global__ void swiglu_bwd_kernel(const T* __restrict__ g, const A* __restrict__ a, const T* __restrict__ b,
                                   T* __restrict__ da, T* __restrict__ db, long long n, long long n8) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -402,11 +405,16 @@ int ew_grid(long long n) { return (int)std::min<long long>(div_up(n, 256), 148LL
 
 }  // namespace
 
-void swiglu_fwd(const void* a, const void* b, void* out, long long n, int dtype, cudaStream_t st) {
+void swiglu_fwd(const void* a, const void* b, void* out, long long n, int a_dtype, int dtype, cudaStream_t st) {
   if (n == 0) return;
   const long long n8 = (aligned32(a) && aligned32(b) && aligned32(out)) ? n / 8 : 0;
-  MB_DISPATCH_DTYPE(dtype, (swiglu_fwd_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
-                               (const scalar_t*)a, (const scalar_t*)b, (scalar_t*)out, n, n8)));
+  const int grid = ew_grid(std::max(n8, n - 8 * n8));
+  MB_DISPATCH_DTYPE(dtype, {
+    if (a_dtype == dtype)
+      swiglu_fwd_kernel<<<grid, 256, 0, st>>>((const scalar_t*)a, (const scalar_t*)b, (scalar_t*)out, n, n8);
+    else
+      swiglu_fwd_kernel<<<grid, 256, 0, st>>>((const float*)a, (const scalar_t*)b, (scalar_t*)out, n, n8);
+  });
 }
 
 void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cudaStream_t st) {
@@ -416,13 +424,19 @@ void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cu
                                (const scalar_t*)g, (const scalar_t*)a, (scalar_t*)da, n, n8)));
 }
 
-void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db, long long n, int dtype,
+void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db, long long n, int a_dtype, int dtype,
                 cudaStream_t st) {
   if (n == 0) return;
   const long long n8 = (aligned32(g) && aligned32(a) && aligned32(b) && aligned32(da) && aligned32(db)) ? n / 8 : 0;
-  MB_DISPATCH_DTYPE(dtype, (swiglu_bwd_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
-                               (const scalar_t*)g, (const scalar_t*)a, (const scalar_t*)b, (scalar_t*)da,
-                               (scalar_t*)db, n, n8)));
+  const int grid = ew_grid(std::max(n8, n - 8 * n8));
+  MB_DISPATCH_DTYPE(dtype, {
+    if (a_dtype == dtype)
+      swiglu_bwd_kernel<<<grid, 256, 0, st>>>((const scalar_t*)g, (const scalar_t*)a, (const scalar_t*)b, (scalar_t*)da,
+                                              (scalar_t*)db, n, n8);
+    else
+      swiglu_bwd_kernel<<<grid, 256, 0, st>>>((const scalar_t*)g, (const float*)a, (const scalar_t*)b, (scalar_t*)da,
+                                              (scalar_t*)db, n, n8);
+  });
 }
 
 void rotary_apply(const void* x, const float* freqs, void* out, long long rows, int L, int H, int Dh,

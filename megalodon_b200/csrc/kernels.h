@@ -65,9 +65,10 @@ void cema_coeffs_bwd(const float* dp, const float* dq, const float* dg, const vo
                      int dtype, cudaStream_t st);
 
 // ---- element-wise (elementwise_kernels.cu)
-void swiglu_fwd(const void* a, const void* b, void* out, long long n, int dtype, cudaStream_t st);
+// a_dtype: that of b or fp32; everything else, the gradient of a included, in the type of b
+void swiglu_fwd(const void* a, const void* b, void* out, long long n, int a_dtype, int dtype, cudaStream_t st);
 void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cudaStream_t st);
-void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db, long long n, int dtype,
+void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db, long long n, int a_dtype, int dtype,
                 cudaStream_t st);
 void rotary_apply(const void* x, const float* freqs, void* out, long long rows, int L, int H, int Dh,
                   bool conj, int dtype, cudaStream_t st);

@@ -203,7 +203,8 @@ class MovingAverageGatedAttention(nn.Module):
         self.znorm = FusedRMSNorm(self.z_head_dim, elementwise_affine=False, eps=norm_eps)
 
         init_fn = get_init_fn(init_mode)
-        # v and r carry a SiLU that is fused into the GEMM epilogue
+        # v and r carry a SiLU that is fused into the GEMM epilogue; as part of a `linear_group` r leaves in fp32 and
+        # its SiLU is taken where the gate is applied
         self.wv = ColumnParallelLinear(mdim, hdim, bias=True, input_is_parallel=True,
                                        gather_output=False, init_method=init_fn, activation="silu")
         self.wz = ColumnParallelLinear(mdim, zdim, bias=True, input_is_parallel=False,
@@ -294,7 +295,7 @@ class MovingAverageGatedAttention(nn.Module):
         fused_adds = get_model_parallel_world_size() == 1 and not (self.training and self.dropout > 0.0)
         if fused_adds and is_plain(self.wz, ColumnParallelLinear) and is_plain(self.wr, ColumnParallelLinear):
             z, r, h = ops.linear_group(mx, [(self.wz.weight, self.wz.bias, None),
-                                            (self.wr.weight, self.wr.bias, None, "silu"),
+                                            (self.wr.weight, self.wr.bias, None, True),
                                             (self.wh1.weight, self.wh1.bias, residual)])
         else:
             z, r = self.wz(mx), self.wr(mx)
@@ -307,7 +308,7 @@ class MovingAverageGatedAttention(nn.Module):
         v = self.wv(out_tsn)          # SiLU fused
 
         attn, cache_attn = self.inner_attention(q, k, v, mask, None, cache_attn)
-        attn = ops.memory_efficient_dropout(attn * r, self.hidden_dropout, self.training)
+        attn = ops.memory_efficient_dropout(ops.gate(r, attn), self.hidden_dropout, self.training)
 
         if fused_adds:
             out = ops.linear_add(attn, self.wh2.weight, None, h)

@@ -75,14 +75,20 @@ def linear_fp32_out(x: Tensor, w: Tensor) -> Tensor:
 
 
 def linear_group(x: Tensor, layers):
-    """Several linear layers of one input: [(w, b, addend or None[, act]), ...] -> [act(x w^T + b) (+ addend), ...]; a
-    layer with an activation takes no addend."""
-    layers = [layer if len(layer) == 4 else (*layer, None) for layer in layers]
-    assert not any(a is not None and act is not None for _, _, a, act in layers)
+    """Several linear layers of one input: [(w, b, addend or None[, gate]), ...] -> [x w^T + b (+ addend), ...].  A
+    layer marked as gate (True; it takes no addend) gives what `gate` multiplies by."""
+    layers = [layer if len(layer) == 4 else (*layer, False) for layer in layers]
+    assert not any(a is not None and is_gate for _, _, a, is_gate in layers)
     if native_for(x):
         return _cuda().linear_group(x, layers)
-    return [reference.linear(x, w, b, act) if a is None else reference.linear(x, w, b, None) + a
-            for w, b, a, act in layers]
+    return [reference.linear(x, w, b, "silu" if is_gate else None) if a is None else reference.linear(x, w, b, None) + a
+            for w, b, a, is_gate in layers]
+
+
+def gate(r, x: Tensor) -> Tensor:
+    """SiLU(x_r w^T + b) * x for the gate `r` of a `linear_group`: its activation rounded to the type of x, or still the
+    fp32 pre-activation."""
+    return x * r if isinstance(r, Tensor) else _cuda().gate(r, x)
 
 
 def qk_rotary(z: Tensor, gamma: Tensor, beta: Tensor, freqs_cis: Tensor, head_dim: int):

@@ -8,7 +8,7 @@ autograd wrappers and native fwd/bwd entry points
 from __future__ import annotations
 
 import os
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 import torch.nn.functional as F
@@ -257,58 +257,63 @@ class _LinearAdd(torch.autograd.Function):
         return dx, dw, db, (dy if ctx.needs_input_grad[3] else None)
 
 
+class GateInput(NamedTuple):
+    """What a gate's SiLU acts on, in fp32, and a 16-bit tensor of the same shape without memory of its own that stands
+    for it in autograd: the gradient of a 16-bit product is 16-bit, as it is wanted by the products behind it."""
+    pre: Tensor
+    handle: Tensor
+
+
 class _LinearGroup(torch.autograd.Function):
-    """Several linear layers of one input: (act_i(x w_i^T + b_i) [+ addend_i])_i, a layer with an activation having no
-    addend.  Backward adds up the input gradients in the epilogues of the data-gradient products, so the sum over the
-    layers costs no pass of its own.  Arguments after x: w, b, addend, act per layer."""
+    """Several linear layers of one input: (x w_i^T + b_i [+ addend_i])_i.  Backward adds up the input gradients in
+    the epilogues of the data-gradient products, so the sum over the layers costs no pass of its own.  Arguments after
+    x: w, b, addend, gate per layer.  A gate leaves as fp32 pre-activation, with its handle (see `GateInput`) among the
+    further outputs; for few rows without gradients as the 16-bit SiLU."""
 
     @staticmethod
     def forward(ctx, x, *layers):
         x2 = x.reshape(-1, x.shape[-1])
-        ws, bs, adds, acts = (layers[i::4] for i in range(4))
-        outs = [torch.empty(*x.shape[:-1], w.shape[0], dtype=x.dtype, device=x.device) for w in ws]
-        ys = [o.view(-1, o.shape[-1]) for o in outs]
+        ws, bs, adds, gates = (layers[i::4] for i in range(4))
         a2 = [None if a is None else a.reshape(-1, a.shape[-1]).contiguous() for a in adds]
-        pres = [None] * len(ws)
-        keep_pre = any(ctx.needs_input_grad) and any(acts)
         pending = any(getattr(w, "_gather_spec", None) is not None and w._gather_spec.pending for w in ws)
-        rc = -1
-        if x2.shape[0] <= _SKINNY_MAX_ROWS and len(ws) <= 4 and not pending and not keep_pre:
-            rc = _C().skinny_gemm([x2] * len(ws), list(ws), [None] * len(ws), list(bs), a2,
-                                  [1 if act == "silu" else 0 for act in acts], ys, False, _err_flag(x.device))
+        few = (x2.shape[0] <= _SKINNY_MAX_ROWS and len(ws) <= 4 and not pending
+               and not (any(gates) and any(ctx.needs_input_grad)))
+        if few:
+            outs = [torch.empty(*x.shape[:-1], w.shape[0], dtype=x.dtype, device=x.device) for w in ws]
+            rc = _C().skinny_gemm([x2] * len(ws), list(ws), [None] * len(ws), list(bs), a2, [int(g) for g in gates],
+                                  [o.view(-1, o.shape[-1]) for o in outs], False, _err_flag(x.device))
             if rc not in (0, -1):
                 raise RuntimeError(f"few-row products: launch failed with code {rc}")
             _bump(1 if rc == 0 else 0)
-        if rc != 0:
-            for i, (w, b, a, act) in enumerate(zip(ws, bs, a2, acts)):
-                if act is not None and keep_pre:
-                    y, pres[i] = _gemm_gathering(x2, w, b, act, want_preact=True)
-                    outs[i] = y.view(outs[i].shape)
-                else:
-                    _gemm_gathering(x2, w, b, act, out=ys[i], **({} if a is None else {"softmax": dict(aux=a)}))
-        ctx.save_for_backward(x2, *ws, *[p for p in pres if p is not None])
+            few = rc == 0
+        handles = []
+        if not few:
+            outs = [torch.empty(*x.shape[:-1], w.shape[0], dtype=torch.float32 if gate else x.dtype, device=x.device)
+                    for w, gate in zip(ws, gates)]
+            for w, b, a, o in zip(ws, bs, a2, outs):
+                _gemm_gathering(x2, w, b, None, out=o.view(-1, o.shape[-1]), **({} if a is None else {"softmax": dict(aux=a)}))
+            handles = [x.new_empty(1).expand(o.shape) for o, gate in zip(outs, gates) if gate]
+            ctx.mark_non_differentiable(*[o for o, gate in zip(outs, gates) if gate])
+        ctx.save_for_backward(x2, *ws)
         ctx.sinks = [getattr(w, "_wgrad_sink", None) for w in ws]
         ctx.bias_dtypes = [None if b is None else b.dtype for b in bs]
-        ctx.has_pre = [p is not None for p in pres]
+        ctx.gates = gates
         ctx.x_shape = x.shape
         ctx.set_materialize_grads(False)
-        return tuple(outs)
+        return (*outs, *handles)
 
     @staticmethod
     def backward(ctx, *dys):
-        n = len(dys)
-        x2, saved = ctx.saved_tensors[0], ctx.saved_tensors[1:]
-        ws, pres = saved[:n], iter(saved[n:])
+        x2, *ws = ctx.saved_tensors
+        handles = iter(dys[len(ws):])
         dx, grads = None, []
-        for i, (dy, w) in enumerate(zip(dys, ws)):
+        for i, w in enumerate(ws):
             need_w, need_b, need_a = ctx.needs_input_grad[1 + 4 * i:4 + 4 * i]
-            pre = next(pres) if ctx.has_pre[i] else None
+            dy = next(handles, None) if ctx.gates[i] else dys[i]
             if dy is None:
                 grads += [None] * 4
                 continue
             g = dy.reshape(-1, dy.shape[-1]).contiguous()
-            if pre is not None:
-                g = silu_bwd(g, pre)
             if ctx.needs_input_grad[0]:
                 if dx is None:
                     dx, _ = gemm(g, w, None, None, b_mn=True)
@@ -321,13 +326,39 @@ class _LinearGroup(torch.autograd.Function):
 
 
 def linear_group(x: Tensor, layers):
-    """[(w, b, addend or None, act or None), ...] of one input -> the list of act(x w^T + b) (+ addend)."""
+    """[(w, b, addend or None, gate), ...] of one input -> the list of x w^T + b (+ addend), of a gate what `gate`
+    takes."""
     x2 = x.reshape(-1, x.shape[-1])
     if (x.dtype == torch.float32 or _GEMM_BACKEND[0] != "tcgen05" or x2.shape[0] <= 1 or not _tma_ok(x2)
             or any(w.dtype != x.dtype or w.shape[0] % 8 != 0 or not _tma_ok(w) or (a is not None and a.dtype != x.dtype)
                    for w, _, a, _ in layers)):
-        return [linear(x, w, b, act) if a is None else linear_add(x, w, b, a) for w, b, a, act in layers]
-    return list(_apply(_LinearGroup, x, *[t for layer in layers for t in layer]))
+        return [linear(x, w, b, "silu" if gate else None) if a is None else linear_add(x, w, b, a)
+                for w, b, a, gate in layers]
+    res = _apply(_LinearGroup, x, *[t for layer in layers for t in layer])
+    handles = iter(res[len(layers):])
+    return [GateInput(y, next(handles)) if gate and len(res) > len(layers) else y
+            for y, (_, _, _, gate) in zip(res, layers)]
+
+
+class _Gate(torch.autograd.Function):
+    """silu(pre) * x, `pre` in fp32."""
+
+    @staticmethod
+    def forward(ctx, pre, handle, x):
+        x = x.contiguous()
+        ctx.save_for_backward(pre, x)
+        _bump()
+        return _C().swiglu_fwd(pre, x)
+
+    @staticmethod
+    def backward(ctx, g):
+        pre, x = ctx.saved_tensors
+        _bump()
+        return (None, *_C().swiglu_bwd(g.contiguous(), pre, x))
+
+
+def gate(r: GateInput, x: Tensor) -> Tensor:
+    return _apply(_Gate, r.pre, r.handle, x)
 
 
 def _weight_grad(g: Tensor, x2: Tensor, w: Tensor, sink) -> Optional[Tensor]:

@@ -267,32 +267,63 @@ def test_gate_is_rounded_after_its_activation(monkeypatch):
 
 
 @pytest.mark.parametrize("rows", [1, 2, 64, 65, 300])
-def test_linear_group_with_an_activation(rows):
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_linear_group_with_a_gate(rows, dtype):
     from megalodon_b200 import ops
     torch.manual_seed(rows)
     K, sizes = 264, (64, 136, 264)
-    x, add = _rand(rows, K), _rand(rows, sizes[2])
-    ws, bs = [_rand(n, K, scale=K ** -0.5) for n in sizes], [_rand(n) for n in sizes]
-    gs = [_rand(rows, n) for n in sizes]
-    leaves = [t.clone().requires_grad_(True) for t in (x, add, *ws, *bs)]
+    x, add, v = _rand(rows, K, dtype=dtype), _rand(rows, sizes[2], dtype=dtype), _rand(rows, sizes[1], dtype=dtype)
+    ws, bs = [_rand(n, K, scale=K ** -0.5, dtype=dtype) for n in sizes], [_rand(n, dtype=dtype) for n in sizes]
+    gs = [_rand(rows, n, dtype=dtype) for n in sizes]
+    leaves = [t.clone().requires_grad_(True) for t in (x, add, *ws, *bs, v)]
 
     def outs(t):
-        return [t[0] @ t[2].t() + t[5], torch.nn.functional.silu(t[0] @ t[3].t() + t[6]), t[0] @ t[4].t() + t[7] + t[1]]
+        return [t[0] @ t[2].t() + t[5], torch.nn.functional.silu(t[0] @ t[3].t() + t[6]) * t[8], t[0] @ t[4].t() + t[7] + t[1]]
 
     def group(t):
-        return ops.linear_group(t[0], [(t[2], t[5], None), (t[3], t[6], None, "silu"), (t[4], t[7], t[1], None)])
+        a, r, c = ops.linear_group(t[0], [(t[2], t[5], None), (t[3], t[6], None, True), (t[4], t[7], t[1], False)])
+        return [a, ops.gate(r, t[8]), c]
     got = group(leaves)
     torch.autograd.backward(got, gs)
-    ref = [t.double().requires_grad_(True) for t in (x, add, *ws, *bs)]
+    ref = [t.double().requires_grad_(True) for t in (x, add, *ws, *bs, v)]
     want = outs(ref)
     torch.autograd.backward(want, [g.double() for g in gs])
     with torch.no_grad():
         again = group(leaves)
-    for o, n, w in zip(got, again, want):
-        assert _rel(o, w) < 2.0 ** -8 and _rel(n, w) < 2.0 ** -8
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for i, (o, n, w) in enumerate(zip(got, again, want)):
+        # one rounding; two where the gate is rounded before it is applied (few rows)
+        assert _rel(o, w) < eps * (1 + (i == 1)) and _rel(n, w) < eps * (1 + (i == 1))
     for i, (a, r) in enumerate(zip(leaves, ref)):
-        # dx and what comes through the activation: rounded once more on the way
-        assert _rel(a.grad, r.grad) < (2.0 ** -7 if i in (0, 3, 6) else 2.0 ** -8), i
+        # dx and what comes through the gate: rounded once more on the way
+        assert _rel(a.grad, r.grad) < (2 if i in (0, 3, 6, 8) else 1) * eps, i
+    # the gate alone, and the group without it
+    a, r, c = ops.linear_group(leaves[0], [(leaves[2], leaves[5], None), (leaves[3], None, None, True)])[:2] + [None]
+    da, = torch.autograd.grad(ops.gate(r, v), leaves[0], gs[1], retain_graph=True)
+    z = x.double() @ ws[1].double().t()
+    s = torch.sigmoid(z)
+    assert _rel(da, (gs[1].double() * v.double() * s * (1 + z * (1 - s))) @ ws[1].double()) < 2 * eps
+    assert _rel(torch.autograd.grad(a, leaves[0], gs[0])[0], gs[0].double() @ ws[0].double()) < 2 * eps
+
+
+@pytest.mark.parametrize("n", [7, 4096, 100003])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_of_a_wider_input(n, dtype):
+    """a in fp32 against b in 16 bits, whole pieces and a tail, aligned and not."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(n)
+    for off in (0, 1):
+        a = _rand(n + off, dtype=torch.float32, scale=3.0)[off:]
+        b, g = _rand(n + off, dtype=dtype)[off:], _rand(n + off, dtype=dtype)[off:]
+        ad, bd = a.double(), b.double()
+        s = torch.sigmoid(ad)
+        eps = 1.01 * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+        out = cuda_ops._C().swiglu_fwd(a, b)
+        da, db = cuda_ops._C().swiglu_bwd(g, a, b)
+        for got, want in ((out, ad * s * bd), (da, g.double() * bd * (s + ad * s * (1 - s))), (db, g.double() * ad * s)):
+            assert got.dtype == dtype and ((got.double() - want).abs() <= eps * want.abs() + 1e-6).all()
+    with pytest.raises(Exception):
+        cuda_ops._C().swiglu_fwd(a, b[:-1])
 
 
 def _coefficient_args(dtype=torch.float32, D=12, N=4):
