@@ -1300,7 +1300,8 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
                       const GemmPeerSpec* peers, bool accumulate, const GemmGatherSpec* gather,
                       const GemmSoftmaxSpec* softmax, const GemmOuterBatch* outer, int tile) {
   const int nb2 = outer != nullptr ? outer->count : 1;
-  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || nb2 <= 0) return 0;
+  if (M <= 0 || N <= 0 || batch <= 0 || nb2 <= 0) return 0;
+  if (K <= 0) return -12;      // (an empty sum is the caller's: no tile would write it)
   // TMA wants 16-byte strides; the vectorised epilogue wants 16-byte aligned rows of C
   if (lda % 8 != 0 || ldb % 8 != 0 || ldc % 8 != 0) return -1;
   if (batch > 1 && (a_bs % 8 != 0 || b_bs % 8 != 0 || c_bs % 8 != 0)) return -1;

@@ -134,7 +134,6 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
     out_dtype = out_dtype or (out.dtype if out is not None else a.dtype)
     native = (_GEMM_BACKEND[0] == "tcgen05" and a.dtype in (torch.bfloat16, torch.float16)
               and _tma_ok(a) and _tma_ok(b)
-              and a.shape[-2 if a_mn else -1] > 0         # (an empty sum: no tile would write the zeros)
               # the epilogue stores 16-byte pieces of rows that start on a 16-byte boundary
               and (_tma_ok(out) if out is not None else (b.shape[-1] if b_mn else b.shape[-2]) % 8 == 0))
     if a_part_ptrs or c_part_ptrs or b_gather:
@@ -154,25 +153,7 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
     if softmax and addend is None and not native:
         raise RuntimeError("fused-softmax epilogues need the tcgen05 backend and TMA-compatible operands")
     if not native:
-        A = a.transpose(-1, -2) if a_mn else a
-        Bm = b if b_mn else b.transpose(-1, -2)
-        pre = torch.matmul(A, Bm)
-        if alpha != 1.0:
-            pre = pre * alpha
-        if bias is not None:
-            pre = pre + bias.to(pre.dtype)
-        res = F.silu(pre) if act == "silu" else pre
-        if addend is not None:
-            res = res + addend
-        if mode == 1:       # the kernel leaves tiles above the diagonal unwritten; nothing reads them
-            pass
-        if out is not None:
-            if accumulate:
-                out.add_(res.to(out.dtype))
-            else:
-                out.copy_(res)
-            res = out
-        return res.to(out_dtype), (pre.to(out_dtype) if want_preact else None)
+        return _matmul(a, b, bias, act, a_mn, b_mn, want_preact, out_dtype, out, alpha, accumulate, addend)
     if (a.dim() == 2 and a.shape[0] <= _SKINNY_MAX_ROWS and not a_mn and not b_mn and mode == 0 and alpha == 1.0
             and not want_preact and not accumulate and (not softmax or addend is not None)):
         res = _few_rows(a, b, bias, act, out_dtype, out, addend)
@@ -183,8 +164,30 @@ def gemm(a: Tensor, b: Tensor, bias: Optional[Tensor] = None, act: Optional[str]
                              _DT[out_dtype], mode, alpha, _err_flag(a.device),
                              accumulate=bool(accumulate and out is not None), **(softmax or {}))
     if rc != 0:
+        if a.shape[-2 if a_mn else -1] == 0 and (not softmax or addend is not None):
+            # an empty sum: no tile would write the zeros
+            return _matmul(a, b, bias, act, a_mn, b_mn, want_preact, out_dtype, out, alpha, accumulate, addend)
         raise RuntimeError(f"tcgen05 GEMM launch failed with code {rc}")
     return res, pre
+
+
+def _matmul(a: Tensor, b: Tensor, bias, act, a_mn, b_mn, want_preact, out_dtype, out, alpha, accumulate, addend):
+    """`gemm` as torch.matmul, for operands that the kernels do not take.  (`mode` only spares work.)"""
+    pre = torch.matmul(a.transpose(-1, -2) if a_mn else a, b if b_mn else b.transpose(-1, -2))
+    if alpha != 1.0:
+        pre = pre * alpha
+    if bias is not None:
+        pre = pre + bias.to(pre.dtype)
+    res = F.silu(pre) if act == "silu" else pre
+    if addend is not None:
+        res = res + addend
+    if out is not None:
+        if accumulate:
+            out.add_(res.to(out.dtype))
+        else:
+            out.copy_(res)
+        res = out
+    return res.to(out_dtype), (pre.to(out_dtype) if want_preact else None)
 
 
 def _few_rows(a: Tensor, b: Tensor, bias, act, out_dtype, out, addend) -> Optional[Tensor]:
