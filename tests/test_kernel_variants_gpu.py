@@ -400,3 +400,58 @@ def test_empty_sums(rows):
     for accumulate, want in ((True, target.clone()), (False, torch.zeros_like(target))):
         cuda_ops.gemm(_rand(0, 32), _rand(0, 64), a_mn=True, b_mn=True, out=target, accumulate=accumulate)
         assert torch.equal(target, want)
+
+
+class _Pending:
+    """What a sharded weight carries while its all-gather is left to the first product (one GPU: the row blocks of two
+    ranks as two tensors)."""
+
+    def __init__(self, w, blocks):
+        self.w, self.blocks, self.pending, self.how = w, blocks, True, None
+
+    def sources(self):
+        return [b.data_ptr() for b in self.blocks], 1
+
+    def done(self):
+        self.pending, self.how = False, "product"
+
+    def pull_now(self):
+        self.w.copy_(torch.cat(self.blocks))
+        self.pending, self.how = False, "pull"
+
+
+@pytest.mark.parametrize("rows", [1, 5, 64, 300])
+@pytest.mark.parametrize("grad", [False, True])
+def test_linear_group_gathers_sharded_weights(rows, grad):
+    """No kernel may read a weight that has not been gathered; where the shape allows it the product gathers it."""
+    from megalodon_b200 import ops
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(rows)
+    K, sizes = 128, (256, 512, 256)
+    x, add, v = _rand(rows, K), _rand(rows, sizes[2]), _rand(rows, sizes[1])
+    true = [_rand(n, K, scale=K ** -0.5) for n in sizes]
+    bs = [_rand(n) for n in sizes]
+    ws, specs = [], []
+    for t in true:
+        w = torch.full_like(t, float("nan"))
+        blocks = [t[: t.shape[0] // 2].clone(), t[t.shape[0] // 2:].clone()]
+        w[t.shape[0] // 2:] = blocks[1]                     # this rank's own rows are in place
+        w._gather_spec = _Pending(w, blocks)
+        specs.append(w._gather_spec)
+        ws.append(w)
+    xl = x.clone().requires_grad_(grad)
+    with torch.set_grad_enabled(grad):
+        a, r, c = ops.linear_group(xl, [(ws[0], bs[0], None), (ws[1], bs[1], None, True), (ws[2], bs[2], add)])
+        b = ops.gate(r, v)
+    torch.cuda.synchronize()
+    assert [s.how for s in specs] == ["product" if rows > 128 else "pull"] * 3
+    lin = [x.double() @ t.double().t() + bias.double() for t, bias in zip(true, bs)]
+    want = [lin[0], torch.nn.functional.silu(lin[1]) * v.double(), lin[2] + add.double()]
+    for got, ref in zip((a, b, c), want):
+        assert _rel(got, ref) < 2.0 ** -7
+    assert all(torch.equal(w, t) for w, t in zip(ws, true))
+    if grad:
+        dx, = torch.autograd.grad([a, c], xl, [a.detach(), c.detach()])
+        ref = a.double() @ true[0].double() + c.double() @ true[2].double()
+        assert _rel(dx, ref) < 2.0 ** -7
+    cuda_ops.check_kernel_errors()
