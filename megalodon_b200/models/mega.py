@@ -27,6 +27,7 @@ from ..modules import (
     RotaryEmbedding,
     TimestepNorm,
 )
+from ..modules.moving_average_gated_attention import _InnerAttention, explicit_causal_mask
 from ..parallel import (
     FullyShardedDataParallel,
     checkpoint_wrapper,
@@ -315,10 +316,18 @@ class Mega(nn.Module):
         return logits, (cache_layers, tuple(out_state))
 
     def _causal_mask(self, x: Tensor, rows: int, past: int):
-        first = self.layers[0]
-        while hasattr(first, "_wrapped"):
-            first = first._wrapped
-        return first.mega.inner_attention.causal_mask(x, rows, past)
+        """Mask argument of the layers: see `_InnerAttention.causal_mask`, whose marker is only for layers that all know
+        it and have no dropout to apply."""
+        if self.efficient_attn:
+            return None
+        inner = []
+        for layer in self.layers:
+            while hasattr(layer, "_wrapped"):
+                layer = layer._wrapped
+            inner.append(layer.mega.inner_attention)
+        if all(is_plain(a, _InnerAttention) for a in inner):
+            return max(inner, key=lambda a: a.training and a.dropout > 0.0).causal_mask(x, rows, past)
+        return explicit_causal_mask(x, rows, past)
 
     def _piece_loss(self, xn: Tensor, targets: Tensor) -> Tensor:
         logits = self.output.output(xn)

@@ -58,6 +58,12 @@ class _CausalMask:
 CAUSAL = _CausalMask()
 
 
+def explicit_causal_mask(x: Tensor, rows: int, past: int) -> Tensor:
+    """Additive mask [1, 1, rows, past + rows] of queries after `past` cached keys, in the type of x."""
+    mask = torch.full((1, 1, rows, rows + past), float("-inf"), device=x.device)
+    return torch.triu(mask, diagonal=past + 1).to(x.dtype)
+
+
 class _InnerAttention(nn.Module):
     """Causal attention restricted to fixed-size chunks.  Sequences longer than
     a chunk are folded to [(B * n_chunks), chunk, H, d]; the KV cache only ever
@@ -152,8 +158,7 @@ class _InnerAttention(nn.Module):
         if not (self.training and self.dropout > 0.0) and ops.attention_native(x, self.z_head_dim, self.v_head_dim,
                                                                                rows + past):
             return CAUSAL
-        mask = torch.full((1, 1, rows, rows + past), float("-inf"), device=x.device)
-        return torch.triu(mask, diagonal=past + 1).to(x.dtype)
+        return explicit_causal_mask(x, rows, past)
 
     def extra_repr(self) -> str:
         return (f"heads={self.n_heads}, z_head_dim={self.z_head_dim}, "

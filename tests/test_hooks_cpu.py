@@ -94,3 +94,60 @@ def test_a_replaced_output_projection_is_called():
         h.remove()
     torch.testing.assert_close(got, want + 1.0)
     torch.testing.assert_close(more, want + 2.0)
+
+
+def _attentions(model):
+    return [_block(model, i).mega for i in range(2)]
+
+
+def test_marker_for_the_causal_mask_stays_among_its_own(monkeypatch):
+    """`CAUSAL` is handed only to layers that know it: a replaced or observed attention gets the mask itself, and dropout
+    in any layer asks for it too."""
+    from megalodon_b200 import ops
+    from megalodon_b200.modules.moving_average_gated_attention import CAUSAL, _InnerAttention
+    model = _model(efficient_attn=None, attention_dropout=0.1)
+    model.eval()
+    toks = torch.randint(0, 96, (2, 12))
+    with torch.no_grad():
+        want, _ = model(toks)
+    monkeypatch.setattr(ops, "attention_native", lambda *a: True)
+    masks = []
+
+    class Recorder(_InnerAttention):
+        def forward(self, xq, xk, xv, mask, *rest):
+            masks.append(mask)
+            return super().forward(xq, xk, xv, mask, *rest)
+
+    class Foreign(torch.nn.Module):                          # knows nothing of the marker
+        def __init__(self, inner):
+            super().__init__()
+            self.call = [inner]
+
+        def forward(self, *args):
+            masks.append(args[3])
+            return self.call[0](*args)
+
+    def run():
+        masks.clear()
+        with torch.no_grad():
+            got, _ = model(toks)
+        torch.testing.assert_close(got, want, rtol=1e-4, atol=1e-4)
+    x = torch.zeros(1, 1, 64)
+    assert model._wrapped._causal_mask(x, 12, 0) is CAUSAL
+    run()
+    last = _attentions(model)[1]
+    last.inner_attention.__class__ = Recorder
+    run()
+    assert torch.is_tensor(masks[0])
+    last.inner_attention.__class__ = _InnerAttention
+    plain = last.inner_attention
+    last.inner_attention = Foreign(plain)
+    run()
+    assert torch.is_tensor(masks[0])
+    last.inner_attention = plain
+    h = plain.register_forward_pre_hook(lambda m, a: masks.append(a[3]))
+    run()
+    h.remove()
+    assert torch.is_tensor(masks[0])
+    plain.train()                                            # dropout acts in this layer alone
+    assert torch.is_tensor(model._wrapped._causal_mask(x, 12, 0))
