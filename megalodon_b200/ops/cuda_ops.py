@@ -77,9 +77,9 @@ def _bump(n: int = 1) -> None:
 
 
 def set_gemm_backend(name: str) -> None:
-    """"tcgen05": this framework's kernel (CTA pairs, 256 x 256 tiles, for more than 128 rows);
-    "tcgen05_1cta": the same kernel family restricted to single-CTA 128 x 256 tiles;
-    "cublas": torch.matmul (baseline only)."""
+    """"tcgen05": this framework's kernels (few-row kernels up to 64 rows; above, CTA pairs with 256 x 256 tiles or
+    single CTAs with 128 x 256, 128 or 64, whichever is estimated to be fastest); "tcgen05_1cta": without the CTA
+    pairs; "cublas": torch.matmul (baseline only)."""
     assert name in ("tcgen05", "tcgen05_1cta", "cublas")
     if name.startswith("tcgen05"):
         require().gemm_set_cta_pairs(name == "tcgen05")
@@ -441,6 +441,8 @@ def linear(x: Tensor, w: Tensor, b: Optional[Tensor] = None, act: Optional[str] 
 
 def linear_fp32_out(x: Tensor, w: Tensor) -> Tensor:
     """x w^T in fp32 as accumulated, without autograd (logits)."""
+    if _transformed():
+        return linear(x, w).float()
     x2 = x.reshape(-1, x.shape[-1])
     y, _ = _gemm_gathering(x2, w, None, None, out_dtype=torch.float32)
     return y.view(*x.shape[:-1], w.shape[0])

@@ -455,3 +455,16 @@ def test_linear_group_gathers_sharded_weights(rows, grad):
         ref = a.double() @ true[0].double() + c.double() @ true[2].double()
         assert _rel(dx, ref) < 2.0 ** -7
     cuda_ops.check_kernel_errors()
+
+
+def test_fp32_products_without_gradients_refuse_what_linear_refuses():
+    from megalodon_b200 import ops
+    x, w = _rand(70, 64), _rand(128, 64, scale=0.1)
+    with torch.no_grad():
+        assert ops.linear_fp32_out(x, w).dtype == torch.float32
+        with torch.autograd.forward_ad.dual_level():
+            dual = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+            with pytest.raises(Exception):
+                ops.linear_fp32_out(dual, w)
+        with pytest.raises(Exception):
+            torch.func.vmap(lambda r: ops.linear_fp32_out(r[None], w))(x)
