@@ -11,7 +11,7 @@
 //   wgrad    dw = dy^T x      A = dy [T, N'] MN-major,  B = x  [T, K'] MN-major
 //
 // CTA = 6 warps: warp 0 issues TMA loads (128B-swizzled tiles, no multicast)
-// into a 4-stage shared-memory ring; warp 1 issues tcgen05.mma (128 x BN x 16)
+// into a shared-memory ring (4, 6 or 8 stages for BN = 256, 128, 64); warp 1 issues tcgen05.mma (128 x BN x 16)
 // into one of two TMEM accumulators; warps 2-5 drain the other accumulator
 // with tcgen05.ld, apply bias / SiLU and store, so the epilogue of tile i
 // overlaps the main loop of tile i+1.  Tiles are walked M-fastest so CTAs that

@@ -186,8 +186,9 @@ def test_native_session_without_cached_coefficients(dtype, training, use_graph):
     with torch.no_grad():
         for i in range(8):
             ref, cache = model(tok[:, i:i + 1], cache=cache)
-            # some ten roundings to `eps` a layer on either side, adding up like a random walk
-            assert _rel(got[i], ref[:, -1]) < 2 * (10 * cfg.num_layers) ** 0.5 * eps, i
+            # some ten roundings a layer on either side, each of about 0.4 eps, adding up like a random walk (0.0143 seen
+            # in bf16, 0.0017 in fp16); half as much again
+            assert _rel(got[i], ref[:, -1]) < 0.6 * (2 * 10 * cfg.num_layers) ** 0.5 * eps, i
     cuda_ops.check_kernel_errors()
 
 
@@ -250,8 +251,9 @@ def test_native_session_with_hooks_adapters_and_new_weights():
                     if undo is not None:
                         undo()
             outs.append(torch.stack(rows))
-        # some ten roundings to 2^-11 a layer on either side, adding up like a random walk
-        assert _rel(*outs) < 2 * (10 * cfg.num_layers) ** 0.5 * 2.0 ** -11
+        # some ten roundings a layer on either side, each of about 0.4 x 2^-11, adding up like a random walk (0.0012 seen);
+        # half as much again
+        assert _rel(*outs) < 0.6 * (2 * 10 * cfg.num_layers) ** 0.5 * 2.0 ** -11
         return sess._native, outs[0]
 
     block = model._wrapped.layers[1]
