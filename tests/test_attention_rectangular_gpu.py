@@ -138,3 +138,25 @@ def test_attention_of_odd_strides(shape, stride, offset):
         res.append([out, *torch.autograd.grad(out, leaves, norm(ts[3]))])
     for a, b in zip(*res):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("pieces", [(512, 511), (300, 700), (5, 900, 100)])
+def test_model_in_pieces_against_the_whole(fused, pieces):
+    """Several tokens at a time against a growing cache give the logits of one call over all of them."""
+    from megalodon_b200.config import ModelConf
+    from megalodon_b200.models.mega import build_model
+    from megalodon_b200.utils import init_cache, set_random_seed
+    cfg = ModelConf(num_layers=2, model_dim=256, num_heads=2, z_dim=128, value_dim=512, ffn_hidden_dim=384, chunk_size=1024,
+                    vocab_size=520, swiglu=True, norm_num_groups=16, efficient_attn="fused" if fused else None)
+    set_random_seed(3)
+    model = build_model(cfg, "fp16", False, True).eval()
+    tok = torch.randint(0, 520, (2, sum(pieces)), device="cuda")
+    with torch.no_grad():
+        want, _ = model(tok, cache=init_cache(2, model, torch.float16))
+        cache, at = init_cache(2, model, torch.float16), 0
+        for n in pieces:
+            got, cache = model(tok[:, at:at + n], cache=cache)
+            # some ten roundings to 2^-11 a layer on either side, adding up like a random walk
+            assert _rel(got, want[:, at:at + n]) < (2 * 10 * cfg.num_layers) ** 0.5 * 2.0 ** -11, n
+            at += n
