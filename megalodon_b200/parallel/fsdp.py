@@ -461,21 +461,12 @@ class FullyShardedDataParallel(nn.Module):
             self._full.untyped_storage().resize_(0)
 
     def _param_views(self, flat: torch.Tensor) -> List[torch.Tensor]:
-        """One view per parameter; the flat buffer is cut in one call, at the parameters and the gaps behind them."""
+        """One view per parameter of the (contiguous) flat buffer.  Each is a view of its own: pieces of one split could
+        not be modified in place where gradients are recorded."""
         if self._cuts is None:
-            sizes, at, pos = [], [], 0
-            for info in self._infos:                      # ascending offsets
-                if info.offset > pos:
-                    sizes.append(info.offset - pos)
-                at.append(len(sizes))
-                sizes.append(info.numel)
-                pos = info.offset + info.numel
-            if pos < self._numel_padded:
-                sizes.append(self._numel_padded - pos)
-            self._cuts = (sizes, at)
-        sizes, at = self._cuts
-        pieces = flat.split_with_sizes(sizes)
-        return [pieces[i].view(info.shape) for i, info in zip(at, self._infos)]
+            self._cuts = [(info.shape, torch.empty(info.shape, device="meta").stride(), info.offset) for info in self._infos]
+        base = flat.storage_offset()
+        return [flat.as_strided(shape, stride, base + offset) for shape, stride, offset in self._cuts]
 
     def _set_views(self, leaf: torch.Tensor, track: bool = False) -> None:
         """Hand the wrapped modules views of `leaf`.  With `track` the views come out of `_FlatViews`

@@ -119,3 +119,16 @@ def test_views_are_handed_out_again_where_a_module_lost_its_own():
         assert torch.equal(twin(x), want)
         unit.flat_param.mul_(2.0)
         assert torch.allclose(unit(x), want * 2.0, rtol=1e-5, atol=1e-6)
+
+
+def test_views_of_frozen_weights_can_be_modified_in_place():
+    """An adapter folded into a frozen weight while gradients are recorded."""
+    unit, ref = _unit(mixed=False)
+    x, delta = torch.randn(4, 48), torch.full((24, 48), 0.5, requires_grad=True)
+    unit.flat_param.requires_grad_(False)
+    unit(x)
+    w = unit._wrapped.weight
+    assert torch.equal(w, ref.weight) and torch.equal(unit._wrapped.bias, ref.bias)
+    w.add_(delta)
+    w.sum().backward()
+    assert torch.equal(delta.grad, torch.ones_like(delta))
