@@ -324,8 +324,8 @@ class Mega(nn.Module):
         for layer in self.layers:
             while hasattr(layer, "_wrapped"):
                 layer = layer._wrapped
-            inner.append(layer.mega.inner_attention)
-        if all(is_plain(a, _InnerAttention) for a in inner):
+            inner.append(getattr(getattr(layer, "mega", None), "inner_attention", None))
+        if inner and all(is_plain(a, _InnerAttention) for a in inner):
             return max(inner, key=lambda a: a.training and a.dropout > 0.0).causal_mask(x, rows, past)
         return explicit_causal_mask(x, rows, past)
 

@@ -151,3 +151,14 @@ def test_marker_for_the_causal_mask_stays_among_its_own(monkeypatch):
     assert torch.is_tensor(masks[0])
     plain.train()                                            # dropout acts in this layer alone
     assert torch.is_tensor(model._wrapped._causal_mask(x, 12, 0))
+
+
+def test_mask_of_layers_that_are_not_the_models_own(monkeypatch):
+    from megalodon_b200 import ops
+    model = _model(efficient_attn=None)._wrapped
+    monkeypatch.setattr(ops, "attention_native", lambda *a: True)
+    x = torch.zeros(1, 1, 64)
+    model.layers = torch.nn.ModuleList([model.layers[0], torch.nn.Identity()])
+    assert torch.is_tensor(model._causal_mask(x, 12, 0))
+    model.layers = torch.nn.ModuleList()
+    assert torch.is_tensor(model._causal_mask(x, 12, 3))
