@@ -685,7 +685,7 @@ class _CEMACoeffs(torch.autograd.Function):
         params = ctx.saved_tensors
         if torch.is_grad_enabled():
             outs = reference.cema_coeffs(*params, ctx.scale)
-            used = [(o, g) for o, g in zip(outs, (dp, dq, dg)) if g is not None]
+            used = [(o, g) for o, g in zip(outs, (dp, dq, dg)) if g is not None and o.requires_grad]
             wanted = [t for t, need in zip(params, ctx.needs_input_grad) if need]
             grads = iter(torch.autograd.grad([o for o, _ in used], wanted, [g for _, g in used], create_graph=True,
                                              allow_unused=True))

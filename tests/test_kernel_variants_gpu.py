@@ -357,6 +357,10 @@ def test_cema_coefficients_differentiate_twice():
     q = ops.cema_coeffs(alpha, *base[1:], 0.5)[1]
     first, = torch.autograd.grad(q.real.sum(), alpha, create_graph=True)
     assert torch.autograd.grad(first.sum(), alpha)[0].abs().sum() > 0
+    theta = base[2].clone().requires_grad_(True)             # p and gamma do not depend on it
+    p, q, g = ops.cema_coeffs(*base[:2], theta, base[3], 0.5)
+    first, = torch.autograd.grad(p.sum() + q.real.sum() + g.abs().sum(), theta, create_graph=True)
+    assert torch.autograd.grad(first.sum(), theta)[0].abs().sum() > 0
 
 
 def test_cema_coefficients_under_transforms_and_other_types():
