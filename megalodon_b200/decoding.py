@@ -135,7 +135,7 @@ class DecodeSession:
         if cuda_ops.gemm_backend() != "tcgen05" or m.embed.weight.shape[1] != m.model_dim:
             return False
         # a sharded unit gives its gathered weights back after every call of its own
-        if hasattr(self.model, "_units") and any(u.reshard_after_forward and not u._is_root for u in self.model._units()):
+        if any(u.reshard_after_forward and not u._is_root for u in self._units()) or not self._weights_current():
             return False
         if not self._as_built():
             return False
@@ -153,6 +153,19 @@ class DecodeSession:
         fn, out = m.output.final_norm, m.output.output
         return (C.decode_norm_ema_ok(m.model_dim, fn.groups_per_partition, 2) and out.weight.shape[1] == m.model_dim
                 and self._params_ok([fn.weight, fn.bias, out.weight]))
+
+    def _units(self):
+        return [u for u in self.model.modules() if hasattr(u, "_full_is_valid")]
+
+    def _weights_current(self) -> bool:
+        """Whether the gathered weights are what the units' own calls would use, after bringing them up to date where
+        the session's model can (it may have been given the model inside its root unit)."""
+        if all(u._full_is_valid() for u in self._units()):
+            return True
+        if not hasattr(self.model, "materialize_views"):
+            return False
+        self.model.materialize_views()
+        return True
 
     def _params_ok(self, params) -> bool:
         return all(p.dtype == self.dtype and p.is_contiguous() and p.data_ptr() % 16 == 0 for p in params)
@@ -286,10 +299,8 @@ class DecodeSession:
 
     # ------------------------------------------------------------------ one token
     def _step_body(self) -> Tensor:
-        if self._native and self._as_built():        # (a hook or an adapter may have come since)
-            # what the units' own calls would bring up to date after an optimiser step or a load
-            if hasattr(self.model, "_units") and not all(u._full_is_valid() for u in self.model._units()):
-                self.model.materialize_views()
+        # (a hook or an adapter may have come since, an optimiser step or a load)
+        if self._native and self._as_built() and self._weights_current():
             return self._native_step()
         m = self.mega
         x = m.embed(self.tok)

@@ -148,3 +148,19 @@ def test_launches_are_counted(monkeypatch):
     # (attention is two launches: the splits and their combination)
     made = sum(2 if name == "decode_attend" else 1 for name, _ in rec.calls if name != "decode_attend_splits")
     assert made == 8 * sess.mega.num_layers + 2 and cuda_ops.count_launches() - before == made
+
+
+def test_a_session_on_the_model_inside_its_root_unit(monkeypatch):
+    """Its units cannot all be brought up to date from here: after an update the step goes through their own calls."""
+    from megalodon_b200.decoding import DecodeSession
+    sess, _ = _session(monkeypatch)
+    inner = DecodeSession(sess.mega, 2, torch.float32, use_graph=False)
+    reached = []
+    inner._native = True
+    monkeypatch.setattr(inner, "_native_step", lambda: (reached.append("chain"), torch.zeros(2, 96))[1])
+    assert inner._weights_current()
+    inner.step(torch.tensor([1, 2]))
+    assert reached == ["chain"]
+    with torch.no_grad():
+        inner._units()[0].flat_param.mul_(1.5)
+    assert not inner._weights_current()
