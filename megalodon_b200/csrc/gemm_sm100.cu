@@ -14,8 +14,8 @@
 // into a shared-memory ring (4, 6 or 8 stages for BN = 256, 128, 64); warp 1 issues tcgen05.mma (128 x BN x 16)
 // into one of two TMEM accumulators; warps 2-5 drain the other accumulator
 // with tcgen05.ld, apply bias / SiLU and store, so the epilogue of tile i
-// overlaps the main loop of tile i+1.  Tiles are walked M-fastest so CTAs that
-// run together share B tiles in L2.
+// overlaps the main loop of tile i+1.  Tiles are walked in bands of rows so that
+// CTAs that run together share A and B tiles in L2 (see `row_band`).
 //
 // All mbarrier waits are bounded; a timeout sets `*err` and the CTA unwinds
 // (releasing its TMEM) instead of hanging.
@@ -71,6 +71,7 @@ struct GemmParams {
   int* err;
   long long ldc;       // elements
   int mode;            // 0 dense, 1..3 see above
+  int band;            // row tiles of a band of the tile walk (`row_band`)
   float alpha;         // C = alpha * acc (+ bias)
   int accumulate;      // 1: C += alpha * acc (+ bias); the old C is read in the epilogue
   int batch;           // independent problems sharing shapes (tensor maps carry their strides)
@@ -118,14 +119,24 @@ struct TmapArray {
   CUtensorMap m[kMaxPeers];
 };
 
+// Tile `t` of a problem, walked band after band of `band` row tiles and inside a band column by column.
+__device__ __forceinline__ void banded_tile(int t, int num_m, int num_n, int band, int& mt, int& nt) {
+  const int b = t / (band * num_n), r = t - b * band * num_n;
+  const int rows = min(band, num_m - b * band);
+  nt = r / rows;
+  mt = b * band + (r - nt * rows);
+}
+
 struct TileCoord {
   int m0, n0, bz;
 };
 template <int BN>
-__device__ __forceinline__ TileCoord decode_tile(int tile, int num_m, int tiles_per_batch) {
+__device__ __forceinline__ TileCoord decode_tile(int tile, int num_m, int num_n, int band) {
+  const int tiles_per_batch = num_m * num_n;
   const int bz = tile / tiles_per_batch;
-  const int t = tile - bz * tiles_per_batch;
-  return {(t % num_m) * BM, (t / num_m) * BN, bz};
+  int mt, nt;
+  banded_tile(tile - bz * tiles_per_batch, num_m, num_n, band, mt, nt);
+  return {mt * BM, nt * BN, bz};
 }
 
 template <int BN>
@@ -311,8 +322,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
   const int lane = threadIdx.x & 31;
   const int num_m = (p.M + BM - 1) / BM;
   const int num_n = (p.N + BN - 1) / BN;
-  const int tiles_per_batch = num_m * num_n;
-  const int num_tiles = tiles_per_batch * p.batch;
+  const int num_tiles = num_m * num_n * p.batch;
   const int num_k = (p.K + BK - 1) / BK;
   constexpr uint32_t kTmemCols = 2 * BN;     // two accumulators (a power of two)
 
@@ -347,7 +357,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TileCoord tc = decode_tile<BN>(tile, num_m, tiles_per_batch);
+        const TileCoord tc = decode_tile<BN>(tile, num_m, num_n, p.band);
         const int m0 = tc.m0, n0 = tc.n0, bo = tc.bz / p.batch_in, bi = tc.bz - bo * p.batch_in;
         if (tile_skipped<BN>(p, m0, n0)) continue;
         int kb0, kb1;
@@ -390,7 +400,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TileCoord tc = decode_tile<BN>(tile, num_m, tiles_per_batch);
+        const TileCoord tc = decode_tile<BN>(tile, num_m, num_n, p.band);
         const int m0 = tc.m0, n0 = tc.n0;
         if (tile_skipped<BN>(p, m0, n0)) continue;
         int kb0, kb1;
@@ -429,7 +439,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
     OutT* C = reinterpret_cast<OutT*>(p.C);
     OutT* P = reinterpret_cast<OutT*>(p.preact);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      const TileCoord tc = decode_tile<BN>(tile, num_m, tiles_per_batch);
+      const TileCoord tc = decode_tile<BN>(tile, num_m, num_n, p.band);
       const int m0 = tc.m0, n0 = tc.n0;
       if (tile_skipped<BN>(p, m0, n0)) continue;
       if (!wait_or_abort(tmem_full + acc, acc_phase, abort_flag)) { ok = false; break; }
@@ -587,12 +597,13 @@ __device__ __forceinline__ void pair_tile_coords(const GemmParams& p, int tile, 
   }
   bz = tile / tiles_per_batch;
   const int t = tile - bz * tiles_per_batch;
-  int nt = t / num_m;
+  int mt, nt;
+  banded_tile(t, num_m, num_n, p.band, mt, nt);
   if (p.g_world > 0) {
     nt += (int)(((long long)p.g_rank * (p.N / p.g_world)) / kPairBN);
     if (nt >= num_n) nt -= num_n;
   }
-  m0 = (t % num_m) * kPairBM;
+  m0 = mt * kPairBM;
   n0 = nt * kPairBN;
 }
 
@@ -1291,6 +1302,18 @@ static int pick_tile(const GemmParams& p, int num_sms) {
   return best;
 }
 
+// Row tiles (of `bm` rows) of a band of the tile walk: equal bands of at most 4096 rows.  What runs together reads a
+// band of A and the few column tiles of B next to each other in the walk.  Without bands, 16384 rows of A (134 MB at
+// K = 4096) pass through L2 once per column of tiles: 4 GB out of memory for a product of 0.4 GB of operands, and the
+// energy of it comes out of the tensor cores' clock.  16384 x 4096 -> 8192, back to back under the power cap: 1057 us
+// at 915 MHz without bands, 875 with bands of 1024 rows, 850 of 2304, 831 of 4096, 839 of 6144; 16384 x 11264 -> 4096
+// 1469 -> 1208; 4096 rows are 2 to 3 % slower in two bands than in one.
+static int row_band(int M, int bm) {
+  const int num_m = (M + bm - 1) / bm, most = 4096 / bm;
+  const int bands = (num_m + most - 1) / most;
+  return (num_m + bands - 1) / bands;
+}
+
 // Returns 0 on success, negative on a host-side failure.  `err` is a device int
 // that the kernel sets non-zero if one of its bounded waits gives up.
 int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const void* bias, int bias_dtype,
@@ -1352,11 +1375,14 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
   if (tile == 0) tile = pick_tile(p, num_sms);
   if (tile != kPairTile && tile != 64 && tile != 128 && tile != 256) return -11;
   const bool pair = tile == kPairTile && g_use_pair;
+  p.band = row_band(M, pair ? kPairBM : BM);
   if (gather != nullptr && gather->world > 0) {
     // B must be the whole K-major weight, contiguous, its row blocks whole 128-row chunks
     if (!gemm_gather_supported(M, N, K, gather->world) || !pair || a_mn || b_mn || p.batch != 1 || mode != 0 ||
         p.a_parts != 1 || ldb != K || gather->world > kMaxPeers || gather->flags == nullptr || B != gather->dst)
       return -9;
+    // (the rows of a chunk are wanted by all row tiles as soon as it has come in)
+    p.band = (M + kPairBM - 1) / kPairBM;
     p.g_world = gather->world; p.g_rank = gather->rank; p.g_dst = gather->dst; p.g_flags = gather->flags;
     for (int i = 0; i < gather->world; ++i) p.g_src[i] = gather->src[i];
   }

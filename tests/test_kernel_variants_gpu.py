@@ -226,6 +226,20 @@ def test_tiles(tile, M, N, K):
             assert _rel(out, ref) < tol
 
 
+@pytest.mark.parametrize("tile", [64, 128, 256, 512])
+@pytest.mark.parametrize("M,batch", [(4096, 1), (4097, 2), (8448, 1), (12301, 1)])
+def test_tiles_in_bands(tile, M, batch):
+    """The tile walk in bands of rows: one band, a last band of one row, equal bands, a ragged last tile."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(M)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, b = _rand(batch, M, 72), _rand(batch, 520, 72, scale=72 ** -0.5)
+    out, _, rc = cuda_ops._C().gemm(a, b, None, None, 0, False, False, False, 1, 0, 1.0, err, tile=tile)
+    assert rc == 0 and err.item() == 0
+    ref = a.double() @ b.double().transpose(1, 2)
+    assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()   # every tile: fp32 sums, one rounding
+
+
 def test_operators_without_gradients_match_the_recorded_ones():
     """The short route under no_grad against the autograd function, and what the latter refuses stays refused."""
     from megalodon_b200 import ops
