@@ -10,9 +10,9 @@
 //   dgrad    dx = dy w        A = dy [M, N'] K-major,   B = w  [N', K'] MN-major
 //   wgrad    dw = dy^T x      A = dy [T, N'] MN-major,  B = x  [T, K'] MN-major
 //
-// CTA = 6 warps: warp 0 issues TMA loads (128B-swizzled tiles, no multicast)
+// CTA = 10 warps (6 for BN = 64): warp 0 issues TMA loads (128B-swizzled tiles, no multicast)
 // into a shared-memory ring (4, 6 or 8 stages for BN = 256, 128, 64); warp 1 issues tcgen05.mma (128 x BN x 16)
-// into one of two TMEM accumulators; warps 2-5 drain the other accumulator
+// into one of two TMEM accumulators; the other warps drain the other accumulator
 // with tcgen05.ld, apply bias / SiLU and store, so the epilogue of tile i
 // overlaps the main loop of tile i+1.  Tiles are walked in bands of rows so that
 // CTAs that run together share A and B tiles in L2 (see `row_band`).
@@ -39,8 +39,7 @@ using namespace ptx;
 constexpr int BM = 128;
 constexpr int BK = 64;          // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int kGemmThreads = 192;
-constexpr int kEpiWarps = 4;
+constexpr int kEpiStageBytes = 32 * 64;   // staging buffer of an epilogue warp: 32 rows of 64 bytes
 constexpr int kMaxPeers = 8;
 
 // Ring of the single-CTA kernel: a tile that walks K alone is bound by one memory latency per ring round, so the
@@ -48,11 +47,14 @@ constexpr int kMaxPeers = 8;
 template <int BN>
 struct SmemLayout {
   static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
+  static constexpr int epi_warps = BN == 64 ? 4 : 8;
+  static constexpr int threads = 64 + 32 * epi_warps;
   static constexpr int a_bytes = BM * BK * 2;       // 16 KiB
   static constexpr int b_bytes = BN * BK * 2;       // 32 KiB at BN = 256
   static constexpr int stage_bytes = a_bytes + b_bytes;
   static constexpr int bar_offset = kStages * stage_bytes;
-  static constexpr int total = bar_offset + 256 + 1024;  // barriers + alignment slack
+  static constexpr int epi_offset = bar_offset + 256;    // barriers
+  static constexpr int total = epi_offset + epi_warps * kEpiStageBytes + 1024;  // + alignment slack
 };
 
 // Triangular (causal) structure, used when the GEMM is one of the products of
@@ -108,6 +110,9 @@ struct GemmParams {
   float* row_out;
   const void* aux;
   int causal_off;
+  // set by the launcher
+  bool staged;         // C, preact and aux suit the 16-byte pieces of `epi_staged`
+  bool bias_vec;       // bias may be read in 16-byte pieces
 };
 
 __device__ __forceinline__ long long c_base(const GemmParams& p, int bz) {
@@ -184,7 +189,9 @@ __device__ __forceinline__ void store_row32<__nv_bfloat16>(__nv_bfloat16* dst, c
       reinterpret_cast<uint4*>(dst)[i] = pk;
     }
   } else {
-    for (int i = 0; i < nvalid; ++i) dst[i] = __float2bfloat16_rn(v[i]);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)      // (unrolled: an index that is not a constant would move v to local memory)
+      if (i < nvalid) dst[i] = __float2bfloat16_rn(v[i]);
   }
 }
 
@@ -205,7 +212,9 @@ __device__ __forceinline__ void store_row32<__half>(__half* dst, const float (&v
       reinterpret_cast<uint4*>(dst)[i] = pk;
     }
   } else {
-    for (int i = 0; i < nvalid; ++i) dst[i] = __float2half_rn(v[i]);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < nvalid) dst[i] = __float2half_rn(v[i]);
   }
 }
 
@@ -216,7 +225,9 @@ __device__ __forceinline__ void store_row32<float>(float* dst, const float (&v)[
     for (int i = 0; i < 8; ++i)
       reinterpret_cast<float4*>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
   } else {
-    for (int i = 0; i < nvalid; ++i) dst[i] = v[i];
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < nvalid) dst[i] = v[i];
   }
 }
 
@@ -232,7 +243,9 @@ __device__ __forceinline__ void add_row32(const OutT* src, float (&v)[32], int n
       for (int j = 0; j < 8; ++j) v[8 * i + j] += t[j];
     }
   } else {
-    for (int i = 0; i < nvalid; ++i) v[i] += to_f(src[i]);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < nvalid) v[i] += to_f(src[i]);
   }
 }
 
@@ -263,17 +276,16 @@ __device__ __forceinline__ void epi_row_end(const GemmParams& p, long long ridx,
   if (p.epi == kEpiRowMax) { if (r.acc > -INFINITY) atomic_max_float(p.row_out + ridx, r.acc); }
   else if (p.epi == kEpiExp) atomicAdd(p.row_out + ridx, r.acc);
 }
-// One 32-column chunk of row `row` (v = alpha * acc).  Returns false when the standard epilogue should run.
+// One 32-column chunk of row `row` (v = alpha * acc).
 template <typename OutT>
-__device__ __forceinline__ bool epi_chunk(const GemmParams& p, float (&v)[32], int row, int col0, int nvalid,
+__device__ __forceinline__ void epi_chunk(const GemmParams& p, float (&v)[32], int row, int col0, int nvalid,
                                           long long off, OutT* C, EpiRow& r) {
-  if (p.epi == kEpiStd) return false;
   const int last = p.mode == 1 ? row + p.causal_off : 0x7fffffff;      // last column that takes part
   if (p.epi == kEpiRowMax) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
       if (i < nvalid && col0 + i <= last) r.acc = fmaxf(r.acc, v[i]);
-    return true;
+    return;
   }
   if (p.epi == kEpiExp) {
 #pragma unroll
@@ -284,13 +296,13 @@ __device__ __forceinline__ bool epi_chunk(const GemmParams& p, float (&v)[32], i
       v[i] = e;
     }
     store_row32<OutT>(C + off, v, nvalid);
-    return true;
+    return;
   }
   if (p.epi == kEpiRowScale) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] *= r.a;
     store_row32<OutT>(C + off, v, nvalid);
-    return true;
+    return;
   }
   // kEpiDS
   float pt[32];
@@ -300,11 +312,312 @@ __device__ __forceinline__ bool epi_chunk(const GemmParams& p, float (&v)[32], i
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = (i < nvalid && col0 + i <= last) ? pt[i] * r.a * (v[i] - r.b) : 0.f;
   store_row32<OutT>(C + off, v, nvalid);
-  return true;
+}
+
+// bias[col, col + 32) added to a thread's 32 columns; columns beyond the last are not read
+__device__ __forceinline__ void add_bias32(const GemmParams& p, int col, float (&v)[32]) {
+  if (p.bias_vec && col + 32 <= p.N) {
+    auto add = [&](auto* bias) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float t[8];
+        load8(bias + col + 8 * i, t);      // the same address in every lane
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[8 * i + j] += t[j];
+      }
+    };
+    if (p.bias_dtype == kF32) add(reinterpret_cast<const float*>(p.bias));
+    else if (p.bias_dtype == kBF16) add(reinterpret_cast<const __nv_bfloat16*>(p.bias));
+    else add(reinterpret_cast<const __half*>(p.bias));
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    if (col + i < p.N) {
+      if (p.bias_dtype == kF32) v[i] += reinterpret_cast<const float*>(p.bias)[col + i];
+      else if (p.bias_dtype == kBF16) v[i] += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i]);
+      else v[i] += __half2float(reinterpret_cast<const __half*>(p.bias)[col + i]);
+    }
+  }
+}
+// SiLU of the epilogues.  A 16-bit result takes the division of two units in the last place of fp32, which is
+// a multiplication and a reciprocal instead of some ten instructions with a branch.
+template <typename OutT>
+__device__ __forceinline__ void silu32(float (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = sizeof(OutT) == 2 ? __fdividef(v[i], 1.f + __expf(-v[i])) : silu_f(v[i]);
+}
+
+// ---- epilogue through staging buffers.  A thread owns one row of the accumulator, so writing its columns straight to
+// global memory makes every warp store touch 32 different lines, 16 bytes each: the load/store unit, not DRAM, then
+// bounds products with short k loops.  Instead a warp collects 64 bytes of each of its 32 rows in shared memory and
+// moves them with instructions that each cover 8 whole segments of 64 bytes; inputs of the epilogue (the accumulated
+// C, an addend, the stored probabilities of the dS epilogue) come in the same way.  Pieces of 16 bytes are
+// XOR-swizzled by the row, which makes both directions conflict-free.  Eight warps, two on each quarter
+// of the accumulator's lanes, so that two instruction streams per scheduler cover one another's latencies; 2 KiB a warp leave the ring of stages as it is and room for a small kernel beside the CTA.
+// us, back to back, before (four warps, bias and pre-activation from scalar accesses in the threads' own rows, the
+// whole tile in local memory where a column index was not a constant; pairs alone staged) and after:
+//   bias + SiLU   6216 x 1024 -> 2048  99 / 33, 6216 x 1024 -> 1024  68 / 25, 4096 x 4096 -> 8192  286 / 209
+//   neither       6216 x 1024 -> 2048  27 / 27, 4096 x 4096 -> 8192  208 / 203
+//   scores of a 4096-token chunk, 4 heads of 256: maxima 36 / 31, exponentials 54 / 45
+__device__ __forceinline__ uint32_t epi_stage_addr(uint32_t base, int row, int piece) {
+  return base + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4);
+}
+__device__ __forceinline__ void lds128(uint32_t addr, uint4& v) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+}
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+template <typename OutT>
+__device__ __forceinline__ uint32_t pack2(float a, float b);
+template <>
+__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+  __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&t);
+}
+template <>
+__device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
+  __half2 t = __floats2half2_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&t);
+}
+template <typename OutT>
+__device__ __forceinline__ void unpack2(uint32_t w, float& a, float& b);
+template <>
+__device__ __forceinline__ void unpack2<__nv_bfloat16>(uint32_t w, float& a, float& b) {
+  a = __uint_as_float(w << 16);
+  b = __uint_as_float(w & 0xffff0000u);
+}
+template <>
+__device__ __forceinline__ void unpack2<__half>(uint32_t w, float& a, float& b) {
+  const __half2 t = *reinterpret_cast<__half2*>(&w);
+  a = __low2float(t);
+  b = __high2float(t);
+}
+// 64 bytes of each of 32 rows, global <-> a warp's staging buffer: lane -> piece (lane & 3) of rows (lane >> 2) + 8 j.
+// Rows from rows_valid and elements from cols_valid on are left alone.  `vec`: the pieces lie on 16-byte boundaries.
+template <typename T>
+__device__ __forceinline__ void epi_load(uint4 (&raw)[4], const T* src, long long ld, int rows_valid, int cols_valid,
+                                         bool vec, int lane) {
+  constexpr int kPiece = 16 / sizeof(T);
+  const int c = (lane & 3) * kPiece;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = 8 * j + (lane >> 2);
+    raw[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (r >= rows_valid) continue;
+    const T* s = src + (long long)r * ld + c;
+    if (vec && c + kPiece <= cols_valid) {
+      raw[j] = *reinterpret_cast<const uint4*>(s);
+    } else if (sizeof(T) == 2) {
+      uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c + i < cols_valid) w[i / 2] |= (uint32_t)reinterpret_cast<const unsigned short*>(s)[i] << (16 * (i & 1));
+      raw[j] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+__device__ __forceinline__ void epi_stage_in(uint32_t stg, const uint4 (&raw)[4], int lane) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sts128(epi_stage_addr(stg, 8 * j + (lane >> 2), lane & 3), raw[j]);
+}
+template <typename T>
+__device__ __forceinline__ void epi_stage_out(uint32_t stg, T* dst, long long ld, int rows_valid, int cols_valid,
+                                              bool vec, int lane) {
+  constexpr int kPiece = 16 / sizeof(T);
+  const int c = (lane & 3) * kPiece;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = 8 * j + (lane >> 2);
+    uint4 v;
+    lds128(epi_stage_addr(stg, r, lane & 3), v);
+    if (r >= rows_valid) continue;
+    T* d = dst + (long long)r * ld + c;
+    if (vec && c + kPiece <= cols_valid) {
+      *reinterpret_cast<uint4*>(d) = v;
+    } else if (sizeof(T) == 2) {
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c + i < cols_valid) reinterpret_cast<unsigned short*>(d)[i] = (unsigned short)(w[i / 2] >> (16 * (i & 1)));
+    } else {
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c + i < cols_valid) reinterpret_cast<uint32_t*>(d)[i] = w[i];
+    }
+  }
+}
+// the thread's own row: 32 columns as floats
+template <typename OutT>
+__device__ __forceinline__ void epi_stage_get(uint32_t stg, int lane, float (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint4 w;
+    lds128(epi_stage_addr(stg, lane, i), w);
+    unpack2<OutT>(w.x, v[8 * i + 0], v[8 * i + 1]);
+    unpack2<OutT>(w.y, v[8 * i + 2], v[8 * i + 3]);
+    unpack2<OutT>(w.z, v[8 * i + 4], v[8 * i + 5]);
+    unpack2<OutT>(w.w, v[8 * i + 6], v[8 * i + 7]);
+  }
+}
+// the thread's 32 columns -> row segments of `dst` (first row and column of the warp's block)
+template <typename OutT>
+__device__ __forceinline__ void epi_store32(uint32_t stg, const float (&v)[32], OutT* dst, long long ld, int rows_valid,
+                                            int cols_valid, bool vec, int lane) {
+  if constexpr (sizeof(OutT) == 2) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      sts128(epi_stage_addr(stg, lane, i),
+             make_uint4(pack2<OutT>(v[8 * i + 0], v[8 * i + 1]), pack2<OutT>(v[8 * i + 2], v[8 * i + 3]),
+                        pack2<OutT>(v[8 * i + 4], v[8 * i + 5]), pack2<OutT>(v[8 * i + 6], v[8 * i + 7])));
+    __syncwarp();
+    epi_stage_out<OutT>(stg, dst, ld, rows_valid, cols_valid, vec, lane);
+    __syncwarp();
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        sts128(epi_stage_addr(stg, lane, i),
+               make_uint4(__float_as_uint(v[16 * h + 4 * i]), __float_as_uint(v[16 * h + 4 * i + 1]),
+                          __float_as_uint(v[16 * h + 4 * i + 2]), __float_as_uint(v[16 * h + 4 * i + 3])));
+      __syncwarp();
+      epi_stage_out<OutT>(stg, dst + 16 * h, ld, rows_valid, cols_valid - 16 * h, vec, lane);
+      __syncwarp();
+    }
+  }
+}
+// Per-row constants of the fused epilogues, folded so that an element costs one FMA plus the operation
+// itself: exp(alpha s - m) = 2^(s * alpha log2e - m log2e); dS = p~ (s * alpha / l - delta / l).
+struct EpiFold {
+  float k1, k2;
+};
+__device__ __forceinline__ EpiFold epi_fold(const GemmParams& p, const EpiRow& er) {
+  if (p.epi == kEpiExp) return {p.alpha * 1.4426950408889634f, er.a * 1.4426950408889634f};
+  if (p.epi == kEpiRowScale) return {p.alpha * er.a, 0.f};
+  if (p.epi == kEpiDS) return {p.alpha * er.a, er.a * er.b};
+  return {p.alpha, 0.f};
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 32 columns of the thread's row: raw accumulator `r` -> values to store in `v`.  MASKED: the tile touches
+// the diagonal or the last column, and columns beyond `last` give zero (and take no part in maxima / sums); other
+// tiles skip the comparison.  The row sum of kEpiExp adds the values before they are rounded to the
+// output type.
+template <bool MASKED>
+__device__ __forceinline__ void epi_compute(const GemmParams& p, const uint32_t (&r)[32], const float (&pt)[32],
+                                            float (&v)[32], int last, int col0, const EpiFold& f, EpiRow& er) {
+  if (p.epi == kEpiRowMax) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (!MASKED || col0 + i <= last) er.acc = fmaxf(er.acc, __uint_as_float(r[i]) * f.k1);
+  } else if (p.epi == kEpiExp) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      float e = ex2_approx(fmaf(__uint_as_float(r[i]), f.k1, -f.k2));
+      if (MASKED && col0 + i > last) e = 0.f;
+      er.acc += e;
+      v[i] = e;
+    }
+  } else if (p.epi == kEpiRowScale) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * f.k1;
+  } else {   // kEpiDS
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const float d = pt[i] * fmaf(__uint_as_float(r[i]), f.k1, -f.k2);
+      v[i] = (MASKED && col0 + i > last) ? 0.f : d;
+    }
+  }
+}
+
+// 32 columns from `col` on of a warp's 32 rows, whose first one lies `off` elements into C.  The read of tensor memory
+// and all global reads are under way before the first wait.  SOFTMAX: one of the fused-softmax epilogues (their kernels
+// are instances of their own: one kernel for both spills registers).
+template <typename OutT, bool SOFTMAX>
+__device__ __forceinline__ void epi_staged(const GemmParams& p, uint32_t t_addr, uint32_t stg, long long off,
+                                           int rows_valid, int col, int row, int lane, const EpiFold& fold, EpiRow& er) {
+  OutT* C = reinterpret_cast<OutT*>(p.C) + off;
+  const int cols_valid = p.N - col;
+  uint32_t r[32];
+  tmem_ld_32x32(t_addr, r);
+  const bool need_in = sizeof(OutT) == 2 && (SOFTMAX ? p.epi == kEpiDS : p.accumulate || p.aux != nullptr);
+  uint4 in[4];
+  if (need_in)
+    epi_load<OutT>(in, !SOFTMAX && p.accumulate ? C : reinterpret_cast<const OutT*>(p.aux) + off, p.ldc, rows_valid,
+                   cols_valid, !SOFTMAX || p.staged, lane);
+  tmem_ld_wait_for(r);
+  float v[32], pt[32];
+  if (need_in) {
+    epi_stage_in(stg, in, lane);
+    __syncwarp();
+    if constexpr (sizeof(OutT) == 2) epi_stage_get<OutT>(stg, lane, pt);
+  }
+  if constexpr (!SOFTMAX) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+    if (p.bias != nullptr) add_bias32(p, col, v);
+    if (need_in) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] += pt[i];
+    }
+    if (p.preact != nullptr)
+      epi_store32<OutT>(stg, v, reinterpret_cast<OutT*>(p.preact) + off, p.ldc, rows_valid, cols_valid, true, lane);
+    if (p.act == 1) silu32<OutT>(v);
+  } else {
+    const int last = p.mode == 1 ? min(row + p.causal_off, p.N - 1) : p.N - 1;
+    // does any row of this warp end inside these columns?  (warp-uniform)
+    if (min(p.mode == 1 ? row - lane + p.causal_off : p.N - 1, p.N - 1) < col + 31)
+      epi_compute<true>(p, r, pt, v, last, col, fold, er);
+    else
+      epi_compute<false>(p, r, pt, v, last, col, fold, er);
+    if (p.epi == kEpiRowMax) return;
+  }
+  epi_store32<OutT>(stg, v, C, p.ldc, rows_valid, cols_valid, !SOFTMAX || p.staged, lane);
+}
+
+// 32 columns written straight from the registers: a C that is split over ranks, rows that start off a 16-byte
+// boundary, fp32 results with inputs, the softmax epilogues of fp32 results and of the single-CTA kernel
+template <typename OutT, bool SOFTMAX>
+__device__ __forceinline__ void epi_direct(const GemmParams& p, uint32_t t_addr, int row, int col0, long long cb,
+                                           EpiRow& er) {
+  OutT* C = reinterpret_cast<OutT*>(p.C);
+  OutT* P = reinterpret_cast<OutT*>(p.preact);
+  uint32_t r[32];
+  tmem_ld_32x32(t_addr, r);
+  tmem_ld_wait_for(r);
+  if (col0 >= p.N || row >= p.M) return;
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+  const int nvalid = min(32, p.N - col0);
+  const long long off = cb + (long long)row * p.ldc + col0;
+  if constexpr (SOFTMAX) {
+    epi_chunk<OutT>(p, v, row, col0, nvalid, off, C, er);
+    return;
+  }
+  if (p.bias != nullptr) add_bias32(p, col0, v);
+  if (p.c_nparts > 1) {
+    // push this 32-column chunk into the slot of the rank that owns these columns
+    const int owner = col0 / p.c_part_cols;
+    OutT* slot = reinterpret_cast<OutT*>(p.c_parts[owner]);
+    store_row32<OutT>(slot + (long long)row * p.c_part_cols + (col0 - owner * p.c_part_cols), v, nvalid);
+    return;
+  }
+  if (p.accumulate) add_row32<OutT>(C + off, v, nvalid);
+  if (p.aux != nullptr) add_row32<OutT>(reinterpret_cast<const OutT*>(p.aux) + off, v, nvalid);   // + addend
+  if (P != nullptr) store_row32<OutT>(P + off, v, nvalid);
+  if (p.act == 1) silu32<OutT>(v);
+  store_row32<OutT>(C + off, v, nvalid);
 }
 
 template <int BN, bool A_MN, bool B_MN, typename OutT>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(SmemLayout<BN>::threads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ GemmParams p, int in_fmt) {
   using L = SmemLayout<BN>;
@@ -333,7 +646,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(tmem_full + i, 1);
-      mbar_init(tmem_empty + i, kEpiWarps);
+      mbar_init(tmem_empty + i, p.epi != kEpiStd ? 4 : L::epi_warps);    // epilogue warps of a tile
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -431,71 +744,45 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
       if (!ok) { *abort_flag = 1; atomicExch(p.err, 2); }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (the other warps)
     const int quarter = warp & 3;              // TMEM lanes [32 * quarter, +32) belong to this warp
+    // Eight warps share a tile's columns; with a softmax epilogue each four take every other tile, whole rows of it, so
+    // that a row's maximum and sum get one contribution from a tile.
+    constexpr int kGroups = L::epi_warps / 4;
+    const bool by_tile = p.epi != kEpiStd;
+    const int group = (warp - 2) / 4;
+    const int cols = by_tile ? BN : BN / kGroups, col_off = by_tile ? 0 : group * cols;
+    const uint32_t stage_buf = smem_u32(smem + L::epi_offset + (warp - 2) * kEpiStageBytes);
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    OutT* C = reinterpret_cast<OutT*>(p.C);
-    OutT* P = reinterpret_cast<OutT*>(p.preact);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const TileCoord tc = decode_tile<BN>(tile, num_m, num_n, p.band);
-      const int m0 = tc.m0, n0 = tc.n0;
-      if (tile_skipped<BN>(p, m0, n0)) continue;
+      const int m0 = tc.m0, n0 = tc.n0 + col_off;
+      if (tile_skipped<BN>(p, m0, tc.n0)) continue;
+      if (kGroups == 2 && by_tile && acc != group) {
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        continue;
+      }
       if (!wait_or_abort(tmem_full + acc, acc_phase, abort_flag)) { ok = false; break; }
       tcgen05_fence_after();
-      const int row = m0 + quarter * 32 + lane;
-      const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
+      const int row_base = m0 + quarter * 32, row = row_base + lane;
+      const uint32_t t_row = tmem_base + acc * BN + col_off + ((uint32_t)(quarter * 32) << 16);
       const long long ridx = (long long)tc.bz * p.M + row;
       const long long cb = c_base(p, tc.bz);
       EpiRow er;
       if (p.epi != kEpiStd) epi_row_begin(p, ridx, row < p.M, er);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (col0 >= p.N) continue;            // warp-uniform
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-        const int nvalid = min(32, p.N - col0);
+      for (int c = 0; c < cols; c += 32) {
+        const int col = n0 + c;
+        if (col >= p.N) break;                // warp-uniform
         if (p.epi != kEpiStd) {
-          if (row < p.M)
-            epi_chunk<OutT>(p, v, row, col0, nvalid, cb + (long long)row * p.ldc + col0,
-                            C, er);
-          continue;
-        }
-        if (p.bias != nullptr) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (i < nvalid) {
-              float bv;
-              if (p.bias_dtype == kF32) bv = reinterpret_cast<const float*>(p.bias)[col0 + i];
-              else if (p.bias_dtype == kBF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col0 + i]);
-              else bv = __half2float(reinterpret_cast<const __half*>(p.bias)[col0 + i]);
-              v[i] += bv;
-            }
-          }
-        }
-        if (row < p.M) {
-          if (p.c_nparts > 1) {
-            // push this 32-column chunk into the slot of the rank that owns these columns
-            const int owner = col0 / p.c_part_cols;
-            OutT* slot = reinterpret_cast<OutT*>(p.c_parts[owner]);
-            store_row32<OutT>(slot + (long long)row * p.c_part_cols + (col0 - owner * p.c_part_cols), v, nvalid);
-          } else {
-            const long long off = cb + (long long)row * p.ldc + col0;
-            if (p.accumulate) add_row32<OutT>(C + off, v, nvalid);
-            if (p.aux != nullptr) add_row32<OutT>(reinterpret_cast<const OutT*>(p.aux) + off, v, nvalid);   // + addend
-            if (P != nullptr) store_row32<OutT>(P + off, v, nvalid);
-            if (p.act == 1) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]);
-            }
-            store_row32<OutT>(C + off, v, nvalid);
-          }
+          epi_direct<OutT, true>(p, t_row + c, row, col, cb, er);
+        } else if (p.staged) {
+          epi_staged<OutT, false>(p, t_row + c, stage_buf, cb + (long long)row_base * p.ldc + col, p.M - row_base, col,
+                                  row, lane, EpiFold{}, er);
+        } else {
+          epi_direct<OutT, false>(p, t_row + c, row, col, cb, er);
         }
       }
       if (p.epi != kEpiStd) epi_row_end(p, ridx, row < p.M, er);
@@ -531,11 +818,11 @@ struct PairSmem {
   static constexpr int b_bytes = (kPairBN / 2) * BK * 2;      // this CTA's 128 rows of B
   static constexpr int stage_bytes = a_bytes + b_bytes;       // 32 KiB
   static constexpr int bar_offset = kPairStages * stage_bytes;
-  // one staging buffer per epilogue warp: 32 rows x 128 bytes (64 columns of a 16-bit output)
-  static constexpr int epi_stage_bytes = 32 * 128;
   static constexpr int epi_offset = bar_offset + 256;
-  static constexpr int total = epi_offset + kEpiWarps * epi_stage_bytes + 1024;
+  static constexpr int total = epi_offset + 8 * kEpiStageBytes + 1024;
 };
+// Epilogue warps; the gathering variant keeps its other four for the copies.
+constexpr int pair_epi_warps(bool gather) { return gather ? 4 : 8; }
 
 __device__ __forceinline__ bool pair_tile_skipped(const GemmParams& p, int m0, int n0) {
   return p.mode == 1 && n0 > m0 + kPairBM - 1;
@@ -549,6 +836,8 @@ __device__ __forceinline__ void pair_k_range(const GemmParams& p, int m0, int nu
 }
 
 constexpr int kGatherWarps = 4;                 // copy warps of the gathering variant
+constexpr int kPairThreads = 64 + 32 * 8;       // producer, MMA issuer and eight epilogue (and copy) warps
+static_assert(pair_epi_warps(true) + kGatherWarps == pair_epi_warps(false), "both variants have ten warps");
 constexpr int kGatherUnitBytes = 8192;          // one claim: 32 lanes x 16 loads of 16 bytes
 
 // Tiles of one batch element that the kernel computes: with mode 1 (causal scores) only those on or below
@@ -666,143 +955,12 @@ __device__ __forceinline__ void gather_copy_warp(const GemmParams& p, int lane) 
   }
 }
 
-// ---- staged epilogue of the pair kernel (16-bit outputs).  A thread owns one row of the accumulator, so
-// writing its 32 columns straight to global memory makes every warp store touch 32 different lines, 16
-// bytes each: the load/store unit, not DRAM, bounds products with short k loops (attention scores: 77 %
-// of the L1 data path busy, tensor pipe 12 %).  Instead the warp collects 64 columns (128 bytes per row)
-// in shared memory and moves them with 8 instructions that each cover 4 whole rows; inputs of the
-// epilogue (the accumulated C, an addend, the stored probabilities of the dS epilogue) come in the same
-// way.  Pieces of 16 bytes are XOR-swizzled by the row, which makes both directions conflict-free.
-__device__ __forceinline__ uint32_t epi_stage_addr(uint32_t base, int row, int piece) {
-  return base + row * 128 + ((piece ^ (row & 7)) << 4);
-}
-__device__ __forceinline__ void lds128(uint32_t addr, uint4& v) {
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-}
-__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-template <typename OutT>
-__device__ __forceinline__ uint32_t pack2(float a, float b);
-template <>
-__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
-  __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&t);
-}
-template <>
-__device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
-  __half2 t = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&t);
-}
-template <>
-__device__ __forceinline__ uint32_t pack2<float>(float a, float) { return __float_as_uint(a); }   // never used
-template <typename OutT>
-__device__ __forceinline__ void unpack2(uint32_t w, float& a, float& b);
-template <>
-__device__ __forceinline__ void unpack2<__nv_bfloat16>(uint32_t w, float& a, float& b) {
-  a = __uint_as_float(w << 16);
-  b = __uint_as_float(w & 0xffff0000u);
-}
-template <>
-__device__ __forceinline__ void unpack2<__half>(uint32_t w, float& a, float& b) {
-  const __half2 t = *reinterpret_cast<__half2*>(&w);
-  a = __low2float(t);
-  b = __high2float(t);
-}
-template <>
-__device__ __forceinline__ void unpack2<float>(uint32_t w, float& a, float& b) { a = b = __uint_as_float(w); }
-// global [32 rows x 64 columns] <-> the warp's staging buffer; rows >= rows_valid are skipped
-template <typename OutT>
-__device__ __forceinline__ void epi_stage_in(uint32_t stg, const OutT* src, long long ld, int rows_valid, int lane) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int r = 4 * j + (lane >> 3), q = lane & 7;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < rows_valid) v = *reinterpret_cast<const uint4*>(src + (long long)r * ld + q * 8);
-    sts128(epi_stage_addr(stg, r, q), v);
-  }
-}
-template <typename OutT>
-__device__ __forceinline__ void epi_stage_out(uint32_t stg, OutT* dst, long long ld, int rows_valid, int lane) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int r = 4 * j + (lane >> 3), q = lane & 7;
-    uint4 v;
-    lds128(epi_stage_addr(stg, r, q), v);
-    if (r < rows_valid) *reinterpret_cast<uint4*>(dst + (long long)r * ld + q * 8) = v;
-  }
-}
-// the thread's own row: 32 columns (half h of the 64) as floats
-template <typename OutT>
-__device__ __forceinline__ void epi_stage_get(uint32_t stg, int lane, int h, float (&v)[32]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 w;
-    lds128(epi_stage_addr(stg, lane, h * 4 + i), w);
-    unpack2<OutT>(w.x, v[8 * i + 0], v[8 * i + 1]);
-    unpack2<OutT>(w.y, v[8 * i + 2], v[8 * i + 3]);
-    unpack2<OutT>(w.z, v[8 * i + 4], v[8 * i + 5]);
-    unpack2<OutT>(w.w, v[8 * i + 6], v[8 * i + 7]);
-  }
-}
-template <typename OutT>
-__device__ __forceinline__ void epi_stage_put(uint32_t stg, int lane, int h, const float (&v)[32]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 w;
-    w.x = pack2<OutT>(v[8 * i + 0], v[8 * i + 1]);
-    w.y = pack2<OutT>(v[8 * i + 2], v[8 * i + 3]);
-    w.z = pack2<OutT>(v[8 * i + 4], v[8 * i + 5]);
-    w.w = pack2<OutT>(v[8 * i + 6], v[8 * i + 7]);
-    sts128(epi_stage_addr(stg, lane, h * 4 + i), w);
-  }
-}
-// Per-row constants of the fused epilogues, folded so that an element costs one FMA plus the operation
-// itself: exp(alpha s - m) = 2^(s * alpha log2e - m log2e); dS = p~ (s * alpha / l - delta / l).
-struct EpiFold {
-  float k1, k2;
-};
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// 32 columns of the thread's row: raw accumulator `r` -> values to store in `v`.  MASKED: the tile touches
-// the diagonal and columns beyond `last` give zero (and take no part in maxima / sums); tiles below the
-// diagonal skip the comparison.  The row sum of kEpiExp adds the values before they are rounded to the
-// output type.
-template <typename OutT, bool MASKED>
-__device__ __forceinline__ void epi_compute(const GemmParams& p, const uint32_t (&r)[32], const float (&pt)[32],
-                                            float (&v)[32], int last, int col0, const EpiFold& f, EpiRow& er) {
-  if (p.epi == kEpiRowMax) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (!MASKED || col0 + i <= last) er.acc = fmaxf(er.acc, __uint_as_float(r[i]));     // raw: scaled by alpha at the end
-  } else if (p.epi == kEpiExp) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      float e = ex2_approx(fmaf(__uint_as_float(r[i]), f.k1, -f.k2));
-      if (MASKED && col0 + i > last) e = 0.f;
-      er.acc += e;
-      v[i] = e;
-    }
-  } else if (p.epi == kEpiRowScale) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * f.k1;
-  } else {   // kEpiDS
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float d = pt[i] * fmaf(__uint_as_float(r[i]), f.k1, -f.k2);
-      v[i] = (MASKED && col0 + i > last) ? 0.f : d;
-    }
-  }
-}
-
-template <bool A_MN, bool B_MN, typename OutT, bool GATHER = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads + (GATHER ? kGatherWarps * 32 : 0), 1)
+template <bool A_MN, bool B_MN, typename OutT, bool GATHER = false, bool SOFTMAX = false>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_constant__ CUtensorMap tmap_b,
                          const __grid_constant__ GemmParams p, int in_fmt) {
   using L = PairSmem;
+  constexpr int kEpi = pair_epi_warps(GATHER);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::bar_offset);     // used in the even CTA only
@@ -831,7 +989,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(tmem_full + i, 1);
-      mbar_init(tmem_empty + i, 2 * kEpiWarps);     // epilogue warps of both CTAs
+      mbar_init(tmem_empty + i, SOFTMAX ? 8 : 2 * kEpi);   // epilogue warps of a tile in both CTAs
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -942,205 +1100,53 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
       }
       if (!ok) { *abort_flag = 1; atomicExch(p.err, 2); }
     }
-  } else if (GATHER && warp >= kGemmThreads / 32) {
+  } else if (GATHER && warp >= 2 + kEpi) {
     // ------------------------------------------------------------ copy warps (gathering variant)
     gather_copy_warp(p, lane);
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+    // ------------------------------------------------------------ epilogue (the other warps, both CTAs)
     const int quarter = warp & 3;
-    const uint32_t stage_buf = smem_u32(smem + L::epi_offset + quarter * L::epi_stage_bytes);
+    // Eight warps share a tile's columns.  With a softmax epilogue each four take every other tile, whole rows of it, so
+    // that a row's maximum and sum get one contribution from a tile.
+    constexpr int kGroups = kEpi / 4;
+    constexpr int kCols = SOFTMAX ? kPairBN : kPairBN / kGroups;
+    constexpr bool kAlways = SOFTMAX && sizeof(OutT) == 2;
+    const int group = (warp - 2) / 4;
+    const int col_off = SOFTMAX ? 0 : group * kCols;
+    const uint32_t stage_buf = smem_u32(smem + L::epi_offset + (warp - 2) * kEpiStageBytes);
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    OutT* C = reinterpret_cast<OutT*>(p.C);
-    OutT* P = reinterpret_cast<OutT*>(p.preact);
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       int m0, n0, bz;
       pair_tile_coords(p, tile, num_m, num_n, tiles_per_batch, num_pairs, m0, n0, bz);
       if (pair_tile_skipped(p, m0, n0)) continue;
+      if (SOFTMAX && kGroups == 2 && acc != group) {
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        continue;
+      }
       if (!wait_or_abort(tmem_full + acc, acc_phase, abort_flag)) { ok = false; break; }
       tcgen05_fence_after();
-      const int row = m0 + (int)rank * BM + quarter * 32 + lane;
-      const uint32_t t_row = tmem_base + acc * kPairBN + ((uint32_t)(quarter * 32) << 16);
+      n0 += col_off;
+      const int row_base = m0 + (int)rank * BM + quarter * 32, row = row_base + lane;
+      const uint32_t t_row = tmem_base + acc * kPairBN + col_off + ((uint32_t)(quarter * 32) << 16);
       const long long ridx = (long long)bz * p.M + row;
       const long long cb = c_base(p, bz);
       EpiRow er;
-      if (p.epi != kEpiStd) epi_row_begin(p, ridx, row < p.M, er);
-      // chunk c (32 columns) written straight from the registers: partial groups, fp32 outputs, split C
-      auto direct_chunk = [&](int c) {
-        uint32_t r[32];
-        tmem_ld_32x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (col0 >= p.N) return;              // warp-uniform
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-        const int nvalid = min(32, p.N - col0);
-        if (p.epi != kEpiStd) {
-          if (row < p.M)
-            epi_chunk<OutT>(p, v, row, col0, nvalid, cb + (long long)row * p.ldc + col0,
-                            C, er);
-          return;
-        }
-        if (p.bias != nullptr) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (i < nvalid) {
-              float bv;
-              if (p.bias_dtype == kF32) bv = reinterpret_cast<const float*>(p.bias)[col0 + i];
-              else if (p.bias_dtype == kBF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col0 + i]);
-              else bv = __half2float(reinterpret_cast<const __half*>(p.bias)[col0 + i]);
-              v[i] += bv;
-            }
-          }
-        }
-        if (row < p.M) {
-          if (p.c_nparts > 1) {
-            const int owner = col0 / p.c_part_cols;
-            OutT* slot = reinterpret_cast<OutT*>(p.c_parts[owner]);
-            store_row32<OutT>(slot + (long long)row * p.c_part_cols + (col0 - owner * p.c_part_cols), v, nvalid);
-          } else {
-            const long long off = cb + (long long)row * p.ldc + col0;
-            if (p.accumulate) add_row32<OutT>(C + off, v, nvalid);
-            if (p.aux != nullptr) add_row32<OutT>(reinterpret_cast<const OutT*>(p.aux) + off, v, nvalid);   // + addend
-            if (P != nullptr) store_row32<OutT>(P + off, v, nvalid);
-            if (p.act == 1) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]);
-            }
-            store_row32<OutT>(C + off, v, nvalid);
-          }
-        }
-            };
-      const int row_base = m0 + (int)rank * BM + quarter * 32;
-      const int rows_valid = p.M - row_base;
-      const bool std_in = p.epi == kEpiStd && (p.accumulate || p.aux != nullptr);
-      // groups of 64 columns: both 32-column reads of tensor memory are issued before the wait, the
-      // results pass through the warp's staging buffer and leave as whole 128-byte row segments
-      const bool can_group = sizeof(OutT) == 2 && P == nullptr && p.c_nparts <= 1 &&
-                             !(p.epi == kEpiStd && p.accumulate && p.aux != nullptr) &&
-                             ((p.ldc | p.c_batch_stride | p.c_outer_stride) & 7) == 0 &&
-                             ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(p.aux)) & 15) == 0 &&
-                             n0 + kPairBN <= p.N && !(p.epi == kEpiRowMax && p.alpha < 0.f);
-      // (the gathering variant, whose 320 threads leave fewer registers each, keeps the direct form: a
-      // register spilled between an asynchronous tensor-memory read and its wait would be read too early)
-      const bool can_group_f32 = !GATHER && sizeof(OutT) == 4 && p.epi == kEpiStd && P == nullptr && p.c_nparts <= 1 &&
-                                 !p.accumulate && p.aux == nullptr && n0 + kPairBN <= p.N &&
-                                 ((p.ldc | p.c_batch_stride | p.c_outer_stride) & 3) == 0 &&
-                                 (reinterpret_cast<uintptr_t>(C) & 15) == 0;
-      if (can_group_f32) {
-        // fp32 results (logits): 32 columns are one staging buffer
-        float* dst = reinterpret_cast<float*>(p.C) + cb + (long long)row_base * p.ldc + n0;
+      if constexpr (SOFTMAX) epi_row_begin(p, ridx, row < p.M, er);
+      const EpiFold fold = SOFTMAX ? epi_fold(p, er) : EpiFold{};
 #pragma unroll 1
-        for (int c = 0; c < kPairBN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_row + c * 32, r);
-          tmem_ld_wait();
-          float v[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int col = n0 + c * 32 + i;
-              float bv;
-              if (p.bias_dtype == kF32) bv = reinterpret_cast<const float*>(p.bias)[col];
-              else if (p.bias_dtype == kBF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col]);
-              else bv = __half2float(reinterpret_cast<const __half*>(p.bias)[col]);
-              v[i] += bv;
-            }
-          }
-          if (p.act == 1) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]);
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint4 w = make_uint4(__float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]),
-                                       __float_as_uint(v[4 * i + 2]), __float_as_uint(v[4 * i + 3]));
-            sts128(epi_stage_addr(stage_buf, lane, i), w);
-          }
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int rr = 4 * j + (lane >> 3), q = lane & 7;
-            uint4 w;
-            lds128(epi_stage_addr(stage_buf, rr, q), w);
-            if (rr < rows_valid) *reinterpret_cast<uint4*>(dst + (long long)rr * p.ldc + c * 32 + q * 4) = w;
-          }
-          __syncwarp();
-        }
-      } else if (GATHER || !can_group) {
-#pragma unroll 1
-        for (int c = 0; c < kPairBN / 32; ++c) direct_chunk(c);
-      } else if constexpr (!GATHER) {
-        const bool need_in = p.epi == kEpiDS || std_in;
-        const OutT* src = (p.epi == kEpiDS || !p.accumulate) ? reinterpret_cast<const OutT*>(p.aux) : C;
-        const long long off_row0 = cb + (long long)row_base * p.ldc + n0;
-        const int last = p.mode == 1 ? row + p.causal_off : 0x7fffffff;
-        // does any row of this warp end inside the tile?  (warp-uniform)
-        const bool masked = p.mode == 1 && n0 + kPairBN - 1 > row_base + p.causal_off;
-        EpiFold fold{p.alpha, 0.f};
-        if (p.epi == kEpiExp) fold = {p.alpha * 1.4426950408889634f, er.a * 1.4426950408889634f};
-        else if (p.epi == kEpiRowScale) fold = {p.alpha * er.a, 0.f};
-        else if (p.epi == kEpiDS) fold = {p.alpha * er.a, er.a * er.b};
-#pragma unroll 1
-        for (int g = 0; g < kPairBN / 64; ++g) {
-          const int colg = n0 + g * 64;
-          const long long off0 = off_row0 + g * 64;
-          uint32_t ra[32], rb[32];
-          tmem_ld_32x32(t_row + g * 64, ra);
-          tmem_ld_32x32(t_row + g * 64 + 32, rb);
-          if (need_in) epi_stage_in<OutT>(stage_buf, src + off0, p.ldc, rows_valid, lane);
-          tmem_ld_wait();
-          if (need_in) __syncwarp();
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int col0 = colg + h * 32;
-            const uint32_t (&rr)[32] = h == 0 ? ra : rb;
-            float v[32], pt[32];
-            if (need_in) epi_stage_get<OutT>(stage_buf, lane, h, pt);
-            if (p.epi != kEpiStd) {
-              if (masked) epi_compute<OutT, true>(p, rr, pt, v, last, col0, fold, er);
-              else epi_compute<OutT, false>(p, rr, pt, v, last, col0, fold, er);
-              if (p.epi == kEpiRowMax) continue;
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(rr[i]) * p.alpha;
-              if (p.bias != nullptr) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                  float bv;
-                  if (p.bias_dtype == kF32) bv = reinterpret_cast<const float*>(p.bias)[col0 + i];
-                  else if (p.bias_dtype == kBF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col0 + i]);
-                  else bv = __half2float(reinterpret_cast<const __half*>(p.bias)[col0 + i]);
-                  v[i] += bv;
-                }
-              }
-              if (need_in) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] += pt[i];
-              }
-              if (p.act == 1) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]);
-              }
-            }
-            epi_stage_put<OutT>(stage_buf, lane, h, v);
-          }
-          if (p.epi != kEpiRowMax) {
-            __syncwarp();
-            epi_stage_out<OutT>(stage_buf, C + off0, p.ldc, rows_valid, lane);
-            __syncwarp();
-          }
-        }
-        if (p.epi == kEpiRowMax) {
-          // the maximum was taken over raw accumulators: alpha >= 0 on this path, so it scales through
-          er.acc = er.acc > -INFINITY ? er.acc * p.alpha : er.acc;
+      for (int c = 0; c < kCols; c += 32) {
+        const int col = n0 + c;
+        if (col >= p.N) break;                // warp-uniform
+        if (kAlways || p.staged) {
+          epi_staged<OutT, SOFTMAX>(p, t_row + c, stage_buf, cb + (long long)row_base * p.ldc + col,
+                                    p.M - row_base, col, row, lane, fold, er);
+        } else {
+          epi_direct<OutT, SOFTMAX>(p, t_row + c, row, col, cb, er);
         }
       }
-      if (p.epi != kEpiStd) epi_row_end(p, ridx, row < p.M, er);
+      if constexpr (SOFTMAX) epi_row_end(p, ridx, row < p.M, er);
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty + acc), 0));
@@ -1224,7 +1230,7 @@ static int launch_gemm(const TmapArray& ta, const CUtensorMap& tb, const GemmPar
   if (!allow_dynamic_smem(kern, L::total, configured)) return -2;
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
   const int grid = tiles < sms ? tiles : sms;
-  kern<<<grid, kGemmThreads, L::total, st>>>(ta, tb, p, in_fmt);
+  kern<<<grid, L::threads, L::total, st>>>(ta, tb, p, in_fmt);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -1241,21 +1247,21 @@ static int launch_gemm_pair_gather(const TmapArray& ta, const CUtensorMap& tb, c
   const int tiles = ((p.M + kPairBM - 1) / kPairBM) * ((p.N + kPairBN - 1) / kPairBN) * p.batch;
   const int pairs = sms / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  kern<<<grid, kGemmThreads + kGatherWarps * 32, L::total, st>>>(ta, tb, p, in_fmt);
+  kern<<<grid, kPairThreads, L::total, st>>>(ta, tb, p, in_fmt);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-template <bool A_MN, bool B_MN, typename OutT>
+template <bool A_MN, bool B_MN, typename OutT, bool SOFTMAX>
 static int launch_gemm_pair(const TmapArray& ta, const CUtensorMap& tb, const GemmParams& p, int in_fmt, int sms,
                             cudaStream_t st) {
   using L = PairSmem;
-  auto kern = gemm_tcgen05_pair_kernel<A_MN, B_MN, OutT>;
+  auto kern = gemm_tcgen05_pair_kernel<A_MN, B_MN, OutT, false, SOFTMAX>;
   static std::atomic<unsigned long long> configured{0};
   if (!allow_dynamic_smem(kern, L::total, configured)) return -2;
   const int tiles = ((p.M + kPairBM - 1) / kPairBM) * ((p.N + kPairBN - 1) / kPairBN) * p.batch;
   const int pairs = sms / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  kern<<<grid, kGemmThreads, L::total, st>>>(ta, tb, p, in_fmt);
+  kern<<<grid, kPairThreads, L::total, st>>>(ta, tb, p, in_fmt);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -1371,6 +1377,16 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
     for (int i = 0; i < p.c_nparts; ++i) p.c_parts[i] = peers->c_ptrs[i];
   }
   if (!ok) return -41;
+  {
+    const bool f32 = out_dtype == kF32;
+    const long long strides = ldc | (batch > 1 ? c_bs : 0) | (nb2 > 1 ? outer->c_stride : 0);
+    const uintptr_t bases = reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(preact) |
+                            reinterpret_cast<uintptr_t>(p.aux);
+    p.staged = p.c_nparts == 1 && (strides & (f32 ? 3 : 7)) == 0 && (bases & 15) == 0 &&
+               !(f32 && (p.epi != kEpiStd || p.accumulate || p.aux != nullptr)) &&
+               !(p.epi == kEpiStd && p.accumulate && p.aux != nullptr);
+    p.bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
+  }
   if (gather != nullptr && gather->world > 0) tile = kPairTile;
   if (tile == 0) tile = pick_tile(p, num_sms);
   if (tile != kPairTile && tile != 64 && tile != 128 && tile != 256) return -11;
@@ -1396,16 +1412,20 @@ int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const
     return launch_gemm_pair_gather<float>(ta, tb, p, fmt, num_sms, st);
   }
   if (pair) {
-#define GEMM_PAIR_CASE(AMN, BMN)                                                                        \
-  if (a_mn == AMN && b_mn == BMN) {                                                                     \
-    if (out_dtype == kBF16) return launch_gemm_pair<AMN, BMN, __nv_bfloat16>(ta, tb, p, fmt, num_sms, st); \
-    if (out_dtype == kF16) return launch_gemm_pair<AMN, BMN, __half>(ta, tb, p, fmt, num_sms, st);      \
-    return launch_gemm_pair<AMN, BMN, float>(ta, tb, p, fmt, num_sms, st);                              \
+#define GEMM_PAIR_CASE(AMN, BMN, SM)                                                                        \
+  if (a_mn == AMN && b_mn == BMN && (p.epi != kEpiStd) == SM) {                                             \
+    if (out_dtype == kBF16) return launch_gemm_pair<AMN, BMN, __nv_bfloat16, SM>(ta, tb, p, fmt, num_sms, st); \
+    if (out_dtype == kF16) return launch_gemm_pair<AMN, BMN, __half, SM>(ta, tb, p, fmt, num_sms, st);      \
+    return launch_gemm_pair<AMN, BMN, float, SM>(ta, tb, p, fmt, num_sms, st);                              \
   }
-    GEMM_PAIR_CASE(false, false)
-    GEMM_PAIR_CASE(false, true)
-    GEMM_PAIR_CASE(true, true)
-    GEMM_PAIR_CASE(true, false)
+#define GEMM_PAIR_CASES(SM)        \
+  GEMM_PAIR_CASE(false, false, SM) \
+  GEMM_PAIR_CASE(false, true, SM)  \
+  GEMM_PAIR_CASE(true, true, SM)   \
+  GEMM_PAIR_CASE(true, false, SM)
+    GEMM_PAIR_CASES(false)
+    GEMM_PAIR_CASES(true)
+#undef GEMM_PAIR_CASES
 #undef GEMM_PAIR_CASE
     return -5;
   }
@@ -1441,7 +1461,7 @@ int gemm_pair_max_active_clusters() {
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::total) != cudaSuccess) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(148, 1, 1);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
+  cfg.blockDim = dim3(kPairThreads, 1, 1);
   cfg.dynamicSmemBytes = PairSmem::total;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -240,6 +240,41 @@ def test_tiles_in_bands(tile, M, batch):
     assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()   # every tile: fp32 sums, one rounding
 
 
+@pytest.mark.parametrize("tile", [64, 128, 256, 512])
+@pytest.mark.parametrize("M,N", [(300, 200), (513, 264), (100, 77)])
+def test_epilogues(tile, M, N):
+    """Bias (vector and scalar reads), SiLU with its pre-activation, addend and accumulation through the staging buffers,
+    last columns that are no whole piece included; nothing beyond them is written."""
+    from megalodon_b200.ops import cuda_ops
+    C = cuda_ops._C()
+    torch.manual_seed(M)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, b = _rand(M, 136), _rand(N, 136, scale=136 ** -0.5)
+    prod = a.double() @ b.double().t()
+    ld = -(-N // 8) * 8 + 8
+
+    def close(got, want):
+        return ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()     # fp32 sums, one rounding
+
+    for dt, off in ((torch.bfloat16, 0), (torch.float32, 0), (torch.float16, 1)):
+        bias = _rand(N + off, dtype=dt)[off:]
+        for add in (None, "aux", "accumulate"):
+            buf = torch.full((M, ld), 7.0, device="cuda", dtype=torch.bfloat16)
+            aux = _rand(M, ld)[:, :N]
+            if add == "accumulate":
+                buf[:, :N] = aux
+            out, _, rc = C.gemm(a, b, buf[:, :N], bias, 0, False, False, False, 1, 0, 0.5, err, tile=tile,
+                                accumulate=add == "accumulate", aux=aux if add == "aux" else None)
+            assert rc == 0 and (buf[:, N:] == 7.0).all()
+            assert close(buf[:, :N], 0.5 * prod + bias.double() + (aux.double() if add else 0.0))
+        if N % 8 == 0:
+            for code, odt in ((1, torch.bfloat16), (0, torch.float32)):
+                out, pre, rc = C.gemm(a, b, None, bias, 1, False, False, True, code, 0, 1.0, err, tile=tile)
+                assert rc == 0 and out.dtype == odt and close(pre, prod + bias.double())
+                assert close(out, torch.nn.functional.silu(prod + bias.double()))
+    assert err.item() == 0
+
+
 def test_operators_without_gradients_match_the_recorded_ones():
     """The short route under no_grad against the autograd function, and what the latter refuses stays refused."""
     from megalodon_b200 import ops
