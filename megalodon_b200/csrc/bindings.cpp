@@ -613,10 +613,12 @@ OptTensor gemv(const Tensor& x, const Tensor& w, const OptTensor& bias, int64_t 
 }
 
 // Up to four products over the same M rows: outs[i] = act_i(xs[i] ws[i]^T + biases[i]) + addends[i], act 0 none,
-// 1 SiLU, 2 SwiGLU with second weight w2s[i]; returns the launch status (0: done, -1: outside what the kernel handles)
+// 1 SiLU, 2 SwiGLU with second weight w2s[i]; row m of xs[i] times rsqrt(sum of row_sqs[i][m] / K + row_eps) where
+// row_sqs is given; returns the launch status (0: done, -1: outside what the kernel handles)
 int64_t skinny_gemm(const std::vector<Tensor>& xs, const std::vector<Tensor>& ws, const std::vector<OptTensor>& w2s,
                     const std::vector<OptTensor>& biases, const std::vector<OptTensor>& addends,
-                    const std::vector<int64_t>& acts, const std::vector<Tensor>& outs, bool pdl, const Tensor& err) {
+                    const std::vector<int64_t>& acts, const std::vector<Tensor>& outs, bool pdl, const Tensor& err,
+                    const std::vector<OptTensor>& row_sqs, double row_eps) {
   const size_t n = xs.size();
   TORCH_CHECK(n >= 1 && n <= (size_t)mb::kSkinnyJobs && ws.size() == n && w2s.size() == n && biases.size() == n &&
               addends.size() == n && acts.size() == n && outs.size() == n);
@@ -649,6 +651,12 @@ int64_t skinny_gemm(const std::vector<Tensor>& xs, const std::vector<Tensor>& ws
       const Tensor& a = *addends[i];
       TORCH_CHECK(a.is_cuda() && a.sizes() == y.sizes() && a.stride(1) == 1 && a.scalar_type() == x.scalar_type());
       j.addend = a.data_ptr(); j.ld_add = a.stride(0);
+    }
+    if (i < row_sqs.size() && row_sqs[i].has_value()) {
+      const Tensor& r = *row_sqs[i];
+      check_cuda_contig(r, "row_sqs");
+      TORCH_CHECK(r.scalar_type() == at::kFloat && r.dim() == 2 && r.size(0) == M);
+      j.row_sq = r.data_ptr<float>(); j.row_parts = (int)r.size(1); j.row_eps = (float)row_eps;
     }
     if (x.scalar_type() == at::kFloat ||
         !mb::skinny_gemm_ok((int)M, j.N, j.K, j.ldx, j.ldw, j.x, j.w, dtype_code(x)))
@@ -767,7 +775,8 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_buf, const Tensor& v_bu
   a.pos = reinterpret_cast<const long long*>(pos.data_ptr<int64_t>());
   a.out = out.data_ptr(); a.part_acc = acc.data_ptr<float>(); a.part_ml = ml.data_ptr<float>();
   a.scale = (float)scale; a.H = H; a.C = C; a.dk = dk; a.dv = dv;
-  TORCH_CHECK(mb::decode_attend(a, B, splits, dtype_code(q), false, stream()) == 0, "decode_attention: launch failed");
+  TORCH_CHECK(mb::decode_attend(a, B, splits, at::cuda::getCurrentDeviceProperties()->multiProcessorCount,
+                                dtype_code(q), false, stream()) == 0, "decode_attention: launch failed");
   return out;
 }
 
@@ -779,11 +788,12 @@ void check_link(const Tensor& t, const char* name, at::ScalarType st, std::vecto
 }
 
 // x [B, D]: TimestepNorm step (count, mean, var updated) -> t_out; with hx also the EMA step (hx updated) and RMSNorm
-// -> mx_out, otherwise `pos` (if given) moves on modulo `chunk`
-void decode_norm_ema(const Tensor& x, const Tensor& w, const Tensor& b, Tensor count, Tensor mean, Tensor var,
+// -> mx_out, otherwise `pos` (if given) moves on modulo `chunk`.  With `sumsq` [B, G] mx_out leaves before the factor
+// 1 / rms of its row, whose sum of squares is that of the row's G parts.
+void decode_norm_ema_parts(const Tensor& x, const Tensor& w, const Tensor& b, Tensor count, Tensor mean, Tensor var,
                      Tensor t_out, const OptTensor& p, const OptTensor& q, const OptTensor& gamma,
                      const OptTensor& omega, const OptTensor& hx, const OptTensor& rms_w, const OptTensor& mx_out,
-                     const OptTensor& pos, int64_t chunk, double eps, double rms_eps, bool pdl) {
+                           const OptTensor& pos, int64_t chunk, double eps, double rms_eps, const OptTensor& sumsq, bool pdl) {
   TORCH_CHECK(x.dim() == 2 && mean.dim() == 2);
   const int64_t B = x.size(0), D = x.size(1), G = mean.size(1);
   const auto T = x.scalar_type();
@@ -814,12 +824,23 @@ void decode_norm_ema(const Tensor& x, const Tensor& w, const Tensor& b, Tensor c
     a.p = p->data_ptr<float>(); a.q = q->data_ptr<float>(); a.gamma = gamma->data_ptr<float>();
     a.omega = omega->data_ptr(); a.hx = hx->data_ptr<float>(); a.rms_w = opt_ptr(rms_w);
     a.mx_out = mx_out->data_ptr(); a.N = (int)N;
+    if (sumsq.has_value()) {
+      check_link(*sumsq, "sumsq", at::kFloat, {B, G});
+      a.sumsq = sumsq->data_ptr<float>();
+    }
   } else if (pos.has_value()) {
     TORCH_CHECK(pos->is_cuda() && pos->scalar_type() == at::kLong && pos->numel() == 1 && chunk > 0);
     a.pos = reinterpret_cast<long long*>(pos->data_ptr<int64_t>());
   }
   TORCH_CHECK(mb::decode_norm_ema_ok(a.D, a.G, a.N), "decode_norm_ema: shape not supported");
   TORCH_CHECK(mb::decode_norm_ema(a, (int)B, dtype_code(x), pdl, stream()) == 0, "decode_norm_ema: launch failed");
+}
+void decode_norm_ema(const Tensor& x, const Tensor& w, const Tensor& b, Tensor count, Tensor mean, Tensor var,
+                     Tensor t_out, const OptTensor& p, const OptTensor& q, const OptTensor& gamma,
+                     const OptTensor& omega, const OptTensor& hx, const OptTensor& rms_w, const OptTensor& mx_out,
+                     const OptTensor& pos, int64_t chunk, double eps, double rms_eps, bool pdl) {
+  decode_norm_ema_parts(x, w, b, count, mean, var, t_out, p, q, gamma, omega, hx, rms_w, mx_out, pos, chunk, eps, rms_eps,
+                        OptTensor(), pdl);
 }
 bool decode_norm_ema_ok(int64_t D, int64_t G, int64_t N) { return mb::decode_norm_ema_ok((int)D, (int)G, (int)N); }
 int64_t decode_attend_splits(int64_t BH, int64_t C) {
@@ -856,7 +877,8 @@ void decode_attend(const Tensor& z, const Tensor& gamma, const Tensor& beta, con
   a.gate = gate.data_ptr(); a.out = out.data_ptr();
   a.part_acc = part.data_ptr<float>(); a.part_ml = a.part_acc + B * H * splits * dv;
   a.scale = 1.f; a.eps = (float)eps; a.H = (int)H; a.C = (int)C; a.dk = (int)dk; a.dv = (int)dv;
-  TORCH_CHECK(mb::decode_attend(a, (int)B, (int)splits, dtype_code(z), pdl, stream()) == 0, "decode_attend: launch failed");
+  TORCH_CHECK(mb::decode_attend(a, (int)B, (int)splits, at::cuda::getCurrentDeviceProperties()->multiProcessorCount,
+                                dtype_code(z), pdl, stream()) == 0, "decode_attend: launch failed");
 }
 
 void decode_layer_norm(const Tensor& x, const OptTensor& w, const OptTensor& b, Tensor y, double eps, bool pdl) {
@@ -1200,7 +1222,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return mb::gemm_gather_supported((int)M, (int)N, (int)K, (int)world);
   });
   m.def("gemv", checked(&gemv));
-  m.def("skinny_gemm", checked(&skinny_gemm));
+  m.def("skinny_gemm", checked(&skinny_gemm), py::arg("xs"), py::arg("ws"), py::arg("w2s"), py::arg("biases"),
+        py::arg("addends"), py::arg("acts"), py::arg("outs"), py::arg("pdl"), py::arg("err"),
+        py::arg("row_sqs") = std::vector<OptTensor>(), py::arg("row_eps") = 0.0);
   m.def("rfft_rows", checked(&rfft_rows), py::arg("x"), py::arg("flip"), py::arg("packed") = -1);
   m.def("irfft_rows", checked(&irfft_rows), py::arg("spec"), py::arg("L"), py::arg("packed") = -1);
   m.def("fftconv_apply", checked(&fftconv_apply), py::arg("x"), py::arg("kf"), py::arg("conj_k"), py::arg("packed") = -1);
@@ -1225,6 +1249,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_bwd_prep", checked(&attn_bwd_prep));
   m.def("decode_attention", checked(&decode_attention));
   m.def("decode_norm_ema", checked(&decode_norm_ema));
+  m.def("decode_norm_ema", checked(&decode_norm_ema_parts));
   m.def("decode_norm_ema_ok", &decode_norm_ema_ok);
   m.def("decode_attend_splits", &decode_attend_splits);
   m.def("decode_attend", checked(&decode_attend));

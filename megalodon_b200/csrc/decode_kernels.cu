@@ -13,7 +13,13 @@
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 
+#include <type_traits>
+
 namespace mb {
+
+bool make_tmap_rows(CUtensorMap* out, const void* base, long long width, long long rows, int box_width, int box_rows,
+                    int elem_dtype);
+
 namespace {
 
 using namespace ptx;
@@ -166,6 +172,134 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
     reinterpret_cast<T*>(p.mx_out)[row0 + i] = from_f<T>(v);
   }
   if (rank == 0 && threadIdx.x == 0) p.count[b] += 1;     // every CTA of the row read it before the barrier above
+}
+
+// The same step for a reader that applies the RMSNorm's factor itself: no CTA then needs the whole row, so a CTA owns
+// one group (or enough of them for 32 features), nothing is exchanged, and a row's state comes through all SMs instead
+// of the eight of a cluster.  Everything but x, the parameters of the norms included, is loaded ahead of the wait.
+// us from this link's wait to the next one's, cluster form and this one (16 states, one row): 1024 features 7.5 / 3.3,
+// 4096 features 15.8 / 4.4; 2048 features, 16 rows: 11.2 / 10.5, with the five CTAs an SM below 7.
+// The number of rows' steps counts the CTAs that have read it in its upper half; the last one takes them off and adds one.
+template <typename T, int PER, int BATCH>      // PER: threads of a feature, two states each; BATCH: items of a thread whose
+__global__ void __launch_bounds__(kDecThreads, BATCH == 1 ? 5 : 3)      // loads are in flight together
+decode_norm_ema_wide_kernel(const __grid_constant__ DecodeNormEma p, int groups) {
+  extern __shared__ float sm[];
+  __shared__ float scratch[32];
+  __shared__ double weight_old, weight_new;
+  const int gs = p.D / p.G, nf = groups * gs, b = blockIdx.y, f0 = blockIdx.x * nf, g0 = blockIdx.x * groups;
+  float* xs = sm;                 // nf: input
+  float* ts = xs + nf;            // nf: normalised input as the products see it
+  float* gm = ts + nf;            // means and reciprocal deviations of the groups
+  float* gr = gm + groups;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long long row0 = (long long)b * p.D + f0;
+  const int total = nf * PER;
+  constexpr int kBatch = BATCH;
+  const long long c0 = (long long)f0 * PER;
+  float4* hx = reinterpret_cast<float4*>(p.hx) + (long long)b * p.D * PER + c0;
+  float4 h[kBatch], q[kBatch], ga[kBatch];
+  float2 pp[kBatch];
+  float om[kBatch], rw[kBatch];
+  auto load_items = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = base + u * kDecThreads + tid;
+      if (i >= total) continue;
+      h[u] = hx[i];
+      q[u] = __ldg(reinterpret_cast<const float4*>(p.q) + c0 + i);
+      ga[u] = __ldg(reinterpret_cast<const float4*>(p.gamma) + c0 + i);
+      pp[u] = __ldg(reinterpret_cast<const float2*>(p.p) + c0 + i);
+      if (i % PER == 0) {
+        om[u] = to_f(reinterpret_cast<const T*>(p.omega)[f0 + i / PER]);
+        rw[u] = p.rms_w != nullptr ? to_f(reinterpret_cast<const T*>(p.rms_w)[f0 + i / PER]) + 1.f : 1.f;
+      }
+    }
+  };
+  load_items(0);
+  float w0 = 0.f, b0 = 0.f, u_old = 0.f, v_old = 0.f;
+  if (tid < nf) {
+    w0 = to_f(reinterpret_cast<const T*>(p.w)[f0 + tid]) + 1.f;
+    b0 = to_f(reinterpret_cast<const T*>(p.b)[f0 + tid]);
+  }
+  if (warp < groups) {             // of this warp's first group
+    u_old = p.mean[(long long)b * p.G + g0 + warp];
+    v_old = p.var[(long long)b * p.G + g0 + warp];
+  }
+  unsigned long long seen = 0;
+  if (tid == 0) {
+    seen = atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull << 32);
+    const double n0 = (double)(unsigned int)seen;
+    weight_old = n0 / (n0 + 1.0);
+    weight_new = 1.0 / (n0 + 1.0);
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = tid; i < nf; i += kDecThreads) xs[i] = to_f(reinterpret_cast<const T*>(p.x)[row0 + i]);
+  __syncthreads();
+  for (int g = warp; g < groups; g += kDecThreads / 32) {
+    float s = 0.f;
+    for (int i = lane; i < gs; i += 32) s += xs[g * gs + i];
+    const float u = warp_sum(s) / gs;
+    float v = 0.f;
+    for (int i = lane; i < gs; i += 32) {
+      const float d = xs[g * gs + i] - u;
+      v = fmaf(d, d, v);
+    }
+    v = warp_sum(v) / gs;
+    if (lane == 0) {
+      // the group's features are one sample of weight one, merged into the running population
+      const long long gi = (long long)b * p.G + g0 + g;
+      const double u0 = g == warp ? u_old : p.mean[gi], v0 = g == warp ? v_old : p.var[gi], ud = u;
+      const double mean = weight_old * u0 + weight_new * ud;
+      const double var = fmax(weight_old * (v0 + u0 * u0) + weight_new * ((double)v + ud * ud) - mean * mean, 0.0);
+      p.mean[gi] = (float)mean;
+      p.var[gi] = (float)var;
+      gm[g] = (float)mean;
+      gr[g] = rsqrtf((float)var + p.eps);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < nf; i += kDecThreads) {
+    const int g = i / gs;
+    if (i != tid) {
+      w0 = to_f(reinterpret_cast<const T*>(p.w)[f0 + i]) + 1.f;
+      b0 = to_f(reinterpret_cast<const T*>(p.b)[f0 + i]);
+    }
+    const T t = from_f<T>((xs[i] - gm[g]) * gr[g] * w0 + b0);
+    reinterpret_cast<T*>(p.t_out)[row0 + i] = t;
+    ts[i] = to_f(t);
+  }
+  __syncthreads();
+  float sq = 0.f;
+  for (int base = 0; base < total; base += kBatch * kDecThreads) {
+    if (base > 0) load_items(base);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = base + u * kDecThreads + tid;
+      const bool on = i < total;
+      float acc = 0.f;
+      const float t = on ? ts[i / PER] : 0.f;
+      if (on) {
+        float4 n;
+        n.x = fmaf(q[u].x, h[u].x, fmaf(-q[u].y, h[u].y, pp[u].x * t));
+        n.y = fmaf(q[u].x, h[u].y, q[u].y * h[u].x);
+        n.z = fmaf(q[u].z, h[u].z, fmaf(-q[u].w, h[u].w, pp[u].y * t));
+        n.w = fmaf(q[u].z, h[u].w, q[u].w * h[u].z);
+        hx[i] = n;
+        acc = ga[u].x * n.x - ga[u].y * n.y + ga[u].z * n.z - ga[u].w * n.w;
+      }
+      acc = subwarp_sum<PER>(acc);
+      if (on && i % PER == 0) {
+        const float y = to_f(from_f<T>(fmaf(om[u], t, acc)));
+        reinterpret_cast<T*>(p.mx_out)[row0 + i / PER] = from_f<T>(y * rw[u]);
+        sq = fmaf(y, y, sq);
+      }
+    }
+  }
+  sq = block_sum(sq, scratch);
+  if (tid < groups) p.sumsq[(long long)b * p.G + g0 + tid] = tid == 0 ? sq : 0.f;
+  if (tid == 0 && (seen >> 32) == gridDim.x - 1)
+    atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull - ((unsigned long long)gridDim.x << 32));
 }
 
 // ---------------------------------------------------------------- attention of one query
@@ -409,42 +543,424 @@ decode_combine_kernel(const __grid_constant__ DecodeAttend p, int splits) {
 }
 
 // ---------------------------------------------------------------- LayerNorm of a few rows
+// A CTA a row; a thread keeps up to kPieces pieces of eight features and their parameters, loaded ahead of the wait, in
+// registers (longer rows go through memory again).
 template <typename T>
 __global__ void __launch_bounds__(kDecThreads)
 decode_layer_norm_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ y,
                          int D, float eps) {
-  extern __shared__ float sm[];
+  constexpr int kPieces = 2, kStep = kDecThreads * 8;
   __shared__ float scratch[32];
   const long long row = (long long)blockIdx.x * D;
+  const int first = threadIdx.x * 8;
+  float v[kPieces][8], wv[kPieces][8], bv[kPieces][8];
+  auto load_params = [&](int i, float (&wp)[8], float (&bp)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { wp[j] = 0.f; bp[j] = 0.f; }
+    if (w != nullptr) load8(w + i, wp);
+    if (b != nullptr) load8(b + i, bp);
+  };
+#pragma unroll
+  for (int u = 0; u < kPieces; ++u)
+    if (first + u * kStep < D) load_params(first + u * kStep, wv[u], bv[u]);
   pdl_wait();
   pdl_launch_dependents();
   float s = 0.f;
-  for (int i = threadIdx.x * 8; i < D; i += kDecThreads * 8) {
-    float v[8];
-    load8(x + row + i, v);
-    store8(sm + i, v);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += v[j];
+  for (int u = 0; u < kPieces; ++u) {
+    if (first + u * kStep >= D) break;
+    load8(x + row + first + u * kStep, v[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < kPieces; ++u) {
+    if (first + u * kStep >= D) break;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += v[u][j];
+  }
+  for (int i = first + kPieces * kStep; i < D; i += kStep) {
+    float t[8];
+    load8(x + row + i, t);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += t[j];
   }
   const float mean = block_sum(s, scratch) / D;
   float q = 0.f;
-  for (int i = threadIdx.x; i < D; i += kDecThreads) {
-    const float d = sm[i] - mean;
-    q = fmaf(d, d, q);
+#pragma unroll
+  for (int u = 0; u < kPieces; ++u) {
+    if (first + u * kStep >= D) break;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q = fmaf(v[u][j] - mean, v[u][j] - mean, q);
+  }
+  for (int i = first + kPieces * kStep; i < D; i += kStep) {
+    float t[8];
+    load8(x + row + i, t);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q = fmaf(t[j] - mean, t[j] - mean, q);
   }
   const float rstd = rsqrtf(block_sum(q, scratch) / D + eps);
-  for (int i = threadIdx.x * 8; i < D; i += kDecThreads * 8) {
-    float o[8], wv[8], bv[8];
-    if (w != nullptr) load8(w + i, wv);
-    if (b != nullptr) load8(b + i, bv);
+  auto finish = [&](int i, const float (&t)[8], const float (&wp)[8], const float (&bp)[8]) {
+    float o[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float v = (sm[i + j] - mean) * rstd;
-      if (w != nullptr) v *= wv[j] + 1.f;
-      if (b != nullptr) v += bv[j];
-      o[j] = v;
-    }
+    for (int j = 0; j < 8; ++j) o[j] = (t[j] - mean) * rstd * (w != nullptr ? wp[j] + 1.f : 1.f) + bp[j];
     store8(y + row + i, o);
+  };
+#pragma unroll
+  for (int u = 0; u < kPieces; ++u)
+    if (first + u * kStep < D) finish(first + u * kStep, v[u], wv[u], bv[u]);
+  for (int i = first + kPieces * kStep; i < D; i += kStep) {
+    float t[8], wp[8], bp[8];
+    load8(x + row + i, t);
+    load_params(i, wp, bp);
+    finish(i, t, wp, bp);
+  }
+}
+
+// ---------------------------------------------------------------- attention of one query, one launch
+// CTA = (split of the keys, block of value columns, sequence x head); the splits of one block form a cluster, whose
+// partial rows meet in distributed shared memory, so neither they nor a second launch go through global memory.
+//   * Keys and values of a split stream through one ring of 16 KiB stages (bulk copies by a warp of its own): the
+//     values follow the keys without a gap, and in the chain the ring is filled before the wait - the older slots were
+//     written by launches long before the predecessor.
+//   * With one or two heads in all the value columns are divided too, and every column block works out the scores again:
+//     its keys come from L2.  Its rows of values are boxes of a tensor map (a copy a row is bound by the number of
+//     copies: 2000 keys of one head 17.9 us, with boxes 14.6, in clusters of 8).
+// One query is bound by bytes where there are many sequences (128 heads, 500 keys: 4.6 TB/s; 3.6 in two launches) and by
+// latencies where there are few.
+constexpr int kAttStage = 16384;
+constexpr int kAttThreads = kDecThreads + 32;      // eight consumer warps and the producer
+constexpr int kAttMaxStages = 8;
+constexpr int kAttMaxSplits = 16;
+constexpr int kAttMaxSmem = 220 * 1024;
+
+struct AttendPlan {
+  int splits, blocks, cw, stages, key_rows, val_rows;
+  int bw;              // columns of one copy of values: whole rows (cw == dv), or the width of `vmap`'s box
+};
+
+__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kDecThreads) : "memory"); }
+// sum / maximum over the consumer warps; `scratch` holds 8 floats
+template <bool MAX>
+__device__ __forceinline__ float consumer_reduce(float v, float* scratch) {
+  v = MAX ? warp_max(v) : warp_sum(v);
+  consumer_sync();                                 // (the scratch of the reduction before this one has been read)
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  consumer_sync();
+  float t = scratch[0];
+#pragma unroll
+  for (int w = 1; w < kDecThreads / 32; ++w) t = MAX ? fmaxf(t, scratch[w]) : t + scratch[w];
+  return t;
+}
+
+// d += a b^T for 16 x 16 of a (rows 8 to 15 zero) and 8 x 16 of b, 16-bit with fp32 sums
+template <typename T>
+__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1);
+template <>
+__device__ __forceinline__ void mma_m16n8k16<__nv_bfloat16>(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0,
+                                                            uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
+}
+template <>
+__device__ __forceinline__ void mma_m16n8k16<__half>(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kAttThreads, 2)
+decode_attend_cluster_kernel(const __grid_constant__ DecodeAttend p, const __grid_constant__ AttendPlan pl,
+                             const __grid_constant__ CUtensorMap vmap) {
+  extern __shared__ uint8_t att_raw[];
+  __shared__ float scratch[8];
+  __shared__ float2 ml[kAttMaxSplits];
+  __shared__ uint64_t full_bar[kAttMaxStages], empty_bar[kAttMaxStages];
+  __shared__ int failed;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(att_raw) + 127) & ~uintptr_t(127));
+  float* qs = reinterpret_cast<float*>(ring + pl.stages * kAttStage);   // dk: query
+  float* kn = qs + p.dk;                                                // dk: this token's key
+  T* qrow = reinterpret_cast<T*>(kn + p.dk);                            // 3 dk: the query as a sum of 16-bit rows
+  float* red = kn + p.dk + (3 * p.dk + 7) / 8 * 4;                      // kDecThreads * 8: rows of the thread groups
+  float* comb = red + kDecThreads * 8;                                  // cw: partial rows of all splits, own columns
+  float* sc = comb + pl.cw;                                             // scores of this split
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int S = pl.splits, split = blockIdx.x;
+  const int bh = blockIdx.z, h = bh % p.H, col0 = blockIdx.y * pl.cw;
+  const bool fused = p.z != nullptr;
+  if (tid == 0) {
+    for (int i = 0; i < pl.stages; ++i) {
+      mbar_init(full_bar + i, 1);
+      mbar_init(empty_bar + i, kDecThreads / 32);
+    }
+    failed = 0;
+    fence_barrier_init();
+    if (pl.cw != p.dv) prefetch_tmap(&vmap);
+  }
+  __syncthreads();
+  if (S > 1) cluster_arrive();     // awaited before the first store into another CTA: by then all have started
+  if (!fused) pdl_wait();          // (nothing is known here about what wrote the position and the slots)
+  const int at = (int)min(p.pos[0], (long long)p.C - 1);
+  const int n = at + 1, per = (n + S - 1) / S;
+  const int lo = min(n, split * per), hi = min(n, lo + per), cnt = hi - lo;
+  const bool mine = fused && at >= lo && at < hi;           // this split has the new slot
+  const int old = mine ? cnt - 1 : cnt;
+  const T* kold = reinterpret_cast<const T*>(p.k_buf) + ((long long)bh * p.C + lo) * p.dk;
+  const T* vold = reinterpret_cast<const T*>(p.v_buf) + ((long long)bh * p.C + lo) * p.dv + col0;
+  const int key_stages = (old + pl.key_rows - 1) / pl.key_rows, val_stages = (old + pl.val_rows - 1) / pl.val_rows;
+
+  if (warp == kDecThreads / 32) {
+    // ------------------------------------------------------------ producer
+    const int total = key_stages + val_stages;
+    int i = 0, st = 0;
+    uint32_t phase = 1;
+    for (; i < total; ++i) {
+      // (all lanes wait: one answer for the warp)
+      const bool room = i < pl.stages || mbar_wait(empty_bar + st, phase);
+      if (!__all_sync(0xffffffffu, room)) {
+        failed = 1;
+        break;
+      }
+      const uint32_t dst = smem_u32(ring + st * kAttStage);
+      const bool keys = i < key_stages;
+      const int per_stage = keys ? pl.key_rows : pl.val_rows, width = keys ? p.dk : pl.cw;
+      const int j = (keys ? i : i - key_stages) * per_stage, rows = min(per_stage, old - j);
+      if (lane == 0) {
+        if (keys || pl.cw == p.dv) {
+          mbar_expect_tx(full_bar + st, rows * width * sizeof(T));
+          bulk_load(dst, keys ? kold + (long long)j * p.dk : vold + (long long)j * p.dv, rows * width * sizeof(T),
+                    full_bar + st);
+        } else {
+          // (whole boxes: what lies behind the split's last key is not used)
+          const int box = pl.val_rows * pl.bw * (int)sizeof(T);
+          mbar_expect_tx(full_bar + st, box * (pl.cw / pl.bw));
+          for (int k = 0; k < pl.cw / pl.bw; ++k)
+            tma_load_4d(ring + st * kAttStage + k * box, &vmap, full_bar + st, col0 + k * pl.bw, bh * p.C + lo + j, 0, 0);
+        }
+      }
+      __syncwarp();
+      if (++st == pl.stages) { st = 0; phase ^= 1; }
+    }
+    for (int k = max(0, i - pl.stages); k < i; ++k)       // no copy is in flight when the CTA leaves
+      if (!mbar_wait(full_bar + k % pl.stages, (k / pl.stages) & 1)) failed = 1;
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ consumers
+    bool ok = true;
+    // the query / key parameters and rotation of this thread's first pair
+    const T *ga = reinterpret_cast<const T*>(p.gamma) + h * p.dk, *be = reinterpret_cast<const T*>(p.beta) + h * p.dk;
+    const float2* freqs = reinterpret_cast<const float2*>(p.freqs) + (long long)at * (p.dk / 2);
+    const int Z = p.H * p.dk;
+    struct Pair { float2 f, gq, gk, bq, bk; };
+    auto load_pair = [&](int i) {
+      auto two = [](const T* s) { return make_float2(to_f(s[0]), to_f(s[1])); };
+      return Pair{freqs[i], two(ga + 2 * i), two(ga + Z + 2 * i), two(be + 2 * i), two(be + Z + 2 * i)};
+    };
+    Pair pair{};
+    if (fused && tid < p.dk / 2) pair = load_pair(tid);
+    pdl_wait();
+    pdl_launch_dependents();
+    // columns of this thread (8 of the block), row groups, and the new value row's piece
+    const int ct = pl.cw / 8, ng = kDecThreads / ct, grp = tid / ct, c = (tid - grp * ct) * 8;
+    uint4 vnew = make_uint4(0u, 0u, 0u, 0u);
+    const bool has_new = mine && grp == 0;
+    if (has_new)
+      vnew = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v_new) + (long long)bh * p.dv + col0 + c);
+    if (fused) {
+      const T* zr = reinterpret_cast<const T*>(p.z) + (long long)bh * p.dk;
+      float s = 0.f;
+      for (int i = tid; i < p.dk; i += kDecThreads) {
+        const float v = to_f(zr[i]);
+        qs[i] = v;
+        s = fmaf(v, v, s);
+      }
+      const float rstd = rsqrtf(consumer_reduce<false>(s, scratch) / p.dk + p.eps);
+      const float inv = rsqrtf((float)p.dk);
+      T* krow = reinterpret_cast<T*>(p.k_buf) + ((long long)bh * p.C + at) * p.dk;
+      for (int i = tid; i < p.dk / 2; i += kDecThreads) {
+        if (i != tid) pair = load_pair(i);
+        const float2 f = pair.f;
+        const float z0 = qs[2 * i] * rstd, z1 = qs[2 * i + 1] * rstd;
+        const float a0 = z0 * (pair.gq.x + 1.f) * inv + pair.bq.x, a1 = z1 * (pair.gq.y + 1.f) * inv + pair.bq.y;
+        const float c0 = z0 * (pair.gk.x + 1.f) * inv + pair.bk.x, c1 = z1 * (pair.gk.y + 1.f) * inv + pair.bk.y;
+        qs[2 * i] = a0 * f.x - a1 * f.y;
+        qs[2 * i + 1] = a0 * f.y + a1 * f.x;
+        const T k0 = from_f<T>(c0 * f.x - c1 * f.y), k1 = from_f<T>(c0 * f.y + c1 * f.x);
+        kn[2 * i] = to_f(k0);
+        kn[2 * i + 1] = to_f(k1);
+        if (mine && blockIdx.y == 0) {
+          krow[2 * i] = k0;
+          krow[2 * i + 1] = k1;
+        }
+      }
+    } else {
+      const T* qr = reinterpret_cast<const T*>(p.q) + (long long)bh * p.dk;
+      for (int i = tid; i < p.dk; i += kDecThreads) qs[i] = to_f(qr[i]);
+    }
+    consumer_sync();
+    for (int i = tid; i < p.dk; i += kDecThreads) {
+      float rest = qs[i];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T part = from_f<T>(rest);
+        qrow[r * p.dk + i] = part;
+        rest -= to_f(part);
+      }
+    }
+    consumer_sync();
+    int st = 0;
+    uint32_t phase = 0;
+    auto wait_stage = [&]() {
+      if (ok && !mbar_wait(full_bar + st, phase)) {
+        ok = false;
+        failed = 1;
+      }
+    };
+    auto free_stage = [&]() {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty_bar + st);
+      if (++st == pl.stages) { st = 0; phase ^= 1; }
+    };
+    // Scores.  With a width that is a multiple of 32 eight keys of a warp at a time on the tensor cores, the query as the
+    // sum of three 16-bit rows of the other operand (its 24 bits; products and sums are fp32): some 40 instructions
+    // for eight keys instead of 400, which with several column blocks bounded the link.  A fragment's places along the
+    // contraction are dealt out so that a lane's part of a key, and of a query row, is 16 contiguous bytes.
+    const bool mma = p.dk % 32 == 0;
+    for (int i = 0; i < key_stages; ++i) {
+      wait_stage();
+      const T* keys = reinterpret_cast<const T*>(ring + st * kAttStage);
+      const int base = i * pl.key_rows, rows = min(pl.key_rows, old - base);
+      if (mma) {
+        const int g = lane >> 2, t8 = (lane & 3) * 8;
+        for (int j0 = warp * 8; j0 < rows; j0 += kDecThreads / 32 * 8) {
+          const T* key = keys + min(j0 + g, rows - 1) * p.dk + t8;
+          float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};
+          for (int e = 0; e < p.dk; e += 32) {
+            uint4 qa = make_uint4(0u, 0u, 0u, 0u);
+            if (g < 3) qa = *reinterpret_cast<const uint4*>(qrow + g * p.dk + e + t8);
+            const uint4 kb = *reinterpret_cast<const uint4*>(key + e);
+            mma_m16n8k16<T>(d, qa.x, qa.y, kb.x, kb.y);
+            mma_m16n8k16<T>(d2, qa.z, qa.w, kb.z, kb.w);
+          }
+          // rows 0 to 2 of the result, columns 2 (lane & 3) and the next
+          float s0 = d[0] + d2[0], s1 = d[1] + d2[1];
+          s0 += __shfl_down_sync(0xffffffffu, s0, 4) + __shfl_down_sync(0xffffffffu, s0, 8);
+          s1 += __shfl_down_sync(0xffffffffu, s1, 4) + __shfl_down_sync(0xffffffffu, s1, 8);
+          const int j = j0 + 2 * lane;
+          if (lane < 4 && j < rows) sc[base + j] = s0 * p.scale;
+          if (lane < 4 && j + 1 < rows) sc[base + j + 1] = s1 * p.scale;
+        }
+      } else {
+        for (int j = warp; j < rows; j += kDecThreads / 32) {
+          float s = 0.f;
+          for (int e = lane * 8; e < p.dk; e += 256) {
+            float q[8], kv[8];
+            load8(qs + e, q);
+            load8(keys + j * p.dk + e, kv);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s = fmaf(q[k], kv[k], s);
+          }
+          s = warp_sum(s);
+          if (lane == 0) sc[base + j] = s * p.scale;
+        }
+      }
+      free_stage();
+    }
+    if (mine && warp == 0) {
+      float s = 0.f;
+      for (int e = lane; e < p.dk; e += 32) s = fmaf(qs[e], kn[e], s);
+      s = warp_sum(s);
+      if (lane == 0) sc[old] = s * p.scale;
+    }
+    consumer_sync();
+    float m = -INFINITY;
+    for (int j = tid; j < cnt; j += kDecThreads) m = fmaxf(m, sc[j]);
+    m = consumer_reduce<true>(m, scratch);
+    const float ref = m == -INFINITY ? 0.f : m;      // a split without keys, or whose keys all have weight zero
+    float sum = 0.f;
+    for (int j = tid; j < cnt; j += kDecThreads) {
+      const float e = __expf(sc[j] - ref);
+      sc[j] = e;
+      sum += e;
+    }
+    sum = consumer_reduce<false>(sum, scratch);      // (its barriers also publish the weights)
+    // values
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int i = 0; i < val_stages; ++i) {
+      wait_stage();
+      const T* vals = reinterpret_cast<const T*>(ring + st * kAttStage) + c / pl.bw * (pl.val_rows * pl.bw) + c % pl.bw;
+      const int base = i * pl.val_rows, rows = min(pl.val_rows, old - base);
+      if (grp < ng) {
+#pragma unroll 4
+        for (int r = grp; r < rows; r += ng) {
+          float v[8];
+          load8(vals + r * pl.bw, v);
+          const float e = sc[base + r];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[k] = fmaf(e, v[k], acc[k]);
+        }
+      }
+      free_stage();
+    }
+    if (has_new) {
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.v_buf) + ((long long)bh * p.C + at) * p.dv + col0 + c) = vnew;
+      float v[8];
+      load8(reinterpret_cast<const T*>(&vnew), v);
+      const float e = sc[old];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] = fmaf(e, v[k], acc[k]);
+    }
+    if (ng > 1) {
+      if (grp < ng) store8(red + tid * 8, acc);
+      consumer_sync();
+      if (grp == 0) {
+        for (int g = 1; g < ng; ++g) {
+          float v[8];
+          load8(red + (g * ct * 8 + tid * 8), v);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[k] += v[k];
+        }
+      }
+    }
+    if (S > 1) cluster_wait();
+    // column k of the block is finished by split k / (cw / S)
+    const int R = pl.cw / S;
+    if (grp == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int owner = (c + k) / R, slot = split * R + (c + k) - owner * R;
+        if (S > 1) st_cluster_f32(map_to_cta(smem_u32(comb + slot), owner), acc[k]);
+        else comb[slot] = acc[k];
+      }
+    }
+    if (tid < S) {
+      if (failed) sum = __int_as_float(0x7fffffff);      // a copy that never came: the result is not a number
+      if (S > 1) {
+        const uint32_t dst = map_to_cta(smem_u32(ml + split), tid);
+        st_cluster_f32(dst, m);
+        st_cluster_f32(dst + 4, sum);
+      } else {
+        ml[0] = make_float2(m, sum);
+      }
+    }
+  }
+  if (S > 1) {
+    if (warp == kDecThreads / 32) cluster_wait();          // (the consumers have come to theirs above)
+    cluster_sync_all();
+  } else {
+    __syncthreads();
+  }
+  if (tid >= kDecThreads) return;
+  float m = ml[0].x;
+  for (int s = 1; s < S; ++s) m = fmaxf(m, ml[s].x);
+  float l = 0.f;
+  for (int s = 0; s < S; ++s) l += __expf(ml[s].x - m) * ml[s].y;
+  const int R = pl.cw / S;
+  for (int k = tid; k < R; k += kDecThreads) {
+    float v = 0.f;
+    for (int s = 0; s < S; ++s) v = fmaf(__expf(ml[s].x - m), comb[s * R + k], v);
+    const long long o = (long long)bh * p.dv + col0 + split * R + k;
+    v /= l;
+    if (p.gate != nullptr) v *= to_f(reinterpret_cast<const T*>(p.gate)[o]);
+    reinterpret_cast<T*>(p.out)[o] = from_f<T>(v);
   }
 }
 
@@ -480,8 +996,35 @@ bool decode_norm_ema_ok(int D, int G, int N) {
   return G >= 1 && D % G == 0 && D <= 16384 && (N == 2 || N == 4 || N == 8 || N == 16 || N == 32);
 }
 
+static int decode_norm_ema_wide(const DecodeNormEma& p, int B, int dtype, bool pdl, cudaStream_t st) {
+  const int gs = p.D / p.G;
+  int groups = 1;                                   // the fewest, dividing G evenly, with 32 features
+  while (groups < p.G && (groups * gs < 32 || p.G % groups != 0)) ++groups;
+  const size_t smem = sizeof(float) * (2 * groups * gs + 2 * groups);
+  cudaError_t e = cudaSuccess;
+  MB_DISPATCH_16BIT(dtype, {
+    auto launch = [&](auto kern) {
+      if (smem > 40 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      if (e == cudaSuccess) e = launch_link(kern, dim3(p.G / groups, B), smem, 1, pdl, st, p, groups);
+    };
+    // One item a thread keeps five CTAs to an SM, which many rows need to start in one or two waves.
+    auto pick = [&](auto per) {
+      constexpr int P = decltype(per)::value;
+      if (groups * gs * P <= kDecThreads) launch(decode_norm_ema_wide_kernel<scalar_t, P, 1>);
+      else launch(decode_norm_ema_wide_kernel<scalar_t, P, 2>);
+    };
+    if (p.N == 2) pick(std::integral_constant<int, 1>());
+    else if (p.N == 4) pick(std::integral_constant<int, 2>());
+    else if (p.N == 8) pick(std::integral_constant<int, 4>());
+    else if (p.N == 16) pick(std::integral_constant<int, 8>());
+    else pick(std::integral_constant<int, 16>());
+  });
+  return e == cudaSuccess ? 0 : -3;
+}
+
 int decode_norm_ema(const DecodeNormEma& p, int B, int dtype, bool pdl, cudaStream_t st) {
   if (B == 0) return 0;
+  if (p.hx != nullptr && p.sumsq != nullptr) return decode_norm_ema_wide(p, B, dtype, pdl, st);
   // as many CTAs per row as share its groups evenly (a cluster of 8 at the most)
   int cl = 8;
   while (cl > 1 && p.G % cl != 0) cl /= 2;
@@ -511,13 +1054,104 @@ int decode_attend_splits(int BH, int C, int num_sms) {
   return s < 1 ? 1 : (s > kDecodeMaxSplits ? kDecodeMaxSplits : s);
 }
 
-int decode_attend(const DecodeAttend& p, int B, int splits, int dtype, bool pdl, cudaStream_t st) {
+// How one launch divides the work, if it takes the shapes and is the better form.  The column blocks of a head repeat its
+// scores, so there are several of them only for one or two heads in all, 128 CTAs in clusters of 16; the next line is
+// where clusters of eight fill the SMs without them.  Between the two, keys split over the whole GPU and a second launch
+// are faster.  us a link, two launches / one (d_qk 256, d_v 2048):
+//   1 head      300 keys  8.9 /  7.5      2000 keys 13.7 / 11.9
+//   2 heads     300 keys  9.0 /  7.9      2000 keys 15.8 / 15.0
+//   4 heads    1111 keys 14.4 / 14.7      4000 keys 26.0 / 31.4
+//   12 heads    700 keys 17.1 / 17.4      2000 keys 33.9 / 38.6
+//   32 heads    700 keys 31.6 / 27.9      2000 keys 71.6 / 63.7
+//   128 heads   500 keys 81.3 / 64.1
+static bool attend_plan(const DecodeAttend& p, int BH, int num_sms, bool wide_clusters, AttendPlan& pl, size_t& smem) {
+  if (p.dv % 8 != 0 || !aligned16(p.v_buf) || !aligned16(p.k_buf) || p.dk > kAttStage / 2) return false;
+  int most;                                             // CTAs
+  if (BH <= 2 && wide_clusters) {
+    pl.splits = kAttMaxSplits;
+    most = 128;
+  } else if (16 * BH > 2 * num_sms) {
+    pl.splits = 8;
+    most = 2 * num_sms;
+    while (pl.splits > 1 && pl.splits * BH > most) pl.splits /= 2;
+  } else {
+    return false;
+  }
+  const int pieces = p.dv / 8;
+  pl.blocks = 0;
+  for (int b = 1; b <= pieces && b <= 64; ++b) {
+    const int cw = p.dv / b;
+    if (pieces % b != 0 || cw > 8 * kDecThreads || cw % pl.splits != 0 || (b > 1 && cw > 256 && cw % 256 != 0)) continue;
+    if (pl.blocks != 0 && (cw < 128 || b * pl.splits * BH > most)) break;
+    pl.blocks = b;
+  }
+  if (pl.blocks == 0) return false;
+  pl.cw = p.dv / pl.blocks;
+  pl.bw = pl.blocks == 1 || pl.cw < 256 ? pl.cw : 256;
+  pl.key_rows = kAttStage / (p.dk * 2);
+  pl.val_rows = kAttStage / (pl.cw * 2);
+  if (pl.val_rows > 256) pl.val_rows = 256;             // (a copy's box)
+  const size_t other = sizeof(float) * (2 * p.dk + (3 * p.dk + 7) / 8 * 4 + kDecThreads * 8 + pl.cw +
+                                        div_up(p.C, pl.splits)) + 128;
+  const size_t room = 112 * 1024;                       // two CTAs to an SM
+  pl.stages = other + 2 * kAttStage > room ? 2 : (int)((room - other) / kAttStage);
+  if (pl.stages > kAttMaxStages) pl.stages = kAttMaxStages;
+  smem = other + (size_t)pl.stages * kAttStage;
+  return smem <= kAttMaxSmem;
+}
+
+// Whether clusters of 16 of the kernel can run on the current device (a size that is not portable).
+template <typename T>
+static bool attend_wide_clusters() {
+  static std::atomic<unsigned long long> known{0}, can{0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+  const unsigned long long bit = 1ull << dev;
+  if ((known.load(std::memory_order_acquire) & bit) == 0) {
+    auto kern = decode_attend_cluster_kernel<T>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kAttMaxSplits, 1, 1);
+    cfg.blockDim = dim3(kAttThreads, 1, 1);
+    cfg.dynamicSmemBytes = kAttMaxSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kAttMaxSplits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttMaxSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
+      can.fetch_or(bit, std::memory_order_release);
+    (void)cudaGetLastError();
+    known.fetch_or(bit, std::memory_order_release);
+  }
+  return (can.load(std::memory_order_acquire) & bit) != 0;
+}
+
+int decode_attend(const DecodeAttend& p, int B, int splits, int num_sms, int dtype, bool pdl, cudaStream_t st) {
   if (B == 0) return 0;
+  cudaError_t e = cudaSuccess;
+  bool done = false;
+  MB_DISPATCH_16BIT(dtype, {
+    auto kern = decode_attend_cluster_kernel<scalar_t>;
+    static std::atomic<unsigned long long> configured{0};
+    AttendPlan pl;
+    size_t bytes;
+    CUtensorMap vmap = {};
+    if (B * p.H <= 65535 && attend_plan(p, B * p.H, num_sms, B * p.H <= 2 && attend_wide_clusters<scalar_t>(), pl, bytes) &&
+        (pl.blocks == 1 || make_tmap_rows(&vmap, p.v_buf, p.dv, (long long)B * p.H * p.C, pl.bw, pl.val_rows, dtype))) {
+      if (!allow_dynamic_smem(kern, kAttMaxSmem, configured)) return -2;
+      e = launch_link<kAttThreads>(kern, dim3(pl.splits, pl.blocks, B * p.H), bytes, pl.splits, pdl, st, p, pl, vmap);
+      done = true;
+    }
+  });
+  if (done) return e == cudaSuccess ? 0 : -3;
   if (p.z != nullptr && (p.dv % 8 != 0 || !aligned16(p.v_buf))) return -1;      // (the new value row leaves in pieces)
   const int BH = B * p.H;
   const int keys = div_up(p.C, splits) < 8 ? 8 : div_up(p.C, splits);
   const size_t smem = sizeof(float) * (2 * p.dk + kDecThreads * 8 + keys);
-  cudaError_t e = cudaSuccess;
   MB_DISPATCH_16BIT(dtype, {
     const bool vec = p.dv % 8 == 0 && aligned16(p.v_buf);
     auto kern = vec ? decode_attend_kernel<scalar_t, true> : decode_attend_kernel<scalar_t, false>;
@@ -534,12 +1168,8 @@ int decode_layer_norm(const void* x, const void* w, const void* b, void* y, int 
   if (rows == 0) return 0;
   cudaError_t e = cudaSuccess;
   MB_DISPATCH_16BIT(dtype, {
-    auto kern = decode_layer_norm_kernel<scalar_t>;
-    if (D * sizeof(float) > 40 * 1024)
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess)
-      e = launch_link(kern, dim3(rows), D * sizeof(float), 1, pdl, st, (const scalar_t*)x, (const scalar_t*)w,
-                      (const scalar_t*)b, (scalar_t*)y, D, eps);
+    e = launch_link(decode_layer_norm_kernel<scalar_t>, dim3(rows), 0, 1, pdl, st, (const scalar_t*)x,
+                    (const scalar_t*)w, (const scalar_t*)b, (scalar_t*)y, D, eps);
   });
   return e == cudaSuccess ? 0 : -3;
 }

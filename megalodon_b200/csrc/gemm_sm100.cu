@@ -1187,10 +1187,10 @@ EncodeTiledFn get_encode_fn() {
 }  // namespace
 
 // 4-D bf16/fp16 tensor map [outer batch, batch, outer, inner] (inner contiguous) with a {1, 1, box_outer,
-// box_inner} box and 128-byte swizzle.  Strides are in elements and must be multiples of 8 (16 bytes).
-bool make_tmap_4d(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
-                  long long batch2, long long row_stride, long long batch_stride, long long batch2_stride,
-                  int box_inner, int box_outer, int elem_dtype) {
+// box_inner} box.  Strides are in elements and must be multiples of 8 (16 bytes).
+static bool encode_tmap(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
+                        long long batch2, long long row_stride, long long batch_stride, long long batch2_stride,
+                        int box_inner, int box_outer, int elem_dtype, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return false;
   // The encoder is a driver entry point and needs a current context; a thread that has made no
@@ -1209,7 +1209,7 @@ bool make_tmap_4d(CUtensorMap* out, const void* base, long long inner, long long
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUtensorMapDataType dt = elem_dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const CUresult res = fn(out, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (res != CUDA_SUCCESS)
     fprintf(stderr,
@@ -1219,6 +1219,21 @@ bool make_tmap_4d(CUtensorMap* out, const void* base, long long inner, long long
             (unsigned long long)dims[3], (unsigned long long)strides[0], (unsigned long long)strides[1],
             (unsigned long long)strides[2], box[0], box[1]);
   return res == CUDA_SUCCESS;
+}
+
+// ... with 128-byte swizzle
+bool make_tmap_4d(CUtensorMap* out, const void* base, long long inner, long long outer, long long batch,
+                  long long batch2, long long row_stride, long long batch_stride, long long batch2_stride,
+                  int box_inner, int box_outer, int elem_dtype) {
+  return encode_tmap(out, base, inner, outer, batch, batch2, row_stride, batch_stride, batch2_stride, box_inner, box_outer,
+                     elem_dtype, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// Map of a contiguous 16-bit matrix [rows, width], box [box_rows, box_width] row by row without swizzle.
+bool make_tmap_rows(CUtensorMap* out, const void* base, long long width, long long rows, int box_width, int box_rows,
+                    int elem_dtype) {
+  return encode_tmap(out, base, width, rows, 1, 1, width, width * rows, width * rows, box_width, box_rows, elem_dtype,
+                     CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 template <int BN, bool A_MN, bool B_MN, typename OutT>

@@ -104,6 +104,9 @@ struct SkinnyJob {
   void* y;              // [M, N], row stride ldy
   long long ldx, ldw, ld_add, ldy;
   int N, K, act, bias_dtype, out_f32;
+  const float* row_sq;  // [M, row_parts] or null: row m of x is multiplied by rsqrt(sum of its parts / K + row_eps)
+  int row_parts;
+  float row_eps;
 };
 bool skinny_gemm_ok(int M, int N, int K, long long ldx, long long ldw, const void* x, const void* w, int in_dtype);
 // pdl: the launch may overlap the end of the kernel before it (only inside a chain of such launches)
@@ -201,6 +204,8 @@ struct DecodeNormEma {
   float* hx;                            // [B, D, N, 2], updated
   const void* rms_w;                    // [D] or null
   void* mx_out;                         // [B, D]
+  float* sumsq;                         // null, or [B, G]: mx_out leaves before its row's factor 1 / rms, which the
+                                        // reader takes from the G parts of the sum of squares
   long long* pos;                       // with hx null: advanced modulo `chunk` after the last layer; or null
   float eps, rms_eps;
   int D, G, N, chunk;
@@ -223,7 +228,7 @@ struct DecodeAttend {
   int H, C, dk, dv;
 };
 int decode_attend_splits(int BH, int C, int num_sms);
-int decode_attend(const DecodeAttend& p, int B, int splits, int dtype, bool pdl, cudaStream_t st);
+int decode_attend(const DecodeAttend& p, int B, int splits, int num_sms, int dtype, bool pdl, cudaStream_t st);
 int decode_layer_norm(const void* x, const void* w, const void* b, void* y, int rows, int D, float eps, int dtype,
                       bool pdl, cudaStream_t st);
 // reduce-scatter fused with the sharded AdamW update (comm_kernels.cu); false if the shapes do not qualify

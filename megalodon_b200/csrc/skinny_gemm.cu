@@ -9,7 +9,8 @@
 // K is split over a cluster of 1..8 CTAs, so that N / 128 tiles fill the machine; the partial accumulators
 // meet in distributed shared memory, each CTA adding up and finishing 128 / S of the tile's features.
 // Up to four products over the same rows share a launch (the four projections of a MEGA layer), and a
-// product may carry a second weight for SwiGLU: y = silu(x w^T) * (x w2^T).
+// product may carry a second weight for SwiGLU: y = silu(x w^T) * (x w2^T).  Rows of x may come without their RMSNorm's
+// factor, which is then applied to the sums (`row_sq`).
 //
 // In a chain of programmatic dependent launches the weight tiles of the first ring round are requested before the
 // previous kernel has finished: weights do not depend on it, x does.  (Prefetching the rest into L2 as well gained
@@ -62,11 +63,15 @@ __device__ __forceinline__ bool sk_wait(uint64_t* bar, uint32_t parity, volatile
 }
 
 template <typename T>
-__device__ __forceinline__ void sk_finish(const SkinnyJob& j, int m, int n, float v, float v2, float bias) {
+__device__ __forceinline__ float sk_addend(const SkinnyJob& j, int m, int n) {
+  return j.addend == nullptr ? 0.f : to_f(reinterpret_cast<const T*>(j.addend)[(long long)m * j.ld_add + n]);
+}
+template <typename T>
+__device__ __forceinline__ void sk_finish(const SkinnyJob& j, int m, int n, float v, float v2, float bias, float addend) {
   v += bias;
   if (j.act == kSkinnySilu) v = silu_f(v);
   else if (j.act == kSkinnySwiGLU) v = silu_f(v) * v2;
-  if (j.addend != nullptr) v += to_f(reinterpret_cast<const T*>(j.addend)[(long long)m * j.ld_add + n]);
+  v += addend;
   if (j.out_f32) reinterpret_cast<float*>(j.y)[(long long)m * j.ldy + n] = v;
   else reinterpret_cast<T*>(j.y)[(long long)m * j.ldy + n] = from_f<T>(v);
 }
@@ -88,6 +93,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
   uint64_t* acc_bar = empty_bar + kSkMaxStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  float* row_scale = reinterpret_cast<float*>(tmem_holder + 2);      // kSkinnyMaxRows
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.split;
@@ -125,6 +131,10 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
 
   if (warp == 0) {
     if (elect_one()) {
+      // (the descriptor of x as well: otherwise its fetch begins only when x is there)
+      prefetch_tmap(&maps.w[ji]);
+      if (dual) prefetch_tmap(&maps.w2[ji]);
+      prefetch_tmap(&maps.x[ji]);
       const int total = kb1 - kb0;
       const int first = min(total, p.stages);
       for (int i = 0; i < first; ++i) {
@@ -187,13 +197,39 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
   const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
   const int nl = quarter * 32 + lane;              // this thread's feature within the tile
   bool ok = true;
+  // Biases (weights, so ahead of the wait) and addends of the first elements that a thread finishes come in while the
+  // product is under way.
+  constexpr int kPre = 2;
+  const int R = kSkRows / S;                       // features finished by each CTA of a cluster
+  float bias_pre[kPre], add_pre[kPre];
+  auto finished = [&](int u, int& m, int& n) {     // element u of this thread; false if it has none
+    const int idx = (int)threadIdx.x - 64 + u * (kSkThreads - 64);
+    m = idx / R;
+    n = n0 + rank * R + idx % R;
+    return m < p.M && n < job.N;
+  };
   if (warp >= 2) {
+    int m, n;
+#pragma unroll
+    for (int u = 0; u < kPre; ++u) bias_pre[u] = S > 1 && finished(u, m, n) ? sk_bias(job, n) : 0.f;
     pdl_wait();
     pdl_launch_dependents();
+#pragma unroll
+    for (int u = 0; u < kPre; ++u) add_pre[u] = S > 1 && finished(u, m, n) ? sk_addend<T>(job, m, n) : 0.f;
+    if (job.row_sq != nullptr) {
+      for (m = warp - 2; m < p.M; m += 4) {
+        float s = 0.f;
+        for (int i = lane; i < job.row_parts; i += 32) s += job.row_sq[m * job.row_parts + i];
+        s = warp_sum(s);
+        if (lane == 0) row_scale[m] = rsqrtf(s / job.K + job.row_eps);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kSkThreads - 64) : "memory");     // the four epilogue warps
+    }
     ok = sk_wait(acc_bar, 0, abort_flag);
     if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 13); }
     tcgen05_fence_after();
   }
+  auto scaled = [&](float v, int m) { return job.row_sq != nullptr ? v * row_scale[m] : v; };
   if (S == 1) {
     if (warp >= 2 && ok) {
       const int n = n0 + nl;
@@ -206,13 +242,14 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
         if (n < job.N) {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            if (c + i < p.M) sk_finish<T>(job, c + i, n, __uint_as_float(r[i]), dual ? __uint_as_float(r2[i]) : 0.f, bias);
+            if (c + i < p.M)
+              sk_finish<T>(job, c + i, n, scaled(__uint_as_float(r[i]), c + i),
+                           dual ? scaled(__uint_as_float(r2[i]), c + i) : 0.f, bias, sk_addend<T>(job, c + i, n));
         }
       }
     }
   } else {
     cluster_wait();
-    const int R = kSkRows / S;                     // features finished by each CTA
     uint8_t* red_smem = smem + p.stages * p.stage_bytes;      // partial sums have memory of their own
     const uint32_t red = smem_u32(red_smem);
     const int plane = p.mpad * R;                  // floats of one (source, accumulator)
@@ -233,17 +270,21 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constan
     cluster_sync_all();
     if (warp >= 2 && ok) {
       const float* part = reinterpret_cast<const float*>(red_smem);
-      for (int idx = threadIdx.x - 64; idx < R * p.M; idx += kSkThreads - 64) {
-        const int fl = idx % R, m = idx / R;
-        const int n = n0 + rank * R + fl;
-        if (n >= job.N) continue;
+      auto finish = [&](int m, int n, float bias, float addend) {
+        const int fl = n - n0 - rank * R;
         float v = 0.f, v2 = 0.f;
         for (int s = 0; s < S; ++s) {
           v += part[s * naccs * plane + m * R + fl];
           if (dual) v2 += part[(s * 2 + 1) * plane + m * R + fl];
         }
-        sk_finish<T>(job, m, n, v, v2, sk_bias(job, n));
-      }
+        sk_finish<T>(job, m, n, scaled(v, m), scaled(v2, m), bias, addend);
+      };
+      int m, n;
+#pragma unroll
+      for (int u = 0; u < kPre; ++u)
+        if (finished(u, m, n)) finish(m, n, bias_pre[u], add_pre[u]);
+      for (int u = kPre; u * (kSkThreads - 64) < R * p.M; ++u)
+        if (finished(u, m, n)) finish(m, n, sk_bias(job, n), sk_addend<T>(job, m, n));
     }
   }
   tcgen05_fence_before();
@@ -333,7 +374,7 @@ int skinny_gemm(const SkinnyJob* jobs, int njobs, int M, int in_dtype, bool pdl,
   const int ring = p.stages * p.stage_bytes;
   p.tmem_cols = 32;
   while (p.tmem_cols < p.mpad * (dual ? 2 : 1)) p.tmem_cols *= 2;
-  const size_t smem = 1024 + ring + p.red_bytes + (2 * kSkMaxStages + 1) * 8 + 16;
+  const size_t smem = 1024 + ring + p.red_bytes + (2 * kSkMaxStages + 1) * 8 + 16 + 4 * kSkinnyMaxRows;
   if (in_dtype == kBF16) return launch_skinny<__nv_bfloat16>(maps, p, tiles, smem, pdl, st);
   return launch_skinny<__half>(maps, p, tiles, smem, pdl, st);
 }

@@ -229,6 +229,7 @@ class DecodeSession:
         splits = require().decode_attend_splits(B * a.num_heads, m.chunk_size)
         self._buf = {n: torch.empty(B, k, dtype=self.dtype, device=dev) for n, k in
                      dict(t=D, mx=D, z=S, r=V, v=V, h=D, attn=V, y=D, f=D, u=F, x0=D, x1=D).items()}
+        self._buf["sq"] = torch.empty(B, a.timenorm.groups_per_partition, dtype=torch.float32, device=dev)
         self._buf["logits"] = torch.empty(B, m.output_size, dtype=torch.float32, device=dev)
         self._buf["part"] = torch.empty(B * a.num_heads * splits * (a.local_v_head_dim + 2), device=dev)
 
@@ -260,9 +261,9 @@ class DecodeSession:
         coeffs = [self._coefficients(_unwrap(layer).mega) for layer in m.layers]
         self._keep = [table, coeffs]     # what a captured graph reads besides the session's buffers and the weights
 
-        def products(xs, ws, biases, addends, acts, outs, w2=None):
+        def products(xs, ws, biases, addends, acts, outs, w2=None, row_sqs=(), row_eps=0.0):
             rc = C.skinny_gemm(xs, ws, [w2] if w2 is not None else [None] * len(xs), biases, addends, acts, outs, True,
-                               err)
+                               err, list(row_sqs), row_eps)
             if rc != 0:
                 raise RuntimeError(f"decode products: launch failed with code {rc}")
 
@@ -276,10 +277,11 @@ class DecodeSession:
             count, mean, var = st["norm"]
             C.decode_norm_ema(x, a.timenorm.weight, a.timenorm.bias, count, mean, var, b["t"], *coeffs[n],
                               torch.view_as_real(st["hx"]), a.rmsnorm.weight, b["mx"], None, 0, a.timenorm.eps,
-                              a.rmsnorm.eps, n > 0)
+                              a.rmsnorm.eps, b["sq"], n > 0)
+            # (b["mx"] is still without the factor of its RMSNorm)
             products([b["mx"], b["mx"], b["t"], b["mx"]], [a.wh1.weight, a.wr.weight, a.wv.weight, a.wz.weight],
                      [a.wh1.bias, a.wr.bias, a.wv.bias, a.wz.bias], [x, None, None, None], [0, 1, 1, 0],
-                     [b["h"], b["r"], b["v"], b["z"]])
+                     [b["h"], b["r"], b["v"], b["z"]], None, [b["sq"], b["sq"], None, b["sq"]], a.rmsnorm.eps)
             C.decode_attend(b["z"], a.gamma, a.beta, table, b["v"], st["k"], st["v"], self.pos, b["r"], b["attn"],
                             b["part"], a.znorm.eps, True)
             products([b["attn"]], [a.wh2.weight], [None], [b["h"]], [0], [b["y"]])

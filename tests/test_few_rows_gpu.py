@@ -128,6 +128,63 @@ def test_decode_attend(B, H, C, dk, dv, pos):
     assert _rel(kb[:, :, pos], qk[1]) < 2.0 ** -8 and torch.equal(vb[:, :, pos].reshape(B, -1), v)
 
 
+@pytest.mark.parametrize("B,H,C,dk,dv,dtype", [(1, 1, 96, 256, 2048, torch.bfloat16), (2, 1, 96, 64, 512, torch.float16),
+                                               (1, 1, 300, 72, 264, torch.bfloat16), (20, 1, 96, 256, 136, torch.bfloat16),
+                                               (50, 2, 40, 32, 4096, torch.float16), (300, 1, 12, 8, 24, torch.bfloat16)])
+def test_decode_attention_in_one_launch(B, H, C, dk, dv, dtype):
+    """Clusters over the keys: fewer keys than splits, the edges of a ring stage and of a box, several column blocks,
+    widths that do and do not suit the tensor cores, more heads than fill the GPU."""
+    from megalodon_b200 import ops
+    torch.manual_seed(dv)
+    q = torch.randn(B, H, dk, device="cuda").to(dtype)
+    k, v = torch.randn(B, H, C, dk, device="cuda").to(dtype), torch.randn(B, H, C, dv, device="cuda").to(dtype)
+    for pos in sorted({0, 1, 14, 15, 16, 31, 32, 33, C // 2, C - 1} & set(range(C))):
+        kn, vn = k.clone(), v.clone()
+        kn[:, :, pos + 1:] = float("nan")
+        vn[:, :, pos + 1:] = float("nan")
+        out = ops.decode_attention(q, kn, vn, torch.tensor([pos], device="cuda"), 0.4)
+        s = torch.einsum("bhd,bhcd->bhc", q.double(), k[:, :, :pos + 1].double()) * 0.4
+        ref = torch.einsum("bhc,bhcd->bhd", torch.softmax(s, -1), v[:, :, :pos + 1].double())
+        # fp32 throughout, one rounding
+        assert _rel(out, ref) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), pos
+
+
+@pytest.mark.parametrize("D,G,N,B", [(512, 32, 16, 1), (96, 3, 4, 2), (4096, 64, 16, 3), (64, 1, 32, 1), (2048, 64, 16, 40),
+                                     (80, 10, 2, 2), (8192, 8, 32, 1)])
+def test_decode_norm_ema_in_parts(D, G, N, B):
+    """The norm + EMA link whose RMSNorm factor is left to the products against the one that applies it, twice in a row
+    (the count, which also tells who came last), and the products that apply it."""
+    from megalodon_b200.ops import cuda_ops
+    C = cuda_ops._C()
+    torch.manual_seed(D)
+
+    def rand(*s):
+        return torch.randn(*s, device="cuda")
+    w, b, rw, omega = (rand(D).mul_(0.1).bfloat16() for _ in range(4))
+    p, q, ga = torch.rand(D, N, device="cuda"), rand(D, N, 2) * 0.4, rand(D, N, 2)
+    state = [torch.arange(B, device="cuda"), rand(B, G) * 0.1, torch.rand(B, G, device="cuda") + 0.5, rand(B, D, N, 2)]
+    other = [t.clone() for t in state]
+    weight, bias = (rand(96, D) * D ** -0.5).bfloat16(), rand(96).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for step in range(2):
+        x = rand(B, D).bfloat16()
+        outs = []
+        for (count, mean, var, hx), sq in ((state, None), (other, torch.empty(B, G, device="cuda"))):
+            t, mx = torch.empty_like(x), torch.empty_like(x)
+            args = (x, w, b, count, mean, var, t, p, q, ga, omega, hx, rw, mx, None, 0, 1e-5, 1e-5)
+            C.decode_norm_ema(*args, *([] if sq is None else [sq]), False)
+            y = torch.empty(B, 96, device="cuda")
+            assert C.skinny_gemm([mx], [weight], [None], [bias], [None], [0], [y], False, err,
+                                 [] if sq is None else [sq], 1e-5) == 0
+            outs.append((t, y))
+        assert torch.equal(state[0], other[0]) and (state[0] == torch.arange(B, device="cuda") + step + 1).all()
+        assert _rel(other[1], state[1]) < 1e-6 and _rel(other[2], state[2]) < 1e-6
+        # (a rounding of t may fall the other way, and so may one of mx)
+        assert _rel(outs[1][0], outs[0][0]) < 2.0 ** -12 and _rel(other[3], state[3]) < 2.0 ** -12
+        assert _rel(outs[1][1], outs[0][1]) < 2.0 ** -7
+    assert err.item() == 0
+
+
 @pytest.mark.parametrize("swiglu,B,D,H,share", [(True, 1, 256, 2, False), (False, 5, 512, 1, True)])
 def test_native_session_matches_cache_path(swiglu, B, D, H, share):
     """The native chain, eager and replayed, against the growing cache; one step across the chunk boundary."""
