@@ -1163,6 +1163,8 @@ void reduce_slots(const Tensor& slots, Tensor& out, int64_t world) {
   mb::reduce_slots(slots.data_ptr(), out.data_ptr(), out.numel(), (int)world, dtype_code(out), stream());
 }
 
+#include "mega_block.h"
+
 }  // namespace
 
 // Every operator below launches kernels on the current stream.  `checked(fn)` wraps a binding so that
@@ -1250,6 +1252,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decode_attention", checked(&decode_attention));
   m.def("decode_norm_ema", checked(&decode_norm_ema));
   m.def("decode_norm_ema", checked(&decode_norm_ema_parts));
+  m.def("mega_block_fwd", checked(&mega_block_fwd));
+  m.def("mega_block_bwd", checked(&mega_block_bwd));
   m.def("decode_norm_ema_ok", &decode_norm_ema_ok);
   m.def("decode_attend_splits", &decode_attend_splits);
   m.def("decode_attend", checked(&decode_attend));

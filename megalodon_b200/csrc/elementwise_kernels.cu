@@ -72,6 +72,25 @@ __global__ void silu_bwd_kernel(const T* __restrict__ g, const T* __restrict__ a
   for (long long i = 8 * n8 + tid; i < n; i += stride) da[i] = from_f<T>(to_f(g[i]) * silu_grad_f(to_f(a[i])));
 }
 
+// dst += a + b, rounded once
+template <typename T>
+__global__ void add_two_kernel(T* __restrict__ dst, const T* __restrict__ a, const T* __restrict__ b, long long n,
+                               long long n8) {
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (long long i = tid; i < n8; i += stride) {
+    float d[8], av[8], bv[8];
+    load8(dst + 8 * i, d);
+    load8(a + 8 * i, av);
+    load8(b + 8 * i, bv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) d[j] += av[j] + bv[j];
+    store8(dst + 8 * i, d);
+  }
+  for (long long i = 8 * n8 + tid; i < n; i += stride) dst[i] = from_f<T>(to_f(dst[i]) + (to_f(a[i]) + to_f(b[i])));
+}
+
 // x [rows, H, Dh]; position of a row is row % L; freqs [L, Dh/2] (cos, sin)
 template <typename T>
 __global__ void rotary_kernel(const T* __restrict__ x, const float2* __restrict__ freqs, T* __restrict__ out,
@@ -422,6 +441,13 @@ void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cu
   const long long n8 = (aligned32(g) && aligned32(a) && aligned32(da)) ? n / 8 : 0;
   MB_DISPATCH_DTYPE(dtype, (silu_bwd_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
                                (const scalar_t*)g, (const scalar_t*)a, (scalar_t*)da, n, n8)));
+}
+
+void add_two(void* dst, const void* a, const void* b, long long n, int dtype, cudaStream_t st) {
+  if (n == 0) return;
+  const long long n8 = (aligned32(dst) && aligned32(a) && aligned32(b)) ? n / 8 : 0;
+  MB_DISPATCH_DTYPE(dtype, (add_two_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+                               (scalar_t*)dst, (const scalar_t*)a, (const scalar_t*)b, n, n8)));
 }
 
 void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db, long long n, int a_dtype, int dtype,

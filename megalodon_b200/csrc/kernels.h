@@ -67,6 +67,7 @@ void cema_coeffs_bwd(const float* dp, const float* dq, const float* dg, const vo
 // ---- element-wise (elementwise_kernels.cu)
 // a_dtype: that of b or fp32; everything else, the gradient of a included, in the type of b
 void swiglu_fwd(const void* a, const void* b, void* out, long long n, int a_dtype, int dtype, cudaStream_t st);
+void add_two(void* dst, const void* a, const void* b, long long n, int dtype, cudaStream_t st);   // dst += a + b
 void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cudaStream_t st);
 void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db, long long n, int a_dtype, int dtype,
                 cudaStream_t st);

@@ -27,6 +27,7 @@ from ..modules import (
     RotaryEmbedding,
     TimestepNorm,
 )
+from ..modules import native_block
 from ..modules.moving_average_gated_attention import _InnerAttention, explicit_causal_mask
 from ..parallel import (
     FullyShardedDataParallel,
@@ -71,6 +72,9 @@ class MegaBlock(nn.Module):
 
     def forward(self, x: Tensor, freqs_cis: Tensor, mask: Optional[Tensor] = None, cache=None,
                 carry=None, piece=None):
+        done = native_block.forward(self, x, freqs_cis, mask, cache, carry, piece)
+        if done is not None:
+            return done
         y, state = self.mega(x, freqs_cis, mask, cache, carry, piece)
         # two-hop residual: the FFN adds the block input, not the attention output
         return self.nffn(y, x), state
