@@ -57,6 +57,7 @@ template <typename T>
 __global__ void attn_softmax_fwd_kernel(T* __restrict__ s, float* __restrict__ lse, int L1, int L2,
                                         long long ld, bool causal, int tile, float drop_p,
                                         unsigned long long seed, unsigned long long offset) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
@@ -99,6 +100,7 @@ __global__ void attn_softmax_fwd_kernel(T* __restrict__ s, float* __restrict__ l
 template <typename T>
 __global__ void attn_softmax_bwd_kernel(const T* __restrict__ p, T* __restrict__ dp, int L1, int L2, long long ld,
                                         bool causal, int tile) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
@@ -137,6 +139,7 @@ template <typename T>
 __global__ void attn_softmax_fwd_vec_kernel(T* __restrict__ s, float* __restrict__ lse, int L1, int L2,
                                             long long ld, bool causal, int tile, float drop_p,
                                             unsigned long long seed, unsigned long long offset) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
@@ -194,6 +197,7 @@ __global__ void attn_softmax_fwd_vec_kernel(T* __restrict__ s, float* __restrict
 template <typename T>
 __global__ void attn_softmax_bwd_vec_kernel(const T* __restrict__ p, T* __restrict__ dp, int L1, int L2,
                                             long long ld, bool causal, int tile) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const int pos = (int)(row % L1);
@@ -244,6 +248,7 @@ template <typename T>
 __global__ void attn_bwd_prep_kernel(const T* __restrict__ dout, const T* __restrict__ out,
                                      const float* __restrict__ rowsum, T* __restrict__ dos,
                                      float* __restrict__ delta, long long rows, int L, int H, int dv) {
+  begin_dependent();
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -281,7 +286,7 @@ void attn_bwd_prep(const void* dout, const void* out, const float* rowsum, void*
   const long long rows = (long long)B * L * H;
   if (rows == 0) return;
   const int warps = 8;
-  MB_DISPATCH_16BIT(dtype, (attn_bwd_prep_kernel<scalar_t><<<(unsigned)div_up(rows, warps), warps * 32, 0, st>>>(
+  MB_DISPATCH_16BIT(dtype, (launch_dependent(attn_bwd_prep_kernel<scalar_t>, (unsigned)div_up(rows, warps), warps * 32, 0, st, 
                                (const scalar_t*)dout, (const scalar_t*)out, rowsum, (scalar_t*)dos, delta, rows, L, H,
                                dv)));
 }
@@ -291,11 +296,11 @@ void attn_softmax_fwd(void* s_inout, float* lse, long long rows, int L1, int L2,
                       cudaStream_t st) {
   if (rows == 0) return;
   if (softmax_vec_ok(s_inout, L2, ld, dtype)) {
-    MB_DISPATCH_DTYPE(dtype, (attn_softmax_fwd_vec_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
+    MB_DISPATCH_DTYPE(dtype, (launch_dependent(attn_softmax_fwd_vec_kernel<scalar_t>, (unsigned)rows, kSmThreads, 0, st, 
                                  (scalar_t*)s_inout, lse, L1, L2, ld, causal, tile, dropkey_p, seed, offset)));
     return;
   }
-  MB_DISPATCH_DTYPE(dtype, (attn_softmax_fwd_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(attn_softmax_fwd_kernel<scalar_t>, (unsigned)rows, kSmThreads, 0, st, 
                                (scalar_t*)s_inout, lse, L1, L2, ld, causal, tile, dropkey_p, seed, offset)));
 }
 
@@ -303,11 +308,11 @@ void attn_softmax_bwd(const void* p, void* dp_inout, long long rows, int L1, int
                       int tile, int dtype, cudaStream_t st) {
   if (rows == 0) return;
   if (softmax_vec_ok(p, L2, ld, dtype) && (reinterpret_cast<uintptr_t>(dp_inout) & 31) == 0) {
-    MB_DISPATCH_DTYPE(dtype, (attn_softmax_bwd_vec_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
+    MB_DISPATCH_DTYPE(dtype, (launch_dependent(attn_softmax_bwd_vec_kernel<scalar_t>, (unsigned)rows, kSmThreads, 0, st, 
                                  (const scalar_t*)p, (scalar_t*)dp_inout, L1, L2, ld, causal, tile)));
     return;
   }
-  MB_DISPATCH_DTYPE(dtype, (attn_softmax_bwd_kernel<scalar_t><<<(unsigned)rows, kSmThreads, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(attn_softmax_bwd_kernel<scalar_t>, (unsigned)rows, kSmThreads, 0, st, 
                                (const scalar_t*)p, (scalar_t*)dp_inout, L1, L2, ld, causal, tile)));
 }
 

@@ -92,6 +92,7 @@ template <typename T, int NPT, int NSPLIT>
 __global__ void cema_fwd_local(const T* __restrict__ x, const float* __restrict__ p,
                                const cfloat* __restrict__ q, const cfloat* __restrict__ g,
                                cfloat* __restrict__ carry, Geo geo) {
+  begin_dependent();
   CEMA_THREAD_SETUP();
   Coef<NPT> c;
   load_coef<NPT, NSPLIT>(c, p, q, g, dd, split, geo.N);
@@ -125,6 +126,7 @@ __global__ void cema_fwd_local(const T* __restrict__ x, const float* __restrict_
 __global__ void cema_combine(cfloat* __restrict__ carry, const cfloat* __restrict__ q,
                              const cfloat* __restrict__ init /* [B, D, N] or null */,
                              cfloat* __restrict__ final_out /* [B, D, N] or null */, Geo geo, bool reverse) {
+  begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long per_b = (long long)geo.N * geo.D;
   if (i >= per_b * geo.B) return;
@@ -157,6 +159,7 @@ __global__ void cema_fwd_final(const T* __restrict__ x, const float* __restrict_
                                const float* __restrict__ omega, const cfloat* __restrict__ incoming,
                                const cfloat* __restrict__ hx, T* __restrict__ y,
                                cfloat* __restrict__ h_last, Geo geo) {
+  begin_dependent();
   CEMA_THREAD_SETUP();
   Coef<NPT> c;
   load_coef<NPT, NSPLIT>(c, p, q, g, dd, split, geo.N);
@@ -202,6 +205,7 @@ template <typename T, int NPT, int NSPLIT>
 __global__ void cema_bwd_rev_local(const T* __restrict__ dy, const float* __restrict__ p,
                                    const cfloat* __restrict__ q, const cfloat* __restrict__ g,
                                    cfloat* __restrict__ carry, Geo geo) {
+  begin_dependent();
   CEMA_THREAD_SETUP();
   Coef<NPT> c;
   load_coef<NPT, NSPLIT>(c, p, q, g, dd, split, geo.N);
@@ -237,6 +241,7 @@ __global__ void cema_bwd_rev_final(const T* __restrict__ dy, const T* __restrict
                                    const cfloat* __restrict__ incoming, const cfloat* __restrict__ dh_last,
                                    T* __restrict__ dx, float* __restrict__ dp, float* __restrict__ domega,
                                    cfloat* __restrict__ dhx, Geo geo) {
+  begin_dependent();
   CEMA_THREAD_SETUP();
   Coef<NPT> c;
   load_coef<NPT, NSPLIT>(c, p, q, g, dd, split, geo.N);
@@ -296,6 +301,7 @@ template <typename T, int NPT, int NSPLIT>
 __global__ void cema_bwd_fwd_local(const T* __restrict__ x, const float* __restrict__ p,
                                    const cfloat* __restrict__ q, const cfloat* __restrict__ g,
                                    cfloat* __restrict__ carry_h, cfloat* __restrict__ carry_u, Geo geo) {
+  begin_dependent();
   CEMA_THREAD_SETUP();
   Coef<NPT> c;
   load_coef<NPT, NSPLIT>(c, p, q, g, dd, split, geo.N);
@@ -333,6 +339,7 @@ __global__ void cema_bwd_fwd_local(const T* __restrict__ x, const float* __restr
 __global__ void cema_bwd_fwd_combine(cfloat* __restrict__ carry_h, cfloat* __restrict__ carry_u,
                                      const cfloat* __restrict__ q, const cfloat* __restrict__ hx,
                                      const cfloat* __restrict__ dh_last, float* __restrict__ dq, Geo geo) {
+  begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long per_b = (long long)geo.N * geo.D;
   if (i >= per_b * geo.B) return;
@@ -374,6 +381,7 @@ __global__ void cema_bwd_fwd_final(const T* __restrict__ dy, const T* __restrict
                                    const cfloat* __restrict__ inc_u, const cfloat* __restrict__ hx,
                                    const cfloat* __restrict__ dh_last, float* __restrict__ dgamma,
                                    float* __restrict__ dq, Geo geo) {
+  begin_dependent();
   CEMA_THREAD_SETUP();
   Coef<NPT> c;
   load_coef<NPT, NSPLIT>(c, p, q, g, dd, split, geo.N);
@@ -580,6 +588,7 @@ template <typename T, int NSPLIT>
 __global__ void __launch_bounds__(kTileFeat* NSPLIT)
 cema_fwd_local_t(const T* __restrict__ x, const float* __restrict__ p, const cfloat* __restrict__ q,
                  cfloat* __restrict__ carry, Geo geo) {
+  begin_dependent();
   constexpr int NPT = 8;
   __shared__ __align__(16) T sm_in[kStages * kTileElems];
   CEMA_TILE_SETUP();
@@ -611,6 +620,7 @@ cema_fwd_final_t(const T* __restrict__ x, const float* __restrict__ p, const cfl
                  const cfloat* __restrict__ g, const float* __restrict__ omega,
                  const cfloat* __restrict__ incoming, const cfloat* __restrict__ hx, T* __restrict__ y,
                  cfloat* __restrict__ h_last, Geo geo) {
+  begin_dependent();
   constexpr int NPT = 8;
   __shared__ __align__(16) T sm_in[kStages * kTileElems];
   __shared__ __align__(16) T sm_out[2 * kTileElems];
@@ -651,6 +661,7 @@ template <typename T, int NSPLIT>
 __global__ void __launch_bounds__(kTileFeat* NSPLIT)
 cema_bwd_rev_local_t(const T* __restrict__ dy, const cfloat* __restrict__ q, const cfloat* __restrict__ g,
                      cfloat* __restrict__ carry, Geo geo) {
+  begin_dependent();
   constexpr int NPT = 8;
   __shared__ __align__(16) T sm_in[kStages * kTileElems];
   CEMA_TILE_SETUP();
@@ -683,6 +694,7 @@ cema_bwd_rev_final_t(const T* __restrict__ dy, const T* __restrict__ x, const fl
                      const cfloat* __restrict__ q, const cfloat* __restrict__ g, const float* __restrict__ omega,
                      const cfloat* __restrict__ incoming, const cfloat* __restrict__ dh_last, T* __restrict__ dx,
                      float* __restrict__ dp, float* __restrict__ domega, cfloat* __restrict__ dhx, Geo geo) {
+  begin_dependent();
   constexpr int NPT = 8;
   __shared__ __align__(16) T sm_in[2 * kStages * kTileElems];
   __shared__ __align__(16) T sm_out[2 * kTileElems];
@@ -736,6 +748,7 @@ template <typename T, int NSPLIT>
 __global__ void __launch_bounds__(kTileFeat* NSPLIT)
 cema_bwd_fwd_local_t(const T* __restrict__ x, const float* __restrict__ p, const cfloat* __restrict__ q,
                      cfloat* __restrict__ carry_h, cfloat* __restrict__ carry_u, Geo geo) {
+  begin_dependent();
   constexpr int NPT = 8;
   __shared__ __align__(16) T sm_in[kStages * kTileElems];
   CEMA_TILE_SETUP();
@@ -776,6 +789,7 @@ cema_bwd_fwd_final_t(const T* __restrict__ dy, const T* __restrict__ x, const fl
                      const cfloat* __restrict__ inc_u, const cfloat* __restrict__ hx,
                      const cfloat* __restrict__ dh_last, float* __restrict__ dgamma, float* __restrict__ dq,
                      Geo geo) {
+  begin_dependent();
   constexpr int NPT = 8;
   __shared__ __align__(16) T sm_in[2 * kStages * kTileElems];
   CEMA_TILE_SETUP();
@@ -913,12 +927,12 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
         if (geo.S > 1) {
           // the end state of the last segment is never needed (fwd_final produces h_last)
           dim3 grid_a(grid.x, geo.S - 1, B);
-          cema_fwd_local_t<T, NSPLIT><<<grid_a, kTileFeat * NSPLIT, 0, st>>>((const T*)x, p, qc, (cfloat*)carry, geo);
+          launch_dependent(cema_fwd_local_t<T, NSPLIT>, grid_a, kTileFeat * NSPLIT, 0, st, (const T*)x, p, qc, (cfloat*)carry, geo);
           const long long n = (long long)B * N * D;
-          cema_combine<<<div_up(n, 256), 256, 0, st>>>((cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
+          launch_dependent(cema_combine, div_up(n, 256), 256, 0, st, (cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
           incoming = (const cfloat*)carry;
         }
-        cema_fwd_final_t<T, NSPLIT><<<grid, kTileFeat * NSPLIT, 0, st>>>(
+        launch_dependent(cema_fwd_final_t<T, NSPLIT>, grid, kTileFeat * NSPLIT, 0, st, 
             (const T*)x, p, qc, gc, omega, incoming, (const cfloat*)hx, (T*)y, (cfloat*)h_last, geo);
       });
     });
@@ -930,12 +944,12 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
       dim3 grid(div_up((long long)D * NSPLIT, kCemaThreads), geo.S, B);
       const cfloat* incoming = nullptr;
       if (geo.S > 1) {
-        cema_fwd_local<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>((const T*)x, p, qc, gc, (cfloat*)carry, geo);
+        launch_dependent(cema_fwd_local<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, (const T*)x, p, qc, gc, (cfloat*)carry, geo);
         const long long n = (long long)B * N * D;
-        cema_combine<<<div_up(n, 256), 256, 0, st>>>((cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
+        launch_dependent(cema_combine, div_up(n, 256), 256, 0, st, (cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
         incoming = (const cfloat*)carry;
       }
-      cema_fwd_final<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>(
+      launch_dependent(cema_fwd_final<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, 
           (const T*)x, p, qc, gc, omega, incoming, (const cfloat*)hx, (T*)y, (cfloat*)h_last, geo);
     });
   });
@@ -958,25 +972,25 @@ void cema_bwd(const void* dy, const void* x, const float* p, const float* q, con
         dim3 grid(div_up(D, kTileFeat), geo.S, B);
         const cfloat* inc = nullptr;
         if (geo.S > 1) {
-          cema_bwd_rev_local_t<T, NSPLIT><<<grid, nthr, 0, st>>>((const T*)dy, qc, gc, (cfloat*)carry_a, geo);
-          cema_combine<<<div_up(nbd, 256), 256, 0, st>>>((cfloat*)carry_a, qc, (const cfloat*)dh_last,
+          launch_dependent(cema_bwd_rev_local_t<T, NSPLIT>, grid, nthr, 0, st, (const T*)dy, qc, gc, (cfloat*)carry_a, geo);
+          launch_dependent(cema_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, qc, (const cfloat*)dh_last,
                                                          (cfloat*)dhx, geo, true);
           inc = (const cfloat*)carry_a;
         }
-        cema_bwd_rev_final_t<T, NSPLIT><<<grid, nthr, 0, st>>>(
+        launch_dependent(cema_bwd_rev_final_t<T, NSPLIT>, grid, nthr, 0, st, 
             (const T*)dy, (const T*)x, p, qc, gc, omega, inc, (const cfloat*)dh_last, (T*)dx, dp, domega,
             (cfloat*)dhx, geo);
         const cfloat* inc_h = nullptr;
         const cfloat* inc_u = nullptr;
         if (geo.S > 1) {
-          cema_bwd_fwd_local_t<T, NSPLIT><<<grid, nthr, 0, st>>>((const T*)x, p, qc, (cfloat*)carry_a,
+          launch_dependent(cema_bwd_fwd_local_t<T, NSPLIT>, grid, nthr, 0, st, (const T*)x, p, qc, (cfloat*)carry_a,
                                                                 (cfloat*)carry_b, geo);
-          cema_bwd_fwd_combine<<<div_up(nbd, 256), 256, 0, st>>>((cfloat*)carry_a, (cfloat*)carry_b, qc,
+          launch_dependent(cema_bwd_fwd_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, (cfloat*)carry_b, qc,
                                                                  (const cfloat*)hx, (const cfloat*)dh_last, dq, geo);
           inc_h = (const cfloat*)carry_a;
           inc_u = (const cfloat*)carry_b;
         }
-        cema_bwd_fwd_final_t<T, NSPLIT><<<grid, nthr, 0, st>>>(
+        launch_dependent(cema_bwd_fwd_final_t<T, NSPLIT>, grid, nthr, 0, st, 
             (const T*)dy, (const T*)x, p, qc, gc, inc_h, inc_u, (const cfloat*)hx, (const cfloat*)dh_last,
             dgamma, dq, geo);
       });
@@ -990,26 +1004,26 @@ void cema_bwd(const void* dy, const void* x, const float* p, const float* q, con
       // adjoint pass
       const cfloat* inc = nullptr;
       if (geo.S > 1) {
-        cema_bwd_rev_local<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>((const T*)dy, p, qc, gc, (cfloat*)carry_a, geo);
-        cema_combine<<<div_up(nbd, 256), 256, 0, st>>>((cfloat*)carry_a, qc, (const cfloat*)dh_last,
+        launch_dependent(cema_bwd_rev_local<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, (const T*)dy, p, qc, gc, (cfloat*)carry_a, geo);
+        launch_dependent(cema_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, qc, (const cfloat*)dh_last,
                                                        (cfloat*)dhx, geo, true);
         inc = (const cfloat*)carry_a;
       }
-      cema_bwd_rev_final<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>(
+      launch_dependent(cema_bwd_rev_final<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, 
           (const T*)dy, (const T*)x, p, qc, gc, omega, inc, (const cfloat*)dh_last, (T*)dx, dp, domega,
           (cfloat*)dhx, geo);
       // forward-time pass for dgamma, dq
       const cfloat* inc_h = nullptr;
       const cfloat* inc_u = nullptr;
       if (geo.S > 1) {
-        cema_bwd_fwd_local<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>((const T*)x, p, qc, gc, (cfloat*)carry_a,
+        launch_dependent(cema_bwd_fwd_local<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, (const T*)x, p, qc, gc, (cfloat*)carry_a,
                                                                         (cfloat*)carry_b, geo);
-        cema_bwd_fwd_combine<<<div_up(nbd, 256), 256, 0, st>>>((cfloat*)carry_a, (cfloat*)carry_b, qc,
+        launch_dependent(cema_bwd_fwd_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, (cfloat*)carry_b, qc,
                                                                (const cfloat*)hx, (const cfloat*)dh_last, dq, geo);
         inc_h = (const cfloat*)carry_a;
         inc_u = (const cfloat*)carry_b;
       }
-      cema_bwd_fwd_final<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>(
+      launch_dependent(cema_bwd_fwd_final<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, 
           (const T*)dy, (const T*)x, p, qc, gc, inc_h, inc_u, (const cfloat*)hx, (const cfloat*)dh_last,
           dgamma, dq, geo);
     });

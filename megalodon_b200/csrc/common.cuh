@@ -187,6 +187,31 @@ __device__ __forceinline__ cfloat cadd(cfloat a, cfloat b) { return {a.re + b.re
     }                                                         \
   } while (0)
 
+// ---- launches that begin under the end of the kernel before them
+// A kernel launched with `launch_dependent` calls `begin_dependent` before anything else: it returns when every kernel
+// ahead of it in the stream is complete and its writes are visible (at once for an ordinary launch), and lets the next
+// such kernel be placed on the SMs as they come free.  What the pair saves is the time from the last CTA of one kernel to
+// the first of the next, some 1.5 us of it a launch: graph-replayed products of 512 features 8.6 -> 6.9 us.
+__device__ __forceinline__ void begin_dependent() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                    Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace mb

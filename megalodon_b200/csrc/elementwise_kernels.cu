@@ -14,6 +14,7 @@ namespace {
 template <typename A, typename T>
 __global__ void swiglu_fwd_kernel(const A* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                                   long long n, long long n8) {
+  begin_dependent();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
@@ -31,6 +32,7 @@ __global__ void swiglu_fwd_kernel(const A* __restrict__ a, const T* __restrict__
 template <typename A, typename T>
 __global__ void swiglu_bwd_kernel(const T* __restrict__ g, const A* __restrict__ a, const T* __restrict__ b,
                                   T* __restrict__ da, T* __restrict__ db, long long n, long long n8) {
+  begin_dependent();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 2
@@ -58,6 +60,7 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ g, const A* __restrict__
 template <typename T>
 __global__ void silu_bwd_kernel(const T* __restrict__ g, const T* __restrict__ a, T* __restrict__ da, long long n,
                                 long long n8) {
+  begin_dependent();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
@@ -76,6 +79,7 @@ __global__ void silu_bwd_kernel(const T* __restrict__ g, const T* __restrict__ a
 template <typename T>
 __global__ void add_two_kernel(T* __restrict__ dst, const T* __restrict__ a, const T* __restrict__ b, long long n,
                                long long n8) {
+  begin_dependent();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
@@ -95,6 +99,7 @@ __global__ void add_two_kernel(T* __restrict__ dst, const T* __restrict__ a, con
 template <typename T>
 __global__ void rotary_kernel(const T* __restrict__ x, const float2* __restrict__ freqs, T* __restrict__ out,
                               long long rows, int L, int H, int Dh, bool conj) {
+  begin_dependent();
   const int half = Dh / 2;
   const long long total = rows * H * half;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -119,6 +124,7 @@ template <typename T, typename W>
 __global__ void qk_rotary_fwd_kernel(const T* __restrict__ z, const W* __restrict__ gamma, const W* __restrict__ beta,
                                      const float2* __restrict__ freqs, T* __restrict__ q, T* __restrict__ k,
                                      long long rows, int S, int Dh, int P, float inv_sqrt) {
+  begin_dependent();
   const int per_row = S / 8;
   const long long total = rows * per_row;
   const int half = Dh / 2;
@@ -153,6 +159,7 @@ __global__ void qk_rotary_bwd_kernel(const T* __restrict__ dq, const T* __restri
                                      const W* __restrict__ gamma, const float2* __restrict__ freqs,
                                      T* __restrict__ dz, float* __restrict__ partial, long long rows, int S, int Dh,
                                      int P, float inv_sqrt) {
+  begin_dependent();
   const int c0 = threadIdx.x * 8;
   if (c0 >= S) return;
   const int half = Dh / 2;
@@ -200,6 +207,7 @@ __global__ void qk_rotary_bwd_kernel(const T* __restrict__ dq, const T* __restri
 template <typename T>
 __global__ void ce_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target,
                               float* __restrict__ loss, float* __restrict__ lse, int V, long long ignore_index) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
@@ -221,6 +229,7 @@ template <typename T>
 __global__ void ce_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target,
                               const float* __restrict__ lse, const float* __restrict__ dloss,
                               T* __restrict__ dlogits, int V, long long ignore_index) {
+  begin_dependent();
   const long long row = blockIdx.x;
   const long long t = target[row];
   const bool skip = (t == ignore_index || t < 0 || t >= V);
@@ -244,6 +253,7 @@ template <typename T>
 __global__ void __launch_bounds__(kCeThreads)
 ce_fwd_vec_kernel(const T* __restrict__ logits, const long long* __restrict__ target, float* __restrict__ loss,
                   float* __restrict__ lse, int V, long long ignore_index) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
@@ -276,6 +286,7 @@ template <typename T>
 __global__ void __launch_bounds__(kCeThreads)
 ce_bwd_vec_kernel(const T* __restrict__ logits, const long long* __restrict__ target, const float* __restrict__ lse,
                   const float* __restrict__ dloss, T* __restrict__ dlogits, int V, long long ignore_index) {
+  begin_dependent();
   const long long row = blockIdx.x;
   const long long t = target[row];
   const bool skip = (t == ignore_index || t < 0 || t >= V);
@@ -336,6 +347,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, flo
                              float* __restrict__ v, Lo* __restrict__ low, long long n, float lr, float beta1,
                              float beta2, float eps, float wd, float bc1, float bc2_sqrt, float grad_scale,
                              const float* __restrict__ scale_ptr) {
+  begin_dependent();
   const float gs = grad_scale * (scale_ptr ? *scale_ptr : 1.f);
   const float step = lr / bc1;
   const float decay = 1.f - lr * wd;
@@ -375,6 +387,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, flo
 
 template <typename T>
 __global__ void sumsq_kernel(const T* __restrict__ g, long long n, long long n8, double* __restrict__ out) {
+  begin_dependent();
   __shared__ float scratch[32];
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
   float part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -397,6 +410,7 @@ __global__ void sumsq_kernel(const T* __restrict__ g, long long n, long long n8,
 // 16-byte accesses: 1.6 GB of bf16 gradients took 1415 us with one element per access, 492 us now
 template <typename T>
 __global__ void scale_by_ptr_kernel(T* __restrict__ g, long long n, long long n8, const float* __restrict__ scale) {
+  begin_dependent();
   const float s = *scale;
   if (s == 1.f) return;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
@@ -414,6 +428,7 @@ __global__ void scale_by_ptr_kernel(T* __restrict__ g, long long n, long long n8
 // coef = min(1, max_norm / (sqrt(sumsq) + 1e-6)); also writes the norm
 __global__ void clip_coef_kernel(const double* __restrict__ sumsq, float max_norm, float* __restrict__ norm_out,
                                  float* __restrict__ coef_out) {
+  begin_dependent();
   const float norm = (float)sqrt(*sumsq);
   *norm_out = norm;
   const float c = max_norm / (norm + 1e-6f);
@@ -430,23 +445,23 @@ void swiglu_fwd(const void* a, const void* b, void* out, long long n, int a_dtyp
   const int grid = ew_grid(std::max(n8, n - 8 * n8));
   MB_DISPATCH_DTYPE(dtype, {
     if (a_dtype == dtype)
-      swiglu_fwd_kernel<<<grid, 256, 0, st>>>((const scalar_t*)a, (const scalar_t*)b, (scalar_t*)out, n, n8);
+      launch_dependent(swiglu_fwd_kernel<scalar_t, scalar_t>, grid, 256, 0, st, (const scalar_t*)a, (const scalar_t*)b, (scalar_t*)out, n, n8);
     else
-      swiglu_fwd_kernel<<<grid, 256, 0, st>>>((const float*)a, (const scalar_t*)b, (scalar_t*)out, n, n8);
+      launch_dependent(swiglu_fwd_kernel<float, scalar_t>, grid, 256, 0, st, (const float*)a, (const scalar_t*)b, (scalar_t*)out, n, n8);
   });
 }
 
 void silu_bwd(const void* g, const void* a, void* da, long long n, int dtype, cudaStream_t st) {
   if (n == 0) return;
   const long long n8 = (aligned32(g) && aligned32(a) && aligned32(da)) ? n / 8 : 0;
-  MB_DISPATCH_DTYPE(dtype, (silu_bwd_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(silu_bwd_kernel<scalar_t>, ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st, 
                                (const scalar_t*)g, (const scalar_t*)a, (scalar_t*)da, n, n8)));
 }
 
 void add_two(void* dst, const void* a, const void* b, long long n, int dtype, cudaStream_t st) {
   if (n == 0) return;
   const long long n8 = (aligned32(dst) && aligned32(a) && aligned32(b)) ? n / 8 : 0;
-  MB_DISPATCH_DTYPE(dtype, (add_two_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(add_two_kernel<scalar_t>, ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st, 
                                (scalar_t*)dst, (const scalar_t*)a, (const scalar_t*)b, n, n8)));
 }
 
@@ -457,10 +472,10 @@ void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db,
   const int grid = ew_grid(std::max(n8, n - 8 * n8));
   MB_DISPATCH_DTYPE(dtype, {
     if (a_dtype == dtype)
-      swiglu_bwd_kernel<<<grid, 256, 0, st>>>((const scalar_t*)g, (const scalar_t*)a, (const scalar_t*)b, (scalar_t*)da,
+      launch_dependent(swiglu_bwd_kernel<scalar_t, scalar_t>, grid, 256, 0, st, (const scalar_t*)g, (const scalar_t*)a, (const scalar_t*)b, (scalar_t*)da,
                                               (scalar_t*)db, n, n8);
     else
-      swiglu_bwd_kernel<<<grid, 256, 0, st>>>((const scalar_t*)g, (const float*)a, (const scalar_t*)b, (scalar_t*)da,
+      launch_dependent(swiglu_bwd_kernel<float, scalar_t>, grid, 256, 0, st, (const scalar_t*)g, (const float*)a, (const scalar_t*)b, (scalar_t*)da,
                                               (scalar_t*)db, n, n8);
   });
 }
@@ -468,7 +483,7 @@ void swiglu_bwd(const void* g, const void* a, const void* b, void* da, void* db,
 void rotary_apply(const void* x, const float* freqs, void* out, long long rows, int L, int H, int Dh,
                   bool conj, int dtype, cudaStream_t st) {
   const long long n = rows * H * (Dh / 2);
-  MB_DISPATCH_DTYPE(dtype, (rotary_kernel<scalar_t><<<ew_grid(n), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(rotary_kernel<scalar_t>, ew_grid(n), 256, 0, st, 
                                (const scalar_t*)x, (const float2*)freqs, (scalar_t*)out, rows, L, H, Dh, conj)));
 }
 
@@ -480,10 +495,10 @@ void qk_rotary_fwd(const void* z, const void* gamma, const void* beta, const flo
   const float inv = 1.f / sqrtf((float)Dh);
   MB_DISPATCH_16BIT(dtype, {
     if (w_dtype == kF32)
-      qk_rotary_fwd_kernel<scalar_t, float><<<ew_grid(n), 256, 0, st>>>((const scalar_t*)z, (const float*)gamma,
+      launch_dependent(qk_rotary_fwd_kernel<scalar_t, float>, ew_grid(n), 256, 0, st, (const scalar_t*)z, (const float*)gamma,
           (const float*)beta, (const float2*)freqs, (scalar_t*)q, (scalar_t*)k, rows, S, Dh, P, inv);
     else
-      qk_rotary_fwd_kernel<scalar_t, scalar_t><<<ew_grid(n), 256, 0, st>>>((const scalar_t*)z, (const scalar_t*)gamma,
+      launch_dependent(qk_rotary_fwd_kernel<scalar_t, scalar_t>, ew_grid(n), 256, 0, st, (const scalar_t*)z, (const scalar_t*)gamma,
           (const scalar_t*)beta, (const float2*)freqs, (scalar_t*)q, (scalar_t*)k, rows, S, Dh, P, inv);
   });
 }
@@ -499,10 +514,10 @@ void qk_rotary_bwd(const void* dq, const void* dk, const void* z, const void* ga
   const int threads = ((S / 8 + 31) / 32) * 32;
   MB_DISPATCH_16BIT(dtype, {
     if (w_dtype == kF32)
-      qk_rotary_bwd_kernel<scalar_t, float><<<grid, threads, 0, st>>>((const scalar_t*)dq, (const scalar_t*)dk,
+      launch_dependent(qk_rotary_bwd_kernel<scalar_t, float>, grid, threads, 0, st, (const scalar_t*)dq, (const scalar_t*)dk,
           (const scalar_t*)z, (const float*)gamma, (const float2*)freqs, (scalar_t*)dz, partial, rows, S, Dh, P, inv);
     else
-      qk_rotary_bwd_kernel<scalar_t, scalar_t><<<grid, threads, 0, st>>>((const scalar_t*)dq, (const scalar_t*)dk,
+      launch_dependent(qk_rotary_bwd_kernel<scalar_t, scalar_t>, grid, threads, 0, st, (const scalar_t*)dq, (const scalar_t*)dk,
           (const scalar_t*)z, (const scalar_t*)gamma, (const float2*)freqs, (scalar_t*)dz, partial, rows, S, Dh, P, inv);
   });
 }
@@ -511,11 +526,11 @@ void cross_entropy_fwd(const void* logits, const long long* target, float* loss,
                        int V, long long ignore_index, int dtype, cudaStream_t st) {
   if (rows == 0) return;
   if (V % 8 == 0 && aligned32(logits)) {
-    MB_DISPATCH_DTYPE(dtype, (ce_fwd_vec_kernel<scalar_t><<<(unsigned)rows, kCeThreads, 0, st>>>(
+    MB_DISPATCH_DTYPE(dtype, (launch_dependent(ce_fwd_vec_kernel<scalar_t>, (unsigned)rows, kCeThreads, 0, st, 
                                  (const scalar_t*)logits, target, loss, lse, V, ignore_index)));
     return;
   }
-  MB_DISPATCH_DTYPE(dtype, (ce_fwd_kernel<scalar_t><<<(unsigned)rows, 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(ce_fwd_kernel<scalar_t>, (unsigned)rows, 256, 0, st, 
                                (const scalar_t*)logits, target, loss, lse, V, ignore_index)));
 }
 
@@ -524,11 +539,11 @@ void cross_entropy_bwd(const void* logits, const long long* target, const float*
                        cudaStream_t st) {
   if (rows == 0) return;
   if (V % 8 == 0 && aligned32(logits) && aligned32(dlogits)) {
-    MB_DISPATCH_DTYPE(dtype, (ce_bwd_vec_kernel<scalar_t><<<(unsigned)rows, kCeThreads, 0, st>>>(
+    MB_DISPATCH_DTYPE(dtype, (launch_dependent(ce_bwd_vec_kernel<scalar_t>, (unsigned)rows, kCeThreads, 0, st, 
                                  (const scalar_t*)logits, target, lse, dloss, (scalar_t*)dlogits, V, ignore_index)));
     return;
   }
-  MB_DISPATCH_DTYPE(dtype, (ce_bwd_kernel<scalar_t><<<(unsigned)rows, 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(ce_bwd_kernel<scalar_t>, (unsigned)rows, 256, 0, st, 
                                (const scalar_t*)logits, target, lse, dloss, (scalar_t*)dlogits, V, ignore_index)));
 }
 
@@ -542,13 +557,13 @@ void adamw_step(float* p, const void* g, float* m, float* v, void* low, long lon
   MB_DISPATCH_DTYPE(g_dtype, {
     using G = scalar_t;
     if (low == nullptr || low_dtype == kBF16) {
-      adamw_kernel<G, __nv_bfloat16><<<grid, 256, 0, st>>>(p, (const G*)g, m, v, (__nv_bfloat16*)low, n, lr,
+      launch_dependent(adamw_kernel<G, __nv_bfloat16>, grid, 256, 0, st, p, (const G*)g, m, v, (__nv_bfloat16*)low, n, lr,
                                                           beta1, beta2, eps, wd, bc1, bc2s, grad_scale, scale_ptr);
     } else if (low_dtype == kF16) {
-      adamw_kernel<G, __half><<<grid, 256, 0, st>>>(p, (const G*)g, m, v, (__half*)low, n, lr, beta1, beta2,
+      launch_dependent(adamw_kernel<G, __half>, grid, 256, 0, st, p, (const G*)g, m, v, (__half*)low, n, lr, beta1, beta2,
                                                    eps, wd, bc1, bc2s, grad_scale, scale_ptr);
     } else {
-      adamw_kernel<G, float><<<grid, 256, 0, st>>>(p, (const G*)g, m, v, (float*)low, n, lr, beta1, beta2, eps,
+      launch_dependent(adamw_kernel<G, float>, grid, 256, 0, st, p, (const G*)g, m, v, (float*)low, n, lr, beta1, beta2, eps,
                                                   wd, bc1, bc2s, grad_scale, scale_ptr);
     }
   });
@@ -557,19 +572,19 @@ void adamw_step(float* p, const void* g, float* m, float* v, void* low, long lon
 void sum_squares(const void* g, long long n, double* out, int dtype, cudaStream_t st) {
   if (n == 0) return;
   const long long n8 = aligned32(g) ? n / 8 : 0;
-  MB_DISPATCH_DTYPE(dtype, (sumsq_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(sumsq_kernel<scalar_t>, ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st, 
                                (const scalar_t*)g, n, n8, out)));
 }
 
 void scale_by_ptr(void* g, long long n, const float* scale, int dtype, cudaStream_t st) {
   if (n == 0) return;
   const long long n8 = aligned32(g) ? n / 8 : 0;
-  MB_DISPATCH_DTYPE(dtype, (scale_by_ptr_kernel<scalar_t><<<ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(scale_by_ptr_kernel<scalar_t>, ew_grid(std::max(n8, n - 8 * n8)), 256, 0, st, 
                                (scalar_t*)g, n, n8, scale)));
 }
 
 void clip_coef(const double* sumsq, float max_norm, float* norm_out, float* coef_out, cudaStream_t st) {
-  clip_coef_kernel<<<1, 1, 0, st>>>(sumsq, max_norm, norm_out, coef_out);
+  launch_dependent(clip_coef_kernel, 1, 1, 0, st, sumsq, max_norm, norm_out, coef_out);
 }
 
 }  // namespace mb

@@ -147,6 +147,7 @@ template <typename T>
 __global__ void cema_coeffs_fwd_kernel(const T* __restrict__ alpha, const T* __restrict__ delta,
                                        const T* __restrict__ theta, const T* __restrict__ gamma, float scale,
                                        float* __restrict__ p, float2* __restrict__ q, float2* __restrict__ g, int D, int N) {
+  begin_dependent();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= D * N) return;
   const int d = i / N, n = i - d * N + 1;
@@ -167,6 +168,7 @@ __global__ void cema_coeffs_bwd_kernel(const float* __restrict__ dp, const float
                                        const T* __restrict__ delta, const T* __restrict__ theta, float scale,
                                        T* __restrict__ dalpha, T* __restrict__ ddelta, T* __restrict__ dtheta,
                                        T* __restrict__ dgamma, int D, int N) {
+  begin_dependent();
   __shared__ float dphi[256];
   const int per = blockDim.x / N;                    // features of a block
   const int fl = threadIdx.x / N, n = threadIdx.x - fl * N;
@@ -201,7 +203,7 @@ __global__ void cema_coeffs_bwd_kernel(const float* __restrict__ dp, const float
 
 void cema_coeffs_fwd(const void* alpha, const void* delta, const void* theta, const void* gamma, float scale, float* p,
                      float* q, float* g, int D, int N, int dtype, cudaStream_t st) {
-  MB_DISPATCH_DTYPE(dtype, (cema_coeffs_fwd_kernel<scalar_t><<<div_up((long long)D * N, 256), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(cema_coeffs_fwd_kernel<scalar_t>, div_up((long long)D * N, 256), 256, 0, st, 
                                (const scalar_t*)alpha, (const scalar_t*)delta, (const scalar_t*)theta,
                                (const scalar_t*)gamma, scale, p, (float2*)q, (float2*)g, D, N)));
 }
@@ -209,7 +211,7 @@ void cema_coeffs_fwd(const void* alpha, const void* delta, const void* theta, co
 void cema_coeffs_bwd(const float* dp, const float* dq, const float* dg, const void* alpha, const void* delta,
                      const void* theta, float scale, void* dalpha, void* ddelta, void* dtheta, void* dgamma, int D, int N,
                      int dtype, cudaStream_t st) {
-  MB_DISPATCH_DTYPE(dtype, (cema_coeffs_bwd_kernel<scalar_t><<<div_up(D, 256 / N), 256, 0, st>>>(
+  MB_DISPATCH_DTYPE(dtype, (launch_dependent(cema_coeffs_bwd_kernel<scalar_t>, div_up(D, 256 / N), 256, 0, st, 
                                dp, (const float2*)dq, (const float2*)dg, (const scalar_t*)alpha, (const scalar_t*)delta,
                                (const scalar_t*)theta, scale, (scalar_t*)dalpha, (scalar_t*)ddelta, (scalar_t*)dtheta,
                                (scalar_t*)dgamma, D, N)));

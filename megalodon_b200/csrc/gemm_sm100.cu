@@ -659,6 +659,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  begin_dependent();        // barriers, tensor memory and descriptors are set up under the end of the kernel before
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -1003,6 +1004,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
   cluster_sync_all();                               // the peer's barriers exist before anything signals them
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  begin_dependent();        // barriers, tensor memory and descriptors are set up under the end of the kernel before
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -1245,8 +1247,7 @@ static int launch_gemm(const TmapArray& ta, const CUtensorMap& tb, const GemmPar
   if (!allow_dynamic_smem(kern, L::total, configured)) return -2;
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
   const int grid = tiles < sms ? tiles : sms;
-  kern<<<grid, L::threads, L::total, st>>>(ta, tb, p, in_fmt);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch_dependent(kern, grid, L::threads, L::total, st, ta, tb, p, in_fmt) == cudaSuccess ? 0 : -3;
 }
 
 // Pair kernel with copy warps that gather the K-major weight operand from its owners while the tensor
@@ -1276,23 +1277,24 @@ static int launch_gemm_pair(const TmapArray& ta, const CUtensorMap& tb, const Ge
   const int tiles = ((p.M + kPairBM - 1) / kPairBM) * ((p.N + kPairBN - 1) / kPairBN) * p.batch;
   const int pairs = sms / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  kern<<<grid, kPairThreads, L::total, st>>>(ta, tb, p, in_fmt);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch_dependent(kern, grid, kPairThreads, L::total, st, ta, tb, p, in_fmt) == cudaSuccess ? 0 : -3;
 }
 
 static bool g_use_pair = true;
 
 // Which tile a product runs on: the one whose estimate is lowest,
 //   (waves - 1) * max(k-blocks * t, e) + k-blocks * t + c,   t = max(latency, bytes of the resident tiles / rate).
-// Constants from graph-replayed launches over 65 shapes from 100 x 256 x 512 to 8192 x 4096 x 256 in three layouts:
-//   latency per k-block   0.285 us as a CTA pair or 128 x 256, 0.19 as 128 x 128, 0.185 as 128 x 64 (what a ring of
-//                         6, 4, 6, 8 stages leaves of a memory latency)
-//   epilogue e            3.5 / 6.3 / 3.5 / 2.0 us a tile, hidden behind the next tile's loop except at the end
-//   start and end c       7.8 / 9.7 / 6.7 / 4.8 us
-//   rate                  18 TB/s out of L2 and memory together, which the narrow tiles reach first
-// Few wide tiles leave most SMs without work: 1024 x 512 x 512 takes 8.6 us in 8 pair tiles and 5.5 us in 64 tiles of
-// 128 x 64, 2048 x 1024 x 4096 26.1 us in pairs and 18.7 us as 128 x 128; 4000 x 2048 x 4096 48 us in pairs, 66 as
-// 128 x 128 and 93 as 128 x 64.
+// Constants fitted to back-to-back launches (each beginning under the end of the one before) of 139 shapes from
+// 512 x 256 x 1024 to 6216 x 4864 x 2048 in two layouts; the choice is 0.1 % off the best tile over all of them, 5 % at
+// the worst shape:
+//   latency per k-block   0.318 us as a CTA pair, 0.277 as 128 x 256, 0.186 as 128 x 128, 0.191 as 128 x 64 (what a ring
+//                         of 6, 4, 6, 8 stages leaves of a memory latency)
+//   epilogue e            4.6 / 5.8 / 3.8 / 2.6 us a tile, hidden behind the next tile's loop except at the end
+//   start and end c       7.4 / 7.9 / 5.1 / 4.6 us
+//   rate                  21.5 TB/s out of L2 and memory together, which the narrow tiles reach first
+// Few wide tiles leave most SMs without work: 1024 x 512 x 512 takes 9.6 us in 8 pair tiles and 6.1 us in 64 tiles of
+// 128 x 64, 2000 x 1024 x 2560 19.4 us in pairs and 13.4 us as 128 x 128; 4000 x 2048 x 4096 48 us in pairs, 59 as
+// 128 x 128 and 87 as 128 x 64.
 static int pick_tile(const GemmParams& p, int num_sms) {
   const bool pair_ok = g_use_pair && p.M > BM && num_sms >= 2;
   if (p.a_parts > 1 || p.c_nparts > 1) return pair_ok ? kPairTile : 256;
@@ -1300,12 +1302,12 @@ static int pick_tile(const GemmParams& p, int num_sms) {
   // what Q K^T skips above the diagonal P V must not contract.  All of them see the same number of rows, so the row
   // tile may depend on nothing else.
   if (p.mode != 0 && pair_ok) return kPairTile;
-  const double nk = (p.K + BK - 1) / BK, rate = 18e6;      // bytes per us
+  const double nk = (p.K + BK - 1) / BK, rate = 21.5e6;      // bytes per us
   struct Tile { int name, bm, bn; double lat, bytes, e, c; };
-  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.285, 65536, 3.5, 7.8},
-                        {256, BM, 256, 0.285, 49152, 6.3, 9.7},
-                        {128, BM, 128, 0.19, 32768, 3.5, 6.7},
-                        {64, BM, 64, 0.185, 24576, 2.0, 4.8}};
+  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.318, 65536, 4.6, 7.4},
+                        {256, BM, 256, 0.277, 49152, 5.8, 7.9},
+                        {128, BM, 128, 0.186, 32768, 3.8, 5.1},
+                        {64, BM, 64, 0.191, 24576, 2.6, 4.6}};
   int best = 256;
   double best_us = 1e30;
   for (const Tile& t : tiles) {

@@ -22,6 +22,7 @@ template <typename T, typename OutT>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_kernel(const T* __restrict__ x, const T* __restrict__ w, const void* __restrict__ bias, int bias_dtype,
             OutT* __restrict__ y, int N, int K, long long ldw, int act) {
+  begin_dependent();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int n0 = (blockIdx.x * (kGemvThreads / 32) + warp) * kGemvNR;
@@ -82,7 +83,7 @@ template <typename T, typename OutT>
 void launch_gemv(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int N, int K, long long ldw,
                  int act, cudaStream_t st) {
   const int grid = div_up(N, (kGemvThreads / 32) * kGemvNR);
-  gemv_kernel<T, OutT><<<grid, kGemvThreads, 0, st>>>((const T*)x, (const T*)w, bias, bias_dtype, (OutT*)y, N, K, ldw,
+  launch_dependent(gemv_kernel<T, OutT>, grid, kGemvThreads, 0, st, (const T*)x, (const T*)w, bias, bias_dtype, (OutT*)y, N, K, ldw,
                                                       act);
 }
 

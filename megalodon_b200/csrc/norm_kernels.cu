@@ -33,6 +33,7 @@ __global__ void norm_fwd_kernel(const T* __restrict__ x, const W* __restrict__ w
                                 const W* __restrict__ bias, float weight_offset, T* __restrict__ y,
                                 float* __restrict__ mean_out, float* __restrict__ rstd_out, long long M,
                                 int D, float eps) {
+  begin_dependent();
   __shared__ float scratch[32];
   const int rows_per_cta = blockDim.x / ROW_THREADS;
   const int sub = threadIdx.x / ROW_THREADS;
@@ -88,6 +89,7 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
                                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                                 T* __restrict__ dx, float* __restrict__ dweight, float* __restrict__ dbias,
                                 long long M, int D) {
+  begin_dependent();
   __shared__ float scratch[32];
   const int rows_per_cta = blockDim.x / ROW_THREADS;
   const int sub = threadIdx.x / ROW_THREADS;
@@ -155,6 +157,7 @@ __global__ void norm_fwd_vec_kernel(const T* __restrict__ x, const W* __restrict
                                     const W* __restrict__ bias, float weight_offset, T* __restrict__ y,
                                     float* __restrict__ mean_out, float* __restrict__ rstd_out, long long M,
                                     int D, float eps) {
+  begin_dependent();
   __shared__ float scratch[32];
   const int rows_per_cta = blockDim.x / ROW_THREADS;
   const int sub = threadIdx.x / ROW_THREADS;
@@ -232,6 +235,7 @@ __global__ void norm_bwd_vec_kernel(const T* __restrict__ dy, const T* __restric
                                     const W* __restrict__ weight, float weight_offset,
                                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                                     T* __restrict__ dx, long long M, int D, float* __restrict__ colsum_ws) {
+  begin_dependent();
   __shared__ float scratch[32];
   const int rows_per_cta = blockDim.x / ROW_THREADS;
   const int sub = threadIdx.x / ROW_THREADS;
@@ -348,6 +352,7 @@ template <typename O>
 __global__ void __launch_bounds__(kFinishWarps * 32)
 colsum_finish_kernel(const float* __restrict__ ws, int rows, int D, O* __restrict__ out0,
                                      O* __restrict__ out1) {
+  begin_dependent();
   __shared__ float part[2][kFinishWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
@@ -395,25 +400,25 @@ void launch_fwd(const void* x, const void* w, const void* b, float off, void* y,
   if (D <= 1024 && vec_ok(D, 32, {x, w, b, y})) {
     const int threads = 128, rows = threads / 32;
     const int grid = (int)std::min<long long>((M + rows - 1) / rows, 148LL * 16);
-    VPT_SWITCH(D, 32, (norm_fwd_vec_kernel<T, W, LAYER, 32, VPT><<<grid, threads, 0, st>>>(
+    VPT_SWITCH(D, 32, (launch_dependent(norm_fwd_vec_kernel<T, W, LAYER, 32, VPT>, grid, threads, 0, st, 
                            (const T*)x, (const W*)w, (const W*)b, off, (T*)y, mean, rstd, M, D, eps)));
     return;
   }
   if (D > 1024 && vec_ok(D, 256, {x, w, b, y})) {
     const int grid = (int)std::min<long long>(M, 148LL * 8);
-    VPT_SWITCH(D, 256, (norm_fwd_vec_kernel<T, W, LAYER, 256, VPT><<<grid, 256, 0, st>>>(
+    VPT_SWITCH(D, 256, (launch_dependent(norm_fwd_vec_kernel<T, W, LAYER, 256, VPT>, grid, 256, 0, st, 
                             (const T*)x, (const W*)w, (const W*)b, off, (T*)y, mean, rstd, M, D, eps)));
     return;
   }
   if (D <= 1024) {
     const int threads = 128, rows = threads / 32;
     const int grid = (int)std::min<long long>((M + rows - 1) / rows, 148LL * 16);
-    norm_fwd_kernel<T, W, LAYER, 32><<<grid, threads, 0, st>>>((const T*)x, (const W*)w, (const W*)b, off,
+    launch_dependent(norm_fwd_kernel<T, W, LAYER, 32>, grid, threads, 0, st, (const T*)x, (const W*)w, (const W*)b, off,
                                                                (T*)y, mean, rstd, M, D, eps);
   } else {
     const int threads = 256;
     const int grid = (int)std::min<long long>(M, 148LL * 8);
-    norm_fwd_kernel<T, W, LAYER, 256><<<grid, threads, 0, st>>>((const T*)x, (const W*)w, (const W*)b, off,
+    launch_dependent(norm_fwd_kernel<T, W, LAYER, 256>, grid, threads, 0, st, (const T*)x, (const W*)w, (const W*)b, off,
                                                                 (T*)y, mean, rstd, M, D, eps);
   }
 }
@@ -428,7 +433,7 @@ void launch_bwd(const void* dy, const void* x, const void* w, float off, const f
   if (D <= 1024 && vec_ok(D, 32, {dy, x, w, dx})) {
     const int rows = kNarrowThreads / 32;
     const int grid = (int)std::min<long long>((M + rows - 1) / rows, (long long)kColsumRows);
-    VPT_SWITCH(D, 32, (norm_bwd_vec_kernel<T, W, LAYER, 32, VPT><<<grid, kNarrowThreads, 0, st>>>(
+    VPT_SWITCH(D, 32, (launch_dependent(norm_bwd_vec_kernel<T, W, LAYER, 32, VPT>, grid, kNarrowThreads, 0, st, 
                            (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, M, D, ws)));
     if (ws != nullptr) colsum_finish(ws, grid, D, dw, LAYER ? db : nullptr, w_dtype, st);
     return;
@@ -436,7 +441,7 @@ void launch_bwd(const void* dy, const void* x, const void* w, float off, const f
   if (D > 1024 && vec_ok(D, 256, {dy, x, w, dx})) {
     // one resident wave (the accumulators of the column sums cap the kernel at two CTAs per SM)
     const int grid = (int)std::min<long long>(M, (long long)kColsumRows);
-    VPT_SWITCH(D, 256, (norm_bwd_vec_kernel<T, W, LAYER, 256, VPT><<<grid, 256, 0, st>>>(
+    VPT_SWITCH(D, 256, (launch_dependent(norm_bwd_vec_kernel<T, W, LAYER, 256, VPT>, grid, 256, 0, st, 
                             (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, M, D, ws)));
     if (ws != nullptr) colsum_finish(ws, grid, D, dw, LAYER ? db : nullptr, w_dtype, st);
     return;
@@ -445,12 +450,12 @@ void launch_bwd(const void* dy, const void* x, const void* w, float off, const f
   if (D <= 1024) {
     const int threads = 128, rows = threads / 32;
     const int grid = (int)std::min<long long>((M + rows - 1) / rows, 148LL * 4);
-    norm_bwd_kernel<T, W, LAYER, 32><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const W*)w, off,
+    launch_dependent(norm_bwd_kernel<T, W, LAYER, 32>, grid, threads, 0, st, (const T*)dy, (const T*)x, (const W*)w, off,
                                                                mean, rstd, (T*)dx, aw, ab, M, D);
   } else {
     const int threads = 256;
     const int grid = (int)std::min<long long>(M, 148LL * 4);
-    norm_bwd_kernel<T, W, LAYER, 256><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const W*)w, off,
+    launch_dependent(norm_bwd_kernel<T, W, LAYER, 256>, grid, threads, 0, st, (const T*)dy, (const T*)x, (const W*)w, off,
                                                                 mean, rstd, (T*)dx, aw, ab, M, D);
   }
   if (ws != nullptr) colsum_finish(ws, 1, D, dw, LAYER ? db : nullptr, w_dtype, st);
@@ -480,6 +485,7 @@ void rms_norm_fwd(const void* x, const void* w, float w_off, void* y, float* rst
 // of rows with 8-column vectors per thread and leaves one row of partial sums; `colsum_finish` adds them.
 template <typename T, int VPT>
 __global__ void colsum_partial_kernel(const T* __restrict__ g, long long M, int N, float* __restrict__ ws) {
+  begin_dependent();
   const int nvec = N / 8;
   float acc[VPT][8];
 #pragma unroll
@@ -515,9 +521,9 @@ bool colsum_16bit(const void* g, long long M, int N, float* ws, void* out, int o
   const int vpt = (N / 8 + 255) / 256;
 #define MB_COLSUM(TT)                                                                                   \
   do {                                                                                                  \
-    if (vpt <= 1) colsum_partial_kernel<TT, 1><<<grid, 256, 0, st>>>((const TT*)g, M, N, ws);           \
-    else if (vpt <= 2) colsum_partial_kernel<TT, 2><<<grid, 256, 0, st>>>((const TT*)g, M, N, ws);      \
-    else colsum_partial_kernel<TT, 4><<<grid, 256, 0, st>>>((const TT*)g, M, N, ws);                    \
+    if (vpt <= 1) launch_dependent(colsum_partial_kernel<TT, 1>, grid, 256, 0, st, (const TT*)g, M, N, ws);           \
+    else if (vpt <= 2) launch_dependent(colsum_partial_kernel<TT, 2>, grid, 256, 0, st, (const TT*)g, M, N, ws);      \
+    else launch_dependent(colsum_partial_kernel<TT, 4>, grid, 256, 0, st, (const TT*)g, M, N, ws);                    \
   } while (0)
   if (dtype == kBF16) MB_COLSUM(__nv_bfloat16);
   else MB_COLSUM(__half);
@@ -527,7 +533,7 @@ bool colsum_16bit(const void* g, long long M, int N, float* ws, void* out, int o
 }
 
 void colsum_finish(const float* ws, int rows, int D, void* out0, void* out1, int out_dtype, cudaStream_t st) {
-  MB_DISPATCH_DTYPE(out_dtype, (colsum_finish_kernel<scalar_t><<<(D + 31) / 32, kFinishWarps * 32, 0, st>>>(
+  MB_DISPATCH_DTYPE(out_dtype, (launch_dependent(colsum_finish_kernel<scalar_t>, (D + 31) / 32, kFinishWarps * 32, 0, st, 
                                    ws, rows, D, (scalar_t*)out0, (scalar_t*)out1)));
 }
 

@@ -33,6 +33,7 @@ constexpr int kSegLen = 32;  // time steps per scan segment
 template <typename T, int LPG>
 __global__ void tsn_group_stats_kernel(const T* __restrict__ x, float* __restrict__ gu,
                                        float* __restrict__ gv, long long rows, int H, int G) {
+  begin_dependent();
   const int Dg = H / G;
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long grp = gid / LPG;  // (row, g) flattened
@@ -66,6 +67,7 @@ __global__ void tsn_group_stats_kernel(const T* __restrict__ x, float* __restric
 __global__ void tsn_seg_sums_kernel(const float* __restrict__ gu, const float* __restrict__ gv,
                                     const bool* __restrict__ mask, double* __restrict__ seg, int B, int L,
                                     int G, int nseg) {
+  begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)B * nseg * G) return;
   const int g = (int)(i % G);
@@ -95,6 +97,7 @@ __global__ void tsn_seg_prefix_kernel(double* __restrict__ seg, const long long*
                                       const T* __restrict__ prev_mean, const T* __restrict__ prev_var,
                                       long long* __restrict__ count_out, T* __restrict__ mean_out,
                                       T* __restrict__ var_out, int B, int G, int nseg) {
+  begin_dependent();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * G) return;
   const int g = i % G, b = i / G;
@@ -129,6 +132,7 @@ __global__ void tsn_seg_apply_kernel(const float* __restrict__ gu, const float* 
                                      const T* __restrict__ prev_mean, const T* __restrict__ prev_var,
                                      float* __restrict__ cummean, float* __restrict__ cumrstd, int B, int L,
                                      int G, int nseg, float eps) {
+  begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long total = (long long)B * nseg * G;
   if (i >= total) return;
@@ -190,6 +194,7 @@ tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv
                       const T* __restrict__ prev_var, long long* __restrict__ count_out, T* __restrict__ mean_out,
                       T* __restrict__ var_out, float* __restrict__ cummean, float* __restrict__ cumrstd, int L, int G,
                       int nseg, int GT, float eps) {
+  begin_dependent();
   __shared__ double sh[3][kScanMaxThreads];
   const int tid = threadIdx.x;
   const int gl = tid % GT, sgi = tid / GT;
@@ -298,6 +303,7 @@ __global__ void tsn_apply_kernel(const T* __restrict__ x, const float* __restric
                                  float gamma_offset, const W* __restrict__ beta,
                                  const bool* __restrict__ mask, T* __restrict__ y, long long rows, int H,
                                  int G) {
+  begin_dependent();
   const int Dg = H / G;
   const long long total = rows * H;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -319,6 +325,7 @@ __global__ void tsn_group_grads_kernel(const T* __restrict__ dy, const T* __rest
                                        const float* __restrict__ cummean, const W* __restrict__ gamma,
                                        float gamma_offset, float* __restrict__ ux, float* __restrict__ ds,
                                        float* __restrict__ db, long long rows, int H, int G) {
+  begin_dependent();
   const int Dg = H / G;
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long grp = gid / LPG;
@@ -363,6 +370,7 @@ __device__ __forceinline__ double count_at(const int* cumvalid, long long first_
 
 // inclusive prefix count of non-padded steps, one thread per batch row (only used with a padding mask)
 __global__ void tsn_cumvalid_kernel(const bool* __restrict__ mask, int* __restrict__ cumvalid, int B, int L) {
+  begin_dependent();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   int c = 0;
@@ -417,6 +425,7 @@ __global__ void tsn_bwd_seg_maps_kernel(StepIn in, const bool* __restrict__ mask
                                         const long long* __restrict__ count_final,
                                         const T* __restrict__ prev_mean, double* __restrict__ maps, int B, int L,
                                         int G, int nseg) {
+  begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long total = (long long)B * nseg * G;
   if (i >= total) return;
@@ -444,6 +453,7 @@ template <typename T>
 __global__ void tsn_bwd_seg_prefix_kernel(double* __restrict__ maps, const T* __restrict__ dmean_out,
                                           const T* __restrict__ dvar_out, T* __restrict__ dprev_mean,
                                           T* __restrict__ dprev_var, int B, int G, int nseg) {
+  begin_dependent();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * G) return;
   const int g = i % G, b = i / G;
@@ -470,6 +480,7 @@ __global__ void tsn_bwd_seg_apply_kernel(StepIn in, const bool* __restrict__ mas
                                          const T* __restrict__ prev_mean, const double* __restrict__ maps,
                                          float* __restrict__ dux, float* __restrict__ dvx, int B, int L, int G,
                                          int nseg) {
+  begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long total = (long long)B * nseg * G;
   if (i >= total) return;
@@ -504,6 +515,7 @@ tsn_bwd_scan_fused_kernel(StepIn in, const bool* __restrict__ mask, const int* _
                           const T* __restrict__ dmean_out, const T* __restrict__ dvar_out,
                           T* __restrict__ dprev_mean, T* __restrict__ dprev_var, float* __restrict__ dux,
                           float* __restrict__ dvx, int L, int G, int nseg, int GT) {
+  begin_dependent();
   __shared__ double sh[4][kScanMaxThreads];
   const int tid = threadIdx.x;
   const int gl = tid % GT, sgi = tid / GT;
@@ -607,6 +619,7 @@ __global__ void tsn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restri
                                      float gamma_offset, const bool* __restrict__ mask, T* __restrict__ dx,
                                      float* __restrict__ dgamma, float* __restrict__ dbeta, long long rows,
                                      int H, int G) {
+  begin_dependent();
   const int Dg = H / G;
   const float inv_d = 1.f / Dg;
   float acc_g[kBwdCols], acc_b[kBwdCols];
@@ -648,6 +661,7 @@ __global__ void tsn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restri
 template <typename T, int VL>
 __global__ void tsn_group_stats_vec_kernel(const T* __restrict__ x, float* __restrict__ gu, float* __restrict__ gv,
                                            long long ngroups) {
+  begin_dependent();
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long grp = gid / VL;
   const int l = (int)(gid % VL);
@@ -681,6 +695,7 @@ __global__ void tsn_apply_vec_kernel(const T* __restrict__ x, const float* __res
                                      const float* __restrict__ cumrstd, const W* __restrict__ gamma,
                                      float gamma_offset, const W* __restrict__ beta, const bool* __restrict__ mask,
                                      T* __restrict__ y, long long rows, int H, int G) {
+  begin_dependent();
   const int Dg = H / G;
   const int hv = H / 8;
   const long long total = rows * hv;
@@ -711,6 +726,7 @@ __global__ void tsn_group_grads_vec_kernel(const T* __restrict__ dy, const T* __
                                            const float* __restrict__ cummean, const W* __restrict__ gamma,
                                            float gamma_offset, float* __restrict__ ux, float* __restrict__ ds,
                                            float* __restrict__ db, long long ngroups, int G) {
+  begin_dependent();
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long grp = gid / VL;
   const int l = (int)(gid % VL);
@@ -750,6 +766,7 @@ __global__ void tsn_bwd_apply_vec_kernel(const T* __restrict__ dy, const T* __re
                                          float gamma_offset, const bool* __restrict__ mask, T* __restrict__ dx,
                                          long long rows,
                                          int H, int G, float* __restrict__ colsum_ws) {
+  begin_dependent();
   const int Dg = H / G;
   const int hv = H / 8;
   const float inv_d = 1.f / Dg;
@@ -876,38 +893,38 @@ void timestep_norm_fwd(const void* x, const long long* prev_count, const void* p
     if (vec) {
       VL_SWITCH(H / G / 8, {
         const long long threads = rows * G * VL;
-        tsn_group_stats_vec_kernel<T, VL><<<div_up(threads, 256), 256, 0, st>>>((const T*)x, gu, gv, rows * G);
+        launch_dependent(tsn_group_stats_vec_kernel<T, VL>, div_up(threads, 256), 256, 0, st, (const T*)x, gu, gv, rows * G);
       });
     } else {
       LPG_SWITCH(lpg, {
         const long long threads = rows * G * LPG;
-        tsn_group_stats_kernel<T, LPG><<<div_up(threads, 256), 256, 0, st>>>((const T*)x, gu, gv, rows, H, G);
+        launch_dependent(tsn_group_stats_kernel<T, LPG>, div_up(threads, 256), 256, 0, st, (const T*)x, gu, gv, rows, H, G);
       });
     }
     const int seg = tsn_fused_seg(L);
     if (seg > 0 && B <= 65535) {
       const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
-      SEG_SWITCH(seg, (tsn_scan_fused_kernel<T, SEG><<<dim3(div_up(G, gt), B), gt * nseg, 0, st>>>(
+      SEG_SWITCH(seg, (launch_dependent(tsn_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
           gu, gv, mask, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
           cummean, cumrstd, L, G, nseg, gt, eps)));
     } else {
     const int nseg = tsn_num_segments(L);
     const long long nsg = (long long)B * nseg * G;
-    tsn_seg_sums_kernel<<<div_up(nsg, 256), 256, 0, st>>>(gu, gv, mask, seg_scratch, B, L, G, nseg);
-    tsn_seg_prefix_kernel<T><<<div_up((long long)B * G, 128), 128, 0, st>>>(
+    launch_dependent(tsn_seg_sums_kernel, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, B, L, G, nseg);
+    launch_dependent(tsn_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
         seg_scratch, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
         B, G, nseg);
-    tsn_seg_apply_kernel<T><<<div_up(nsg, 256), 256, 0, st>>>(gu, gv, mask, seg_scratch, (const T*)prev_mean,
+    launch_dependent(tsn_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, (const T*)prev_mean,
                                                             (const T*)prev_var, cummean, cumrstd, B, L, G, nseg,
                                                             eps);
     }
     if (vec) {
       const int grid = (int)std::min<long long>(div_up(rows * (H / 8), 256), 148LL * 16);
-      tsn_apply_vec_kernel<T, W><<<grid, 256, 0, st>>>((const T*)x, cummean, cumrstd, (const W*)gamma,
+      launch_dependent(tsn_apply_vec_kernel<T, W>, grid, 256, 0, st, (const T*)x, cummean, cumrstd, (const W*)gamma,
                                                        gamma_offset, (const W*)beta, mask, (T*)y, rows, H, G);
     } else {
       const int grid = (int)std::min<long long>(div_up(rows * H, 256), 148LL * 16);
-      tsn_apply_kernel<T, W><<<grid, 256, 0, st>>>((const T*)x, cummean, cumrstd, (const W*)gamma,
+      launch_dependent(tsn_apply_kernel<T, W>, grid, 256, 0, st, (const T*)x, cummean, cumrstd, (const W*)gamma,
                                                    gamma_offset, (const W*)beta, mask, (T*)y, rows, H, G);
     }
   });
@@ -927,54 +944,54 @@ void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_o
     if (vec) {
       VL_SWITCH(H / G / 8, {
         const long long threads = rows * G * VL;
-        tsn_group_grads_vec_kernel<T, W, VL><<<div_up(threads, 256), 256, 0, st>>>(
+        launch_dependent(tsn_group_grads_vec_kernel<T, W, VL>, div_up(threads, 256), 256, 0, st, 
             (const T*)dy, (const T*)x, cummean, (const W*)gamma, gamma_offset, ux, ds, db, rows * G, G);
       });
     } else {
       LPG_SWITCH(lpg, {
         const long long threads = rows * G * LPG;
-        tsn_group_grads_kernel<T, W, LPG><<<div_up(threads, 256), 256, 0, st>>>(
+        launch_dependent(tsn_group_grads_kernel<T, W, LPG>, div_up(threads, 256), 256, 0, st, 
             (const T*)dy, (const T*)x, cummean, (const W*)gamma, gamma_offset, ux, ds, db, rows, H, G);
       });
     }
-    if (mask != nullptr) tsn_cumvalid_kernel<<<div_up(B, 32), 32, 0, st>>>(mask, cumvalid, B, L);
+    if (mask != nullptr) launch_dependent(tsn_cumvalid_kernel, div_up(B, 32), 32, 0, st, mask, cumvalid, B, L);
     const int* cv = mask != nullptr ? cumvalid : nullptr;
     const StepIn in{ux, ds, db, cummean, cumrstd};
     const int seg = tsn_fused_seg(L);
     if (seg > 0 && B <= 65535) {
       const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
-      SEG_SWITCH(seg, (tsn_bwd_scan_fused_kernel<T, SEG><<<dim3(div_up(G, gt), B), gt * nseg, 0, st>>>(
+      SEG_SWITCH(seg, (launch_dependent(tsn_bwd_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
           in, mask, cv, count_final, (const T*)prev_mean, (const T*)dmean_out, (const T*)dvar_out, (T*)dprev_mean,
           (T*)dprev_var, dux, dvx, L, G, nseg, gt)));
     } else {
     const int nseg = tsn_num_segments(L);
     const long long nsg = (long long)B * nseg * G;
-    tsn_bwd_seg_maps_kernel<T><<<div_up(nsg, 256), 256, 0, st>>>(in, mask, cv, count_final, (const T*)prev_mean,
+    launch_dependent(tsn_bwd_seg_maps_kernel<T>, div_up(nsg, 256), 256, 0, st, in, mask, cv, count_final, (const T*)prev_mean,
                                                                seg_scratch, B, L, G, nseg);
-    tsn_bwd_seg_prefix_kernel<T><<<div_up((long long)B * G, 128), 128, 0, st>>>(
+    launch_dependent(tsn_bwd_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
         seg_scratch, (const T*)dmean_out, (const T*)dvar_out, (T*)dprev_mean, (T*)dprev_var, B, G, nseg);
-    tsn_bwd_seg_apply_kernel<T><<<div_up(nsg, 256), 256, 0, st>>>(in, mask, cv, count_final, (const T*)prev_mean,
+    launch_dependent(tsn_bwd_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, in, mask, cv, count_final, (const T*)prev_mean,
                                                                 seg_scratch, dux, dvx, B, L, G, nseg);
     }
     const int grid = (int)std::min<long long>(rows, vec ? (long long)kColsumRows : 148LL * 4);
     if (vec) {
       const int hv = H / 8;
       if (hv <= kBwdThreads)
-        tsn_bwd_apply_vec_kernel<T, W, 1><<<grid, kBwdThreads, 0, st>>>(
+        launch_dependent(tsn_bwd_apply_vec_kernel<T, W, 1>, grid, kBwdThreads, 0, st, 
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
             rows, H, G, colsum_ws);
       else if (hv <= 2 * kBwdThreads)
-        tsn_bwd_apply_vec_kernel<T, W, 2><<<grid, kBwdThreads, 0, st>>>(
+        launch_dependent(tsn_bwd_apply_vec_kernel<T, W, 2>, grid, kBwdThreads, 0, st, 
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
             rows, H, G, colsum_ws);
       else
-        tsn_bwd_apply_vec_kernel<T, W, 4><<<grid, kBwdThreads, 0, st>>>(
+        launch_dependent(tsn_bwd_apply_vec_kernel<T, W, 4>, grid, kBwdThreads, 0, st, 
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
             rows, H, G, colsum_ws);
       colsum_finish(colsum_ws, grid, H, dgamma, dbeta, w_dtype, st);
     } else {
     cudaMemsetAsync(colsum_ws, 0, sizeof(float) * 2 * H, st);
-    tsn_bwd_apply_kernel<T, W><<<grid, kBwdThreads, 0, st>>>((const T*)dy, (const T*)x, cummean, cumrstd, ux, dux,
+    launch_dependent(tsn_bwd_apply_kernel<T, W>, grid, kBwdThreads, 0, st, (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux,
                                                      dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
                                                      colsum_ws, colsum_ws + H, rows, H, G);
     colsum_finish(colsum_ws, 1, H, dgamma, dbeta, w_dtype, st);
