@@ -914,6 +914,7 @@ int cema_num_segments(int L) { return (L + kCemaSegLen - 1) / kCemaSegLen; }
 void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, const float* omega,
               const float* hx, void* y, float* h_last, float* carry, int B, int L, int D, int N,
               int x_dtype, cudaStream_t st) {
+  if (cema_fwd_tensor(x, p, q, gamma, omega, hx, y, h_last, B, L, D, N, x_dtype, st)) return;
   Geo geo{B, L, D, N, cema_num_segments(L), kCemaSegLen};
   const cfloat* qc = (const cfloat*)q;
   const cfloat* gc = (const cfloat*)gamma;

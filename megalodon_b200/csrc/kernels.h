@@ -50,6 +50,9 @@ int cema_num_segments(int L);
 void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, const float* omega,
               const float* hx, void* y, float* h_last, float* carry, int B, int L, int D, int N,
               int x_dtype, cudaStream_t st);
+// the same on the tensor cores (cema_tensor_kernels.cu); false where it does not take the call
+bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, const float* omega, const float* hx,
+                     void* y, float* h_last, int B, int L, int D, int N, int x_dtype, cudaStream_t st);
 // dp [D,N], dq/dgamma [D,N,2], domega [D] must be zero-initialised (accumulated with atomics)
 void cema_bwd(const void* dy, const void* x, const float* p, const float* q, const float* gamma,
               const float* omega, const float* hx, const float* dh_last, void* dx, float* dp, float* dq,

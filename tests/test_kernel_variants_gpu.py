@@ -275,6 +275,67 @@ def test_epilogues(tile, M, N):
     assert err.item() == 0
 
 
+@pytest.mark.parametrize("B,L,D", [(1, 1, 8), (2, 15, 24), (1, 16, 16), (3, 17, 40), (1, 255, 264), (2, 256, 16), (1, 257, 8),
+                                   (1, 700, 32), (2, 1024, 48)])
+@pytest.mark.parametrize("carried", [False, True])
+def test_ema_on_tensor_cores(B, L, D, carried):
+    """Chunks, tiles and features that are no whole ones, against the recurrence in 64 bits: outputs rounded once, the last
+    state to 32-bit sums."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(L)
+    N, dev = 16, "cuda"
+    x = _rand(B, L, D)
+    p = torch.rand(D, N, device=dev) * 0.8 + 0.1
+    q = torch.polar(1.0 - torch.rand(D, N, device=dev).pow(3) * 0.9, torch.rand(D, N, device=dev) * 3.0)
+    gamma = torch.view_as_complex(torch.randn(D, N, 2, device=dev) * 0.25)
+    omega = torch.randn(D, device=dev)
+    hx = torch.view_as_complex(torch.randn(B, D, N, 2, device=dev)) if carried else None
+    y, last = cuda_ops._C().cema_fwd(x, p, torch.view_as_real(q), torch.view_as_real(gamma), omega,
+                                     None if hx is None else torch.view_as_real(hx), True)
+    h = torch.zeros(B, D, N, dtype=torch.complex128, device=dev) if hx is None else hx.to(torch.complex128)
+    want, size = (torch.empty(B, L, D, dtype=torch.float64, device=dev) for _ in range(2))
+    for t in range(L):
+        h = q.to(torch.complex128) * h + p.double() * x[:, t].double().unsqueeze(-1)
+        want[:, t] = (gamma.to(torch.complex128) * h).sum(-1).real + omega.double() * x[:, t].double()
+        size[:, t] = (gamma.abs().double() * h.abs()).sum(-1) + omega.abs().double() * x[:, t].abs().double()
+    assert _rel(last, torch.view_as_real(h)) < 2e-6
+    # one rounding of the result, and of 32 + 16 terms summed in fp32 what they cancel (2^-24 each, and of their powers)
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -24 * 64 * size).all()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
+def test_ema_with_infinities_stays_causal(bad):
+    """What comes before an infinity or NaN in a feature, and the other features, do not see it."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(3)
+    B, L, D, N = 2, 600, 32, 16
+    x = _rand(B, L, D)
+    p, q = torch.rand(D, N, device="cuda"), torch.rand(D, N, 2, device="cuda") * 0.6
+    gamma, omega = torch.randn(D, N, 2, device="cuda") * 0.25, torch.randn(D, device="cuda")
+    clean, _ = cuda_ops._C().cema_fwd(x, p, q, gamma, omega, None, True)
+    x2 = x.clone()
+    x2[1, 300, 5] = bad
+    y, last = cuda_ops._C().cema_fwd(x2, p, q, gamma, omega, None, True)
+    keep = torch.ones(B, L, D, dtype=torch.bool, device="cuda")
+    keep[1, 300:, 5] = False
+    assert torch.isfinite(y[keep]).all() and _rel(y[keep], clean[keep]) < 2.0 ** -9
+    assert not torch.isfinite(y[1, 300:, 5]).any() and not torch.isfinite(last[1, 5]).all()
+
+
+def test_ema_with_growing_states():
+    """Powers that overflow within a tile, where the recurrence itself does not: only the last steps have inputs."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(4)
+    B, L, D, N = 1, 500, 16, 16
+    x = torch.zeros(B, L, D, device="cuda", dtype=torch.bfloat16)
+    x[:, 480:] = _rand(B, 20, D)
+    p, q = torch.rand(D, N, device="cuda"), torch.randn(D, N, 2, device="cuda") * 2
+    gamma, omega = torch.randn(D, N, 2, device="cuda") * 0.25, torch.randn(D, device="cuda")
+    y, last = cuda_ops._C().cema_fwd(x, p, q, gamma, omega, None, True)
+    tail, tail_last = cuda_ops._C().cema_fwd(x[:, 480:].float().contiguous(), p, q, gamma, omega, None, True)
+    assert (y[:, :480] == 0).all() and _rel(y[:, 480:], tail) < 2.0 ** -8 and _rel(last, tail_last) < 1e-5
+
+
 def test_operators_without_gradients_match_the_recorded_ones():
     """The short route under no_grad against the autograd function, and what the latter refuses stays refused."""
     from megalodon_b200 import ops
