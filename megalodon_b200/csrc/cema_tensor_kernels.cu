@@ -22,8 +22,8 @@
 // A tile of a feature with infinities or NaN, and all of one whose powers overflow, takes the recurrence step by step: in
 // the products a zero of K times an infinity would reach back in time.
 //
-// us, scan / this (B x L x D): 1 x 300 x 1024 35 / 12, 8 x 777 x 1024 88 / 67, 1 x 907 x 2048 39 / 18, 2 x 2048 x 2048
-// 97 / 57, 1 x 4096 x 4096 169 / 102, 1 x 16384 x 4096 586 / 371.  What bounds it is latency: sixteen warps fill an SM's
+// us, scan / this (B x L x D): 1 x 300 x 1024 35 / 12, 8 x 777 x 1024 88 / 52, 1 x 907 x 2048 39 / 18, 2 x 2048 x 2048
+// 97 / 53, 1 x 4096 x 4096 169 / 104, 1 x 16384 x 4096 586 / 376.  What bounds it is latency: sixteen warps fill an SM's
 // registers (128 a thread), a scheduler issues in 42 % of the cycles, the tensor pipe is busy in 23 %, the wavefronts of
 // shared memory in 45 %.  Setting a warp up takes some 5 us, a tile 2.9.
 #include "common.cuh"
@@ -124,12 +124,13 @@ __device__ __forceinline__ bool odd_bf16(uint32_t w) {       // an infinity or N
 __global__ void __launch_bounds__(kFeat * 32, 1)
 cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ p, const float2* __restrict__ q,
                        const float2* __restrict__ gamma, const float* __restrict__ omega, const float2* __restrict__ hx,
-                       __nv_bfloat16* __restrict__ y, float2* __restrict__ h_last, int L, int D) {
+                       __nv_bfloat16* __restrict__ y, float2* __restrict__ h_last, int B, int L, int D, int per) {
   begin_dependent();
   extern __shared__ uint8_t raw[];
   Smem& sm = *reinterpret_cast<Smem*>(raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int f0 = blockIdx.x * kFeat, b = blockIdx.y;
+  const int f0 = blockIdx.x * kFeat, b0 = blockIdx.y * per, tiles = (L + kSteps - 1) / kSteps;
+  const int all = tiles * min(per, B - b0);               // tiles of this CTA: sequences b0, b0 + 1, ... one after another
   const bool live = f0 + warp < D;
   const int d = live ? f0 + warp : D - 1;
   const float om = omega[d];
@@ -140,11 +141,24 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
   // this thread's piece of a tile: eight features of one step
   const int oct = lane & 1, step = warp * 16 + (lane >> 1);
   const bool has = f0 + 8 * oct < D;
-  const long long base = (long long)b * L * D + f0 + 8 * oct;
-  const int tiles = (L + kSteps - 1) / kSteps;
-  auto load = [&](int k) {
-    const int s = k * kSteps + step;
-    return has && s < L ? *reinterpret_cast<const uint4*>(x + base + (long long)s * D) : make_uint4(0u, 0u, 0u, 0u);
+  struct Place {                     // of that piece, from tile to tile
+    int s;
+    long long i;
+  };
+  const long long first = ((long long)b0 * L + step) * D + f0 + 8 * oct, skip = (long long)(L - tiles * kSteps) * D;
+  Place from{step, first}, to = from;
+  auto advance = [&](Place& p) {
+    p.s += kSteps;
+    p.i += (long long)kSteps * D;
+    if (p.s >= tiles * kSteps) {
+      p.s = step;
+      p.i += skip;
+    }
+  };
+  auto load = [&]() {
+    const uint4 v = has && from.s < L ? *reinterpret_cast<const uint4*>(x + from.i) : make_uint4(0u, 0u, 0u, 0u);
+    advance(from);
+    return v;
   };
   auto put = [&](int k, const uint4& v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -153,23 +167,25 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
       reinterpret_cast<unsigned short&>(sm.x[k & 1][8 * oct + i][step]) = (unsigned short)(w[i / 2] >> (16 * (i & 1)));
   };
   auto store = [&](int k) {
-    const int s = k * kSteps + step;
-    if (!has || s >= L) return;
     uint32_t w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       w[i] = (uint32_t) reinterpret_cast<const unsigned short&>(sm.x[k & 1][8 * oct + 2 * i][step]) |
              (uint32_t) reinterpret_cast<const unsigned short&>(sm.x[k & 1][8 * oct + 2 * i + 1][step]) << 16;
-    *reinterpret_cast<uint4*>(y + base + (long long)s * D) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (has && to.s < L) *reinterpret_cast<uint4*>(y + to.i) = make_uint4(w[0], w[1], w[2], w[3]);
+    advance(to);
   };
-  uint4 next = load(0);
+  uint4 next = load();
   float H0[4][2];                 // state before the tile, states 4 j + t
+  auto start = [&](int b) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 z = hx != nullptr ? hx[((long long)b * D + d) * kStates + 4 * j + t] : make_float2(0.f, 0.f);
-    H0[j][0] = z.x;
-    H0[j][1] = z.y;
-  }
+    for (int j = 0; j < 4; ++j) {
+      const float2 z = hx != nullptr ? hx[((long long)b * D + d) * kStates + 4 * j + t] : make_float2(0.f, 0.f);
+      H0[j][0] = z.x;
+      H0[j][1] = z.y;
+    }
+  };
+  start(b0);
 
   // ---------------------------------------------------------------- fragments of E, K and F
   // Powers and what is made of them carry some 48 bits: a factor that is off is off by the same amount in every chunk,
@@ -251,13 +267,14 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
 
   // One barrier a tile: a thread takes the outputs of tile k - 1 from where it then puts the inputs of tile k + 1.
   put(0, next);
-  if (tiles > 1) next = load(1);
-  for (int k = 0; k < tiles; ++k) {
+  if (all > 1) next = load();
+  int b = b0, seq_k = 0;          // the tile's sequence, its number there
+  for (int k = 0; k < all; ++k) {
     __syncthreads();
     if (k > 0) store(k - 1);
-    if (k + 1 < tiles) put(k + 1, next);
-    if (k + 2 < tiles) next = load(k + 2);
-    const int valid = min(kSteps, L - k * kSteps);
+    if (k + 1 < all) put(k + 1, next);
+    if (k + 2 < all) next = load();
+    const int valid = min(kSteps, L - seq_k * kSteps);
     __nv_bfloat16* row = sm.x[k & 1][warp];
     uint2* plo = reinterpret_cast<uint2*>(row + 32 * g + 4 * t);            // chunk 2 g
     uint2* phi = reinterpret_cast<uint2*>(row + 32 * g + 16 + 4 * t);       // chunk 2 g + 1
@@ -309,7 +326,7 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
         H0[j][0] = er;
         H0[j][1] = ei;
       }
-      if (h_last != nullptr && k == tiles - 1) {
+      if (h_last != nullptr && seq_k == tiles - 1) {
         // the state after the last step: that before its chunk, and the chunk's steps one by one
         const int c = (valid - 1) / 16, rest = valid - 16 * c;
         if (g == c / 2) {
@@ -379,7 +396,7 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
       }
       __syncwarp();
       if (lane < 16) tb.state[n] = z;
-      if (h_last != nullptr && k == tiles - 1 && lane < 16 && live)
+      if (h_last != nullptr && seq_k == tiles - 1 && lane < 16 && live)
         h_last[((long long)b * D + d) * kStates + n] = z;
       __syncwarp();
 #pragma unroll
@@ -389,9 +406,13 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
         H0[j][1] = s.y;
       }
     }
+    if (++seq_k == tiles && k + 1 < all) {
+      seq_k = 0;
+      start(++b);
+    }
   }
   __syncthreads();
-  store(tiles - 1);
+  store(all - 1);
 }
 
 }  // namespace
@@ -399,7 +420,9 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
 // y (and h_last, if given) of the EMA; false where the scan is to run.  That is also where few features have a long
 // sequence, which only the scan divides: 16384 x 1024 167 us there, 185 here; 16384 x 512 109 and 184; 4096 x 1024 64 and
 // 51; 2048 x 512 41 and 28.  The lines in between: the scan takes 32 us and 8 for a million elements, this 5 and 2.85 a tile
-// of 256 steps for every wave of CTAs (16 features of a sequence each).
+// of 256 steps for every wave of CTAs.  A CTA has 16 features of as many sequences as make that least: it is set up once
+// for all of them, and waves are filled better (8 x 777 x 1024 67 -> 52 us, 2 x 2048 x 2048 57 -> 53, 32 x 1000 x 1024
+// 240 -> 196; of one sequence each, 1 % the slower for the bookkeeping).
 bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, const float* omega, const float* hx,
                      void* y, float* h_last, int B, int L, int D, int N, int x_dtype, cudaStream_t st) {
   if (N != kStates || x_dtype != kBF16 || D % 8 != 0 || L < 1 || B < 1 || B > 65535 || !aligned16(x) || !aligned16(y))
@@ -407,13 +430,20 @@ bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float*
   int dev = 0, sms = 1;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
-  const double waves = div_up((long long)div_up(D, kFeat) * B, sms);
-  if (waves * (5.0 + 2.85 * div_up(L, kSteps)) > 32.0 + 8e-6 * B * L * D) return false;
+  const int groups = div_up(D, kFeat), tiles = div_up(L, kSteps);
+  int per = 1;
+  double us = 1e30;
+  for (int n = 1; n <= B; ++n) {                  // n sequences a CTA
+    if (n > 1 && div_up(B, n) == div_up(B, n - 1)) continue;
+    const double t = div_up((long long)groups * div_up(B, n), sms) * (5.0 + 2.85 * tiles * n);
+    if (t < us) us = t, per = n;
+  }
+  if (us > 32.0 + 8e-6 * B * L * D) return false;
   static std::atomic<unsigned long long> configured{0};
   if (!allow_dynamic_smem(cema_fwd_tensor_kernel, sizeof(Smem), configured)) return false;
-  launch_dependent(cema_fwd_tensor_kernel, dim3(div_up(D, kFeat), B), dim3(kFeat * 32), sizeof(Smem), st,
+  launch_dependent(cema_fwd_tensor_kernel, dim3(groups, div_up(B, per)), dim3(kFeat * 32), sizeof(Smem), st,
                    (const __nv_bfloat16*)x, p, (const float2*)q, (const float2*)gamma, omega, (const float2*)hx,
-                   (__nv_bfloat16*)y, (float2*)h_last, L, D);
+                   (__nv_bfloat16*)y, (float2*)h_last, B, L, D, per);
   return true;
 }
 

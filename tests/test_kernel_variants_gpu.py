@@ -276,11 +276,11 @@ def test_epilogues(tile, M, N):
 
 
 @pytest.mark.parametrize("B,L,D", [(1, 1, 8), (2, 15, 24), (1, 16, 16), (3, 17, 40), (1, 255, 264), (2, 256, 16), (1, 257, 8),
-                                   (1, 700, 32), (2, 1024, 48)])
+                                   (1, 700, 32), (2, 1024, 48), (3, 17, 1024), (5, 300, 648)])
 @pytest.mark.parametrize("carried", [False, True])
 def test_ema_on_tensor_cores(B, L, D, carried):
-    """Chunks, tiles and features that are no whole ones, against the recurrence in 64 bits: outputs rounded once, the last
-    state to 32-bit sums."""
+    """Chunks, tiles and features that are no whole ones, several sequences to a CTA, against the recurrence in 64 bits:
+    outputs rounded once, the last state to 32-bit sums."""
     from megalodon_b200.ops import cuda_ops
     torch.manual_seed(L)
     N, dev = 16, "cuda"
