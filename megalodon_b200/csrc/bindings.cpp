@@ -143,9 +143,10 @@ std::tuple<Tensor, OptTensor, OptTensor> layer_norm_bwd(const Tensor& dy, const 
 
 // ------------------------------------------------------------------ TimestepNorm
 // returns y, count, mean, var, cummean, cumrstd
-std::vector<Tensor> timestep_norm_fwd(const Tensor& x, const Tensor& prev_count, const Tensor& prev_mean,
-                                      const Tensor& prev_var, const Tensor& gamma, double gamma_off,
-                                      const Tensor& beta, const OptTensor& mask, int64_t G, double eps) {
+// prior: the statistics before x are prev_count [], prev_mean [G] and exp(prev_var [G]) for every sequence
+std::vector<Tensor> timestep_norm_fwd_from(const Tensor& x, const Tensor& prev_count, const Tensor& prev_mean,
+                                           const Tensor& prev_var, const Tensor& gamma, double gamma_off,
+                                           const Tensor& beta, const OptTensor& mask, int64_t G, double eps, bool prior) {
   check_cuda_contig(x, "x");
   check_cuda_contig(prev_mean, "prev_mean");
   check_cuda_contig(prev_var, "prev_var");
@@ -161,9 +162,9 @@ std::vector<Tensor> timestep_norm_fwd(const Tensor& x, const Tensor& prev_count,
   if (mask.has_value()) TORCH_CHECK(mask->scalar_type() == at::kBool && mask->is_contiguous());
   auto f32 = x.options().dtype(at::kFloat);
   Tensor y = torch::empty_like(x);
-  Tensor count = torch::empty_like(prev_count);
-  Tensor mean = torch::empty_like(prev_mean);
-  Tensor var = torch::empty_like(prev_var);
+  Tensor count = prior ? torch::empty({B}, prev_count.options()) : torch::empty_like(prev_count);
+  Tensor mean = prior ? torch::empty({B, G}, x.options()) : torch::empty_like(prev_mean);
+  Tensor var = torch::empty_like(mean);
   Tensor cummean = torch::empty({B, L, G}, f32);
   Tensor cumrstd = torch::empty({B, L, G}, f32);
   Tensor gu = torch::empty({B, L, G}, f32);
@@ -175,8 +176,14 @@ std::vector<Tensor> timestep_norm_fwd(const Tensor& x, const Tensor& prev_count,
                         (long long*)count.data_ptr<int64_t>(), mean.data_ptr(), var.data_ptr(),
                         cummean.data_ptr<float>(), cumrstd.data_ptr<float>(), gu.data_ptr<float>(),
                         gv.data_ptr<float>(), seg.data_ptr<double>(), B, L, H, (int)G, (float)eps, dtype_code(x),
-                        weight_code(x, gamma), stream());
+                        weight_code(x, gamma), stream(), prior);
   return {y, count, mean, var, cummean, cumrstd};
+}
+
+std::vector<Tensor> timestep_norm_fwd(const Tensor& x, const Tensor& prev_count, const Tensor& prev_mean,
+                                      const Tensor& prev_var, const Tensor& gamma, double gamma_off,
+                                      const Tensor& beta, const OptTensor& mask, int64_t G, double eps) {
+  return timestep_norm_fwd_from(x, prev_count, prev_mean, prev_var, gamma, gamma_off, beta, mask, G, eps, false);
 }
 
 // returns dx, dprev_mean, dprev_var, dgamma, dbeta (in gamma's type)
@@ -214,13 +221,16 @@ std::vector<Tensor> timestep_norm_bwd(const Tensor& dy, const OptTensor& dmean, 
 
 // ------------------------------------------------------------------ CEMA
 // p [D,N] f32, q/gamma [D,N,2] f32, omega [D] f32, hx [B,D,N,2] f32 or none
-std::tuple<Tensor, OptTensor> cema_fwd(const Tensor& x, const Tensor& p, const Tensor& q, const Tensor& gamma,
-                                       const Tensor& omega, const OptTensor& hx, bool want_last) {
+// (cema_fwd_any, cema_bwd_any: omega in 16 bits as well)
+mb::OmegaRef omega_ref(const Tensor& omega) { return {omega.data_ptr(), dtype_code(omega)}; }
+std::tuple<Tensor, OptTensor> cema_fwd_any(const Tensor& x, const Tensor& p, const Tensor& q, const Tensor& gamma,
+                                           const Tensor& omega, const OptTensor& hx, bool want_last) {
   check_cuda_contig(x, "x");
+  check_cuda_contig(omega, "omega");
   c10::cuda::CUDAGuard guard(x.device());
   const int B = x.size(0), L = x.size(1), D = x.size(2), N = p.size(1);
   TORCH_CHECK(mb::cema_supported_ndim(N), "cema: ndim must be one of 1,2,4,8,16,32");
-  for (const Tensor* t : {&p, &q, &gamma, &omega}) {
+  for (const Tensor* t : {&p, &q, &gamma}) {
     TORCH_CHECK(t->is_cuda() && t->is_contiguous() && t->scalar_type() == at::kFloat, "cema coefficients must be contiguous fp32");
   }
   auto f32 = x.options().dtype(at::kFloat);
@@ -230,14 +240,19 @@ std::tuple<Tensor, OptTensor> cema_fwd(const Tensor& x, const Tensor& p, const T
   const int S = mb::cema_num_segments(L);
   Tensor carry = torch::empty({S > 1 ? (long long)B * S * N * D * 2 : 0}, f32);
   mb::cema_fwd(x.data_ptr(), p.data_ptr<float>(), q.data_ptr<float>(), gamma.data_ptr<float>(),
-               omega.data_ptr<float>(), hx.has_value() ? hx->data_ptr<float>() : nullptr, y.data_ptr(),
+               omega_ref(omega), hx.has_value() ? hx->data_ptr<float>() : nullptr, y.data_ptr(),
                h_last.has_value() ? h_last->data_ptr<float>() : nullptr, carry.data_ptr<float>(), B, L, D, N,
                dtype_code(x), stream());
   return {y, h_last};
 }
+std::tuple<Tensor, OptTensor> cema_fwd(const Tensor& x, const Tensor& p, const Tensor& q, const Tensor& gamma,
+                                       const Tensor& omega, const OptTensor& hx, bool want_last) {
+  TORCH_CHECK(omega.scalar_type() == at::kFloat, "cema coefficients must be contiguous fp32");
+  return cema_fwd_any(x, p, q, gamma, omega, hx, want_last);
+}
 
 // returns dx, dp, dq, dgamma, domega, dhx
-std::vector<Tensor> cema_bwd(const Tensor& dy, const Tensor& x, const Tensor& p, const Tensor& q,
+std::vector<Tensor> cema_bwd_any(const Tensor& dy, const Tensor& x, const Tensor& p, const Tensor& q,
                              const Tensor& gamma, const Tensor& omega, const OptTensor& hx,
                              const OptTensor& dh_last) {
   check_cuda_contig(dy, "dy");
@@ -259,11 +274,16 @@ std::vector<Tensor> cema_bwd(const Tensor& dy, const Tensor& x, const Tensor& p,
   Tensor carry = torch::empty({2 * cn}, f32);
   if (dh_last.has_value()) TORCH_CHECK(dh_last->is_contiguous() && dh_last->scalar_type() == at::kFloat);
   mb::cema_bwd(dy.data_ptr(), x.data_ptr(), p.data_ptr<float>(), q.data_ptr<float>(), gamma.data_ptr<float>(),
-               omega.data_ptr<float>(), hx.has_value() ? hx->data_ptr<float>() : nullptr,
+               omega_ref(omega), hx.has_value() ? hx->data_ptr<float>() : nullptr,
                dh_last.has_value() ? dh_last->data_ptr<float>() : nullptr, dx.data_ptr(), dp.data_ptr<float>(),
                dq.data_ptr<float>(), dgamma.data_ptr<float>(), domega.data_ptr<float>(), dhx.data_ptr<float>(),
                carry.data_ptr<float>(), carry.data_ptr<float>() + cn, B, L, D, N, dtype_code(x), stream());
   return {dx, dp, dq, dgamma, domega, dhx};
+}
+std::vector<Tensor> cema_bwd(const Tensor& dy, const Tensor& x, const Tensor& p, const Tensor& q, const Tensor& gamma,
+                             const Tensor& omega, const OptTensor& hx, const OptTensor& dh_last) {
+  TORCH_CHECK(omega.scalar_type() == at::kFloat, "cema coefficients must be contiguous fp32");
+  return cema_bwd_any(dy, x, p, q, gamma, omega, hx, dh_last);
 }
 
 // alpha, delta [D, N, 1], theta [D, 1, 1], gamma [D, N, 2] of one type -> p [D, N, 1], q, gamma [D, N, 2] (fp32)
@@ -357,8 +377,9 @@ Tensor rotary(const Tensor& x, const Tensor& freqs, bool conj) {
 }
 
 // z [..., S] (16-bit, S = H * Dh), gamma / beta [2, S] (fp32 or z's dtype), freqs [P, Dh/2, 2] fp32 -> (q, k) like z
-std::tuple<Tensor, Tensor> qk_rotary_fwd(const Tensor& z, const Tensor& gamma, const Tensor& beta, const Tensor& freqs,
-                                         int64_t Dh) {
+// row_max, row_sum (fp32, an element per row and head): set to -inf and 0
+std::tuple<Tensor, Tensor> qk_rotary_fwd_rows(const Tensor& z, const Tensor& gamma, const Tensor& beta, const Tensor& freqs,
+                                              int64_t Dh, const OptTensor& row_max, const OptTensor& row_sum) {
   check_cuda_contig(z, "z");
   check_cuda_contig(gamma, "gamma");
   check_cuda_contig(beta, "beta");
@@ -372,8 +393,14 @@ std::tuple<Tensor, Tensor> qk_rotary_fwd(const Tensor& z, const Tensor& gamma, c
               (gamma.scalar_type() == at::kFloat || gamma.scalar_type() == z.scalar_type()));
   Tensor q = torch::empty_like(z), k = torch::empty_like(z);
   mb::qk_rotary_fwd(z.data_ptr(), gamma.data_ptr(), beta.data_ptr(), freqs.data_ptr<float>(), q.data_ptr(), k.data_ptr(),
-                    z.numel() / S, S, (int)Dh, P, dtype_code(z), dtype_code(gamma), stream());
+                    z.numel() / S, S, (int)Dh, P, dtype_code(z), dtype_code(gamma), stream(),
+                    row_max.has_value() ? row_max->data_ptr<float>() : nullptr,
+                    row_sum.has_value() ? row_sum->data_ptr<float>() : nullptr);
   return {q, k};
+}
+std::tuple<Tensor, Tensor> qk_rotary_fwd(const Tensor& z, const Tensor& gamma, const Tensor& beta, const Tensor& freqs,
+                                         int64_t Dh) {
+  return qk_rotary_fwd_rows(z, gamma, beta, freqs, Dh, OptTensor(), OptTensor());
 }
 
 // -> (dz like z, dgamma [2, S] fp32, dbeta [2, S] fp32)

@@ -156,7 +156,7 @@ __global__ void cema_combine(cfloat* __restrict__ carry, const cfloat* __restric
 template <typename T, int NPT, int NSPLIT>
 __global__ void cema_fwd_final(const T* __restrict__ x, const float* __restrict__ p,
                                const cfloat* __restrict__ q, const cfloat* __restrict__ g,
-                               const float* __restrict__ omega, const cfloat* __restrict__ incoming,
+                               const OmegaRef omega, const cfloat* __restrict__ incoming,
                                const cfloat* __restrict__ hx, T* __restrict__ y,
                                cfloat* __restrict__ h_last, Geo geo) {
   begin_dependent();
@@ -171,7 +171,7 @@ __global__ void cema_fwd_final(const T* __restrict__ x, const float* __restrict_
     else if (hx != nullptr) h[i] = hx[((long long)b * geo.D + dd) * geo.N + n];
     else h[i] = {0.f, 0.f};
   }
-  const float om = omega[dd];
+  const float om = load_any(omega.p, omega.dtype, dd);
   const long long base = (long long)b * geo.L * geo.D + dd;
   for (int tb = t0; tb < t1; tb += kPf) {
     float xs[kPf];
@@ -237,7 +237,7 @@ __global__ void cema_bwd_rev_local(const T* __restrict__ dy, const float* __rest
 template <typename T, int NPT, int NSPLIT>
 __global__ void cema_bwd_rev_final(const T* __restrict__ dy, const T* __restrict__ x,
                                    const float* __restrict__ p, const cfloat* __restrict__ q,
-                                   const cfloat* __restrict__ g, const float* __restrict__ omega,
+                                   const cfloat* __restrict__ g, const OmegaRef omega,
                                    const cfloat* __restrict__ incoming, const cfloat* __restrict__ dh_last,
                                    T* __restrict__ dx, float* __restrict__ dp, float* __restrict__ domega,
                                    cfloat* __restrict__ dhx, Geo geo) {
@@ -255,7 +255,7 @@ __global__ void cema_bwd_rev_final(const T* __restrict__ dy, const T* __restrict
     else st[i] = {0.f, 0.f};
     acc_p[i] = 0.f;
   }
-  const float om = omega[dd];
+  const float om = load_any(omega.p, omega.dtype, dd);
   float acc_om = 0.f;
   const long long base = (long long)b * geo.L * geo.D + dd;
   for (int tb = t1 - 1; tb >= t0; tb -= kPf) {
@@ -617,7 +617,7 @@ cema_fwd_local_t(const T* __restrict__ x, const float* __restrict__ p, const cfl
 template <typename T, int NSPLIT>
 __global__ void __launch_bounds__(kTileFeat* NSPLIT)
 cema_fwd_final_t(const T* __restrict__ x, const float* __restrict__ p, const cfloat* __restrict__ q,
-                 const cfloat* __restrict__ g, const float* __restrict__ omega,
+                 const cfloat* __restrict__ g, const OmegaRef omega,
                  const cfloat* __restrict__ incoming, const cfloat* __restrict__ hx, T* __restrict__ y,
                  cfloat* __restrict__ h_last, Geo geo) {
   begin_dependent();
@@ -639,7 +639,7 @@ cema_fwd_final_t(const T* __restrict__ x, const float* __restrict__ p, const cfl
     else if (hx != nullptr) hin = hx[((long long)b * geo.D + dd) * geo.N + n];
     h[i] = {hin.re / pe[i], hin.im / pe[i]};
   }
-  const float om = omega[dd];
+  const float om = load_any(omega.p, omega.dtype, dd);
   tiled_scan<T, 1, true, false, NSPLIT>(x, nullptr, y, geo, b, t0, t1, f0, sm_in, sm_out, [&](float xv, float) {
     float acc = 0.f;
 #pragma unroll
@@ -691,7 +691,7 @@ cema_bwd_rev_local_t(const T* __restrict__ dy, const cfloat* __restrict__ q, con
 template <typename T, int NSPLIT>
 __global__ void __launch_bounds__(kTileFeat* NSPLIT)
 cema_bwd_rev_final_t(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ p,
-                     const cfloat* __restrict__ q, const cfloat* __restrict__ g, const float* __restrict__ omega,
+                     const cfloat* __restrict__ q, const cfloat* __restrict__ g, const OmegaRef omega,
                      const cfloat* __restrict__ incoming, const cfloat* __restrict__ dh_last, T* __restrict__ dx,
                      float* __restrict__ dp, float* __restrict__ domega, cfloat* __restrict__ dhx, Geo geo) {
   begin_dependent();
@@ -714,7 +714,7 @@ cema_bwd_rev_final_t(const T* __restrict__ dy, const T* __restrict__ x, const fl
     st[i] = {in.re * pe[i], in.im * pe[i]};
     acc_p[i] = 0.f;
   }
-  const float om = omega[dd];
+  const float om = load_any(omega.p, omega.dtype, dd);
   float acc_om = 0.f;
   tiled_scan<T, 2, true, true, NSPLIT>(dy, x, dx, geo, b, t0, t1, f0, sm_in, sm_out, [&](float gy, float xv) {
     float acc = 0.f;
@@ -914,7 +914,7 @@ int cema_num_segments(int L) { return (L + kCemaSegLen - 1) / kCemaSegLen; }
 // Passes over the segments are launched the ordinary way: their grid fills the chip about once, and CTAs placed while the
 // kernel before them drains crowd on the SMs that came free first (4096 x 1024, N = 8: forward 41 us, 65 to 86 so; 32-bit
 // N = 16 backward 278 and 311).  What follows the few threads of a combination does not suffer so in the tiled forward.
-void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, const float* omega,
+void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega,
               const float* hx, void* y, float* h_last, float* carry, int B, int L, int D, int N,
               int x_dtype, cudaStream_t st) {
   if (cema_fwd_tensor(x, p, q, gamma, omega, hx, y, h_last, B, L, D, N, x_dtype, st)) return;
@@ -960,7 +960,7 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
 }
 
 void cema_bwd(const void* dy, const void* x, const float* p, const float* q, const float* gamma,
-              const float* omega, const float* hx, const float* dh_last, void* dx, float* dp, float* dq,
+              OmegaRef omega, const float* hx, const float* dh_last, void* dx, float* dp, float* dq,
               float* dgamma, float* domega, float* dhx, float* carry_a, float* carry_b, int B, int L,
               int D, int N, int x_dtype, cudaStream_t st) {
   Geo geo{B, L, D, N, cema_num_segments(L), kCemaSegLen};

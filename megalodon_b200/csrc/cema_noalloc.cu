@@ -52,6 +52,6 @@ extern "C" int mb_cema_fwd_noalloc(const void* x, const float* p, const float* q
   float* scratch = nullptr;
   const int rc = scratch_for_current_device(&scratch);
   if (rc != MB_NOALLOC_OK) return rc;
-  mb::cema_fwd(x, p, q, gamma, omega, hx, y, h_last, scratch, B, L, D, N, dtype, stream);
+  mb::cema_fwd(x, p, q, gamma, mb::OmegaRef{omega, 0}, hx, y, h_last, scratch, B, L, D, N, dtype, stream);
   return cudaGetLastError() == cudaSuccess ? MB_NOALLOC_OK : MB_NOALLOC_CUDA_ERROR;
 }

@@ -123,7 +123,7 @@ __device__ __forceinline__ bool odd_bf16(uint32_t w) {       // an infinity or N
 
 __global__ void __launch_bounds__(kFeat * 32, 1)
 cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ p, const float2* __restrict__ q,
-                       const float2* __restrict__ gamma, const float* __restrict__ omega, const float2* __restrict__ hx,
+                       const float2* __restrict__ gamma, const OmegaRef omega, const float2* __restrict__ hx,
                        __nv_bfloat16* __restrict__ y, float2* __restrict__ h_last, int B, int L, int D, int per) {
   begin_dependent();
   extern __shared__ uint8_t raw[];
@@ -133,7 +133,7 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
   const int all = tiles * min(per, B - b0);               // tiles of this CTA: sequences b0, b0 + 1, ... one after another
   const bool live = f0 + warp < D;
   const int d = live ? f0 + warp : D - 1;
-  const float om = omega[d];
+  const float om = load_any(omega.p, omega.dtype, d);
   WarpTables& tb = sm.t[warp];
   const float2 *qd = tb.q, *gd = tb.gamma;
   const float* pd = tb.p;
@@ -423,7 +423,7 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
 // of 256 steps for every wave of CTAs.  A CTA has 16 features of as many sequences as make that least: it is set up once
 // for all of them, and waves are filled better (8 x 777 x 1024 67 -> 52 us, 2 x 2048 x 2048 57 -> 53, 32 x 1000 x 1024
 // 240 -> 196; of one sequence each, 1 % the slower for the bookkeeping).
-bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, const float* omega, const float* hx,
+bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega, const float* hx,
                      void* y, float* h_last, int B, int L, int D, int N, int x_dtype, cudaStream_t st) {
   if (N != kStates || x_dtype != kBF16 || D % 8 != 0 || L < 1 || B < 1 || B > 65535 || !aligned16(x) || !aligned16(y))
     return false;

@@ -187,6 +187,12 @@ __device__ __forceinline__ cfloat cadd(cfloat a, cfloat b) { return {a.re + b.re
     }                                                         \
   } while (0)
 
+// element i of a vector whose type is known at run time
+__device__ __forceinline__ float load_any(const void* p, int dtype, int i) {
+  return dtype == kF32 ? static_cast<const float*>(p)[i]
+                       : dtype == kBF16 ? to_f(static_cast<const __nv_bfloat16*>(p)[i]) : to_f(static_cast<const __half*>(p)[i]);
+}
+
 // ---- launches that begin under the end of the kernel before them
 // A kernel launched with `launch_dependent` calls `begin_dependent` before anything else: it returns when every kernel
 // ahead of it in the stream is complete and its writes are visible (at once for an ordinary launch), and lets the next

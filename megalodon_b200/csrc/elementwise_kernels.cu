@@ -120,16 +120,24 @@ __global__ void rotary_kernel(const T* __restrict__ x, const float2* __restrict_
 //   q = rot(z * (gamma_q + 1) / sqrt(Dh) + beta_q),  k = rot(z * (gamma_k + 1) / sqrt(Dh) + beta_k)
 // z, q, k [rows, S] with S = H * Dh, gamma / beta [2, S] (row 0 for q, row 1 for k), rot = the rotary
 // rotation of pairs (2j, 2j + 1) by freqs[row % P, j % (Dh / 2)].  One thread per 4 pairs (16-byte accesses).
+// row_max, row_sum (may be null): the row maxima and sums of the softmax over q k, set to where they start from; as two
+// fills of their own they cost the host 10 us a block, which bounds the smaller models.
 template <typename T, typename W>
 __global__ void qk_rotary_fwd_kernel(const T* __restrict__ z, const W* __restrict__ gamma, const W* __restrict__ beta,
                                      const float2* __restrict__ freqs, T* __restrict__ q, T* __restrict__ k,
-                                     long long rows, int S, int Dh, int P, float inv_sqrt) {
+                                     long long rows, int S, int Dh, int P, float inv_sqrt, float* __restrict__ row_max,
+                                     float* __restrict__ row_sum) {
   begin_dependent();
   const int per_row = S / 8;
+  const long long heads = rows * (S / Dh);                 // (no more than `total`: Dh >= 8)
   const long long total = rows * per_row;
   const int half = Dh / 2;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
+    if (row_max != nullptr && i < heads) {
+      row_max[i] = -INFINITY;
+      row_sum[i] = 0.f;
+    }
     const long long row = i / per_row;
     const int c0 = (int)(i - row * per_row) * 8;
     const int pos = (int)(row % P);
@@ -489,17 +497,18 @@ void rotary_apply(const void* x, const float* freqs, void* out, long long rows, 
 
 // gamma / beta are fp32 or of the activation dtype (w_dtype)
 void qk_rotary_fwd(const void* z, const void* gamma, const void* beta, const float* freqs, void* q, void* k,
-                   long long rows, int S, int Dh, int P, int dtype, int w_dtype, cudaStream_t st) {
+                   long long rows, int S, int Dh, int P, int dtype, int w_dtype, cudaStream_t st, float* row_max,
+                   float* row_sum) {
   if (rows == 0) return;
   const long long n = rows * (S / 8);
   const float inv = 1.f / sqrtf((float)Dh);
   MB_DISPATCH_16BIT(dtype, {
     if (w_dtype == kF32)
       launch_dependent(qk_rotary_fwd_kernel<scalar_t, float>, ew_grid(n), 256, 0, st, (const scalar_t*)z, (const float*)gamma,
-          (const float*)beta, (const float2*)freqs, (scalar_t*)q, (scalar_t*)k, rows, S, Dh, P, inv);
+          (const float*)beta, (const float2*)freqs, (scalar_t*)q, (scalar_t*)k, rows, S, Dh, P, inv, row_max, row_sum);
     else
       launch_dependent(qk_rotary_fwd_kernel<scalar_t, scalar_t>, ew_grid(n), 256, 0, st, (const scalar_t*)z, (const scalar_t*)gamma,
-          (const scalar_t*)beta, (const float2*)freqs, (scalar_t*)q, (scalar_t*)k, rows, S, Dh, P, inv);
+          (const scalar_t*)beta, (const float2*)freqs, (scalar_t*)q, (scalar_t*)k, rows, S, Dh, P, inv, row_max, row_sum);
   });
 }
 

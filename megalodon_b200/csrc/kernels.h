@@ -26,11 +26,12 @@ void layer_norm_bwd(const void* dy, const void* x, const void* w, float w_off, c
                     int w_dtype, cudaStream_t st, float* colsum_ws);
 
 // ---- TimestepNorm (timestep_norm_kernels.cu)
+// prior: prev_count [1], prev_mean [G] and prev_var [G], a log variance, are those of every sequence
 void timestep_norm_fwd(const void* x, const long long* prev_count, const void* prev_mean,
                        const void* prev_var, const void* gamma, float gamma_offset, const void* beta,
                        const bool* mask, void* y, long long* count_out, void* mean_out, void* var_out,
                        float* cummean, float* cumrstd, float* gu, float* gv, double* seg_scratch, int B, int L,
-                       int H, int G, float eps, int x_dtype, int w_dtype, cudaStream_t st);
+                       int H, int G, float eps, int x_dtype, int w_dtype, cudaStream_t st, bool prior = false);
 // scan segments per sequence; the forward pass needs 3 * B * nseg * G doubles of scratch, the backward
 // pass 4 * B * nseg * G doubles (+ B * L ints when a padding mask is given)
 int tsn_num_segments(int L);
@@ -42,20 +43,26 @@ void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_o
                        int* cumvalid, int B, int L, int H, int G, int x_dtype, int w_dtype, cudaStream_t st,
                        float* colsum_ws);
 
+// omega [D] of the EMA, in fp32 or as the 16-bit parameter it is
+struct OmegaRef {
+  const void* p;
+  int dtype;
+};
+
 // ---- CEMA (cema_kernels.cu); complex tensors are interleaved (re, im) fp32
 constexpr int kCemaSegLen = 128;
 bool cema_supported_ndim(int N);
 int cema_num_segments(int L);
 // carry: scratch of B * S * N * D complex (S = cema_num_segments(L)); unused when S == 1
-void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, const float* omega,
+void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega,
               const float* hx, void* y, float* h_last, float* carry, int B, int L, int D, int N,
               int x_dtype, cudaStream_t st);
 // the same on the tensor cores (cema_tensor_kernels.cu); false where it does not take the call
-bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, const float* omega, const float* hx,
+bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega, const float* hx,
                      void* y, float* h_last, int B, int L, int D, int N, int x_dtype, cudaStream_t st);
 // dp [D,N], dq/dgamma [D,N,2], domega [D] must be zero-initialised (accumulated with atomics)
 void cema_bwd(const void* dy, const void* x, const float* p, const float* q, const float* gamma,
-              const float* omega, const float* hx, const float* dh_last, void* dx, float* dp, float* dq,
+              OmegaRef omega, const float* hx, const float* dh_last, void* dx, float* dp, float* dq,
               float* dgamma, float* domega, float* dhx, float* carry_a, float* carry_b, int B, int L,
               int D, int N, int x_dtype, cudaStream_t st);
 
@@ -78,8 +85,10 @@ void rotary_apply(const void* x, const float* freqs, void* out, long long rows, 
                   bool conj, int dtype, cudaStream_t st);
 // q, k = rotary(z * (gamma + 1) / sqrt(Dh) + beta) for the two rows of gamma / beta [2, S]; z [rows, S], S = H * Dh a
 // multiple of 8 (and at most 8192), position of a row = row % P, freqs [P, Dh / 2] (cos, sin); 16-bit activations
+// row_max, row_sum (null: not asked for): [rows * heads], set to -inf and 0 for the softmax that follows
 void qk_rotary_fwd(const void* z, const void* gamma, const void* beta, const float* freqs, void* q, void* k,
-                   long long rows, int S, int Dh, int P, int dtype, int w_dtype, cudaStream_t st);
+                   long long rows, int S, int Dh, int P, int dtype, int w_dtype, cudaStream_t st, float* row_max = nullptr,
+                   float* row_sum = nullptr);
 int qk_rotary_bwd_ctas(long long rows);
 void qk_rotary_bwd(const void* dq, const void* dk, const void* z, const void* gamma, const float* freqs, void* dz,
                    float* partial, long long rows, int S, int Dh, int P, int dtype, int w_dtype, cudaStream_t st);

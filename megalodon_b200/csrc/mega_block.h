@@ -66,7 +66,7 @@ class Launcher {
 
 // Every size that the kernels take on trust.
 void check_block(const Tensor& x, const Tensor& count, const Tensor& mean, const Tensor& var, const OptTensor& hx,
-                 const Tensor& p, const Params& w, const BlockDims& d) {
+                 const Tensor& p, const Params& w, const BlockDims& d, bool prior) {
   const int64_t B = x.size(0), D = x.size(2), N = p.size(1), V = d.heads * d.dv, S = d.heads * d.dk;
   auto is = [&](int i, std::vector<int64_t> shape) {
     TORCH_CHECK(w[i].has_value() && w[i]->sizes() == at::IntArrayRef(shape) && w[i]->is_contiguous(),
@@ -82,7 +82,8 @@ void check_block(const Tensor& x, const Tensor& count, const Tensor& mean, const
   is(kFc1, {F, D}); is(kFc2, {D, F});
   if (w[kFc3].has_value()) is(kFc3, {F, D});
   of(kOmega, D); of(kRmsW, D); of(kBv, V); of(kBz, S); of(kBr, V); of(kBh1, D); of(kLnW, D); of(kLnB, D);
-  TORCH_CHECK(count.numel() == B && mean.numel() == B * d.groups && var.numel() == B * d.groups && p.numel() == D * N &&
+  const int64_t n = prior ? 1 : B;
+  TORCH_CHECK(count.numel() == n && mean.numel() == n * d.groups && var.numel() == n * d.groups && p.numel() == D * N &&
               (!hx.has_value() || hx->numel() == 2 * B * D * N), "mega_block: state of another size");
   TORCH_CHECK(x.size(1) <= d.chunk || x.size(1) % d.chunk == 0, "mega_block: not a whole number of chunks");
 }
@@ -90,39 +91,42 @@ void check_block(const Tensor& x, const Tensor& count, const Tensor& mean, const
 Tensor heads_view(const Tensor& t) { return t.permute({0, 2, 1, 3}); }
 
 // x [B, L, D] etc. -> {out, count, mean, var, k, v[, h]}, what the backward pass needs (empty without `keep`), launches.
-// count, mean, var: the running statistics before x; hx [B, D, N, 2]; p, q, gamma: EMA coefficients (fp32, real pairs)
+// count, mean, var: the running statistics before x, or with `prior` one count, mean and log variance; hx [B, D, N, 2]; p, q, gamma: EMA coefficients (fp32, real pairs)
 std::tuple<std::vector<Tensor>, Params, int64_t> mega_block_fwd(
     const Tensor& x, const Tensor& count, const Tensor& mean, const Tensor& var, const OptTensor& hx, const Tensor& p,
     const Tensor& q, const Tensor& gamma, const Tensor& freqs, const Params& w, const std::vector<int64_t>& dims,
-    const std::vector<double>& eps, bool want_last, bool keep, const Tensor& err) {
-  TORCH_CHECK(w.size() == kBlockParams && x.dim() == 3 && x.numel() > 0, "mega_block: arguments");
+    const std::vector<double>& eps, bool want_last, bool keep, bool prior, const Tensor& err) {
+  TORCH_CHECK(w.size() == kBlockParams && x.dim() == 3 && x.numel() > 0 && !(keep && prior), "mega_block: arguments");
   c10::cuda::CUDAGuard guard(x.device());
   const BlockDims d = block_dims(dims, eps);
-  check_block(x, count, mean, var, hx, p, w, d);
+  check_block(x, count, mean, var, hx, p, w, d, prior);
   Launcher run(err);
   const auto T = x.scalar_type();
   const auto f32 = x.options().dtype(at::kFloat);
   const Tensor xc = x.contiguous();
   const int64_t B = xc.size(0), L = xc.size(1), D = xc.size(2), rows = B * L;
   const Tensor pm = mean.to(T).contiguous(), pv = var.to(T).contiguous();
-  const std::vector<Tensor> tsn = timestep_norm_fwd(xc, count.contiguous(), pm, pv, *w[kTsnW], 1.0, *w[kTsnB], OptTensor(),
-                                                    d.groups, d.tsn_eps);
+  const std::vector<Tensor> tsn = timestep_norm_fwd_from(xc, count.contiguous(), pm, pv, *w[kTsnW], 1.0, *w[kTsnB],
+                                                         OptTensor(), d.groups, d.tsn_eps, prior);
   const Tensor& t = tsn[0];
-  const Tensor omega = w[kOmega]->reshape({D}).to(at::kFloat);
-  const auto [ema, h] = cema_fwd(t, p, q, gamma, omega, hx, want_last);
+  const Tensor omega = w[kOmega]->view({D});
+  const auto [ema, h] = cema_fwd_any(t, p, q, gamma, omega, hx, want_last);
   const auto [mx, mx_rstd] = rms_norm_fwd(ema, w[kRmsW], 1.0, d.rms_eps);
   run.count += 7;
   const Tensor x2 = xc.view({rows, D}), t2 = t.view({rows, D}), m2 = mx.view({rows, D});
 
   // the projections of mx; the gate leaves as fp32 pre-activation, for few rows without gradients as its 16-bit SiLU
   const int64_t S = d.heads * d.dk, V = d.heads * d.dv;
-  Tensor z = torch::empty({rows, S}, x.options()), r, hres = torch::empty({rows, D}, x.options());
+  Tensor z = torch::empty({rows, S}, x.options()), r, hres = torch::empty({rows, D}, x.options()), v;
+  OptTensor v_pre;
   bool few = rows <= mb::kSkinnyMaxRows && !keep;
   if (few) {
     r = torch::empty({rows, V}, x.options());
-    const int64_t rc = skinny_gemm({m2, m2, m2}, {*w[kWz], *w[kWr], *w[kWh1]}, {OptTensor(), OptTensor(), OptTensor()},
-                                   {w[kBz], w[kBr], w[kBh1]}, {OptTensor(), OptTensor(), x2}, {0, 1, 0}, {z, r, hres}, false,
-                                   err, {}, 0.0);
+    v = torch::empty({rows, V}, x.options());
+    const OptTensor none;
+    const int64_t rc = skinny_gemm({m2, m2, m2, t2}, {*w[kWz], *w[kWr], *w[kWh1], *w[kWv]}, {none, none, none, none},
+                                   {w[kBz], w[kBr], w[kBh1], w[kBv]}, {none, none, x2, none}, {0, 1, 0, 1}, {z, r, hres, v},
+                                   false, err, {}, 0.0);
     TORCH_CHECK(rc == 0 || rc == -1, "few-row products: launch failed with code ", rc);
     few = rc == 0;
     run.count += few;
@@ -139,19 +143,20 @@ std::tuple<std::vector<Tensor>, Params, int64_t> mega_block_fwd(
   }
   const auto [zn, z_rstd] = rms_norm_fwd(z.view({rows * d.heads, d.dk}), OptTensor(), 1.0, d.z_eps);
   const Tensor zn3 = zn.view({B, L, S});
-  const auto [qr, kr] = qk_rotary_fwd(zn3, *w[kGamma], *w[kBeta], freqs, d.dk);
-  GemmArgs gv;
-  gv.bias = w[kBv]; gv.act = 1; gv.want_pre = keep;
-  const auto [v, v_pre] = run.linear(t2, *w[kWv], gv);
+  const int64_t c = std::min(L, d.chunk), n = rows / c, ld = (c + 127) / 128 * 128;
+  const Tensor rmax = torch::empty({n, d.heads, c}, f32), rsum = torch::empty({n, d.heads, c}, f32);
+  const auto [qr, kr] = qk_rotary_fwd_rows(zn3, *w[kGamma], *w[kBeta], freqs, d.dk, rmax, rsum);
+  if (!few) {
+    GemmArgs gv;
+    gv.bias = w[kBv]; gv.act = 1; gv.want_pre = keep;
+    std::tie(v, v_pre) = run.linear(t2, *w[kWv], gv);
+  }
 
   // chunk-local causal attention: scores twice (row maxima, then exponentials and row sums), P V over the row sums
-  const int64_t c = std::min(L, d.chunk), n = rows / c, ld = (c + 127) / 128 * 128;
   const Tensor qh = heads_view(qr.view({n, c, d.heads, d.dk})), kh = heads_view(kr.view({n, c, d.heads, d.dk}));
   const Tensor vh = heads_view(v.view({n, c, d.heads, d.dv}));
   const Tensor P = torch::empty({n, d.heads, c, ld}, x.options()), attn = torch::empty({n, c, d.heads, d.dv}, x.options());
   const Tensor Pv = P.narrow(-1, 0, c);
-  const Tensor rmax = torch::full({n, d.heads, c}, -std::numeric_limits<float>::infinity(), f32);
-  const Tensor rsum = torch::zeros({n, d.heads, c}, f32);
   GemmArgs gs;
   gs.out = Pv; gs.mode = 1; gs.epi = 1; gs.row_out = rmax;
   run.gemm(qh, kh, gs);
@@ -310,7 +315,7 @@ std::tuple<Params, int64_t> mega_block_bwd(const Tensor& dout, const OptTensor& 
   // norms and EMA
   const auto [dema, drms] = rms_norm_bwd(dmx.view({B, L, D}), ema, w[kRmsW], 1.0, mx_rstd);
   dw[kRmsW] = drms;
-  const std::vector<Tensor> ce = cema_bwd(dema, t, p, q, gamma, omega, hx, dh);
+  const std::vector<Tensor> ce = cema_bwd_any(dema, t, p, q, gamma, omega, hx, dh);
   dw[kOmega] = ce[4].view(w[kOmega]->sizes()).to(w[kOmega]->scalar_type());
   const Tensor dt = ce[0];
   input_grad(gv, kWv, dt.view({rows, D}));

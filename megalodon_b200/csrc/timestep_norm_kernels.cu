@@ -58,6 +58,22 @@ __global__ void tsn_group_stats_kernel(const T* __restrict__ x, float* __restric
   }
 }
 
+// The statistics before a sequence: of each sequence, or (prior) one prior mean and log variance per group and one count
+// for all, which saves the five small launches that would spread them over the batch first.  The variance is rounded as
+// stored statistics are.
+template <typename T>
+struct Before {
+  const long long* count;
+  const T *mean, *var;
+  bool prior;
+  __device__ __forceinline__ double n(int b) const { return (double)count[prior ? 0 : b]; }
+  __device__ __forceinline__ double u(int b, int g, int G) const { return to_f(mean[prior ? g : b * G + g]); }
+  __device__ __forceinline__ double v(int b, int g, int G) const {
+    const float x = to_f(var[prior ? g : b * G + g]);
+    return prior ? to_f(from_f<T>(expf(x))) : x;
+  }
+};
+
 // ---- forward scan in three small kernels over segments of kSegLen steps:
 //   seg_sums   : (b, seg, g)  sums of (1, gu, gv + gu^2) over the segment's valid steps
 //   seg_prefix : (b, g)       exclusive prefix over segments, seeded with the carried statistics
@@ -93,17 +109,14 @@ __global__ void tsn_seg_sums_kernel(const float* __restrict__ gu, const float* _
 }
 
 template <typename T>
-__global__ void tsn_seg_prefix_kernel(double* __restrict__ seg, const long long* __restrict__ prev_count,
-                                      const T* __restrict__ prev_mean, const T* __restrict__ prev_var,
-                                      long long* __restrict__ count_out, T* __restrict__ mean_out,
+__global__ void tsn_seg_prefix_kernel(double* __restrict__ seg, const Before<T> before, long long* __restrict__ count_out, T* __restrict__ mean_out,
                                       T* __restrict__ var_out, int B, int G, int nseg) {
   begin_dependent();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * G) return;
   const int g = i % G, b = i / G;
   const long long total = (long long)B * nseg * G;
-  const double n0 = (double)prev_count[b];
-  const double u0 = to_f(prev_mean[i]), v0 = to_f(prev_var[i]);
+  const double n0 = before.n(b), u0 = before.u(b, g, G), v0 = before.v(b, g, G);
   double cn = n0, s1 = n0 * u0, s2 = n0 * (v0 + u0 * u0);
 #pragma unroll 4
   for (int k = 0; k < nseg; ++k) {
@@ -129,8 +142,7 @@ __global__ void tsn_seg_prefix_kernel(double* __restrict__ seg, const long long*
 template <typename T>
 __global__ void tsn_seg_apply_kernel(const float* __restrict__ gu, const float* __restrict__ gv,
                                      const bool* __restrict__ mask, const double* __restrict__ seg,
-                                     const T* __restrict__ prev_mean, const T* __restrict__ prev_var,
-                                     float* __restrict__ cummean, float* __restrict__ cumrstd, int B, int L,
+                                     const Before<T> before, float* __restrict__ cummean, float* __restrict__ cumrstd, int B, int L,
                                      int G, int nseg, float eps) {
   begin_dependent();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -143,7 +155,7 @@ __global__ void tsn_seg_apply_kernel(const float* __restrict__ gu, const float* 
   const long long off = (long long)b * L * G + g;
   const bool* mb_ = mask ? mask + (long long)b * L : nullptr;
   double cn = seg[i], s1 = seg[total + i], s2 = seg[2 * total + i];
-  double mean = to_f(prev_mean[b * G + g]), var = to_f(prev_var[b * G + g]);
+  double mean = before.u(b, g, G), var = before.v(b, g, G);
   if (cn > 0.5) {
     mean = s1 / cn;
     var = fmax(s2 / cn - mean * mean, 0.0);
@@ -190,8 +202,7 @@ constexpr int kScanMaxThreads = 512;   // 128 registers per thread: the segment'
 template <typename T, int SEG>
 __global__ void __launch_bounds__(kScanMaxThreads)
 tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv, const bool* __restrict__ mask,
-                      const long long* __restrict__ prev_count, const T* __restrict__ prev_mean,
-                      const T* __restrict__ prev_var, long long* __restrict__ count_out, T* __restrict__ mean_out,
+                      const Before<T> before, long long* __restrict__ count_out, T* __restrict__ mean_out,
                       T* __restrict__ var_out, float* __restrict__ cummean, float* __restrict__ cumrstd, int L, int G,
                       int nseg, int GT, float eps) {
   begin_dependent();
@@ -242,8 +253,7 @@ tsn_scan_fused_kernel(const float* __restrict__ gu, const float* __restrict__ gv
     __syncthreads();
   }
   if (!live) return;
-  const double n0 = (double)prev_count[b];
-  const double u0 = to_f(prev_mean[b * G + g]), v0 = to_f(prev_var[b * G + g]);
+  const double n0 = before.n(b), u0 = before.u(b, g, G), v0 = before.v(b, g, G);
   double cn = n0, s1 = n0 * u0, s2 = n0 * (v0 + u0 * u0);
   if (sgi == nseg - 1) {   // the sequence's final statistics
     const double fn = cn + sh[0][tid], f1 = s1 + sh[1][tid], f2 = s2 + sh[2][tid];
@@ -885,10 +895,11 @@ void timestep_norm_fwd(const void* x, const long long* prev_count, const void* p
                        const void* prev_var, const void* gamma, float gamma_offset, const void* beta,
                        const bool* mask, void* y, long long* count_out, void* mean_out, void* var_out,
                        float* cummean, float* cumrstd, float* gu, float* gv, double* seg_scratch, int B, int L,
-                       int H, int G, float eps, int x_dtype, int w_dtype, cudaStream_t st) {
+                       int H, int G, float eps, int x_dtype, int w_dtype, cudaStream_t st, bool prior) {
   const long long rows = (long long)B * L;
   const int lpg = pick_lpg(H / G);
   TSN_DISPATCH(x_dtype, w_dtype, {
+    const Before<T> before{prev_count, (const T*)prev_mean, (const T*)prev_var, prior};
     const bool vec = tsn_vec_ok(H, G, {x, y, gamma, beta});
     if (vec) {
       VL_SWITCH(H / G / 8, {
@@ -905,17 +916,16 @@ void timestep_norm_fwd(const void* x, const long long* prev_count, const void* p
     if (seg > 0 && B <= 65535) {
       const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
       SEG_SWITCH(seg, (launch_dependent(tsn_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
-          gu, gv, mask, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
+          gu, gv, mask, before, count_out, (T*)mean_out, (T*)var_out,
           cummean, cumrstd, L, G, nseg, gt, eps)));
     } else {
     const int nseg = tsn_num_segments(L);
     const long long nsg = (long long)B * nseg * G;
     launch_dependent(tsn_seg_sums_kernel, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, B, L, G, nseg);
     launch_dependent(tsn_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
-        seg_scratch, prev_count, (const T*)prev_mean, (const T*)prev_var, count_out, (T*)mean_out, (T*)var_out,
+        seg_scratch, before, count_out, (T*)mean_out, (T*)var_out,
         B, G, nseg);
-    launch_dependent(tsn_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, (const T*)prev_mean,
-                                                            (const T*)prev_var, cummean, cumrstd, B, L, G, nseg,
+    launch_dependent(tsn_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, before, cummean, cumrstd, B, L, G, nseg,
                                                             eps);
     }
     if (vec) {

@@ -108,12 +108,12 @@ class _MegaBlock(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, meta, x, count, mean, var, hx, p, q, gamma, *params):
-        dims, eps, freqs, want_last, keep = meta
+        dims, eps, freqs, want_last, keep, prior = meta
         D = x.shape[-1]
         p2, q2, g2 = p.reshape(D, -1).float().contiguous(), cuda_ops._c2r(q.reshape(D, -1)), cuda_ops._c2r(gamma.reshape(D, -1))
         h2 = None if hx is None else cuda_ops._c2r(hx)
         outs, saved, launches = require().mega_block_fwd(x, count, mean, var, h2, p2, q2, g2, freqs, list(params), dims, eps,
-                                                         want_last, keep, cuda_ops._err_flag(x.device))
+                                                         want_last, keep, prior, cuda_ops._err_flag(x.device))
         cuda_ops._bump(launches)
         out, count, mean_out, var_out, k, v = outs[:6]
         h = torch.view_as_complex(outs[6]) if want_last else None
@@ -169,14 +169,19 @@ def forward(block, x: Tensor, freqs_cis: Tensor, mask=None, cache=None, carry=No
         _, (count, mean, var), hx = cache
     elif carry is not None:
         count, mean, var, hx = carry
-    if count is None or mean is None or var is None:
+    grad = torch.is_grad_enabled()
+    # without gradients the kernel spreads the prior over the batch itself
+    prior = (not grad and count is None and mean is None and var is None and "initial_stats" not in norm.__dict__
+             and norm.prior_mean.dtype == norm.prior_logv.dtype == x.dtype)
+    if prior:
+        count, mean, var = norm.prior_count, norm.prior_mean, norm.prior_logv
+    elif count is None or mean is None or var is None:
         c0, m0, v0 = norm.initial_stats(bsz, x.dtype)
         count, mean, var = (c0 if count is None else count, m0 if mean is None else mean, v0 if var is None else var)
     want_last = cache is not None or (streaming and not last_piece) or emit
-    grad = torch.is_grad_enabled()
     freqs = torch.view_as_real(freqs_cis.to(torch.complex64).contiguous())
     meta = ([norm.groups_per_partition, a.num_heads, a.z_head_dim, a.v_head_dim, a.chunk_size],
-            [norm.eps, am["rmsnorm"].eps, am["znorm"].eps, fm["norm"].eps], freqs, want_last, grad)
+            [norm.eps, am["rmsnorm"].eps, am["znorm"].eps, fm["norm"].eps], freqs, want_last, grad, prior)
     args = (meta, x, count, mean, var, hx, *am["cema"].coeffs(), *params)
     if grad:
         out, count, mean, var, h = _MegaBlock.apply(*args)

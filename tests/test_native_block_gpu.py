@@ -78,6 +78,26 @@ def test_without_gradients(monkeypatch, B, L, dtype, swiglu, fused, affine):
                 assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("B,L", [(3, 2), (2, 512), (2, 16640)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_prior_statistics(monkeypatch, B, L, dtype):
+    """The prior that the kernel spreads over the batch, in both forms of the scan (one launch up to 16384 steps), against
+    the expanded one: the same bits, and another prior gives others."""
+    block = _block(dtype).eval()
+    calls = _calls(monkeypatch)
+    x, freqs = torch.randn(B, L, 256, device="cuda").to(dtype), _freqs(block, L)
+    with torch.no_grad():
+        block.mega.timenorm.prior_count.fill_(3)
+        block.mega.timenorm.prior_logv.uniform_(-2.0, 2.0)
+        got = _flat(block(x, freqs, piece=(0, 2, 2 * L)))
+        assert calls
+        want = _flat(_through_modules(monkeypatch, lambda: block(x, freqs, piece=(0, 2, 2 * L))))
+        for a, b in zip(got, want):
+            assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+        block.mega.timenorm.prior_logv.add_(1.0)
+        assert not torch.equal(_flat(block(x, freqs, piece=(0, 2, 2 * L)))[0], got[0])
+
+
 @pytest.mark.parametrize("B,L,swiglu,fused,affine,dtype", [(2, 40, True, "fused", True, torch.bfloat16),
                                                            (1, 37, False, None, True, torch.bfloat16),
                                                            (2, 256, True, None, False, torch.float16),
