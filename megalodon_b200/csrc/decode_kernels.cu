@@ -1,12 +1,14 @@
 // One token through a MEGA block with a fixed-shape state: everything between the matrix products.
 //
-//   decode_norm_ema   TimestepNorm step -> complex-EMA step -> RMSNorm, state updated in place
+//   decode_norm_ema   TimestepNorm step -> complex-EMA step -> RMSNorm, state updated in place (the RMSNorm's factor left
+//                     to the products that follow, where groups of features can do without each other)
 //   decode_attend     per-head RMSNorm of z, query / key affine and rotary, key / value appended to the
 //                     buffers, attention of one query over the filled slots split over the keys
-//   decode_combine    the partial results of the splits put together, times the gate
+//   decode_combine    the partial results of the splits put together, times the gate; attention in one
+//                     launch (`attend_plan`) does without it
 //   decode_layer_norm LayerNorm of the feed-forward branch
 //
-// A step is bound by its chain of launches, not by bytes: per layer these four and four products
+// A step is bound by its chain of launches, not by bytes: per layer these three or four and four products
 // (skinny_gemm.cu) replace some thirty-five launches.  All of them are written as links of a programmatic
 // dependent launch chain: `pdl_wait` before the first access to anything another kernel writes.
 #include "common.cuh"

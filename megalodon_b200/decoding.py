@@ -296,7 +296,7 @@ class DecodeSession:
         C.decode_norm_ema(x, norm.weight, norm.bias, count, mean, var, b["t"], None, None, None, None, None, None, None,
                           self.pos, m.chunk_size, norm.eps, 0.0, True)
         products([b["t"]], [m.output.output.weight], [None], [None], [0], [b["logits"]])
-        cuda_ops._bump(8 * n + 2)        # (the EMA coefficients count themselves)
+        cuda_ops._bump(8 * n + 2)        # (attention as two launches, its most; the EMA coefficients count themselves)
         return b["logits"]
 
     # ------------------------------------------------------------------ one token
