@@ -299,7 +299,8 @@ decode_norm_ema_wide_kernel(const __grid_constant__ DecodeNormEma p, int groups)
     }
   }
   sq = block_sum(sq, scratch);
-  if (tid < groups) p.sumsq[(long long)b * p.G + g0 + tid] = tid == 0 ? sq : 0.f;
+  // (a group of one or two features that has no small divisor to be bundled by: more groups than threads)
+  for (int g = tid; g < groups; g += kDecThreads) p.sumsq[(long long)b * p.G + g0 + g] = g == 0 ? sq : 0.f;
   if (tid == 0 && (seen >> 32) == gridDim.x - 1)
     atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull - ((unsigned long long)gridDim.x << 32));
 }

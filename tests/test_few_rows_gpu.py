@@ -185,6 +185,39 @@ def test_decode_norm_ema_in_parts(D, G, N, B):
     assert err.item() == 0
 
 
+@pytest.mark.parametrize("D,G,N,B", [(2056, 257, 16, 2), (4112, 514, 4, 3)])
+def test_decode_norm_ema_in_parts_with_more_groups_than_threads(D, G, N, B):
+    """Groups that only a prime over 256 of them bundles into 32 features: every part of the sum of squares is written.
+    Against the step in 64 bits."""
+    _norm_ema_in_parts(D, G, N, B, 3)
+
+
+def _norm_ema_in_parts(D, G, N, B, steps_before):
+    """The link and a product behind it, once, against the step in 64 bits from a count of `steps_before` on."""
+    from megalodon_b200.ops import cuda_ops, reference
+    C = cuda_ops._C()
+    torch.manual_seed(D)
+
+    def rand(*s):
+        return torch.randn(*s, device="cuda")
+    w, b, rw, omega = (rand(D).mul_(0.1).bfloat16() for _ in range(4))
+    p, q, ga, hx = torch.rand(D, N, device="cuda"), rand(D, N, 2) * 0.4, rand(D, N, 2), rand(B, D, N, 2)
+    count, mean, var = torch.full((B,), steps_before, device="cuda"), rand(B, G) * 0.1, torch.rand(B, G, device="cuda") + 0.5
+    x, weight = rand(B, D).bfloat16(), (rand(96, D) * D ** -0.5).bfloat16()
+    ty, _, m1, v1 = reference.timestep_norm(x.double()[:, None], count, mean.double(), var.double(), w.double(), b.double(),
+                                            None, G, 1e-5, 1.0)
+    t64 = ty[:, 0].bfloat16().double()
+    ga64, q64, h64 = (torch.view_as_complex(z.double()) for z in (ga, q, hx))
+    y = (ga64 * (q64 * h64 + p.double() * t64[:, :, None])).sum(-1).real + omega.double() * t64
+    want = (y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * (rw.double() + 1.0)) @ weight.double().t()
+    t, mx, sq = torch.empty_like(x), torch.empty_like(x), torch.full((B, G), float("nan"), device="cuda")
+    C.decode_norm_ema(x, w, b, count, mean, var, t, p, q, ga, omega, hx, rw, mx, None, 0, 1e-5, 1e-5, sq, False)
+    out, err = torch.empty(B, 96, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert C.skinny_gemm([mx], [weight], [None], [None], [None], [0], [out], False, err, [sq], 1e-5) == 0 and err.item() == 0
+    assert (count == steps_before + 1).all() and _rel(mean, m1) < 1e-6 and _rel(var, v1) < 1e-6
+    assert _rel(out, want) < 2.0 ** -7               # roundings of t, of y and of y (1 + w) to 8 bits
+
+
 @pytest.mark.parametrize("swiglu,B,D,H,share", [(True, 1, 256, 2, False), (False, 5, 512, 1, True)])
 def test_native_session_matches_cache_path(swiglu, B, D, H, share):
     """The native chain, eager and replayed, against the growing cache; one step across the chunk boundary."""
