@@ -181,7 +181,9 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
 // of the eight of a cluster.  Everything but x, the parameters of the norms included, is loaded ahead of the wait.
 // us from this link's wait to the next one's, cluster form and this one (16 states, one row): 1024 features 7.5 / 3.3,
 // 4096 features 15.8 / 4.4; 2048 features, 16 rows: 11.2 / 10.5, with the five CTAs an SM below 7.
-// The number of rows' steps counts the CTAs that have read it in its upper half; the last one takes them off and adds one.
+// A row's count of steps also counts the CTAs that have read it, from bit kArrivalBit on (there are 512 at the most: 16384
+// features, 32 of them to a CTA); the last one takes them off and adds the step.
+constexpr int kArrivalBit = 52;
 template <typename T, int PER, int BATCH>      // PER: threads of a feature, two states each; BATCH: items of a thread whose
 __global__ void __launch_bounds__(kDecThreads, BATCH == 1 ? 5 : 3)      // loads are in flight together
 decode_norm_ema_wide_kernel(const __grid_constant__ DecodeNormEma p, int groups) {
@@ -229,8 +231,8 @@ decode_norm_ema_wide_kernel(const __grid_constant__ DecodeNormEma p, int groups)
   }
   unsigned long long seen = 0;
   if (tid == 0) {
-    seen = atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull << 32);
-    const double n0 = (double)(unsigned int)seen;
+    seen = atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull << kArrivalBit);
+    const double n0 = (double)(seen & ((1ull << kArrivalBit) - 1));
     weight_old = n0 / (n0 + 1.0);
     weight_new = 1.0 / (n0 + 1.0);
   }
@@ -301,8 +303,8 @@ decode_norm_ema_wide_kernel(const __grid_constant__ DecodeNormEma p, int groups)
   sq = block_sum(sq, scratch);
   // (a group of one or two features that has no small divisor to be bundled by: more groups than threads)
   for (int g = tid; g < groups; g += kDecThreads) p.sumsq[(long long)b * p.G + g0 + g] = g == 0 ? sq : 0.f;
-  if (tid == 0 && (seen >> 32) == gridDim.x - 1)
-    atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull - ((unsigned long long)gridDim.x << 32));
+  if (tid == 0 && (seen >> kArrivalBit) == gridDim.x - 1)
+    atomicAdd(reinterpret_cast<unsigned long long*>(p.count + b), 1ull - ((unsigned long long)gridDim.x << kArrivalBit));
 }
 
 // ---------------------------------------------------------------- attention of one query

@@ -192,6 +192,13 @@ def test_decode_norm_ema_in_parts_with_more_groups_than_threads(D, G, N, B):
     _norm_ema_in_parts(D, G, N, B, 3)
 
 
+@pytest.mark.parametrize("D,G,N,B,steps", [(512, 32, 16, 2, 2 ** 32 - 1), (1024, 8, 2, 3, 2 ** 40 + 5), (16384, 512, 2, 1, 2 ** 32 + 1)])
+def test_decode_norm_ema_in_parts_after_many_steps(D, G, N, B, steps):
+    """Counts beyond 32 bits, with as many CTAs to a row as there can be."""
+    _norm_ema_in_parts(D, G, N, B, steps)
+    _norm_ema_in_parts(D, G, N, B, steps + 1)
+
+
 def _norm_ema_in_parts(D, G, N, B, steps_before):
     """The link and a product behind it, once, against the step in 64 bits from a count of `steps_before` on."""
     from megalodon_b200.ops import cuda_ops, reference
