@@ -179,8 +179,10 @@ decode_norm_ema_kernel(const __grid_constant__ DecodeNormEma p, int cl) {
 // The same step for a reader that applies the RMSNorm's factor itself: no CTA then needs the whole row, so a CTA owns
 // one group (or enough of them for 32 features), nothing is exchanged, and a row's state comes through all SMs instead
 // of the eight of a cluster.  Everything but x, the parameters of the norms included, is loaded ahead of the wait.
-// us from this link's wait to the next one's, cluster form and this one (16 states, one row): 1024 features 7.5 / 3.3,
-// 4096 features 15.8 / 4.4; 2048 features, 16 rows: 11.2 / 10.5, with the five CTAs an SM below 7.
+// The link alone, 16 states, cluster form / this one, us: 8 rows of 1024 features 6.9 / 4.7, 32 rows 7.8 / 8.1, 64 rows
+// 14.7 / 11.7; 16 rows of 2048 10.7 / 7.8, 64 rows 21.6 / 19.2; 8 rows of 4096 11.6 / 5.7, 32 rows 18.6 / 15.3.  With one or
+// two groups a row has as many CTAs as the cluster form and takes as long (8192 features in one group 119.7 / 119.3), from
+// nine rows on less (102 / 65 us for 16 rows of 4096), where a cluster's CTAs have 256 threads too.
 // A row's count of steps also counts the CTAs that have read it, from bit kArrivalBit on (there are 512 at the most: 16384
 // features, 32 of them to a CTA); the last one takes them off and adds the step.
 constexpr int kArrivalBit = 52;
@@ -1003,8 +1005,11 @@ bool decode_norm_ema_ok(int D, int G, int N) {
 
 static int decode_norm_ema_wide(const DecodeNormEma& p, int B, int dtype, bool pdl, cudaStream_t st) {
   const int gs = p.D / p.G;
-  int groups = 1;                                   // the fewest, dividing G evenly, with 32 features
-  while (groups < p.G && (groups * gs < 32 || p.G % groups != 0)) ++groups;
+  // Features of a CTA: 32, or 64 where that would be more CTAs than the five to an SM that run at once (us, 32 / 64:
+  // 24 x 1024 8.1 / 7.6, 32 x 1024 8.5 / 8.1, 64 x 1024 12.8 / 11.7, 16 x 2048 8.7 / 7.8, 64 x 2048 23.4 / 19.2).
+  const int least = (long long)B * p.D > 32 * 5 * 148 ? 64 : 32;
+  int groups = 1;                                   // the fewest, dividing G evenly, with that many
+  while (groups < p.G && (groups * gs < least || p.G % groups != 0)) ++groups;
   const size_t smem = sizeof(float) * (2 * groups * gs + 2 * groups);
   cudaError_t e = cudaSuccess;
   MB_DISPATCH_16BIT(dtype, {
