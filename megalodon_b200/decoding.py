@@ -229,7 +229,10 @@ class DecodeSession:
         splits = require().decode_attend_splits(B * a.num_heads, m.chunk_size)
         self._buf = {n: torch.empty(B, k, dtype=self.dtype, device=dev) for n, k in
                      dict(t=D, mx=D, z=S, r=V, v=V, h=D, attn=V, y=D, f=D, u=F, x0=D, x1=D).items()}
-        self._buf["sq"] = torch.empty(B, a.timenorm.groups_per_partition, dtype=torch.float32, device=dev)
+        # bf16: the EMA output leaves the norm + EMA link before its RMSNorm's factor, which the products apply.  In fp16 it
+        # may be an infinity or lose bits below 6e-5 without the factor, so there the link applies it.
+        self._buf["sq"] = (torch.empty(B, a.timenorm.groups_per_partition, dtype=torch.float32, device=dev)
+                           if self.dtype == torch.bfloat16 else None)
         self._buf["logits"] = torch.empty(B, m.output_size, dtype=torch.float32, device=dev)
         self._buf["part"] = torch.empty(B * a.num_heads * splits * (a.local_v_head_dim + 2), device=dev)
 
@@ -278,7 +281,6 @@ class DecodeSession:
             C.decode_norm_ema(x, a.timenorm.weight, a.timenorm.bias, count, mean, var, b["t"], *coeffs[n],
                               torch.view_as_real(st["hx"]), a.rmsnorm.weight, b["mx"], None, 0, a.timenorm.eps,
                               a.rmsnorm.eps, b["sq"], n > 0)
-            # (b["mx"] is still without the factor of its RMSNorm)
             products([b["mx"], b["mx"], b["t"], b["mx"]], [a.wh1.weight, a.wr.weight, a.wv.weight, a.wz.weight],
                      [a.wh1.bias, a.wr.bias, a.wv.bias, a.wz.bias], [x, None, None, None], [0, 1, 1, 0],
                      [b["h"], b["r"], b["v"], b["z"]], None, [b["sq"], b["sq"], None, b["sq"]], a.rmsnorm.eps)

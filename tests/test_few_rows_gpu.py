@@ -289,6 +289,33 @@ def test_native_session_without_cached_coefficients(dtype, training, use_graph):
     cuda_ops.check_kernel_errors()
 
 
+def test_native_session_in_fp16_with_large_ema_outputs():
+    """EMA outputs that are over 65504 when multiplied by 1 + w but not normalised, against the modules."""
+    from megalodon_b200.config import ModelConf
+    from megalodon_b200.decoding import DecodeSession
+    from megalodon_b200.models.mega import build_model
+    from megalodon_b200.utils import init_cache, set_random_seed
+    cfg = ModelConf(num_layers=1, model_dim=256, num_heads=1, z_dim=64, value_dim=256, ffn_hidden_dim=256, chunk_size=64,
+                    vocab_size=264, swiglu=True, norm_num_groups=8, efficient_attn="fused")
+    set_random_seed(5)
+    model = build_model(cfg, "fp16", False, False).eval()
+    block = model._wrapped.layers[0]
+    while hasattr(block, "_wrapped"):
+        block = block._wrapped
+    tok = torch.randint(0, 264, (2, 6), device="cuda")
+    with torch.no_grad():
+        model.materialize_views()
+        block.mega.cema.omega.fill_(6000.0)
+        block.mega.rmsnorm.weight.fill_(9.0)
+        sess = DecodeSession(model, 2, torch.float16, use_graph=False)
+        assert sess._native
+        cache = init_cache(2, model, torch.float16)
+        for i in range(4):
+            ref, cache = model(tok[:, i:i + 1], cache=cache)
+            # some ten roundings on either side, each of about 0.4 x 2^-11, adding up like a random walk; half as much again
+            assert _rel(sess.step(tok[:, i]), ref[:, -1]) < 0.6 * 20 ** 0.5 * 2.0 ** -11
+
+
 @pytest.mark.parametrize("D,G,B", [(2048, 32, 64), (4096, 64, 40), (1024, 2, 64)])
 def test_decode_norm_ema_with_more_clusters_than_fit(D, G, B):
     """Clusters that wait for room start late and one by one; every row still gets the whole row's sum of squares."""
