@@ -658,25 +658,16 @@ __device__ __forceinline__ float consumer_reduce(float v, float* scratch) {
   return t;
 }
 
-// d += a b^T for 16 x 16 of a (rows 8 to 15 zero) and 8 x 16 of b, 16-bit with fp32 sums
-template <typename T>
-__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_m16n8k16<__nv_bfloat16>(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0,
-                                                            uint32_t b1) {
+// d += a b^T for 16 x 16 of a (rows 8 to 15 zero) and 8 x 16 of b, bf16 with fp32 sums
+__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
 }
-template <>
-__device__ __forceinline__ void mma_m16n8k16<__half>(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
-}
 
-template <typename T>
 __global__ void __launch_bounds__(kAttThreads, 2)
 decode_attend_cluster_kernel(const __grid_constant__ DecodeAttend p, const __grid_constant__ AttendPlan pl,
                              const __grid_constant__ CUtensorMap vmap) {
+  using T = __nv_bfloat16;
   extern __shared__ uint8_t att_raw[];
   __shared__ float scratch[8];
   __shared__ float2 ml[kAttMaxSplits];
@@ -827,8 +818,8 @@ decode_attend_cluster_kernel(const __grid_constant__ DecodeAttend p, const __gri
       if (++st == pl.stages) { st = 0; phase ^= 1; }
     };
     // Scores.  With a width that is a multiple of 32 eight keys of a warp at a time on the tensor cores, the query as the
-    // sum of three 16-bit rows of the other operand (its 24 bits; products and sums are fp32): some 40 instructions
-    // for eight keys instead of 400, which with several column blocks bounded the link.  A fragment's places along the
+    // sum of three bf16 rows of the other operand (its 24 bits; products and sums are fp32): some 40 instructions for
+    // eight keys instead of 400, which with several column blocks bounded the link.  A fragment's places along the
     // contraction are dealt out so that a lane's part of a key, and of a query row, is 16 contiguous bytes.
     const bool mma = p.dk % 32 == 0;
     for (int i = 0; i < key_stages; ++i) {
@@ -844,8 +835,8 @@ decode_attend_cluster_kernel(const __grid_constant__ DecodeAttend p, const __gri
             uint4 qa = make_uint4(0u, 0u, 0u, 0u);
             if (g < 3) qa = *reinterpret_cast<const uint4*>(qrow + g * p.dk + e + t8);
             const uint4 kb = *reinterpret_cast<const uint4*>(key + e);
-            mma_m16n8k16<T>(d, qa.x, qa.y, kb.x, kb.y);
-            mma_m16n8k16<T>(d2, qa.z, qa.w, kb.z, kb.w);
+            mma_m16n8k16(d, qa.x, qa.y, kb.x, kb.y);
+            mma_m16n8k16(d2, qa.z, qa.w, kb.z, kb.w);
           }
           // rows 0 to 2 of the result, columns 2 (lane & 3) and the next
           float s0 = d[0] + d2[0], s1 = d[1] + d2[1];
@@ -1064,18 +1055,18 @@ int decode_attend_splits(int BH, int C, int num_sms) {
   return s < 1 ? 1 : (s > kDecodeMaxSplits ? kDecodeMaxSplits : s);
 }
 
-// How one launch divides the work, if it takes the shapes and is the better form.  The column blocks of a head repeat its
-// scores, so there are several of them only for one or two heads in all, 128 CTAs in clusters of 16; the next line is
-// where clusters of eight fill the SMs without them.  Between the two, keys split over the whole GPU and a second launch
-// are faster.  us a link, two launches / one (d_qk 256, d_v 2048):
-//   1 head      300 keys  8.9 /  7.5      2000 keys 13.7 / 11.9
-//   2 heads     300 keys  9.0 /  7.9      2000 keys 15.8 / 15.0
-//   4 heads    1111 keys 14.4 / 14.7      4000 keys 26.0 / 31.4
-//   12 heads    700 keys 17.1 / 17.4      2000 keys 33.9 / 38.6
-//   32 heads    700 keys 31.6 / 27.9      2000 keys 71.6 / 63.7
-//   128 heads   500 keys 81.3 / 64.1
-static bool attend_plan(const DecodeAttend& p, int BH, int num_sms, bool wide_clusters, AttendPlan& pl, size_t& smem) {
-  if (p.dv % 8 != 0 || !aligned16(p.v_buf) || !aligned16(p.k_buf) || p.dk > kAttStage / 2) return false;
+// How one launch divides the work, if it takes the shapes and is the better form; bf16 only, since three 16-bit parts of a
+// query are its 24 bits in bf16 alone (fp16 ones end at 2^-24), and with the scores as fp32 FMAs two launches are as fast.
+//   * The column blocks of a head repeat its scores, so there are several of them only for one or two heads in all, 128
+//     CTAs in clusters of 16.
+//   * More heads: from where clusters of eight fill the SMs.  Between the two, keys split over the whole GPU and a second
+//     launch are faster.
+// us a link, two launches / one (d_qk 256, d_v 2048): 4 heads 1111 keys 14.4 / 14.7, 12 heads 700 keys 17.1 / 17.4, 32 heads
+// 700 keys 31.6 / 27.9, 128 heads 500 keys 81.3 / 64.1.
+// One or two heads (d_qk 256, d_v 2048): 300 keys 8.9 / 7.5 and 9.0 / 7.9, 2000 keys 13.7 / 11.9 and 15.8 / 15.0.
+static bool attend_plan(const DecodeAttend& p, int BH, int num_sms, int dtype, bool wide_clusters, AttendPlan& pl,
+                        size_t& smem) {
+  if (dtype != kBF16 || p.dv % 8 != 0 || !aligned16(p.v_buf) || !aligned16(p.k_buf) || p.dk > kAttStage / 2) return false;
   int most;                                             // CTAs
   if (BH <= 2 && wide_clusters) {
     pl.splits = kAttMaxSplits;
@@ -1111,14 +1102,13 @@ static bool attend_plan(const DecodeAttend& p, int BH, int num_sms, bool wide_cl
 }
 
 // Whether clusters of 16 of the kernel can run on the current device (a size that is not portable).
-template <typename T>
 static bool attend_wide_clusters() {
   static std::atomic<unsigned long long> known{0}, can{0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
   const unsigned long long bit = 1ull << dev;
   if ((known.load(std::memory_order_acquire) & bit) == 0) {
-    auto kern = decode_attend_cluster_kernel<T>;
+    auto kern = decode_attend_cluster_kernel;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kAttMaxSplits, 1, 1);
     cfg.blockDim = dim3(kAttThreads, 1, 1);
@@ -1143,21 +1133,17 @@ static bool attend_wide_clusters() {
 int decode_attend(const DecodeAttend& p, int B, int splits, int num_sms, int dtype, bool pdl, cudaStream_t st) {
   if (B == 0) return 0;
   cudaError_t e = cudaSuccess;
-  bool done = false;
-  MB_DISPATCH_16BIT(dtype, {
-    auto kern = decode_attend_cluster_kernel<scalar_t>;
+  AttendPlan pl;
+  size_t bytes;
+  CUtensorMap vmap = {};
+  if (B * p.H <= 65535 && attend_plan(p, B * p.H, num_sms, dtype, B * p.H <= 2 && attend_wide_clusters(), pl, bytes) &&
+      (pl.blocks == 1 || make_tmap_rows(&vmap, p.v_buf, p.dv, (long long)B * p.H * p.C, pl.bw, pl.val_rows, dtype))) {
+    auto kern = decode_attend_cluster_kernel;
     static std::atomic<unsigned long long> configured{0};
-    AttendPlan pl;
-    size_t bytes;
-    CUtensorMap vmap = {};
-    if (B * p.H <= 65535 && attend_plan(p, B * p.H, num_sms, B * p.H <= 2 && attend_wide_clusters<scalar_t>(), pl, bytes) &&
-        (pl.blocks == 1 || make_tmap_rows(&vmap, p.v_buf, p.dv, (long long)B * p.H * p.C, pl.bw, pl.val_rows, dtype))) {
-      if (!allow_dynamic_smem(kern, kAttMaxSmem, configured)) return -2;
-      e = launch_link<kAttThreads>(kern, dim3(pl.splits, pl.blocks, B * p.H), bytes, pl.splits, pdl, st, p, pl, vmap);
-      done = true;
-    }
-  });
-  if (done) return e == cudaSuccess ? 0 : -3;
+    if (!allow_dynamic_smem(kern, kAttMaxSmem, configured)) return -2;
+    e = launch_link<kAttThreads>(kern, dim3(pl.splits, pl.blocks, B * p.H), bytes, pl.splits, pdl, st, p, pl, vmap);
+    return e == cudaSuccess ? 0 : -3;
+  }
   if (p.z != nullptr && (p.dv % 8 != 0 || !aligned16(p.v_buf))) return -1;      // (the new value row leaves in pieces)
   const int BH = B * p.H;
   const int keys = div_up(p.C, splits) < 8 ? 8 : div_up(p.C, splits);

@@ -149,6 +149,34 @@ def test_decode_attention_in_one_launch(B, H, C, dk, dv, dtype):
         assert _rel(out, ref) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), pos
 
 
+@pytest.mark.parametrize("B,H", [(1, 1), (1, 2), (32, 1), (64, 2), (200, 1)])
+def test_decode_attend_with_a_small_query_in_fp16(B, H):
+    """Query entries of 4e-6 (the query is held in fp32) against keys of 2e4: scores of about one, which 16-bit parts of
+    the query would get wrong by a hundredth."""
+    from megalodon_b200.ops import cuda_ops
+    torch.manual_seed(B)
+    dk, dv, C, pos, dev, dt = 64, 256, 96, 80, "cuda", torch.float16
+
+    def rand(*s):
+        return torch.randn(*s, device=dev)
+    z, v, gate = rand(B, H * dk).to(dt), rand(B, H * dv).to(dt), rand(B, H * dv).to(dt)
+    gamma, beta = torch.full((2, H * dk), -1.0, device=dev, dtype=dt), (rand(2, H * dk) * 4e-6).to(dt)      # q, k = beta, rotated
+    kb, vb = (rand(B, H, C, dk) * 2e4).clamp(-6e4, 6e4).to(dt), rand(B, H, C, dv).to(dt)
+    ang = torch.outer(torch.arange(C, device=dev).float(), torch.rand(dk // 2, device=dev))
+    freqs = torch.polar(torch.ones_like(ang), ang)
+    q, k = (torch.view_as_real(torch.view_as_complex(b.double().view(H, dk // 2, 2)) * freqs[pos].to(torch.complex128))
+            .reshape(1, H, dk).expand(B, H, dk) for b in beta)
+    keys = torch.cat([kb[:, :, :pos].double(), k.half().double()[:, :, None]], 2)
+    vals = torch.cat([vb[:, :, :pos].double(), v.double().view(B, H, 1, dv)], 2)
+    pr = torch.softmax(torch.einsum("bhd,bhcd->bhc", q, keys), -1)
+    ref = torch.einsum("bhc,bhcd->bhd", pr, vals).reshape(B, -1) * gate.double()
+    out = torch.empty(B, H * dv, device=dev, dtype=dt)
+    part = torch.empty(B * H * cuda_ops._C().decode_attend_splits(B * H, C) * (dv + 2), device=dev)
+    cuda_ops._C().decode_attend(z, gamma, beta, torch.view_as_real(freqs), v, kb, vb, torch.tensor([pos], device=dev), gate,
+                                out, part, 1e-5, False)
+    assert _rel(out, ref) < 2.0 ** -11               # fp32 throughout, one rounding
+
+
 @pytest.mark.parametrize("D,G,N,B", [(512, 32, 16, 1), (96, 3, 4, 2), (4096, 64, 16, 3), (64, 1, 32, 1), (2048, 64, 16, 40),
                                      (80, 10, 2, 2), (8192, 8, 32, 1)])
 def test_decode_norm_ema_in_parts(D, G, N, B):
