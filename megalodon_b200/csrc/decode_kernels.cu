@@ -1059,24 +1059,28 @@ int decode_attend_splits(int BH, int C, int num_sms) {
 // query are its 24 bits in bf16 alone (fp16 ones end at 2^-24), and with the scores as fp32 FMAs two launches are as fast.
 //   * The column blocks of a head repeat its scores, so there are several of them only for one or two heads in all, 128
 //     CTAs in clusters of 16.
-//   * More heads: from where clusters of eight fill the SMs.  Between the two, keys split over the whole GPU and a second
-//     launch are faster.
-// us a link, two launches / one (d_qk 256, d_v 2048): 4 heads 1111 keys 14.4 / 14.7, 12 heads 700 keys 17.1 / 17.4, 32 heads
-// 700 keys 31.6 / 27.9, 128 heads 500 keys 81.3 / 64.1.
+//   * More heads: the largest cluster of 8, 4, 2 whose CTAs run at once - two to an SM, but clusters of four and eight leave
+//     SMs of a GPC over: 264 CTAs of 296 fit in eights, 272 in fours - and fill the SMs.  A wave that is not full and one
+//     CTA too many are what loses: us, two launches / one, d_qk 256, d_v 1024, 1000 keys: 19 heads 18.2 / 21.5,
+//     24 22.5 / 22.5, 28 26.2 / 23.5, 32 28.6 / 24.5, 36 28.3 / 37.3, 48 36.0 / 36.4, 64 48.5 / 36.9, 72 1.18 times two
+//     launches, 104 to 180 0.74 to 0.75 times.  Rows of at most 640 columns pay from one CTA an SM on: d_qk 64, d_v 256,
+//     19 heads 0.71 times, 48 0.61; single CTAs do so at any width (150 heads 0.68 to 0.77).
+//   * A width that is no multiple of 32 has its scores from FMAs, which only pairs and single CTAs keep up with: d_qk 72,
+//     2000 keys, 32 heads 1.20 times two launches, 56 1.31, 104 0.91.
 // One or two heads (d_qk 256, d_v 2048): 300 keys 8.9 / 7.5 and 9.0 / 7.9, 2000 keys 13.7 / 11.9 and 15.8 / 15.0.
 static bool attend_plan(const DecodeAttend& p, int BH, int num_sms, int dtype, bool wide_clusters, AttendPlan& pl,
                         size_t& smem) {
   if (dtype != kBF16 || p.dv % 8 != 0 || !aligned16(p.v_buf) || !aligned16(p.k_buf) || p.dk > kAttStage / 2) return false;
-  int most;                                             // CTAs
+  int most;                                             // CTAs up to which there are several column blocks
   if (BH <= 2 && wide_clusters) {
     pl.splits = kAttMaxSplits;
     most = 128;
-  } else if (16 * BH > 2 * num_sms) {
-    pl.splits = 8;
-    most = 2 * num_sms;
-    while (pl.splits > 1 && pl.splits * BH > most) pl.splits /= 2;
   } else {
-    return false;
+    pl.splits = p.dk % 32 == 0 ? 8 : 2;
+    while (pl.splits > 1 && pl.splits * BH > (pl.splits == 2 ? 2 * num_sms : 7 * num_sms / 4)) pl.splits /= 2;
+    const int least = pl.splits == 1 || p.dk + p.dv <= 640 ? num_sms : 29 * num_sms / 20;
+    if (pl.splits * BH < least) return false;
+    most = 0;
   }
   const int pieces = p.dv / 8;
   pl.blocks = 0;
@@ -1128,6 +1132,14 @@ static bool attend_wide_clusters() {
     known.fetch_or(bit, std::memory_order_release);
   }
   return (can.load(std::memory_order_acquire) & bit) != 0;
+}
+
+int decode_attend_plan(int BH, int C, int dk, int dv, int dtype, int num_sms) {
+  DecodeAttend p = {};
+  p.C = C; p.dk = dk; p.dv = dv;
+  AttendPlan pl;
+  size_t bytes;
+  return attend_plan(p, BH, num_sms, dtype, true, pl, bytes) ? pl.splits * pl.blocks : 0;
 }
 
 int decode_attend(const DecodeAttend& p, int B, int splits, int num_sms, int dtype, bool pdl, cudaStream_t st) {

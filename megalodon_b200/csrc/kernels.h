@@ -241,6 +241,8 @@ struct DecodeAttend {
   int H, C, dk, dv;
 };
 int decode_attend_splits(int BH, int C, int num_sms);
+// CTAs to a head of attention in one launch; 0 where it is two
+int decode_attend_plan(int BH, int C, int dk, int dv, int dtype, int num_sms);
 int decode_attend(const DecodeAttend& p, int B, int splits, int num_sms, int dtype, bool pdl, cudaStream_t st);
 int decode_layer_norm(const void* x, const void* w, const void* b, void* y, int rows, int D, float eps, int dtype,
                       bool pdl, cudaStream_t st);

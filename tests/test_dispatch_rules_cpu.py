@@ -1,0 +1,26 @@
+"""Rules by which a launcher chooses among its kernels, asked without a GPU (148 SMs)."""
+import pytest
+
+from megalodon_b200.ops._ext import have_ext, require
+
+pytestmark = pytest.mark.skipif(not have_ext(), reason="extension not built")
+_BF16, _FP16 = 1, 2
+
+
+def test_attention_of_one_query_in_one_launch():
+    """Where its clusters run at once and fill the SMs (figures beside the rule); fp16 not at all."""
+    plan = require().decode_attend_plan
+    for heads, want in ((1, 128), (2, 64), (3, 0), (18, 0), (19, 0), (24, 0), (28, 8), (32, 8), (34, 0), (36, 0), (40, 0),
+                        (48, 0), (60, 4), (64, 4), (68, 0), (72, 0), (96, 0), (112, 2), (148, 2), (150, 1), (400, 1)):
+        ctas = plan(heads, 2048, 256, 2048 if heads < 3 else 1024, _BF16, 148)
+        assert ctas == want, (heads, ctas)
+        assert plan(heads, 2048, 256, 1024, _FP16, 148) == 0
+    for heads, want in ((19, 8), (32, 8), (36, 0), (37, 4), (64, 4), (72, 0), (75, 2)):      # narrow rows
+        assert plan(heads, 2048, 64, 256, _BF16, 148) == want, heads
+    for heads, want in ((28, 0), (64, 0), (128, 2), (200, 1)):                              # scores from FMAs
+        assert plan(heads, 2048, 72, 264, _BF16, 148) == want, heads
+    # whatever the heads: never more CTAs in clusters than run at once, never too few for the SMs
+    for heads in range(3, 600):
+        ctas = plan(heads, 2048, 128, 1024, _BF16, 148)
+        if ctas > 1:
+            assert 214 <= ctas * heads <= (296 if ctas == 2 else 259), heads
