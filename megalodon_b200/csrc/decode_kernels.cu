@@ -664,6 +664,13 @@ __device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
 }
 
+// the score of one key by one thread
+__device__ __noinline__ float fma_score(const float* q, const __nv_bfloat16* key, int dk) {
+  float s = 0.f;
+  for (int e = 0; e < dk; ++e) s = fmaf(q[e], to_f(key[e]), s);
+  return s;
+}
+
 __global__ void __launch_bounds__(kAttThreads, 2)
 decode_attend_cluster_kernel(const __grid_constant__ DecodeAttend p, const __grid_constant__ AttendPlan pl,
                              const __grid_constant__ CUtensorMap vmap) {
@@ -870,7 +877,13 @@ decode_attend_cluster_kernel(const __grid_constant__ DecodeAttend p, const __gri
     }
     consumer_sync();
     float m = -INFINITY;
-    for (int j = tid; j < cnt; j += kDecThreads) m = fmaxf(m, sc[j]);
+    for (int j = tid; j < cnt; j += kDecThreads) {
+      float v = sc[j];
+      // An infinity in a key is NaN after the products with the query's parts, one of which is zero or of the other sign.
+      // (Where the products are, a look at them costs up to 8 % with many heads.)
+      if (mma && isnan(v) && j < old) sc[j] = v = fma_score(qs, kold + (long long)j * p.dk, p.dk) * p.scale;
+      m = fmaxf(m, v);
+    }
     m = consumer_reduce<true>(m, scratch);
     const float ref = m == -INFINITY ? 0.f : m;      // a split without keys, or whose keys all have weight zero
     float sum = 0.f;

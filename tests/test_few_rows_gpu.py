@@ -149,6 +149,21 @@ def test_decode_attention_in_one_launch(B, H, C, dk, dv, dtype):
         assert _rel(out, ref) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), pos
 
 
+@pytest.mark.parametrize("B,dk", [(1, 256), (2, 64), (28, 32), (64, 128), (1, 72), (12, 64)])
+def test_decode_attention_with_infinite_keys(B, dk):
+    """A key with an infinity against the query has no weight (its score is minus infinity) and spoils nothing."""
+    from megalodon_b200 import ops
+    torch.manual_seed(dk)
+    q = torch.rand(B, 1, dk, device="cuda").bfloat16() + 0.5
+    k, v = torch.randn(B, 1, 40, dk, device="cuda").bfloat16(), torch.randn(B, 1, 40, 256, device="cuda").bfloat16()
+    k[:, :, 3, 1] = float("-inf")
+    k[:, :, 17, dk - 1] = float("-inf")
+    s = torch.einsum("bhd,bhcd->bhc", q.double(), k.double()) * 0.1
+    ref = torch.einsum("bhc,bhcd->bhd", torch.softmax(s, -1), v.double())
+    out = ops.decode_attention(q, k, v, torch.tensor([39], device="cuda"), 0.1)
+    assert _rel(out, ref) < 2.0 ** -8                # fp32 throughout, one rounding
+
+
 @pytest.mark.parametrize("B,H", [(1, 1), (1, 2), (32, 1), (64, 2), (200, 1)])
 def test_decode_attend_with_a_small_query_in_fp16(B, H):
     """Query entries of 4e-6 (the query is held in fp32) against keys of 2e4: scores of about one, which 16-bit parts of
