@@ -281,15 +281,17 @@ std::tuple<Params, int64_t> mega_block_bwd(const Tensor& dout, const OptTensor& 
     GemmArgs a;
     a.out = heads_view(dv); a.mode = 3; a.a_mn = a.b_mn = true;
     run.gemm(Pv, heads_view(dos), a);
-    GemmArgs s;          // dS over the probabilities, which nothing reads any more
-    s.out = Pv; s.mode = 1; s.epi = 4; s.row_in = rsum; s.row_in2 = delta; s.aux = Pv;
+    // dS in memory of its own: a graph that is kept is walked again, and then wants the probabilities
+    const Tensor dS = torch::empty_like(P).narrow(-1, 0, c);
+    GemmArgs s;
+    s.out = dS; s.mode = 1; s.epi = 4; s.row_in = rsum; s.row_in2 = delta; s.aux = Pv;
     run.gemm(heads_view(do4), heads_view(v4), s);
     GemmArgs qg;
     qg.out = heads_view(dq); qg.mode = 2; qg.b_mn = true;
-    run.gemm(Pv, heads_view(k4), qg);
+    run.gemm(dS, heads_view(k4), qg);
     GemmArgs kg;
     kg.out = heads_view(dk); kg.mode = 3; kg.a_mn = kg.b_mn = true;
-    run.gemm(Pv, heads_view(q4), kg);
+    run.gemm(dS, heads_view(q4), kg);
   }
   const Tensor gv = silu_bwd(dv.view({rows, V}), v_pre);
   weight_grad(kWv, gv, t2);

@@ -961,12 +961,14 @@ class _Attention(torch.autograd.Function):
             # delta_i = dO_i . O_i (what sum_j P_ij dP_ij equals) and dO' = dO / rowsum, in one pass
             _bump()
             dos, delta = _C().attn_bwd_prep(dout, out, rsum)                                      # delta [B, H, L1]
-            # dV = P~^T (dO / l); dS = P~ / l * (dO V^T - delta) written over P~; dQ, dK from dS
+            # dV = P~^T (dO / l); dS = P~ / l * (dO V^T - delta); dQ, dK from dS.  dS has memory of its own where P~ is
+            # kept: the graph may be walked again (`retain_graph`).
             gemm(Pv, _heads_view(dos), a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)
-            gemm(doh, vh, out=Pv, mode=m1, softmax=dict(epi_kind=4, row_in=rsum, row_in2=delta, aux=Pv))
+            dS = torch.empty_like(P)[..., :L2] if ctx.scores_kept else Pv
+            gemm(doh, vh, out=dS, mode=m1, softmax=dict(epi_kind=4, row_in=rsum, row_in2=delta, aux=Pv))
             # dQ = scale dS K ; dK = scale dS^T Q
-            gemm(Pv, _heads_view(k), b_mn=True, out=_heads_view(dq), mode=m2, alpha=scale)
-            gemm(Pv, _heads_view(q), a_mn=True, b_mn=True, out=_heads_view(dk_), mode=m3, alpha=scale)
+            gemm(dS, _heads_view(k), b_mn=True, out=_heads_view(dq), mode=m2, alpha=scale)
+            gemm(dS, _heads_view(q), a_mn=True, b_mn=True, out=_heads_view(dk_), mode=m3, alpha=scale)
             return dq, dk_, dv_, None, None, None
         # dV = P^T dO   (A = P stored [q, key] = [K, M]; B = dO stored [q, dv] = [K, N])
         gemm(Pv, doh, a_mn=True, b_mn=True, out=_heads_view(dv_), mode=m3)

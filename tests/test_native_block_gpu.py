@@ -129,6 +129,22 @@ def test_gradients(monkeypatch, B, L, swiglu, fused, affine, dtype):
         assert _rel(a, b) < 2.0 ** -6, (a.shape, _rel(a, b))
 
 
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("L", [64, 512])
+def test_a_kept_graph_is_walked_again(monkeypatch, native, L):
+    """Two backward passes over one graph, the block's own and its attention's: the same gradients."""
+    from megalodon_b200.modules import native_block
+    if not native:
+        monkeypatch.setattr(native_block, "forward", lambda *a, **k: None)
+    block = _block()
+    x = torch.randn(2, L, 256, device="cuda").bfloat16().requires_grad_(True)
+    y, _ = block(x, _freqs(block, L))
+    g = torch.randn_like(y)
+    first = torch.autograd.grad(y, [x, *block.parameters()], g, retain_graph=True)
+    for a, b in zip(first, torch.autograd.grad(y, [x, *block.parameters()], g)):
+        assert _rel(b, a) < 1e-5             # (column sums are added in any order)
+
+
 def test_what_stays_with_the_modules(monkeypatch):
     """Hooks, replaced modules, dropout, frozen parameters, one token, cached keys, doubles and other options."""
     from megalodon_b200.ops import cuda_ops
