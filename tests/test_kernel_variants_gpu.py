@@ -582,3 +582,40 @@ def test_fp32_products_without_gradients_refuse_what_linear_refuses():
                 ops.linear_fp32_out(dual, w)
         with pytest.raises(Exception):
             torch.func.vmap(lambda r: ops.linear_fp32_out(r[None], w))(x)
+
+
+@pytest.mark.parametrize("tile", [64, 128, 256, 512])
+def test_silu_of_large_negative_values(tile):
+    """SiLU(x) down to where exp(-x) leaves fp32: results that bf16 holds are not flushed to zero."""
+    from megalodon_b200.ops import cuda_ops
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, w = torch.zeros(130, 64, device="cuda").bfloat16(), torch.zeros(72, 64, device="cuda").bfloat16()
+    a[:, 0] = 1.0
+    w[:, 0] = -torch.linspace(80.0, 88.5, 72, device="cuda").bfloat16()
+    out, _, rc = cuda_ops._C().gemm(a, w, None, None, 1, False, False, False, 1, 0, 1.0, err, tile=tile)
+    x = w[:, 0].double()
+    # one rounding to 8 bits; exp in fp32 is off by some 88 steps of 2^-23
+    assert rc == 0 and ((out.double() / (x * torch.sigmoid(x)) - 1.0).abs() < 2.0 ** -8).all()
+
+
+def test_silu_of_the_epilogue_in_fp32():
+    """Against 64 bits over all of fp32's useful range, and at its ends."""
+    from megalodon_b200.ops import cuda_ops
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def silu(x):
+        a, w = torch.zeros(8, 64, device="cuda").bfloat16(), torch.zeros(x.numel(), 64, device="cuda").bfloat16()
+        out, _, rc = cuda_ops._C().gemm(a, w, None, x, 1, False, False, False, 0, 0, 1.0, err)
+        assert rc == 0
+        return out[0]
+    torch.manual_seed(0)
+    x = torch.rand(1 << 16, device="cuda") * 176.0 - 88.0
+    want = x.double() * torch.sigmoid(x.double())
+    # exp in fp32 is a power of two whose exponent x log2(e) has two roundings, of the constant and of the product, half a
+    # step each: |x| steps of 2^-23 of the result; the power is off by two, and three roundings more
+    assert ((silu(x).double() / want - 1.0).abs() <= (x.double().abs() + 5) * 2.0 ** -23).all()
+    inf = float("inf")
+    got = silu(torch.tensor([0.0, inf, 3e38, -100.0, -3e38, 1e-38, -1e-38, 1e-40], device="cuda")).tolist()
+    assert got[:5] == [0.0, inf, 3.0000000054977558e38, 0.0, 0.0]
+    assert all(abs(g - w) <= 2.0 ** -149 for g, w in zip(got[5:], (5e-39, -5e-39, 5e-41)))
+    assert silu(torch.tensor([-inf, float("nan")] * 4, device="cuda")).isnan().all()
