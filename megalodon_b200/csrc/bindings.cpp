@@ -1284,6 +1284,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decode_norm_ema_ok", &decode_norm_ema_ok);
   m.def("decode_attend_splits", &decode_attend_splits);
   m.def("decode_attend_plan", &mb::decode_attend_plan);
+  m.def("cema_tensor_plan", &mb::cema_tensor_plan);
   m.def("decode_attend", checked(&decode_attend));
   m.def("decode_layer_norm", checked(&decode_layer_norm));
   m.def("p2p_send", checked(&p2p_send));

@@ -417,12 +417,26 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
 
 }  // namespace
 
-// y (and h_last, if given) of the EMA; false where the scan is to run.  That is also where few features have a long
-// sequence, which only the scan divides: 16384 x 1024 167 us there, 185 here; 16384 x 512 109 and 184; 4096 x 1024 64 and
-// 51; 2048 x 512 41 and 28.  The lines in between: the scan takes 32 us and 8 for a million elements, this 5 and 2.85 a tile
-// of 256 steps for every wave of CTAs.  A CTA has 16 features of as many sequences as make that least: it is set up once
-// for all of them, and waves are filled better (8 x 777 x 1024 67 -> 52 us, 2 x 2048 x 2048 57 -> 53, 32 x 1000 x 1024
-// 240 -> 196; of one sequence each, 1 % the slower for the bookkeeping).
+// Sequences of a CTA; 0 where the scan is the faster one.  That is where few features have a long sequence, which only the
+// scan divides: 16384 x 1024 167 us there, 185 here; 16384 x 512 109 and 184; 4096 x 1024 64 and 51; 2048 x 512 41 and 28.
+// The lines in between: the scan takes 32 us and 8 for a million elements, this 5 and 2.85 a tile of 256 steps for every
+// wave of CTAs.  A CTA has 16 features of as many sequences as make that least: it is set up once for all of them, and
+// waves are filled better (8 x 777 x 1024 67 -> 52 us, 2 x 2048 x 2048 57 -> 53, 32 x 1000 x 1024 240 -> 196; of one sequence
+// each, 1 % the slower for the bookkeeping).
+int cema_tensor_plan(int B, int L, int D, int sms) {
+  const int groups = div_up(D, kFeat), tiles = div_up(L, kSteps);
+  int per = 1;
+  double us = 1e30;
+  for (int n = 1; n <= B;) {                      // n sequences a CTA, the fewest that make so many CTAs
+    const int ctas = div_up(B, n);
+    const double t = div_up((long long)groups * ctas, sms) * (5.0 + 2.85 * tiles * n);
+    if (t < us) us = t, per = n;
+    n = ctas == 1 ? B + 1 : (B - 1) / (ctas - 1) + 1;
+  }
+  return us > 32.0 + 8e-6 * B * L * D ? 0 : per;
+}
+
+// y (and h_last, if given) of the EMA; false where the scan is to run
 bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega, const float* hx,
                      void* y, float* h_last, int B, int L, int D, int N, int x_dtype, cudaStream_t st) {
   if (N != kStates || x_dtype != kBF16 || D % 8 != 0 || L < 1 || B < 1 || B > 65535 || !aligned16(x) || !aligned16(y))
@@ -430,15 +444,8 @@ bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float*
   int dev = 0, sms = 1;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
-  const int groups = div_up(D, kFeat), tiles = div_up(L, kSteps);
-  int per = 1;
-  double us = 1e30;
-  for (int n = 1; n <= B; ++n) {                  // n sequences a CTA
-    if (n > 1 && div_up(B, n) == div_up(B, n - 1)) continue;
-    const double t = div_up((long long)groups * div_up(B, n), sms) * (5.0 + 2.85 * tiles * n);
-    if (t < us) us = t, per = n;
-  }
-  if (us > 32.0 + 8e-6 * B * L * D) return false;
+  const int groups = div_up(D, kFeat), per = cema_tensor_plan(B, L, D, sms);
+  if (per == 0) return false;
   static std::atomic<unsigned long long> configured{0};
   if (!allow_dynamic_smem(cema_fwd_tensor_kernel, sizeof(Smem), configured)) return false;
   launch_dependent(cema_fwd_tensor_kernel, dim3(groups, div_up(B, per)), dim3(kFeat * 32), sizeof(Smem), st,

@@ -58,6 +58,7 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
               const float* hx, void* y, float* h_last, float* carry, int B, int L, int D, int N,
               int x_dtype, cudaStream_t st);
 // the same on the tensor cores (cema_tensor_kernels.cu); false where it does not take the call
+int cema_tensor_plan(int B, int L, int D, int sms);      // its sequences to a CTA; 0: the scan is the faster one
 bool cema_fwd_tensor(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega, const float* hx,
                      void* y, float* h_last, int B, int L, int D, int N, int x_dtype, cudaStream_t st);
 // dp [D,N], dq/dgamma [D,N,2], domega [D] must be zero-initialised (accumulated with atomics)

@@ -1,4 +1,6 @@
 """Rules by which a launcher chooses among its kernels, asked without a GPU (148 SMs)."""
+import time
+
 import pytest
 
 from megalodon_b200.ops._ext import have_ext, require
@@ -24,3 +26,21 @@ def test_attention_of_one_query_in_one_launch():
         ctas = plan(heads, 2048, 128, 1024, _BF16, 148)
         if ctas > 1:
             assert 214 <= ctas * heads <= (296 if ctas == 2 else 259), heads
+
+
+def test_sequences_to_a_cta_of_the_ema():
+    """Every number of CTAs is looked at, and nothing else: a batch of 65535 costs a call less than its launches."""
+    plan = require().cema_tensor_plan
+
+    def want(B, L, D, sms=148):
+        groups, tiles = -(-D // 16), -(-L // 256)
+        cost, per = min((-(-groups * -(-B // n) // sms) * (5.0 + 2.85 * tiles * n), n) for n in range(1, B + 1))
+        return cost, per
+    for B in (*range(1, 70), 100, 777, 1000, 4097):
+        for L, D in ((300, 1024), (777, 1024), (2048, 2048), (5003, 512), (600, 64)):
+            cost, per = want(B, L, D)
+            assert plan(B, L, D, 148) == (0 if cost > 32.0 + 8e-6 * B * L * D else per), (B, L, D)
+    t0 = time.perf_counter()
+    for B in range(65436, 65536):
+        plan(B, 2, 16, 148)
+    assert time.perf_counter() - t0 < 100 * 50e-6
