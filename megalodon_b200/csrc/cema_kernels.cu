@@ -913,7 +913,7 @@ int cema_num_segments(int L) { return (L + kCemaSegLen - 1) / kCemaSegLen; }
 
 // Passes over the segments are launched the ordinary way: their grid fills the chip about once, and CTAs placed while the
 // kernel before them drains crowd on the SMs that came free first (4096 x 1024, N = 8: forward 41 us, 65 to 86 so; 32-bit
-// N = 16 backward 278 and 311).  What follows the few threads of a combination does not suffer so in the tiled forward.
+// N = 16 backward 278 and 311; the last pass alone so, 16 states in fp16: 33 x 500 x 1000 112 and 164, 2 x 256 x 4096 41 and 66).
 void cema_fwd(const void* x, const float* p, const float* q, const float* gamma, OmegaRef omega,
               const float* hx, void* y, float* h_last, float* carry, int B, int L, int D, int N,
               int x_dtype, cudaStream_t st) {
@@ -936,7 +936,7 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
           launch_dependent(cema_combine, div_up(n, 256), 256, 0, st, (cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
           incoming = (const cfloat*)carry;
         }
-        launch_dependent(cema_fwd_final_t<T, NSPLIT>, grid, kTileFeat * NSPLIT, 0, st,
+        cema_fwd_final_t<T, NSPLIT><<<grid, kTileFeat * NSPLIT, 0, st>>>(
             (const T*)x, p, qc, gc, omega, incoming, (const cfloat*)hx, (T*)y, (cfloat*)h_last, geo);
       });
     });
