@@ -419,8 +419,9 @@ cema_fwd_tensor_kernel(const __nv_bfloat16* __restrict__ x, const float* __restr
 
 // Sequences of a CTA; 0 where the scan is the faster one.  That is where few features have a long sequence, which only the
 // scan divides: 16384 x 1024 167 us there, 185 here; 16384 x 512 109 and 184; 4096 x 1024 64 and 51; 2048 x 512 41 and 28.
-// The lines in between: the scan takes 32 us and 8 for a million elements, this 5 and 2.85 a tile of 256 steps for every
-// wave of CTAs.  A CTA has 16 features of as many sequences as make that least: it is set up once for all of them, and
+// The lines in between: the scan takes 32 us and 8 for a million elements, or in one pass (up to 128 steps) 7.5 and 0.13 a
+// step, this 5 and 2.85 a tile of 256 steps for every wave of CTAs.  One pass, scan / this: 1 x 2 x 1024 7.6 / 9.0 us,
+// 1 x 37 x 1024 12.3 / 9.0, 4 x 128 x 1024 23.9 / 12.3, 16 x 128 x 1024 24.4 / 30.6, 128 x 100 x 128 20.9 / 28.6.  A CTA has 16 features of as many sequences as make that least: it is set up once for all of them, and
 // waves are filled better (8 x 777 x 1024 67 -> 52 us, 2 x 2048 x 2048 57 -> 53, 32 x 1000 x 1024 240 -> 196; of one sequence
 // each, 1 % the slower for the bookkeeping).
 int cema_tensor_plan(int B, int L, int D, int sms) {
@@ -433,7 +434,7 @@ int cema_tensor_plan(int B, int L, int D, int sms) {
     if (t < us) us = t, per = n;
     n = ctas == 1 ? B + 1 : (B - 1) / (ctas - 1) + 1;
   }
-  return us > 32.0 + 8e-6 * B * L * D ? 0 : per;
+  return us > (L <= kCemaSegLen ? 7.5 + 0.13 * L : 32.0 + 8e-6 * B * L * D) ? 0 : per;
 }
 
 // y (and h_last, if given) of the EMA; false where the scan is to run

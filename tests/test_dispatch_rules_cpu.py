@@ -40,6 +40,10 @@ def test_sequences_to_a_cta_of_the_ema():
         for L, D in ((300, 1024), (777, 1024), (2048, 2048), (5003, 512), (600, 64)):
             cost, per = want(B, L, D)
             assert plan(B, L, D, 148) == (0 if cost > 32.0 + 8e-6 * B * L * D else per), (B, L, D)
+    # one pass of the scan: few sequences on the tensor cores, many not
+    for B, L, D, tensor in ((1, 2, 1024, False), (1, 37, 1024, True), (4, 64, 512, True), (4, 128, 1024, True),
+                            (16, 128, 1024, False), (128, 100, 128, False), (8, 40, 1024, False), (4, 100, 4096, False)):
+        assert (plan(B, L, D, 148) > 0) == tensor, (B, L, D)
     t0 = time.perf_counter()
     for B in range(65436, 65536):
         plan(B, 2, 16, 148)
