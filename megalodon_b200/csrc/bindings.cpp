@@ -1283,6 +1283,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mega_block_bwd", checked(&mega_block_bwd));
   m.def("decode_norm_ema_ok", &decode_norm_ema_ok);
   m.def("decode_attend_splits", &decode_attend_splits);
+  m.def("gemm_tile", &mb::gemm_tile);
   m.def("decode_attend_plan", &mb::decode_attend_plan);
   m.def("cema_tensor_plan", &mb::cema_tensor_plan);
   m.def("decode_attend", checked(&decode_attend));

@@ -179,6 +179,8 @@ struct GemmOuterBatch {
   int count = 1;
   long long a_stride = 0, b_stride = 0, c_stride = 0;
 };
+// the tile that a dense product of these sizes runs on (named as below)
+int gemm_tile(int M, int N, int K, int batch, int num_sms);
 // `tile`: 0 picks one; 512: 256 x 256 by a CTA pair; 64, 128, 256: 128 x tile by one CTA
 int gemm_bf16_tcgen05(const void* A, const void* B, void* C, void* preact, const void* bias, int bias_dtype,
                       int act, int M, int N, int K, long long lda, long long ldb, long long ldc, bool a_mn,

@@ -48,3 +48,20 @@ def test_sequences_to_a_cta_of_the_ema():
     for B in range(65436, 65536):
         plan(B, 2, 16, 148)
     assert time.perf_counter() - t0 < 100 * 50e-6
+
+
+@pytest.mark.parametrize("M,N,K,tiles", [
+    # us measured as 128 x 64, 128 x 128, 128 x 256 and CTA pair (512); what may be chosen is within 4 % of the best
+    (130, 4096, 16384, {64}),               # 50.5  61.0 101.2  78.8
+    (513, 4096, 16384, {512}),              # 140   111  101    84
+    (1000, 512, 20000, {64}),               # 59.6  70.5 110    94
+    (1000, 4096, 8192, {512}),              # 95.6  62.7  57.3  50.0
+    (600, 4096, 11264, {512}),              # 104   82.2  75.3  64.7
+    (2000, 2048, 512, {128, 256}),          # 11.4   8.5   8.5   9.2
+    (2000, 1024, 4096, {128}),              # 27.4  16.5  24.1  24.1
+    (1000, 512, 4096, {64}),                # 15.1  15.5  23.6  23.8
+    (4096, 4096, 4096, {512}),              # 172   109   111    92
+    (513, 1024, 16384, {64, 128}),          # 51.2  49.8  77.6  77.8
+])
+def test_tile_of_a_product(M, N, K, tiles):
+    assert require().gemm_tile(M, N, K, 1, 148) in tiles
