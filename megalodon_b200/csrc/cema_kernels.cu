@@ -937,12 +937,12 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
         if (geo.S > 1) {
           // the end state of the last segment is never needed (fwd_final produces h_last)
           dim3 grid_a(grid.x, geo.S - 1, B);
-          cema_fwd_local_t<T, NSPLIT><<<grid_a, kTileFeat * NSPLIT, 0, st>>>((const T*)x, p, qc, (cfloat*)carry, geo);
+          launch_plain(cema_fwd_local_t<T, NSPLIT>, grid_a, kTileFeat * NSPLIT, 0, st, (const T*)x, p, qc, (cfloat*)carry, geo);
           const long long n = (long long)B * N * D;
           launch_dependent(cema_combine, div_up(n, 256), 256, 0, st, (cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
           incoming = (const cfloat*)carry;
         }
-        cema_fwd_final_t<T, NSPLIT><<<grid, kTileFeat * NSPLIT, 0, st>>>(
+        launch_plain(cema_fwd_final_t<T, NSPLIT>, grid, kTileFeat * NSPLIT, 0, st,
             (const T*)x, p, qc, gc, omega, incoming, (const cfloat*)hx, (T*)y, (cfloat*)h_last, geo);
       });
     });
@@ -954,12 +954,12 @@ void cema_fwd(const void* x, const float* p, const float* q, const float* gamma,
       dim3 grid(div_up((long long)D * NSPLIT, kCemaThreads), geo.S, B);
       const cfloat* incoming = nullptr;
       if (geo.S > 1) {
-        cema_fwd_local<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>((const T*)x, p, qc, gc, (cfloat*)carry, geo);
+        launch_plain(cema_fwd_local<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, (const T*)x, p, qc, gc, (cfloat*)carry, geo);
         const long long n = (long long)B * N * D;
         launch_dependent(cema_combine, div_up(n, 256), 256, 0, st, (cfloat*)carry, qc, (const cfloat*)hx, nullptr, geo, false);
         incoming = (const cfloat*)carry;
       }
-      cema_fwd_final<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>(
+      launch_plain(cema_fwd_final<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st,
           (const T*)x, p, qc, gc, omega, incoming, (const cfloat*)hx, (T*)y, (cfloat*)h_last, geo);
     });
   });
@@ -982,25 +982,25 @@ void cema_bwd(const void* dy, const void* x, const float* p, const float* q, con
         dim3 grid(div_up(D, kTileFeat), geo.S, B);
         const cfloat* inc = nullptr;
         if (geo.S > 1) {
-          cema_bwd_rev_local_t<T, NSPLIT><<<grid, nthr, 0, st>>>((const T*)dy, qc, gc, (cfloat*)carry_a, geo);
+          launch_plain(cema_bwd_rev_local_t<T, NSPLIT>, grid, nthr, 0, st, (const T*)dy, qc, gc, (cfloat*)carry_a, geo);
           launch_dependent(cema_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, qc, (const cfloat*)dh_last,
                                                          (cfloat*)dhx, geo, true);
           inc = (const cfloat*)carry_a;
         }
-        cema_bwd_rev_final_t<T, NSPLIT><<<grid, nthr, 0, st>>>(
+        launch_plain(cema_bwd_rev_final_t<T, NSPLIT>, grid, nthr, 0, st,
             (const T*)dy, (const T*)x, p, qc, gc, omega, inc, (const cfloat*)dh_last, (T*)dx, dp, domega,
             (cfloat*)dhx, geo);
         const cfloat* inc_h = nullptr;
         const cfloat* inc_u = nullptr;
         if (geo.S > 1) {
-          cema_bwd_fwd_local_t<T, NSPLIT><<<grid, nthr, 0, st>>>((const T*)x, p, qc, (cfloat*)carry_a,
+          launch_plain(cema_bwd_fwd_local_t<T, NSPLIT>, grid, nthr, 0, st, (const T*)x, p, qc, (cfloat*)carry_a,
                                                                 (cfloat*)carry_b, geo);
           launch_dependent(cema_bwd_fwd_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, (cfloat*)carry_b, qc,
                                                                  (const cfloat*)hx, (const cfloat*)dh_last, dq, geo);
           inc_h = (const cfloat*)carry_a;
           inc_u = (const cfloat*)carry_b;
         }
-        cema_bwd_fwd_final_t<T, NSPLIT><<<grid, nthr, 0, st>>>(
+        launch_plain(cema_bwd_fwd_final_t<T, NSPLIT>, grid, nthr, 0, st,
             (const T*)dy, (const T*)x, p, qc, gc, inc_h, inc_u, (const cfloat*)hx, (const cfloat*)dh_last,
             dgamma, dq, geo);
       });
@@ -1014,26 +1014,26 @@ void cema_bwd(const void* dy, const void* x, const float* p, const float* q, con
       // adjoint pass
       const cfloat* inc = nullptr;
       if (geo.S > 1) {
-        cema_bwd_rev_local<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>((const T*)dy, p, qc, gc, (cfloat*)carry_a, geo);
+        launch_plain(cema_bwd_rev_local<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, (const T*)dy, p, qc, gc, (cfloat*)carry_a, geo);
         launch_dependent(cema_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, qc, (const cfloat*)dh_last,
                                                        (cfloat*)dhx, geo, true);
         inc = (const cfloat*)carry_a;
       }
-      cema_bwd_rev_final<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>(
+      launch_plain(cema_bwd_rev_final<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st,
           (const T*)dy, (const T*)x, p, qc, gc, omega, inc, (const cfloat*)dh_last, (T*)dx, dp, domega,
           (cfloat*)dhx, geo);
       // forward-time pass for dgamma, dq
       const cfloat* inc_h = nullptr;
       const cfloat* inc_u = nullptr;
       if (geo.S > 1) {
-        cema_bwd_fwd_local<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>((const T*)x, p, qc, gc, (cfloat*)carry_a,
+        launch_plain(cema_bwd_fwd_local<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st, (const T*)x, p, qc, gc, (cfloat*)carry_a,
                                                                         (cfloat*)carry_b, geo);
         launch_dependent(cema_bwd_fwd_combine, div_up(nbd, 256), 256, 0, st, (cfloat*)carry_a, (cfloat*)carry_b, qc,
                                                                (const cfloat*)hx, (const cfloat*)dh_last, dq, geo);
         inc_h = (const cfloat*)carry_a;
         inc_u = (const cfloat*)carry_b;
       }
-      cema_bwd_fwd_final<T, NPT, NSPLIT><<<grid, kCemaThreads, 0, st>>>(
+      launch_plain(cema_bwd_fwd_final<T, NPT, NSPLIT>, grid, kCemaThreads, 0, st,
           (const T*)dy, (const T*)x, p, qc, gc, inc_h, inc_u, (const cfloat*)hx, (const cfloat*)dh_last,
           dgamma, dq, geo);
     });

@@ -3,6 +3,7 @@
 // the kernel translation units compile in seconds.
 #pragma once
 
+#include "kernels.h"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -193,6 +194,13 @@ __device__ __forceinline__ float load_any(const void* p, int dtype, int i) {
                        : dtype == kBF16 ? to_f(static_cast<const __nv_bfloat16*>(p)[i]) : to_f(static_cast<const __half*>(p)[i]);
 }
 
+// an ordinary launch
+template <typename... KArgs, typename... Args>
+inline void launch_plain(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  ++thread_launches();
+  kern<<<grid, block, smem, st>>>(KArgs(args)...);
+}
+
 // ---- launches that begin under the end of the kernel before them
 // A kernel launched with `launch_dependent` calls `begin_dependent` before anything else: it returns when every kernel
 // ahead of it in the stream is complete and its writes are visible (at once for an ordinary launch), and lets the next
@@ -215,6 +223,7 @@ inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 bloc
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  ++thread_launches();
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 

@@ -6,6 +6,13 @@
 
 namespace mb {
 
+// Kernels that this host thread has launched through `launch_plain`, `launch_dependent` (common.cuh) and the few-row
+// products: all of a block's, whose native call reports how many it were.
+inline long long& thread_launches() {
+  static thread_local long long n = 0;
+  return n;
+}
+
 // ---- row-wise norms (norm_kernels.cu); weight dtype is fp32 or the activation dtype
 void rms_norm_fwd(const void* x, const void* w, float w_off, void* y, float* rstd, long long M, int D,
                   float eps, int x_dtype, int w_dtype, cudaStream_t st);

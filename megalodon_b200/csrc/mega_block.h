@@ -31,11 +31,11 @@ struct GemmArgs {
 };
 class Launcher {
  public:
-  explicit Launcher(const Tensor& err) : err_(err) {}
-  int64_t count = 0;
+  explicit Launcher(const Tensor& err) : err_(err), before_(mb::thread_launches()) {}
+  // kernels launched since
+  int64_t count() const { return mb::thread_launches() - before_; }
 
   std::tuple<Tensor, OptTensor> gemm(const Tensor& a, const Tensor& b, const GemmArgs& g) {
-    ++count;
     const at::ScalarType t = g.out.has_value() ? g.out->scalar_type()
                                                : (g.out_type == at::ScalarType::Undefined ? a.scalar_type() : g.out_type);
     const int64_t code = t == at::kFloat ? 0 : (t == at::kBFloat16 ? 1 : 2);
@@ -51,10 +51,7 @@ class Launcher {
       if (!g.out.has_value()) g.out = torch::empty({x.size(0), w.size(0)}, x.options().dtype(t));
       const int64_t rc = skinny_gemm({x}, {w}, {OptTensor()}, {g.bias}, {g.aux}, {g.act}, {*g.out}, false, err_, {}, 0.0);
       TORCH_CHECK(rc == 0 || rc == -1, "few-row product: launch failed with code ", rc);
-      if (rc == 0) {
-        ++count;
-        return {*g.out, OptTensor()};
-      }
+      if (rc == 0) return {*g.out, OptTensor()};
     }
     return gemm(x, w, g);
   }
@@ -62,6 +59,7 @@ class Launcher {
 
  private:
   Tensor err_;
+  long long before_;
 };
 
 // Every size that the kernels take on trust.
@@ -112,7 +110,6 @@ std::tuple<std::vector<Tensor>, Params, int64_t> mega_block_fwd(
   const Tensor omega = w[kOmega]->view({D});
   const auto [ema, h] = cema_fwd_any(t, p, q, gamma, omega, hx, want_last);
   const auto [mx, mx_rstd] = rms_norm_fwd(ema, w[kRmsW], 1.0, d.rms_eps);
-  run.count += 7;
   const Tensor x2 = xc.view({rows, D}), t2 = t.view({rows, D}), m2 = mx.view({rows, D});
 
   // the projections of mx; the gate leaves as fp32 pre-activation, for few rows without gradients as its 16-bit SiLU
@@ -129,7 +126,6 @@ std::tuple<std::vector<Tensor>, Params, int64_t> mega_block_fwd(
                                    false, err, {}, 0.0);
     TORCH_CHECK(rc == 0 || rc == -1, "few-row products: launch failed with code ", rc);
     few = rc == 0;
-    run.count += few;
   }
   if (!few) {
     r = torch::empty({rows, V}, f32);
@@ -174,13 +170,11 @@ std::tuple<std::vector<Tensor>, Params, int64_t> mega_block_fwd(
 
   // feed-forward branch; the block's input is its residual
   const auto [f, ln_mean, ln_rstd] = layer_norm_fwd(y, w[kLnW], w[kLnB], 1.0, d.ln_eps);
-  run.count += 4;
   Tensor a, b, u;
   if (w[kFc3].has_value()) {
     a = std::get<0>(run.linear(f, *w[kFc1], {}));
     b = std::get<0>(run.linear(f, *w[kFc3], {}));
     u = swiglu_fwd(a, b);
-    ++run.count;
   } else {
     GemmArgs g1;
     g1.act = 1; g1.want_pre = keep;
@@ -198,7 +192,7 @@ std::tuple<std::vector<Tensor>, Params, int64_t> mega_block_fwd(
   if (keep)
     saved = {xc, pm, tsn[1], tsn[4], tsn[5], t, omega, ema, mx_rstd, mx, z, z_rstd, zn, qr, kr, v, v_pre, P, rsum, attn, r,
              gated, y, ln_mean, ln_rstd, f, a, b.defined() ? OptTensor(b) : OptTensor(), u};
-  return {outs, saved, run.count};
+  return {outs, saved, run.count()};
 }
 
 // Gradients of x, mean, var, hx, p, q, gamma (hx's also where it was absent) and of the parameters, and the launches.
@@ -244,7 +238,6 @@ std::tuple<Params, int64_t> mega_block_bwd(const Tensor& dout, const OptTensor& 
   auto bias_grad = [&](int i, const Tensor& g) {
     if (!w[i].has_value()) return;
     dw[i] = colsum(g, dtype_code(*w[i]));
-    run.count += 2;
   };
 
   // feed-forward branch
@@ -329,9 +322,8 @@ std::tuple<Params, int64_t> mega_block_bwd(const Tensor& dout, const OptTensor& 
   // both residual additions hand their gradient on
   const Tensor dx = ts[0];
   mb::add_two(dx.data_ptr(), dy.data_ptr(), g.data_ptr(), dx.numel(), dtype_code(dx), stream());
-  run.count += 24;
 
   Params out{dx, ts[1], ts[2], ce[5], ce[1], ce[2], ce[3]};
   out.insert(out.end(), dw.begin(), dw.end());
-  return {out, run.count};
+  return {out, run.count()};
 }

@@ -345,6 +345,7 @@ int launch_skinny(const SkinnyMaps& maps, const SkinnyParams& p, int tiles, size
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
+  ++thread_launches();
   return cudaLaunchKernelEx(&cfg, kern, maps, p) == cudaSuccess ? 0 : -3;
 }
 

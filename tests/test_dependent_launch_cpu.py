@@ -34,15 +34,22 @@ def _launched():
     for f, text in _sources():
         bodies = _bodies(text)
         for name in sorted(set(re.findall(r"launch_dependent\(\s*(\w+)", text))):
-            if name == "kern":                             # (the products, whose kernels prepare before they wait)
-                out += [(f, k, b, False) for k, b in bodies.items() if k.startswith("gemm_tcgen05")]
-            else:
+            if name in bodies:
                 out.append((f, name, bodies[name], True))
+                continue
+            # a variable: the kernels that it is set to anywhere in the file (the products, which prepare before they wait)
+            kernels = sorted(set(re.findall(rf"\b{name}\s*=\s*(\w+)", text)))
+            assert kernels and all(k in bodies for k in kernels), (f, name, kernels)
+            out += [(f, k, bodies[k], False) for k in kernels]
     return out
 
 
 def test_the_launches_are_found():
-    assert len(_launched()) > 40
+    found = {(f, name) for f, name, _, _ in _launched()}
+    assert len(found) > 40
+    assert {("gemm_sm100.cu", "gemm_tcgen05_kernel"), ("gemm_sm100.cu", "gemm_tcgen05_pair_kernel")} <= found
+    # (the launcher's own text is not among the sources) every launch names a kernel or a variable of its file
+    assert all(re.match(r"[A-Za-z_]\w*\s*[<,]", m) for _, t in _sources() for m in re.findall(r"launch_dependent\(\s*([^;]{1,60})", t))
 
 
 @pytest.mark.parametrize("file,name,body,first", _launched(), ids=lambda v: v if isinstance(v, str) and len(v) < 45 else "")

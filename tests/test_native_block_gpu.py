@@ -219,3 +219,17 @@ def test_a_model_with_the_native_block_through_checkpoints_and_units(monkeypatch
     assert torch.equal(got[0], want[0])
     for a, b in zip(got[1:], want[1:]):
         assert _rel(a, b) < 2.0 ** -6
+
+
+@pytest.mark.parametrize("L,swiglu,kernels", [(256, True, 21), (256, False, 19), (37, True, 17)])
+def test_launches_are_counted_where_they_are_made(L, swiglu, kernels):
+    """TimestepNorm three, EMA one, six norms and element-wise ones (without the gate, which is torch's, for few rows, and
+    without SwiGLU), three of attention, eight products (seven; few rows: the four projections in one)."""
+    from megalodon_b200.ops import cuda_ops
+    block = _block(swiglu=swiglu).eval()
+    x, freqs = torch.randn(1, L, 256, device="cuda").bfloat16(), _freqs(block, L)
+    with torch.no_grad():
+        block(x, freqs)                          # (in eval mode the EMA's coefficients are computed once)
+        before = cuda_ops.count_launches()
+        block(x, freqs)
+    assert cuda_ops.count_launches() - before == kernels
