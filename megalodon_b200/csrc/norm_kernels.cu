@@ -441,7 +441,7 @@ void launch_bwd(const void* dy, const void* x, const void* w, float off, const f
   if (D > 1024 && vec_ok(D, 256, {dy, x, w, dx})) {
     // one resident wave (the accumulators of the column sums cap the kernel at two CTAs per SM)
     const int grid = (int)std::min<long long>(M, (long long)kColsumRows);
-    VPT_SWITCH(D, 256, (launch_dependent(norm_bwd_vec_kernel<T, W, LAYER, 256, VPT>, grid, 256, 0, st, 
+    VPT_SWITCH(D, 256, (launch_plain(norm_bwd_vec_kernel<T, W, LAYER, 256, VPT>, grid, 256, 0, st, 
                             (const T*)dy, (const T*)x, (const W*)w, off, mean, rstd, (T*)dx, M, D, ws)));
     if (ws != nullptr) colsum_finish(ws, grid, D, dw, LAYER ? db : nullptr, w_dtype, st);
     return;
@@ -455,7 +455,7 @@ void launch_bwd(const void* dy, const void* x, const void* w, float off, const f
   } else {
     const int threads = 256;
     const int grid = (int)std::min<long long>(M, 148LL * 4);
-    launch_dependent(norm_bwd_kernel<T, W, LAYER, 256>, grid, threads, 0, st, (const T*)dy, (const T*)x, (const W*)w, off,
+    launch_plain(norm_bwd_kernel<T, W, LAYER, 256>, grid, threads, 0, st, (const T*)dy, (const T*)x, (const W*)w, off,
                                                                 mean, rstd, (T*)dx, aw, ab, M, D);
   }
   if (ws != nullptr) colsum_finish(ws, 1, D, dw, LAYER ? db : nullptr, w_dtype, st);
@@ -521,9 +521,9 @@ bool colsum_16bit(const void* g, long long M, int N, float* ws, void* out, int o
   const int vpt = (N / 8 + 255) / 256;
 #define MB_COLSUM(TT)                                                                                   \
   do {                                                                                                  \
-    if (vpt <= 1) launch_dependent(colsum_partial_kernel<TT, 1>, grid, 256, 0, st, (const TT*)g, M, N, ws);           \
-    else if (vpt <= 2) launch_dependent(colsum_partial_kernel<TT, 2>, grid, 256, 0, st, (const TT*)g, M, N, ws);      \
-    else launch_dependent(colsum_partial_kernel<TT, 4>, grid, 256, 0, st, (const TT*)g, M, N, ws);                    \
+    if (vpt <= 1) launch_plain(colsum_partial_kernel<TT, 1>, grid, 256, 0, st, (const TT*)g, M, N, ws);           \
+    else if (vpt <= 2) launch_plain(colsum_partial_kernel<TT, 2>, grid, 256, 0, st, (const TT*)g, M, N, ws);      \
+    else launch_plain(colsum_partial_kernel<TT, 4>, grid, 256, 0, st, (const TT*)g, M, N, ws);                    \
   } while (0)
   if (dtype == kBF16) MB_COLSUM(__nv_bfloat16);
   else MB_COLSUM(__half);

@@ -915,17 +915,17 @@ void timestep_norm_fwd(const void* x, const long long* prev_count, const void* p
     const int seg = tsn_fused_seg(L);
     if (seg > 0 && B <= 65535) {
       const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
-      SEG_SWITCH(seg, (launch_dependent(tsn_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
+      SEG_SWITCH(seg, (launch_plain(tsn_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
           gu, gv, mask, before, count_out, (T*)mean_out, (T*)var_out,
           cummean, cumrstd, L, G, nseg, gt, eps)));
     } else {
     const int nseg = tsn_num_segments(L);
     const long long nsg = (long long)B * nseg * G;
-    launch_dependent(tsn_seg_sums_kernel, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, B, L, G, nseg);
-    launch_dependent(tsn_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
+    launch_plain(tsn_seg_sums_kernel, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, B, L, G, nseg);
+    launch_plain(tsn_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
         seg_scratch, before, count_out, (T*)mean_out, (T*)var_out,
         B, G, nseg);
-    launch_dependent(tsn_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, before, cummean, cumrstd, B, L, G, nseg,
+    launch_plain(tsn_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, gu, gv, mask, seg_scratch, before, cummean, cumrstd, B, L, G, nseg,
                                                             eps);
     }
     if (vec) {
@@ -970,38 +970,38 @@ void timestep_norm_bwd(const void* dy, const void* dmean_out, const void* dvar_o
     const int seg = tsn_fused_seg(L);
     if (seg > 0 && B <= 65535) {
       const int nseg = div_up(L, seg), gt = tsn_fused_groups(nseg);
-      SEG_SWITCH(seg, (launch_dependent(tsn_bwd_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
+      SEG_SWITCH(seg, (launch_plain(tsn_bwd_scan_fused_kernel<T, SEG>, dim3(div_up(G, gt), B), gt * nseg, 0, st, 
           in, mask, cv, count_final, (const T*)prev_mean, (const T*)dmean_out, (const T*)dvar_out, (T*)dprev_mean,
           (T*)dprev_var, dux, dvx, L, G, nseg, gt)));
     } else {
     const int nseg = tsn_num_segments(L);
     const long long nsg = (long long)B * nseg * G;
-    launch_dependent(tsn_bwd_seg_maps_kernel<T>, div_up(nsg, 256), 256, 0, st, in, mask, cv, count_final, (const T*)prev_mean,
+    launch_plain(tsn_bwd_seg_maps_kernel<T>, div_up(nsg, 256), 256, 0, st, in, mask, cv, count_final, (const T*)prev_mean,
                                                                seg_scratch, B, L, G, nseg);
-    launch_dependent(tsn_bwd_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
+    launch_plain(tsn_bwd_seg_prefix_kernel<T>, div_up((long long)B * G, 128), 128, 0, st, 
         seg_scratch, (const T*)dmean_out, (const T*)dvar_out, (T*)dprev_mean, (T*)dprev_var, B, G, nseg);
-    launch_dependent(tsn_bwd_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, in, mask, cv, count_final, (const T*)prev_mean,
+    launch_plain(tsn_bwd_seg_apply_kernel<T>, div_up(nsg, 256), 256, 0, st, in, mask, cv, count_final, (const T*)prev_mean,
                                                                 seg_scratch, dux, dvx, B, L, G, nseg);
     }
     const int grid = (int)std::min<long long>(rows, vec ? (long long)kColsumRows : 148LL * 4);
     if (vec) {
       const int hv = H / 8;
       if (hv <= kBwdThreads)
-        launch_dependent(tsn_bwd_apply_vec_kernel<T, W, 1>, grid, kBwdThreads, 0, st, 
+        launch_plain(tsn_bwd_apply_vec_kernel<T, W, 1>, grid, kBwdThreads, 0, st, 
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
             rows, H, G, colsum_ws);
       else if (hv <= 2 * kBwdThreads)
-        launch_dependent(tsn_bwd_apply_vec_kernel<T, W, 2>, grid, kBwdThreads, 0, st, 
+        launch_plain(tsn_bwd_apply_vec_kernel<T, W, 2>, grid, kBwdThreads, 0, st, 
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
             rows, H, G, colsum_ws);
       else
-        launch_dependent(tsn_bwd_apply_vec_kernel<T, W, 4>, grid, kBwdThreads, 0, st, 
+        launch_plain(tsn_bwd_apply_vec_kernel<T, W, 4>, grid, kBwdThreads, 0, st, 
             (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux, dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
             rows, H, G, colsum_ws);
       colsum_finish(colsum_ws, grid, H, dgamma, dbeta, w_dtype, st);
     } else {
     cudaMemsetAsync(colsum_ws, 0, sizeof(float) * 2 * H, st);
-    launch_dependent(tsn_bwd_apply_kernel<T, W>, grid, kBwdThreads, 0, st, (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux,
+    launch_plain(tsn_bwd_apply_kernel<T, W>, grid, kBwdThreads, 0, st, (const T*)dy, (const T*)x, cummean, cumrstd, ux, dux,
                                                      dvx, (const W*)gamma, gamma_offset, mask, (T*)dx,
                                                      colsum_ws, colsum_ws + H, rows, H, G);
     colsum_finish(colsum_ws, 1, H, dgamma, dbeta, w_dtype, st);

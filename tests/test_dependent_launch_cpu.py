@@ -46,7 +46,7 @@ def _launched():
 
 def test_the_launches_are_found():
     found = {(f, name) for f, name, _, _ in _launched()}
-    assert len(found) > 40
+    assert len(found) >= 40
     assert {("gemm_sm100.cu", "gemm_tcgen05_kernel"), ("gemm_sm100.cu", "gemm_tcgen05_pair_kernel")} <= found
     # (the launcher's own text is not among the sources) every launch names a kernel or a variable of its file
     assert all(re.match(r"[A-Za-z_]\w*\s*[<,]", m) for _, t in _sources() for m in re.findall(r"launch_dependent\(\s*([^;]{1,60})", t))
