@@ -1295,14 +1295,14 @@ static bool g_use_pair = true;
 
 // Which tile a product runs on: the one whose estimate is lowest,
 //   (waves - 1) * max(k-blocks * t, e) + k-blocks * t + c,   t = max(latency, bytes of the resident tiles / rate).
-// Constants fitted to back-to-back launches (each beginning under the end of the one before) of 170 shapes from
-// 64 x 64 to 20000 rows and 32000 columns, K from 64 to 65536, in three layouts; the choice is 0.1 % off the best tile over
-// all of them, 6 % at the worst shape (constants fitted to K up to 4864 alone: 2.8 and 21 %):
-//   latency per k-block   0.283 us as a CTA pair, 0.293 as 128 x 256, 0.187 as 128 x 128, 0.178 as 128 x 64 (what a ring
-//                         of 6, 4, 6, 8 stages leaves of a memory latency)
-//   epilogue e            5.1 / 5.1 / 3.0 / 2.3 us a tile, hidden behind the next tile's loop except at the end
-//   start and end c       6.4 / 5.7 / 4.2 / 3.9 us
-//   rate                  19.4 TB/s out of L2 and memory together, which the narrow tiles reach first
+// Constants fitted to back-to-back launches (each beginning under the end of the one before) of 849 products: 64 to 20000
+// rows, 64 to 32000 columns, K from 64 to 65536, in three layouts; the choice is 0.1 % off the best tile over all of them and
+// 9 % at the worst (constants fitted to K up to 4864 alone: 2.2 and 29 %):
+//   latency per k-block   0.280 us as a CTA pair, 0.320 as 128 x 256, 0.189 as 128 x 128 and 128 x 64 (what a ring of
+//                         6, 4, 6, 8 stages leaves of a memory latency)
+//   epilogue e            2.85 / 5.08 / 2.30 / 1.91 us a tile, hidden behind the next tile's loop except at the end
+//   start and end c       7.30 / 4.71 / 4.39 / 3.80 us
+//   rate                  19.6 TB/s out of L2 and memory together, which the narrow tiles reach first
 // Few wide tiles leave most SMs without work: 1024 x 512 x 512 takes 9.6 us in 8 pair tiles and 6.1 us in 64 tiles of
 // 128 x 64, 2000 x 1024 x 2560 19.4 us in pairs and 13.4 us as 128 x 128; 4000 x 2048 x 4096 48 us in pairs, 59 as
 // 128 x 128 and 87 as 128 x 64; with a long sum pairs lose least to a k-block: 513 x 4096 x 16384 84 us in pairs, 101 as
@@ -1314,12 +1314,12 @@ static int pick_tile(const GemmParams& p, int num_sms) {
   // what Q K^T skips above the diagonal P V must not contract.  All of them see the same number of rows, so the row
   // tile may depend on nothing else.
   if (p.mode != 0 && pair_ok) return kPairTile;
-  const double nk = (p.K + BK - 1) / BK, rate = 19.4e6;      // bytes per us
+  const double nk = (p.K + BK - 1) / BK, rate = 19.6e6;      // bytes per us
   struct Tile { int name, bm, bn; double lat, bytes, e, c; };
-  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.283, 65536, 5.1, 6.4},
-                        {256, BM, 256, 0.293, 49152, 5.1, 5.7},
-                        {128, BM, 128, 0.187, 32768, 3.0, 4.2},
-                        {64, BM, 64, 0.178, 24576, 2.3, 3.9}};
+  const Tile tiles[] = {{kPairTile, kPairBM, kPairBN, 0.280, 65536, 2.85, 7.30},
+                        {256, BM, 256, 0.320, 49152, 5.08, 4.71},
+                        {128, BM, 128, 0.189, 32768, 2.30, 4.39},
+                        {64, BM, 64, 0.189, 24576, 1.91, 3.80}};
   int best = 256;
   double best_us = 1e30;
   for (const Tile& t : tiles) {

@@ -62,6 +62,7 @@ def test_sequences_to_a_cta_of_the_ema():
     (1000, 512, 4096, {64}),                # 15.1  15.5  23.6  23.8
     (4096, 4096, 4096, {512}),              # 172   109   111    92
     (513, 1024, 16384, {64, 128}),          # 51.2  49.8  77.6  77.8
+    (6216, 1024, 2048, {128, 512}),         # 40.3  24.3  26.2  24.7
 ])
 def test_tile_of_a_product(M, N, K, tiles):
     assert require().gemm_tile(M, N, K, 1, 148) in tiles
