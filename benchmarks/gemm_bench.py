@@ -37,6 +37,7 @@ def main():
     ap.add_argument("--tokens", type=int, default=4096)
     ap.add_argument("--only", default=None, help="run a single projection, e.g. wv/wr (for profiler captures)")
     ap.add_argument("--no-cublas", action="store_true", help="skip the torch.matmul comparison")
+    ap.add_argument("--silu", action="store_true", help="forward products with bias and SiLU in the epilogue, and nothing else")
     args = ap.parse_args()
     T = args.tokens
     dev = torch.device("cuda")
@@ -57,6 +58,10 @@ def main():
             ("wgrad", n_out, k_in, T, lambda: cuda_ops.gemm(dy, x, a_mn=True, b_mn=True),
              lambda: torch.matmul(dy.t(), x)),
         ]
+        if args.silu:
+            bias = torch.randn(n_out, device=dev).bfloat16()
+            cases = [("silu", T, n_out, k_in, lambda: cuda_ops.gemm(x, w, bias, "silu"),
+                      lambda: torch.nn.functional.silu(torch.nn.functional.linear(x, w, bias)))]
         for pname, M, N, K, mine, ref in cases:
             t0 = time_it(mine, flush)
             t1 = t0 if args.no_cublas else time_it(ref, flush)

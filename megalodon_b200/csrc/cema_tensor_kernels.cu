@@ -24,8 +24,8 @@
 //
 // us, scan / this (B x L x D): 1 x 300 x 1024 35 / 12, 8 x 777 x 1024 88 / 52, 1 x 907 x 2048 39 / 18, 2 x 2048 x 2048
 // 97 / 53, 1 x 4096 x 4096 169 / 104, 1 x 16384 x 4096 586 / 376.  What bounds it is latency: sixteen warps fill an SM's
-// registers (128 a thread), a scheduler issues in 42 % of the cycles, the tensor pipe is busy in 23 %, the wavefronts of
-// shared memory in 45 %.  Setting a warp up takes some 5 us, a tile 2.9.
+// registers (128 a thread), a scheduler issues in 48 % of the cycles, the tensor pipe is busy in 24 %, the wavefronts of
+// shared memory in 39 %.  Setting a warp up takes some 5 us, a tile 2.9.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -80,7 +80,8 @@ __device__ __forceinline__ void split3(ff a, ff b, uint32_t& p0, uint32_t& p1, u
   p2 = pack_bf16(a.h - __uint_as_float(p0 << 16) - __uint_as_float(p1 << 16) + a.l,
                  b.h - __uint_as_float(p0 & 0xffff0000u) - __uint_as_float(p1 & 0xffff0000u) + b.l);
 }
-// s + e and a + b without loss (the second for any order of sizes); the intrinsics keep the compiler from contracting
+// Sums and products without loss (Knuth's and Dekker's, the latter with a fused multiply-add); the intrinsics keep the
+// compiler from contracting
 __device__ __forceinline__ ff two_sum(float a, float b) {
   const float s = __fadd_rn(a, b), v = __fsub_rn(s, a);
   return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v))};

@@ -670,7 +670,7 @@ gemm_tcgen05_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid_cons
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  begin_dependent();        // barriers, tensor memory and descriptors are set up under the end of the kernel before
+  begin_dependent();        // barriers and tensor memory are set up under the end of the kernel before
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -1015,7 +1015,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ TmapArray tmaps_a, const __grid
   cluster_sync_all();                               // the peer's barriers exist before anything signals them
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  begin_dependent();        // barriers, tensor memory and descriptors are set up under the end of the kernel before
+  begin_dependent();        // barriers and tensor memory are set up under the end of the kernel before
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)

@@ -2,8 +2,8 @@
 // file in its unnamed namespace): the same kernels in the same order as the modules launch them, without an interpreter,
 // a module call and an autograd node between two of them.
 //
-// A launch through the modules costs the host 20 to 27 us, more than most kernels of a small model take; from here 5 to
-// 7.  Modules / native, ms: a training step of two 512-wide layers 9.8 / 5.9, of four 1024-wide ones 8.6 / 6.7; scoring
+// A launch through the modules costs the host 20 to 27 us, more than most kernels of a small model take; from here some
+// 9 without gradients (21 launches of a block in 178 us, Python's checks among them; 15 a launch both ways with autograd).  Modules / native, ms: a training step of two 512-wide layers 9.8 / 5.9, of four 1024-wide ones 8.6 / 6.7; scoring
 // 8 x 777 tokens in twelve 1024-wide layers 8.4 / 6.2; a prompt of 37 tokens there 6.7 / 3.2.
 #pragma once
 

@@ -1,7 +1,7 @@
 """A MEGA block as one native call each way (csrc/mega_block.h).
 
 A launch through the modules costs the host 20 to 27 us, which bounds everything but the largest models; the native
-block launches the same kernels at 4 to 6 us each.  It stands for the calls of the block's own modules, so it is taken
+block launches the same kernels at some 9 us each.  It stands for the calls of the block's own modules, so it is taken
 only where those are what the model was built with, without hooks, and where every operator would run on the kernels,
 which is asked anew at every call.
 """

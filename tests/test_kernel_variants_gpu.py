@@ -303,6 +303,16 @@ def test_ema_on_tensor_cores(B, L, D, carried):
     assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -24 * 64 * size).all()
 
 
+@pytest.mark.parametrize("B,L,D", [(1, 3, 8), (2, 16, 48), (4, 128, 1024), (2, 129, 24), (3, 257, 1024)])
+def test_ema_on_tensor_cores_for_short_sequences(B, L, D):
+    """Around the length up to which the scan needs one pass, where the choice between the two follows another line, and
+    several short sequences to a CTA."""
+    from megalodon_b200.ops import cuda_ops
+    per = cuda_ops._C().cema_tensor_plan(B, L, D, torch.cuda.get_device_properties(0).multi_processor_count)
+    assert per == (2 if D == 1024 else 1)
+    test_ema_on_tensor_cores(B, L, D, True)
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
 def test_ema_with_infinities_stays_causal(bad):
     """What comes before an infinity or NaN in a feature, and the other features, do not see it."""
